@@ -366,22 +366,222 @@ __global__ void k_flags_singular(DevMesh M, const SingularTask* tasks, uint8_t* 
 
 // ------------------------------------------------------------------ local-block kernels
 
-// General pair number q (strictly lower pairs, in the builder's distance order when
-// it made one) of mesh M for one job: p x p Gauss points, the pair's local blocks
-// written to locj (the job's block array).
-template <int D, bool RK, bool CURVED>
+// ---- general pairs, real wavenumber
+//
+// What bounds it: the FP64 pipe (two lanes per cycle and SM; see hankel_u.cuh), so the
+// count of FP64 instructions per quadrature point.  One thread per (pair, Gauss node a of
+// panel i), looping over the p nodes b of panel j; a CTA of 128 threads takes
+// floor(128 / p) pairs.  Per point:
+//   * v = gamma_i(x_a) - gamma_j(y_b), |v|^2, u = ks^2 |v|^2: 5 instructions, and f(u),
+//     g(u) from the table: 17 (no distance, reciprocal, logarithm or sine);
+//   * every kernel value is f, g, |v|^2 f or |v|^2 g up to factors of the job, and along b
+//     only two moments of each are needed (weights w_b and w_b y_b); the powers of x_a and
+//     the factors of node a enter once per row.  On straight panels v x tau_j does not
+//     depend on b, so the double layer shares the sums of the single layer.
+// At order 2 that is 58 FP64 instructions on lines and 84 on arcs where a thread per pair
+// with the four moments per kernel value, the distance and the branches of
+// hankel01_real took about 230 and 300.
+// The rows' sums are then combined through shared memory: 2 p instructions per value.
+
+// value sets of a thread's row sums, each with D + 1 functions and 2 powers of y:
+// 0: {f, v2 g, v2 f} (single layer, hypersingular), 1: {g, f, v2 g} x (v x tau_j)|tau_i|,
+// 2: {g, f, v2 g} x (tau_i x v)|tau_j|, 3 (curved): set 0 x 2 tau_i . tau_j
+template <int D, bool CURVED>
+struct GenDims {
+    static constexpr int F = D + 1, SETS = CURVED ? 4 : 3, NV = SETS * F * 2, THREADS = 128;
+    static constexpr size_t kRows = (size_t)NV * THREADS * sizeof(cplx);
+    static size_t smem(int p) { return kRows + (size_t)(THREADS / p) * NV * 2 * sizeof(cplx); }
+};
+
+__device__ __forceinline__ void row_add(cplx (&s)[2], double w, double wy, cplx k) {
+    axpy(s[0], w, k);
+    axpy(s[1], wy, k);
+}
+
+// entry (a, b) of the moments m = {1, x, y, xy}: shape functions (t, 1 - t) in x and y
+__device__ __forceinline__ cplx entry_fwd(const cplx* m, int a, int b) {
+    const cplx r0 = b ? m[0] - m[2] : m[2];      // sum w psi_b
+    const cplx r1 = b ? m[1] - m[3] : m[3];      // sum w x psi_b
+    return a ? r0 - r1 : r1;
+}
+
+// The pairs q0 .. of mesh M that one CTA takes, for the job K; locj: the job's blocks.
+template <int D, bool CURVED>
+__device__ __forceinline__ void general_rows(const DevMesh& M, const KConst& K, long long q0, const double* sx,
+                                             const double* sw, cplx* smem, cplx* locj) {
+    typedef GenDims<D, CURVED> G;
+    constexpr int F = G::F;
+    const int p = M.p, ppc = G::THREADS / p;
+    const int lp = threadIdx.x / p, a = threadIdx.x - lp * p;
+    const long long q = q0 + lp;
+    cplx* rows = smem;                              // [value][thread]
+    cplx* mom = smem + G::NV * G::THREADS;          // [pair][set][function][4]
+    if (lp < ppc && q < M.ngen) {
+        const unsigned pr = M.gpairs[q];
+        const int i = pr >> 16, j = pr & 0xffffu;
+        const uint8_t fl = M.flags[tri_index(i, j)];
+        const cplx xi = M.gpt[i * p + a], ti = M.gtan[i * p + a];
+        const double tin = M.gtn[i * p + a], ks2 = K.ks.re * K.ks.re;
+        const cplx* ptj = M.gpt + j * p;
+        const cplx* tgj = M.gtan + j * p;
+        const double* tnj = M.gtn + j * p;
+        cplx S[F][2], L[CURVED ? F : 1][2], T[F][2], W[CURVED ? F : 1][2];
+#pragma unroll
+        for (int t = 0; t < F; ++t) {
+            S[t][0] = S[t][1] = T[t][0] = T[t][1] = mk(0.);
+            if (CURVED || t == 0) L[CURVED ? t : 0][0] = L[CURVED ? t : 0][1] = mk(0.);
+            if (CURVED) W[CURVED ? t : 0][0] = W[CURVED ? t : 0][1] = mk(0.);
+        }
+        for (int b = 0; b < p; ++b) {
+            const cplx v = xi - ptj[b];
+            const double v2 = norm2(v);
+            cplx f, g;
+            hk_pair(M.hk, ks2 * v2, f, g);
+            const double w = sw[b], y = sx[b], wy = sw[p + b];   // sw[p + b] = w_b y_b
+            const cplx vg = D > 0 ? v2 * g : mk(0.), vf = D > 1 ? v2 * f : mk(0.);
+            const cplx ks[3] = {f, vg, vf}, kd[3] = {g, f, vg};
+#pragma unroll
+            for (int t = 0; t < F; ++t) row_add(S[t], w, wy, ks[t]);
+            const double ct = v.im * ti.re - v.re * ti.im;       // tau_i x v
+            if (CURVED) {
+                const cplx tj = tgj[b];
+                const double wt = w * tnj[b] * ct, wd = w * (v.re * tj.im - v.im * tj.re);
+                const double wc = w * (ti.im * tj.im + ti.re * tj.re);
+#pragma unroll
+                for (int t = 0; t < F; ++t) {
+                    row_add(T[t], wt, wt * y, kd[t]);
+                    row_add(L[CURVED ? t : 0], wd, wd * y, kd[t]);
+                    row_add(W[CURVED ? t : 0], wc, wc * y, ks[t]);
+                }
+            } else {
+                const double wt = w * ct, wty = wy * ct;
+#pragma unroll
+                for (int t = 0; t < F; ++t) row_add(T[t], wt, wty, kd[t]);
+                row_add(L[0], w, wy, g);
+            }
+        }
+        // the factors of node a; a pair whose geometric factor vanishes at every point (the
+        // builder's flags, galerkin_builder.cpp:475-499) adds nothing to that operator
+        const double wa = sw[a];
+        const cplx v0 = xi - ptj[0], t0j = tgj[0];
+        const double fd = (fl & PF_DL0_ZERO) ? 0. : CURVED ? wa * tin : wa * tin * (v0.re * t0j.im - v0.im * t0j.re);
+        const double ft = (fl & PF_DLT0_ZERO) ? 0. : CURVED ? wa : wa * tnj[0];
+        const double fw = (fl & PF_TDT0_ZERO) ? 0. : 2. * wa;
+        cplx* r = rows + threadIdx.x;
+#pragma unroll
+        for (int t = 0; t < F; ++t)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int e = 2 * t + h;
+                r[e * G::THREADS] = wa * S[t][h];
+                r[(2 * F + e) * G::THREADS] = fd * (CURVED ? L[CURVED ? t : 0][h] : t == 0 ? L[0][h] : S[t > 0 ? t - 1 : 0][h]);
+                r[(4 * F + e) * G::THREADS] = ft * T[t][h];
+                if (CURVED) r[(6 * F + e) * G::THREADS] = fw * W[CURVED ? t : 0][h];
+            }
+    }
+    __syncthreads();
+    const int npairs = (int)(M.ngen - q0 < ppc ? M.ngen - q0 : ppc);
+    for (int it = threadIdx.x; it < npairs * G::NV; it += G::THREADS) {
+        const int e = it / npairs, l = it - e * npairs;
+        const cplx* r = rows + e * G::THREADS + l * p;
+        cplx m0 = mk(0.), m1 = mk(0.);
+        for (int c = 0; c < p; ++c) {
+            const cplx z = r[c];
+            m0 += z;
+            axpy(m1, sx[c], z);
+        }
+        cplx* m = mom + ((long long)l * (G::NV / 2) + (e >> 1)) * 4 + 2 * (e & 1);
+        m[0] = m0;
+        m[1] = m1;
+    }
+    __syncthreads();
+    // the pair's blocks: 4 kinds x 4 shape-function pairs, the kind slowest so that a warp
+    // mostly has one
+    const double ks = K.ks.re, ks2 = ks * ks, kc = K.c * K.k.re;
+    for (int it = threadIdx.x; it < npairs * 16; it += G::THREADS) {
+        const int kind = it / (4 * npairs), rest = it - kind * 4 * npairs, l = rest >> 2, e = rest & 3;
+        const int sa = e >> 1, sb = e & 1;
+        const unsigned pr = M.gpairs[q0 + l];
+        const int i = pr >> 16, j = pr & 0xffffu;
+        const cplx* m = mom + (long long)l * (G::NV / 2) * 4;
+        cplx* dst = locj + tri_index(i, j) * (D + 1) * kLocPerD + 4 * kind + e;
+        if (kind < 2) {        // double layer, transposed double layer (test function on the y panel)
+            const cplx* md = m + (kind == 0 ? 1 : 2) * F * 4;
+            const int ex = kind == 0 ? sa : sb, ey = kind == 0 ? sb : sa;
+            dst[0] = ks2 * entry_fwd(md, ex, ey);
+            if (D > 0) {
+                const cplx d1 = entry_fwd(md + 4, ex, ey);
+                dst[kLocPerD] = kc * d1;
+                if (D > 1) dst[2 * kLocPerD] = K.c * (d1 - ks2 * entry_fwd(md + 8, ex, ey));
+            }
+        } else {
+            const cplx t0i = M.gtan[i * p], t0j = M.gtan[j * p];
+            const double ttp = M.gtn[i * p] * M.gtn[j * p];
+            // s: {h0, |v| h1, |v|^2 h0 - |v| h1 / ks} from {f, v2 g, v2 f}
+            const cplx* mw = m + (CURVED ? 3 * F * 4 : 0);
+            const bool tz = (M.flags[tri_index(i, j)] & PF_TDT0_ZERO) != 0;
+            const double tw = CURVED ? 1. : tz ? 0. : 2. * (t0i.im * t0j.im + t0i.re * t0j.re);
+            const double fct = kind == 3 ? ttp : tw;
+            const cplx* mm = kind == 3 ? m : mw;
+            cplx E[3];
+            E[0] = fct * entry_fwd(mm, sa, sb);
+            if (D > 0) {
+                const cplx vg = fct * entry_fwd(mm + 4, sa, sb);
+                E[1] = ks * vg;
+                if (D > 1) E[2] = fct * entry_fwd(mm + 8, sa, sb) - vg;
+            }
+            if (kind == 2) {   // hypersingular: b'_a b'_b h0 moments and the k^2 term
+                const double dd = (sa == sb) ? 1. : -1., k2h = 0.5 * ks2;
+                const cplx W0 = E[0];
+                E[0] = dd * m[0] - k2h * W0;
+                if (D > 0) {
+                    const cplx W1 = E[1];
+                    E[1] = (dd * ks) * m[4] - k2h * W1 + ks * W0;
+                    if (D > 1) E[2] = dd * (m[8] - m[4]) - k2h * E[2] - (2. * ks) * W1 + W0;
+                }
+            }
+            dst[0] = E[0];
+            if (D > 0) dst[kLocPerD] = -K.sqrtc * E[1];
+            if (D > 1) dst[2 * kLocPerD] = -K.c * E[2];
+        }
+    }
+}
+
+// the Gauss nodes sx[p] and weights sw[p], w_b x_b behind the weights
+__device__ __forceinline__ void load_rule(const DevMesh& M, double* sx, double* sw) {
+    for (int t = threadIdx.x; t < M.p; t += blockDim.x) {
+        const double x = M.xg[t], w = M.wg[t];
+        sx[t] = x;
+        sw[t] = w;
+        sw[M.p + t] = w * x;
+    }
+}
+
+template <int D, bool CURVED>
+__global__ void __launch_bounds__(128, 2) k_general(DevMesh M, const Job* jobs, cplx* loc, long long npair) {
+    extern __shared__ __align__(16) unsigned char gsm[];
+    __shared__ double sx[32], sw[64];
+    load_rule(M, sx, sw);
+    __syncthreads();
+    const int job = blockIdx.y;
+    const KConst K = make_kconst(jobs[job]);
+    general_rows<D, CURVED>(M, K, blockIdx.x * (long long)(128 / M.p), sx, sw, reinterpret_cast<cplx*>(gsm),
+                            loc + (long long)job * npair * (D + 1) * kLocPerD);
+}
+
+// Complex wavenumbers: general pair number q of mesh M (in the builder's order by
+// distance) for one job: p x p Gauss points, the pair's local blocks written to locj
+// (the job's block array).
+template <int D, bool CURVED>
 __device__ __forceinline__ void general_pair(const DevMesh& M, const KConst& K, long long q, const double* sx,
                                              const double* sw, cplx* locj) {
+    constexpr bool RK = false;
     // neighbouring threads take pairs of similar panel distance, so a warp's lanes
     // mostly follow the same Hankel branch and series length
-    if (M.gorder) q = M.gorder[q];
-    long long i = (long long)((1.0 + sqrt(8.0 * (double)q + 1.0)) * 0.5);
-    while (i * (i - 1) / 2 > q) --i;
-    while ((i + 1) * i / 2 <= q) ++i;
-    long long j = q - i * (i - 1) / 2;
-    long long pid = tri_index(i, j);
-    uint8_t fl = M.flags[pid];
-    if (fl & 0x80) return;   // coincident / adjacent: singular kernel
+    const unsigned pr = M.gpairs[q];
+    const long long i = pr >> 16, j = pr & 0xffffu;
+    const long long pid = tri_index(i, j);
+    const uint8_t fl = M.flags[pid];
     const bool use_dl = !(fl & PF_DL0_ZERO), use_dlt = !(fl & PF_DLT0_ZERO), tz = (fl & PF_TDT0_ZERO) != 0;
     const int p = M.p;
     const cplx* pti = M.gpt + i * p;
@@ -417,43 +617,39 @@ __device__ __forceinline__ void general_pair(const DevMesh& M, const KConst& K, 
                            locj + pid * (D + 1) * kLocPerD);
 }
 
-// General pairs, one thread per pair.
-template <int D, bool RK, bool CURVED>
-__global__ void __launch_bounds__(128) k_general(DevMesh M, const Job* jobs, cplx* loc, long long npair) {
+// Complex wavenumbers, one thread per pair.
+template <int D, bool CURVED>
+__global__ void __launch_bounds__(128) k_general_z(DevMesh M, const Job* jobs, cplx* loc, long long npair) {
     __shared__ double sx[64], sw[64];
     for (int t = threadIdx.x; t < M.p; t += blockDim.x) { sx[t] = M.xg[t]; sw[t] = M.wg[t]; }
     __syncthreads();
     long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    long long nlow = (long long)M.n * (M.n - 1) / 2;   // strictly lower pairs
-    if (q >= nlow) return;
+    if (q >= M.ngen) return;
     const int job = blockIdx.y;
     KConst K = make_kconst(jobs[job]);
-    general_pair<D, RK, CURVED>(M, K, q, sx, sw, loc + (long long)job * npair * (D + 1) * kLocPerD);
+    general_pair<D, CURVED>(M, K, q, sx, sw, loc + (long long)job * npair * (D + 1) * kLocPerD);
 }
 
-template <int D, bool RK, bool CURVED>
-__global__ void __launch_bounds__(128) k_general_w(DevMesh M, const Job* jobs, cplx* loc, long long npair, int ppw) {
+template <int D, bool CURVED>
+__global__ void __launch_bounds__(128) k_general_zw(DevMesh M, const Job* jobs, cplx* loc, long long npair, int ppw) {
     __shared__ double sx[64], sw[64];
     for (int t = threadIdx.x; t < M.p; t += blockDim.x) { sx[t] = M.xg[t]; sw[t] = M.wg[t]; }
     __syncthreads();
-    // k_general with one warp per pair, its lanes over the p x p Gauss points: for
+    // k_general_z with one warp per pair, its lanes over the p x p Gauss points: for
     // launches with few pairs x media (the Newton rounds of a small scatterer) a thread
     // per pair leaves most of the GPU idle.  Each warp takes ppw consecutive pairs.
     const int lane = threadIdx.x & 31;
-    const long long nlow = (long long)M.n * (M.n - 1) / 2;   // strictly lower pairs
+    constexpr bool RK = false;
     const long long q0 = (blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5)) * ppw;
-    if (q0 >= nlow) return;   // whole warp
+    if (q0 >= M.ngen) return;   // whole warp
     const int job = blockIdx.y;
     const KConst K = make_kconst(jobs[job]);
     const int p = M.p;
-    for (long long q = q0; q < q0 + ppw && q < nlow; ++q) {
-        long long i = (long long)((1.0 + sqrt(8.0 * (double)q + 1.0)) * 0.5);
-        while (i * (i - 1) / 2 > q) --i;
-        while ((i + 1) * i / 2 <= q) ++i;
-        const long long j = q - i * (i - 1) / 2;
+    for (long long q = q0; q < q0 + ppw && q < M.ngen; ++q) {
+        const unsigned pr = M.gpairs[q];
+        const long long i = pr >> 16, j = pr & 0xffffu;
         const long long pid = tri_index(i, j);
         const uint8_t fl = M.flags[pid];
-        if (fl & 0x80) continue;   // coincident / adjacent: singular kernel (whole warp)
         const bool use_dl = !(fl & PF_DL0_ZERO), use_dlt = !(fl & PF_DLT0_ZERO), tz = (fl & PF_TDT0_ZERO) != 0;
         const cplx* pti = M.gpt + i * p;
         const cplx* ptj = M.gpt + j * p;
@@ -801,11 +997,12 @@ __device__ __forceinline__ int job_of_block(const long long* start, int njobs, l
     return lo;
 }
 
-template <int D, bool RK, bool CURVED>
-__global__ void __launch_bounds__(128) k_general_multi(const MultiMesh* meshes, const MultiJob* jobs,
-                                                       const long long* start, int njobs, cplx* loc) {
+template <int D, bool CURVED>
+__global__ void __launch_bounds__(128, 2) k_general_multi(const MultiMesh* meshes, const MultiJob* jobs,
+                                                          const long long* start, int njobs, cplx* loc) {
+    extern __shared__ __align__(16) unsigned char gsm[];
     __shared__ DevMesh sM;
-    __shared__ double sx[64], sw[64];
+    __shared__ double sx[32], sw[64];
     __shared__ int sjob;
     if (threadIdx.x == 0) {
         sjob = job_of_block(start, njobs, blockIdx.x);
@@ -813,17 +1010,15 @@ __global__ void __launch_bounds__(128) k_general_multi(const MultiMesh* meshes, 
     }
     __syncthreads();
     const int job = sjob;
-    for (int t = threadIdx.x; t < sM.p; t += blockDim.x) { sx[t] = sM.xg[t]; sw[t] = sM.wg[t]; }
+    load_rule(sM, sx, sw);
     __syncthreads();
-    const long long q = (blockIdx.x - start[job]) * (long long)blockDim.x + threadIdx.x;
-    const long long nlow = (long long)sM.n * (sM.n - 1) / 2;
-    if (q >= nlow) return;
     const MultiJob J = jobs[job];
     const KConst K = make_kconst(J.job);
-    general_pair<D, RK, CURVED>(sM, K, q, sx, sw, loc + J.loc);
+    general_rows<D, CURVED>(sM, K, (blockIdx.x - start[job]) * (long long)(128 / sM.p), sx, sw,
+                            reinterpret_cast<cplx*>(gsm), loc + J.loc);
 }
 
-template <int D, bool RK, bool CURVED>
+template <int D, bool CURVED>
 __global__ void __launch_bounds__(128) k_singular_multi(const MultiMesh* meshes, const MultiJob* jobs,
                                                         const long long* start, int njobs, cplx* loc) {
     extern __shared__ double sm[];
@@ -846,7 +1041,7 @@ __global__ void __launch_bounds__(128) k_singular_multi(const MultiMesh* meshes,
     const MultiJob J = jobs[sjob];
     const KConst K = make_kconst(J.job);
     const SingularTask T = sT;
-    singular_pair<D, RK, CURVED>(sM, T, (int)(blockIdx.x - start[sjob]), K, sxc, swc, red, loc + J.loc);
+    singular_pair<D, true, CURVED>(sM, T, (int)(blockIdx.x - start[sjob]), K, sxc, swc, red, loc + J.loc);
 }
 
 // ------------------------------------------------------------------ gather
@@ -1014,10 +1209,18 @@ cudaError_t launch_hankel01(int n, const cplx* z, int complex_arg, cplx* h0, cpl
 
 // ------------------------------------------------------------------ launchers
 
-// General-pair layout of a launch: kLayoutAuto picks by size (a thread per pair
-// once pairs x jobs fill the GPU, else a warp per pair with ppw pairs per warp);
-// 0 forces a thread per pair, ppw > 0 a warp per pair with that many pairs.
+// General-pair layout of a complex-wavenumber launch: kLayoutAuto picks by size (a
+// thread per pair once pairs x jobs fill the GPU, else a warp per pair with ppw pairs per
+// warp); 0 forces a thread per pair, ppw > 0 a warp per pair with that many pairs.  Real
+// wavenumbers have one layout (k_general).
 constexpr int kLayoutAuto = -1;
+
+// dynamic shared memory above 48 KB is asked for once per kernel and device
+template <class Kernel>
+static cudaError_t allow_smem(Kernel kernel, size_t bytes) {
+    return bytes <= 48 * 1024 ? cudaSuccess
+                              : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
 
 // Parts per point set (q) of the split singular launch: about four CTAs per SM (152
 // SMs) counting an adjacent pair's two sets, at most 8; 0 when the launch has that
@@ -1043,25 +1246,32 @@ template <int D, bool RK, bool CURVED>
 static cudaError_t launch_local_c(const DevMesh& M, const SingularTask* tasks, int ntasks, const Job* jobs, int njobs,
                                   cplx* loc, cudaStream_t st, int layout, int which, double* part) {
     long long npair = (long long)M.n * (M.n + 1) / 2;
-    long long nlow = (long long)M.n * (M.n - 1) / 2;
     constexpr int NV = (int)(sizeof(Acc<D, CURVED>) / sizeof(double));
     const size_t ssmem = (2 * (size_t)M.nc + 4 * NV) * sizeof(double);
     const int q = (part && (which & 2)) ? singular_parts(ntasks, njobs) : 0;
     if (q > 0)
         k_singular_part<D, RK, CURVED><<<dim3(ntasks * 2 * q, njobs), 128, ssmem, st>>>(M, tasks, jobs, q, part);
-    if (nlow > 0 && (which & 1)) {
-        int ppw = layout;
-        if (layout == kLayoutAuto) {
-            if (nlow * njobs >= 152LL * 16 * 32) ppw = 0;   // enough pairs x media for a thread per pair
-            else ppw = (int)std::min(16LL, std::max(1LL, nlow * njobs / 8192));   // ~8k warps in the launch
-        }
-        if (ppw == 0) {
-            dim3 g((unsigned)((nlow + 127) / 128), njobs);
-            k_general<D, RK, CURVED><<<g, 128, 0, st>>>(M, jobs, loc, npair);
+    if (M.ngen > 0 && (which & 1)) {
+        if constexpr (RK) {
+            const size_t smem = GenDims<D, CURVED>::smem(M.p);
+            if (cudaError_t e = allow_smem(k_general<D, CURVED>, smem); e != cudaSuccess) return e;
+            const int ppc = 128 / M.p;
+            k_general<D, CURVED><<<dim3((unsigned)((M.ngen + ppc - 1) / ppc), njobs), 128, smem, st>>>(M, jobs, loc,
+                                                                                                     npair);
         } else {
-            const long long per_cta = 4LL * ppw;
-            dim3 g((unsigned)((nlow + per_cta - 1) / per_cta), njobs);
-            k_general_w<D, RK, CURVED><<<g, 128, 0, st>>>(M, jobs, loc, npair, ppw);
+            int ppw = layout;
+            if (layout == kLayoutAuto) {
+                if (M.ngen * njobs >= 152LL * 16 * 32) ppw = 0;   // enough pairs x media for a thread per pair
+                else ppw = (int)std::min(16LL, std::max(1LL, M.ngen * njobs / 8192));   // ~8k warps in the launch
+            }
+            if (ppw == 0) {
+                dim3 g((unsigned)((M.ngen + 127) / 128), njobs);
+                k_general_z<D, CURVED><<<g, 128, 0, st>>>(M, jobs, loc, npair);
+            } else {
+                const long long per_cta = 4LL * ppw;
+                dim3 g((unsigned)((M.ngen + per_cta - 1) / per_cta), njobs);
+                k_general_zw<D, CURVED><<<g, 128, 0, st>>>(M, jobs, loc, npair, ppw);
+            }
         }
     }
     if (q > 0) {
@@ -1098,15 +1308,19 @@ cudaError_t launch_flags(const DevMesh& M, const SingularTask* tasks, int ntasks
     return cudaGetLastError();
 }
 
-template <int D, bool RK, bool CURVED>
+template <int D, bool CURVED>
 static cudaError_t launch_multi_c(const MultiMesh* meshes, const MultiJob* jobs, int njobs, const long long* gstart,
-                                  long long gblocks, const long long* sstart, long long sblocks, int max_nc, cplx* loc,
-                                  cudaStream_t st) {
-    if (gblocks > 0) k_general_multi<D, RK, CURVED><<<(unsigned)gblocks, 128, 0, st>>>(meshes, jobs, gstart, njobs, loc);
+                                  long long gblocks, const long long* sstart, long long sblocks, int max_nc, int min_p,
+                                  cplx* loc, cudaStream_t st) {
+    if (gblocks > 0) {
+        const size_t smem = GenDims<D, CURVED>::smem(min_p);
+        if (cudaError_t e = allow_smem(k_general_multi<D, CURVED>, smem); e != cudaSuccess) return e;
+        k_general_multi<D, CURVED><<<(unsigned)gblocks, 128, smem, st>>>(meshes, jobs, gstart, njobs, loc);
+    }
     if (sblocks > 0) {
         constexpr int NV = (int)(sizeof(Acc<D, CURVED>) / sizeof(double));
         const size_t smem = (2 * (size_t)max_nc + 4 * NV) * sizeof(double);
-        k_singular_multi<D, RK, CURVED><<<(unsigned)sblocks, 128, smem, st>>>(meshes, jobs, sstart, njobs, loc);
+        k_singular_multi<D, CURVED><<<(unsigned)sblocks, 128, smem, st>>>(meshes, jobs, sstart, njobs, loc);
     }
     return cudaGetLastError();
 }
@@ -1114,23 +1328,20 @@ static cudaError_t launch_multi_c(const MultiMesh* meshes, const MultiJob* jobs,
 // The pair blocks of njobs jobs over several meshes in two launches (see the
 // many-mesh kernels): gstart / sstart (njobs + 1 entries, device) are the jobs'
 // first CTA numbers of the general and singular launch.
+// min_p: the lowest quadrature order among the meshes (the most pairs per CTA).  The
+// wavenumbers are real and positive.
 cudaError_t launch_local_multi(const MultiMesh* meshes, const MultiJob* jobs, int njobs, const long long* gstart,
-                               long long gblocks, const long long* sstart, long long sblocks, int max_nc, bool curved,
-                               bool real_k, int d, cplx* loc, cudaStream_t st) {
+                               long long gblocks, const long long* sstart, long long sblocks, int max_nc, int min_p,
+                               bool curved, int d, cplx* loc, cudaStream_t st) {
     if (gblocks > 0x7fffffffLL || sblocks > 0x7fffffffLL) return cudaErrorInvalidValue;
-#define HB_MULTI(D_, RK_)                                                                                        \
-    return curved ? launch_multi_c<D_, RK_, true>(meshes, jobs, njobs, gstart, gblocks, sstart, sblocks, max_nc, \
-                                                  loc, st)                                                       \
-                  : launch_multi_c<D_, RK_, false>(meshes, jobs, njobs, gstart, gblocks, sstart, sblocks, max_nc, \
-                                                   loc, st)
-    if (real_k) {
-        if (d == 0) HB_MULTI(0, true);
-        if (d == 1) HB_MULTI(1, true);
-        HB_MULTI(2, true);
-    }
-    if (d == 0) HB_MULTI(0, false);
-    if (d == 1) HB_MULTI(1, false);
-    HB_MULTI(2, false);
+#define HB_MULTI(D_)                                                                                            \
+    return curved ? launch_multi_c<D_, true>(meshes, jobs, njobs, gstart, gblocks, sstart, sblocks, max_nc, min_p, \
+                                             loc, st)                                                           \
+                  : launch_multi_c<D_, false>(meshes, jobs, njobs, gstart, gblocks, sstart, sblocks, max_nc, min_p, \
+                                              loc, st)
+    if (d == 0) HB_MULTI(0);
+    if (d == 1) HB_MULTI(1);
+    HB_MULTI(2);
 #undef HB_MULTI
 }
 

@@ -3,7 +3,8 @@
 //
 // Work decomposition (square P1 spaces, panel pairs i >= j as in
 // galerkin_builder.cpp:958-1013):
-//   * general pairs   -- one thread per (pair, job), p x p tensor Gauss points;
+//   * general pairs   -- one thread per (pair, Gauss node of panel i, job), p points each
+//                        (complex k: one thread or one warp per pair);
 //   * singular pairs  -- one CTA per (coincident | adjacent pair, job), the
 //                        n_c x n_c Duffy-mapped composite points (x2 for adjacent)
 //                        split over the CTA and reduced in shared memory;
@@ -14,7 +15,7 @@
 #pragma once
 #include <cstdint>
 
-#include "hbem_device.cuh"
+#include "hankel_u.cuh"
 
 namespace hbem {
 
@@ -51,7 +52,9 @@ struct DevMesh {
     const double* gtn;        // [n][p] tangent norms
     const cplx* ends;         // [n][2] start/end (the [-1,1] map at -1/+1)
     const uint8_t* flags;     // [n(n+1)/2] per lower-triangle pair
-    const int* gorder = nullptr;   // [n(n-1)/2] strictly-lower pairs by distance (thread-per-pair order), or null
+    long long ngen = 0;                  // general (neither coincident nor adjacent) pairs
+    const unsigned* gpairs = nullptr;    // [ngen] i << 16 | j (i > j) in order of the panels' distance
+    const HkEntry* hk = nullptr;         // the Hankel table (hankel_u.cuh)
     const double* sgeo = nullptr;   // [ntasks][2][kSGeoFields][nc*nc] singular-pair point data, or null
 };
 

@@ -31,8 +31,8 @@ size_t singular_part_bytes(int ntasks, int njobs, int d, bool curved);
 cudaError_t launch_gather_T(int N, int d, const cplx* loc, const double* Mmass, int nk, int sp, cplx* T,
                             cudaStream_t st);
 cudaError_t launch_local_multi(const MultiMesh* meshes, const MultiJob* jobs, int njobs, const long long* gstart,
-                               long long gblocks, const long long* sstart, long long sblocks, int max_nc, bool curved,
-                               bool real_k, int d, cplx* loc, cudaStream_t st);
+                               long long gblocks, const long long* sstart, long long sblocks, int max_nc, int min_p,
+                               bool curved, int d, cplx* loc, cudaStream_t st);
 cudaError_t launch_gather_layers(int N, int d, int layers, const cplx* loc, int job, int sp, cplx* out,
                                  cudaStream_t st);
 cudaError_t launch_gather_layers_sub(int N, int d, int layers, const cplx* loc, int job, int row, int rows, int col,
@@ -283,8 +283,9 @@ double dist(cplx a, cplx b) { return std::hypot(a.re - b.re, a.im - b.im); }
 // timing on the launching stream
 // ---- autotuner of the general-pair layout (option "autotune", default 0)
 //
-// The general pairs of a launch run a thread per pair or a warp per pair with ppw
-// pairs per warp; the built-in rule picks by the number of pairs x jobs.  With the
+// The general pairs of a complex-wavenumber launch run a thread per pair or a warp per
+// pair with ppw pairs per warp; the built-in rule picks by the number of pairs x jobs (real
+// wavenumbers have one layout, number 0).  With the
 // autotuner on, the first launch of each (panels, order, jobs rounded up to a power
 // of two, derivative order, real k, curved) times every layout once on the launch's
 // own data (CUDA events on its stream) and keeps the fastest; later launches of the
@@ -331,6 +332,7 @@ int tuned_layout(const DevMesh& M, const SingularTask* tasks, int ntasks, const 
     int best = kLayoutAuto;
     float best_ms = 0.f;
     for (int lay : kTuneLayouts) {
+        if (real_k && lay > 0) break;   // one layout for real wavenumbers
         cudaEventRecord(a, st);
         if (launch_local(M, tasks, ntasks, jobs, njobs, real_k, d, loc, st, lay, 1, nullptr) != cudaSuccess) break;
         cudaEventRecord(b, st);
@@ -399,7 +401,9 @@ struct hbem_builder_s {
     DBuf d_kind, d_par, d_xg, d_wg, d_xc, d_wc, d_gpt, d_gtan, d_gtn, d_ends, d_flags, d_tasks;
     DBuf d_loc, d_jobs, d_layers;
     DBuf d_sgeo;   // k-independent point data of the singular pairs (when within kSingularTableMax)
-    DBuf d_gorder; // strictly-lower pair indices sorted by panel-midpoint distance
+    DBuf d_gpairs; // general pairs (i << 16 | j) sorted by panel-midpoint distance
+    long long ngen = 0;
+    const HkEntry* hk = nullptr;
     int asm_layers = 0, asm_d = -1, asm_rows = 0, asm_cols = 0;
 
     long long npair() const { return (long long)n * (n + 1) / 2; }
@@ -415,7 +419,9 @@ struct hbem_builder_s {
         M.gpt = d_gpt.as<cplx>(); M.gtan = d_gtan.as<cplx>(); M.gtn = d_gtn.as<double>();
         M.ends = d_ends.as<cplx>(); M.flags = d_flags.as<uint8_t>();
         M.sgeo = g_singular_table ? d_sgeo.as<double>() : nullptr;
-        M.gorder = d_gorder.as<int>();
+        M.gpairs = d_gpairs.as<unsigned>();
+        M.ngen = ngen;
+        M.hk = hk;
         return M;
     }
     // BuilderData::is_adjacent (galerkin_builder.cpp:189-201)
@@ -427,7 +433,7 @@ struct hbem_builder_s {
     }
     ~hbem_builder_s() {
         for (DBuf* b : {&d_kind, &d_par, &d_xg, &d_wg, &d_xc, &d_wc, &d_gpt, &d_gtan, &d_gtn, &d_ends, &d_flags,
-                        &d_tasks, &d_loc, &d_jobs, &d_layers, &d_sgeo, &d_gorder})
+                        &d_tasks, &d_loc, &d_jobs, &d_layers, &d_sgeo, &d_gpairs})
             b->release();
         if (st) cudaStreamDestroy(st);
     }
@@ -733,20 +739,25 @@ int hbem_builder_create(int npanels, const int* kinds, const double* params, int
     if (e == cudaSuccess) e = launch_flags(b->view(), b->d_tasks.as<SingularTask>(), (int)b->tasks.size(),
                                            b->d_flags.as<uint8_t>(), b->st);
     // general pairs in order of the distance between their panels' middle Gauss points
-    // (ties by index): the thread-per-pair kernel's warps then see similar distances
-    if (e == cudaSuccess && n > 1 && (long long)n * (n - 1) / 2 < (1LL << 31)) {
-        const long long nlow = (long long)n * (n - 1) / 2;
-        std::vector<float> key((size_t)nlow);
-        std::vector<int> ord((size_t)nlow);
-        for (long long i = 1, q = 0; i < n; ++i)
-            for (long long j = 0; j < i; ++j, ++q) {
+    // (ties by index): a warp's points then lie in neighbouring intervals of the Hankel table
+    if (e == cudaSuccess && n <= 65536) {
+        std::vector<std::pair<float, unsigned>> ord;
+        ord.reserve((size_t)b->npair());
+        for (int i = 1; i < n; ++i)
+            for (int j = 0; j < i; ++j) {
+                if (flags[tri_index(i, j)]) continue;
                 const cplx a = gpt[(size_t)i * p + p / 2], c = gpt[(size_t)j * p + p / 2];
-                key[(size_t)q] = (float)std::hypot(a.re - c.re, a.im - c.im);
-                ord[(size_t)q] = (int)q;
+                const double dx = a.re - c.re, dy = a.im - c.im;
+                ord.emplace_back((float)(dx * dx + dy * dy), (unsigned)i << 16 | (unsigned)j);
             }
-        std::stable_sort(ord.begin(), ord.end(), [&](int x, int y) { return key[(size_t)x] < key[(size_t)y]; });
-        e = upload(b->d_gorder, ord, b->st);
+        std::sort(ord.begin(), ord.end());
+        std::vector<unsigned> pairs(ord.size());
+        for (size_t q = 0; q < ord.size(); ++q) pairs[q] = ord[q].second;
+        b->ngen = (long long)pairs.size();
+        e = upload(b->d_gpairs, pairs, b->st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(b->st);   // the host copy ends here
     }
+    if (e == cudaSuccess) b->hk = hankel_table(&e);
     const size_t geo_bytes = singular_geo_bytes(b->nc, (int)b->tasks.size());
     if (e == cudaSuccess && geo_bytes > 0 && geo_bytes <= kSingularTableMax) {
         e = b->d_sgeo.ensure(geo_bytes);
@@ -1073,10 +1084,11 @@ int hbem_gen_sol_op_multi_device(const hbem_solop* ops, int nops, const int* cou
     DBuf& d_jobs = b0->d_jobs;
     DBuf& d_loc = b0->d_loc;
     std::vector<MultiMesh> meshes(nops);
-    int max_nc = 0;
+    int max_nc = 0, min_p = 32;
     for (int i = 0; i < nops; ++i) {
         meshes[i] = MultiMesh{ops[i]->b->view(), ops[i]->b->d_tasks.as<SingularTask>(), (int)ops[i]->b->tasks.size()};
         max_nc = std::max(max_nc, ops[i]->b->nc);
+        min_p = std::min(min_p, ops[i]->b->p);
     }
     HB_CK(upload(d_meshes, meshes, st));
     const size_t per_pair = (size_t)(d + 1) * kLocPerD;   // complex entries per pair and job
@@ -1101,13 +1113,12 @@ int hbem_gen_sol_op_multi_device(const hbem_solop* ops, int nops, const int* cou
                 if ((b->lines == 0) != (curved == 1) || (size_t)counts[i] <= q0) continue;
                 nk[i] = std::min(chunk, (size_t)counts[i] - q0);
                 first[i] = jobs.size();
-                const long long nlow = (long long)b->n * (b->n - 1) / 2;
                 for (size_t q = 0; q < nk[i]; ++q) {
                     const double k = k_host[koff[i] + q0 + q];
                     for (double c : {c_i_host[i], c_o}) {
                         jobs.push_back(MultiJob{Job{k, 0., c}, i, off});
                         off += (long long)(b->npair() * per_pair);
-                        gstart.push_back(gstart.back() + (nlow + 127) / 128);
+                        gstart.push_back(gstart.back() + (b->ngen + 128 / b->p - 1) / (128 / b->p));
                         sstart.push_back(sstart.back() + (long long)b->tasks.size());
                     }
                 }
@@ -1124,7 +1135,7 @@ int hbem_gen_sol_op_multi_device(const hbem_solop* ops, int nops, const int* cou
             if (timed) timing_begin(&e0, st);
             HB_CK(launch_local_multi(d_meshes.as<MultiMesh>(), d_jobs.as<MultiJob>(), njobs, d_start.as<long long>(),
                                      gstart.back(), d_start.as<long long>() + gstart.size(), sstart.back(), max_nc,
-                                     curved == 1, true, (int)d, d_loc.as<cplx>(), st));
+                                     min_p, curved == 1, (int)d, d_loc.as<cplx>(), st));
             g_launches += (gstart.back() > 0 ? 1 : 0) + (sstart.back() > 0 ? 1 : 0);
             if (timed) {
                 timing_end(e0, st);
