@@ -405,6 +405,55 @@ __device__ __forceinline__ cplx entry_fwd(const cplx* m, int a, int b) {
     return a ? r0 - r1 : r1;
 }
 
+// Entry e = 2 a + b (shape functions a on panel i, b on panel j) of block `kind` (0 double
+// layer, 1 transposed double layer, 2 hypersingular, 3 single layer) of a pair, all
+// derivative orders, from its moments m[set][function][4] (sets as above); rx, ry: the
+// shape functions on panel i / j run the other way (adjacent pairs); ttp: |tau_i||tau_j|;
+// tw: 2 tau_i . tau_j on straight panels (0 where it vanishes).  out: the pair's blocks.
+template <int D, bool CURVED>
+__device__ __forceinline__ void block_entry(const KConst& K, const cplx* m, int kind, int e, bool rx, bool ry,
+                                            double ttp, double tw, cplx* out) {
+    constexpr int F = D + 1;
+    const double ks = K.ks.re, ks2 = ks * ks, kc = K.c * K.k.re;
+    const int sa = e >> 1, sb = e & 1;
+    cplx* dst = out + 4 * kind + e;
+    if (kind < 2) {        // the transposed double layer has its test function on the y panel
+        const cplx* md = m + (kind == 0 ? 1 : 2) * F * 4;
+        const int ex = (kind == 0 ? sa : sb) ^ (int)rx, ey = (kind == 0 ? sb : sa) ^ (int)ry;
+        dst[0] = ks2 * entry_fwd(md, ex, ey);
+        if (D > 0) {
+            const cplx d1 = entry_fwd(md + 4, ex, ey);
+            dst[kLocPerD] = kc * d1;
+            if (D > 1) dst[2 * kLocPerD] = K.c * (d1 - ks2 * entry_fwd(md + 8, ex, ey));
+        }
+        return;
+    }
+    // {h0, |v| h1, |v|^2 h0 - |v| h1 / ks} from {f, v2 g, v2 f}
+    const int ex = sa ^ (int)rx, ey = sb ^ (int)ry;
+    const double fct = kind == 3 ? ttp : CURVED ? 1. : tw;
+    const cplx* mm = m + (kind == 2 && CURVED ? 3 * F * 4 : 0);
+    cplx E[3];
+    E[0] = fct * entry_fwd(mm, ex, ey);
+    if (D > 0) {
+        const cplx vg = fct * entry_fwd(mm + 4, ex, ey);
+        E[1] = ks * vg;
+        if (D > 1) E[2] = fct * entry_fwd(mm + 8, ex, ey) - vg;
+    }
+    if (kind == 2) {   // b'_a b'_b times the plain moments, and the k^2 term
+        const double dd = (sa == sb) ? 1. : -1., k2h = 0.5 * ks2;
+        const cplx W0 = E[0];
+        E[0] = dd * m[0] - k2h * W0;
+        if (D > 0) {
+            const cplx W1 = E[1];
+            E[1] = (dd * ks) * m[4] - k2h * W1 + ks * W0;
+            if (D > 1) E[2] = dd * (m[8] - m[4]) - k2h * E[2] - (2. * ks) * W1 + W0;
+        }
+    }
+    dst[0] = E[0];
+    if (D > 0) dst[kLocPerD] = -K.sqrtc * E[1];
+    if (D > 1) dst[2 * kLocPerD] = -K.c * E[2];
+}
+
 // The pairs q0 .. of mesh M that one CTA takes, for the job K; locj: the job's blocks.
 template <int D, bool CURVED>
 __device__ __forceinline__ void general_rows(const DevMesh& M, const KConst& K, long long q0, const double* sx,
@@ -497,53 +546,15 @@ __device__ __forceinline__ void general_rows(const DevMesh& M, const KConst& K, 
     __syncthreads();
     // the pair's blocks: 4 kinds x 4 shape-function pairs, the kind slowest so that a warp
     // mostly has one
-    const double ks = K.ks.re, ks2 = ks * ks, kc = K.c * K.k.re;
     for (int it = threadIdx.x; it < npairs * 16; it += G::THREADS) {
         const int kind = it / (4 * npairs), rest = it - kind * 4 * npairs, l = rest >> 2, e = rest & 3;
-        const int sa = e >> 1, sb = e & 1;
         const unsigned pr = M.gpairs[q0 + l];
         const int i = pr >> 16, j = pr & 0xffffu;
-        const cplx* m = mom + (long long)l * (G::NV / 2) * 4;
-        cplx* dst = locj + tri_index(i, j) * (D + 1) * kLocPerD + 4 * kind + e;
-        if (kind < 2) {        // double layer, transposed double layer (test function on the y panel)
-            const cplx* md = m + (kind == 0 ? 1 : 2) * F * 4;
-            const int ex = kind == 0 ? sa : sb, ey = kind == 0 ? sb : sa;
-            dst[0] = ks2 * entry_fwd(md, ex, ey);
-            if (D > 0) {
-                const cplx d1 = entry_fwd(md + 4, ex, ey);
-                dst[kLocPerD] = kc * d1;
-                if (D > 1) dst[2 * kLocPerD] = K.c * (d1 - ks2 * entry_fwd(md + 8, ex, ey));
-            }
-        } else {
-            const cplx t0i = M.gtan[i * p], t0j = M.gtan[j * p];
-            const double ttp = M.gtn[i * p] * M.gtn[j * p];
-            // s: {h0, |v| h1, |v|^2 h0 - |v| h1 / ks} from {f, v2 g, v2 f}
-            const cplx* mw = m + (CURVED ? 3 * F * 4 : 0);
-            const bool tz = (M.flags[tri_index(i, j)] & PF_TDT0_ZERO) != 0;
-            const double tw = CURVED ? 1. : tz ? 0. : 2. * (t0i.im * t0j.im + t0i.re * t0j.re);
-            const double fct = kind == 3 ? ttp : tw;
-            const cplx* mm = kind == 3 ? m : mw;
-            cplx E[3];
-            E[0] = fct * entry_fwd(mm, sa, sb);
-            if (D > 0) {
-                const cplx vg = fct * entry_fwd(mm + 4, sa, sb);
-                E[1] = ks * vg;
-                if (D > 1) E[2] = fct * entry_fwd(mm + 8, sa, sb) - vg;
-            }
-            if (kind == 2) {   // hypersingular: b'_a b'_b h0 moments and the k^2 term
-                const double dd = (sa == sb) ? 1. : -1., k2h = 0.5 * ks2;
-                const cplx W0 = E[0];
-                E[0] = dd * m[0] - k2h * W0;
-                if (D > 0) {
-                    const cplx W1 = E[1];
-                    E[1] = (dd * ks) * m[4] - k2h * W1 + ks * W0;
-                    if (D > 1) E[2] = dd * (m[8] - m[4]) - k2h * E[2] - (2. * ks) * W1 + W0;
-                }
-            }
-            dst[0] = E[0];
-            if (D > 0) dst[kLocPerD] = -K.sqrtc * E[1];
-            if (D > 1) dst[2 * kLocPerD] = -K.c * E[2];
-        }
+        const cplx t0i = M.gtan[i * p], t0j = M.gtan[j * p];
+        const bool tz = (M.flags[tri_index(i, j)] & PF_TDT0_ZERO) != 0;
+        block_entry<D, CURVED>(K, mom + (long long)l * (G::NV / 2) * 4, kind, e, false, false,
+                               M.gtn[i * p] * M.gtn[j * p], tz ? 0. : 2. * (t0i.im * t0j.im + t0i.re * t0j.re),
+                               locj + tri_index(i, j) * (D + 1) * kLocPerD);
     }
 }
 
@@ -792,51 +803,9 @@ __device__ __forceinline__ void singular_accumulate(Acc<D, CURVED>& A, const KCo
     }
 }
 
-// One coincident / adjacent pair (task index ti of mesh M) for one job, reduced over
-// the CTA: its local blocks written to out.  sxc, swc: the composite nodes and
-// weights in shared memory; red: reduction space.
-template <int D, bool RK, bool CURVED>
-__device__ __forceinline__ void singular_pair(const DevMesh& M, const SingularTask& T, int ti, const KConst& K,
-                                              const double* sxc, const double* swc, double* red, cplx* out) {
-    const long long pid = tri_index(T.i, T.j);
-    const uint8_t fl = M.flags[pid];
-    const int nc = M.nc, tot = nc * nc;
-    const int nset = T.kind == PK_COINC ? 1 : 2;
-    // point data from the table when the builder made one, else computed here
-    const double* G = M.sgeo ? M.sgeo + (long long)ti * 2 * kSGeoFields * tot : nullptr;
-    Acc<D, CURVED> A;
-    A.zero();
-    for (int e = threadIdx.x; e < tot; e += blockDim.x) {
-        const int a = e % nc, b = e / nc;
-#pragma unroll 1
-        for (int Kset = 0; Kset < nset; ++Kset) {
-            double f[kSGeoFields];
-            if (G) {
-#pragma unroll
-                for (int q = 0; q < kSGeoFields; ++q) f[q] = __ldg(G + ((long long)Kset * kSGeoFields + q) * tot + e);
-            } else {
-                singular_fields(M, T, Kset, sxc[a], sxc[b], swc[a], swc[b], f);
-            }
-            singular_accumulate<D, RK, CURVED>(A, K, T.kind, fl, Kset, f);
-        }
-    }
-    block_reduce(A, red);
-    if (threadIdx.x == 0) {
-        // per-pair constants: tangent norms (constant on lines and arcs) and, for
-        // straight panels, the tangent product
-        SPoint P;
-        singular_point(M, T, 0, sxc[0], sxc[0], P);
-        const bool adj = T.kind == PK_ADJ;
-        const bool tz = CURVED ? false : (fl & PF_TDT0_ZERO) != 0;
-        store_local<D, CURVED>(A, K, adj && !T.swap, adj && T.swap, P.tin * P.tjn,
-                               2. * (P.ti.im * P.tj.im + P.ti.re * P.tj.re), tz, out + pid * (D + 1) * kLocPerD);
-    }
-}
-
-// (the per-pair code of singular_pair, kept inline here: the order-0 instance keeps
-// its register allocation of 128 per thread)
-template <int D, bool RK, bool CURVED>
-__global__ void __launch_bounds__(128) k_singular(DevMesh M, const SingularTask* tasks, const Job* jobs, cplx* loc,
+// Complex wavenumbers: one CTA per coincident / adjacent pair and job.
+template <int D, bool CURVED>
+__global__ void __launch_bounds__(128) k_singular_z(DevMesh M, const SingularTask* tasks, const Job* jobs, cplx* loc,
                                                   long long npair) {
     extern __shared__ double sm[];
     double* sxc = sm;
@@ -866,7 +835,7 @@ __global__ void __launch_bounds__(128) k_singular(DevMesh M, const SingularTask*
             } else {
                 singular_fields(M, T, Kset, sxc[a], sxc[b], swc[a], swc[b], f);
             }
-            singular_accumulate<D, RK, CURVED>(A, K, T.kind, fl, Kset, f);
+            singular_accumulate<D, false, CURVED>(A, K, T.kind, fl, Kset, f);
         }
     }
     block_reduce(A, red);
@@ -887,14 +856,14 @@ __global__ void __launch_bounds__(128) k_singular(DevMesh M, const SingularTask*
 //
 // A launch of a few wavenumbers (one Newton point of the plain search: 2 media) has
 // fewer singular CTAs than 4 per SM, and an adjacent pair's CTA (two point sets) takes
-// twice a coincident pair's time, so k_singular ends in a tail on part of the GPU.
+// twice a coincident pair's time, so one CTA per pair ends in a tail on part of the GPU.
 // Here each (pair, job) is split into CTAs of 1/q of a point set each: q parts for a
 // coincident pair, 2q for an adjacent one (blocks 2q t .. 2q t + 2q - 1 of pair t,
 // the upper q of a coincident pair empty), so that every CTA has the same work.  Their block sums go to `part`
 // ([job][pair x 2q][NV] doubles) and k_singular_join adds them in part order and forms
 // the pair blocks.
 
-template <int D, bool RK, bool CURVED>
+template <int D, bool CURVED>
 __global__ void __launch_bounds__(128) k_singular_part(DevMesh M, const SingularTask* tasks, const Job* jobs, int q,
                                                        double* part) {
     extern __shared__ double sm[];
@@ -926,7 +895,7 @@ __global__ void __launch_bounds__(128) k_singular_part(DevMesh M, const Singular
             const int a = e % nc, b = e / nc;
             singular_fields(M, T, Kset, sxc[a], sxc[b], swc[a], swc[b], f);
         }
-        singular_accumulate<D, RK, CURVED>(A, K, T.kind, fl, Kset, f);
+        singular_accumulate<D, false, CURVED>(A, K, T.kind, fl, Kset, f);
     }
     block_reduce(A, red);
     constexpr int NV = (int)(sizeof(Acc<D, CURVED>) / sizeof(double));
@@ -977,6 +946,10 @@ __global__ void __launch_bounds__(128) k_singular_join(DevMesh M, const Singular
                               loc + ((long long)job * npair + pid) * (D + 1) * kLocPerD, lane >> 1, lane & 1);
 }
 
+}  // namespace hbem
+#include "singular_rows.cuh"
+namespace hbem {
+
 // ------------------------------------------------------------------ many meshes in one launch
 //
 // The batching path: the jobs of several meshes (scatterers of uneven panel counts,
@@ -1019,9 +992,10 @@ __global__ void __launch_bounds__(128, 2) k_general_multi(const MultiMesh* meshe
 }
 
 template <int D, bool CURVED>
-__global__ void __launch_bounds__(128) k_singular_multi(const MultiMesh* meshes, const MultiJob* jobs,
-                                                        const long long* start, int njobs, cplx* loc) {
-    extern __shared__ double sm[];
+__global__ void __launch_bounds__(128, 2) k_singular_multi(const MultiMesh* meshes, const MultiJob* jobs,
+                                                           const long long* start, int njobs, cplx* loc) {
+    typedef RowDims<D, CURVED> R;
+    extern __shared__ __align__(16) unsigned char ssm[];
     __shared__ DevMesh sM;
     __shared__ int sjob;
     __shared__ SingularTask sT;
@@ -1032,16 +1006,45 @@ __global__ void __launch_bounds__(128) k_singular_multi(const MultiMesh* meshes,
         sT = MM.tasks[blockIdx.x - start[sjob]];
     }
     __syncthreads();
-    const int nc = sM.nc;
-    double* sxc = sm;
-    double* swc = sm + nc;
-    double* red = sm + 2 * nc;
-    for (int t = threadIdx.x; t < nc; t += blockDim.x) { sxc[t] = sM.xc[t]; swc[t] = sM.wc[t]; }
-    __syncthreads();
+    cplx* acc = reinterpret_cast<cplx*>(ssm);
+    cplx* mom = acc + R::NA * 128;
+    double* sxc = reinterpret_cast<double*>(mom + R::NA);
+    double* swc = sxc + sM.nc;
     const MultiJob J = jobs[sjob];
     const KConst K = make_kconst(J.job);
     const SingularTask T = sT;
-    singular_pair<D, true, CURVED>(sM, T, (int)(blockIdx.x - start[sjob]), K, sxc, swc, red, loc + J.loc);
+    if (nodes_serve(sM, (int)(blockIdx.x - start[sjob]), K)) return;   // whole CTA
+    load_composite(sM, sxc, swc);
+    __syncthreads();
+    singular_moments<D, CURVED>(sM, T, K, 0, 1, sxc, swc, acc, mom);
+    singular_store<D, CURVED>(sM, T, K, mom, threadIdx.x, 128,
+                              loc + J.loc + tri_index(T.i, T.j) * (D + 1) * kLocPerD);
+}
+
+template <int D, bool CURVED>
+__global__ void __launch_bounds__(128) k_singular_nodes_multi(const MultiMesh* meshes, const MultiJob* jobs,
+                                                              const long long* start, int njobs, cplx* loc) {
+    __shared__ DevMesh sM;
+    __shared__ int sjob, sn;
+    __shared__ const SingularTask* stasks;
+    __shared__ double vals[4][4][2][kSN];
+    __shared__ cplx mom[4][RowDims<D, CURVED>::NA];
+    if (threadIdx.x == 0) {
+        sjob = job_of_block(start, njobs, blockIdx.x);
+        const MultiMesh& MM = meshes[jobs[sjob].mesh];
+        sM = MM.M;
+        sn = MM.ntasks;
+        stasks = MM.tasks;
+    }
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, task = (int)(blockIdx.x - start[sjob]) * 4 + warp;
+    if (task >= sn) return;   // whole warp
+    const MultiJob J = jobs[sjob];
+    const KConst K = make_kconst(J.job);
+    if (!nodes_serve(sM, task, K)) return;
+    const SingularTask T = stasks[task];
+    singular_node_pair<D, CURVED>(sM, T, task, K, vals[warp], mom[warp],
+                                  loc + J.loc + tri_index(T.i, T.j) * (D + 1) * kLocPerD);
 }
 
 // ------------------------------------------------------------------ gather
@@ -1215,10 +1218,10 @@ cudaError_t launch_hankel01(int n, const cplx* z, int complex_arg, cplx* h0, cpl
 // wavenumbers have one layout (k_general).
 constexpr int kLayoutAuto = -1;
 
-// dynamic shared memory above 48 KB is asked for once per kernel and device
+// more than 48 KB of shared memory (with the static part) has to be asked for
 template <class Kernel>
 static cudaError_t allow_smem(Kernel kernel, size_t bytes) {
-    return bytes <= 48 * 1024 ? cudaSuccess
+    return bytes <= 40 * 1024 ? cudaSuccess
                               : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
@@ -1241,16 +1244,24 @@ size_t singular_part_bytes(int ntasks, int njobs, int d, bool curved) {
 }
 
 // part: scratch of singular_part_bytes for the split singular launch of few jobs, or
-// null (one CTA per pair and job)
+// null (one CTA per pair and job); which: bit 0 the general pairs, bit 1 the singular
+// pairs, bit 2 some singular pair of a mesh with a node table is beyond its range
 template <int D, bool RK, bool CURVED>
 static cudaError_t launch_local_c(const DevMesh& M, const SingularTask* tasks, int ntasks, const Job* jobs, int njobs,
                                   cplx* loc, cudaStream_t st, int layout, int which, double* part) {
     long long npair = (long long)M.n * (M.n + 1) / 2;
-    constexpr int NV = (int)(sizeof(Acc<D, CURVED>) / sizeof(double));
-    const size_t ssmem = (2 * (size_t)M.nc + 4 * NV) * sizeof(double);
     const int q = (part && (which & 2)) ? singular_parts(ntasks, njobs) : 0;
-    if (q > 0)
-        k_singular_part<D, RK, CURVED><<<dim3(ntasks * 2 * q, njobs), 128, ssmem, st>>>(M, tasks, jobs, q, part);
+    const bool rows = (which & 2) && ntasks > 0 && (!RK || !M.snode || (which & 4));
+    constexpr int NV = (int)(sizeof(Acc<D, CURVED>) / sizeof(double));
+    const size_t ssmem = RK ? RowDims<D, CURVED>::kSmem + 2 * (size_t)M.nc * sizeof(double)
+                            : (2 * (size_t)M.nc + 4 * NV) * sizeof(double);
+    if (rows && RK) {
+        if (cudaError_t e = allow_smem(k_singular_rows<D, CURVED>, ssmem); e != cudaSuccess) return e;
+        k_singular_rows<D, CURVED><<<dim3(q ? ntasks * 2 * q : ntasks, njobs), 128, ssmem, st>>>(M, tasks, jobs, q, part,
+                                                                                                loc, npair);
+    } else if (rows && q > 0) {
+        k_singular_part<D, CURVED><<<dim3(ntasks * 2 * q, njobs), 128, ssmem, st>>>(M, tasks, jobs, q, part);
+    }
     if (M.ngen > 0 && (which & 1)) {
         if constexpr (RK) {
             const size_t smem = GenDims<D, CURVED>::smem(M.p);
@@ -1274,12 +1285,14 @@ static cudaError_t launch_local_c(const DevMesh& M, const SingularTask* tasks, i
             }
         }
     }
-    if (q > 0) {
-        k_singular_join<D, CURVED><<<dim3((ntasks + 3) / 4, njobs), 128, 0, st>>>(M, tasks, jobs, ntasks, q, part, loc,
-                                                                                   npair);
-    } else if (ntasks > 0 && (which & 2)) {
-        dim3 g(ntasks, njobs);
-        k_singular<D, RK, CURVED><<<g, 128, ssmem, st>>>(M, tasks, jobs, loc, npair);
+    if (RK && M.snode && ntasks > 0 && (which & 2))
+        k_singular_nodes<D, CURVED><<<dim3((ntasks + 3) / 4, njobs), 128, 0, st>>>(M, tasks, ntasks, jobs, loc, npair);
+    if (rows && q > 0) {
+        const dim3 g((ntasks + 3) / 4, njobs);
+        if (RK) k_singular_rows_join<D, CURVED><<<g, 128, 0, st>>>(M, tasks, jobs, ntasks, q, part, loc, npair);
+        else k_singular_join<D, CURVED><<<g, 128, 0, st>>>(M, tasks, jobs, ntasks, q, part, loc, npair);
+    } else if (rows && !RK) {
+        k_singular_z<D, CURVED><<<dim3(ntasks, njobs), 128, ssmem, st>>>(M, tasks, jobs, loc, npair);
     }
     return cudaGetLastError();
 }
@@ -1301,6 +1314,30 @@ cudaError_t launch_singular_geo(const DevMesh& M, const SingularTask* tasks, int
     return cudaGetLastError();
 }
 
+// The node table (see k_singular_nodes): bytes, and its making on st.  scratch:
+// snode_scratch_bytes.
+size_t snode_bytes(int ntasks) { return (size_t)ntasks * kSNodeStride * sizeof(double); }
+double snode_limit() { return kSNodeX; }
+
+// CTAs per pair: about four per SM over the whole launch
+static int snode_split(int ntasks) { return std::max(1, std::min(16, (4 * 152 + ntasks - 1) / std::max(1, ntasks))); }
+
+size_t snode_scratch_bytes(int ntasks) {
+    return (size_t)ntasks * snode_split(ntasks) * kSNodePart * sizeof(double);
+}
+
+cudaError_t launch_snode(const DevMesh& M, const SingularTask* tasks, int ntasks, double* nodes, double* scratch,
+                         cudaStream_t st) {
+    if (ntasks <= 0) return cudaSuccess;
+    const int ns = snode_split(ntasks);
+    if (cudaError_t e = allow_smem(k_snode_part<false>, kSNodeSmem); e != cudaSuccess) return e;
+    if (cudaError_t e = allow_smem(k_snode_part<true>, kSNodeSmem); e != cudaSuccess) return e;
+    if (M.lines) k_snode_part<false><<<ntasks * ns, 128, kSNodeSmem, st>>>(M, tasks, ns, scratch);
+    else k_snode_part<true><<<ntasks * ns, 128, kSNodeSmem, st>>>(M, tasks, ns, scratch);
+    k_snode_join<<<ntasks, 128, 0, st>>>(M, tasks, ns, scratch, nodes);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_flags(const DevMesh& M, const SingularTask* tasks, int ntasks, uint8_t* flags, cudaStream_t st) {
     long long npair = (long long)M.n * (M.n + 1) / 2;
     k_flags_general<<<(unsigned)((npair + 127) / 128), 128, 0, st>>>(M, flags);
@@ -1310,43 +1347,45 @@ cudaError_t launch_flags(const DevMesh& M, const SingularTask* tasks, int ntasks
 
 template <int D, bool CURVED>
 static cudaError_t launch_multi_c(const MultiMesh* meshes, const MultiJob* jobs, int njobs, const long long* gstart,
-                                  long long gblocks, const long long* sstart, long long sblocks, int max_nc, int min_p,
-                                  cplx* loc, cudaStream_t st) {
+                                  long long gblocks, const long long* sstart, long long sblocks, const long long* nstart,
+                                  long long nblocks, int max_nc, int min_p, cplx* loc, cudaStream_t st) {
     if (gblocks > 0) {
         const size_t smem = GenDims<D, CURVED>::smem(min_p);
         if (cudaError_t e = allow_smem(k_general_multi<D, CURVED>, smem); e != cudaSuccess) return e;
         k_general_multi<D, CURVED><<<(unsigned)gblocks, 128, smem, st>>>(meshes, jobs, gstart, njobs, loc);
     }
     if (sblocks > 0) {
-        constexpr int NV = (int)(sizeof(Acc<D, CURVED>) / sizeof(double));
-        const size_t smem = (2 * (size_t)max_nc + 4 * NV) * sizeof(double);
+        const size_t smem = RowDims<D, CURVED>::kSmem + 2 * (size_t)max_nc * sizeof(double);
+        if (cudaError_t e = allow_smem(k_singular_multi<D, CURVED>, smem); e != cudaSuccess) return e;
         k_singular_multi<D, CURVED><<<(unsigned)sblocks, 128, smem, st>>>(meshes, jobs, sstart, njobs, loc);
     }
+    if (nblocks > 0)
+        k_singular_nodes_multi<D, CURVED><<<(unsigned)nblocks, 128, 0, st>>>(meshes, jobs, nstart, njobs, loc);
     return cudaGetLastError();
 }
 
-// The pair blocks of njobs jobs over several meshes in two launches (see the
-// many-mesh kernels): gstart / sstart (njobs + 1 entries, device) are the jobs'
-// first CTA numbers of the general and singular launch.
+// The pair blocks of njobs jobs over several meshes in up to three launches (see the
+// many-mesh kernels): gstart / sstart / nstart (njobs + 1 entries, device) are the jobs'
+// first CTA numbers of the general, the singular and the node-table launch.
 // min_p: the lowest quadrature order among the meshes (the most pairs per CTA).  The
 // wavenumbers are real and positive.
 cudaError_t launch_local_multi(const MultiMesh* meshes, const MultiJob* jobs, int njobs, const long long* gstart,
-                               long long gblocks, const long long* sstart, long long sblocks, int max_nc, int min_p,
-                               bool curved, int d, cplx* loc, cudaStream_t st) {
-    if (gblocks > 0x7fffffffLL || sblocks > 0x7fffffffLL) return cudaErrorInvalidValue;
-#define HB_MULTI(D_)                                                                                            \
-    return curved ? launch_multi_c<D_, true>(meshes, jobs, njobs, gstart, gblocks, sstart, sblocks, max_nc, min_p, \
-                                             loc, st)                                                           \
-                  : launch_multi_c<D_, false>(meshes, jobs, njobs, gstart, gblocks, sstart, sblocks, max_nc, min_p, \
-                                              loc, st)
+                               long long gblocks, const long long* sstart, long long sblocks,
+                               const long long* nstart, long long nblocks, int max_nc, int min_p, bool curved, int d,
+                               cplx* loc, cudaStream_t st) {
+    if (gblocks > 0x7fffffffLL || sblocks > 0x7fffffffLL || nblocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+#define HB_MULTI(D_)                                                                                             \
+    return curved ? launch_multi_c<D_, true>(meshes, jobs, njobs, gstart, gblocks, sstart, sblocks, nstart, nblocks, \
+                                             max_nc, min_p, loc, st)                                             \
+                  : launch_multi_c<D_, false>(meshes, jobs, njobs, gstart, gblocks, sstart, sblocks, nstart, nblocks, \
+                                              max_nc, min_p, loc, st)
     if (d == 0) HB_MULTI(0);
     if (d == 1) HB_MULTI(1);
     HB_MULTI(2);
 #undef HB_MULTI
 }
 
-// layout: kLayoutAuto or a forced general-pair layout (see launch_local_c); which:
-// bit 0 the general pairs, bit 1 the singular pairs; part: see launch_local_c
+// layout: kLayoutAuto or a forced general-pair layout; which, part: see launch_local_c
 cudaError_t launch_local(const DevMesh& M, const SingularTask* tasks, int ntasks, const Job* jobs, int njobs,
                          bool real_k, int d, cplx* loc, cudaStream_t st, int layout, int which, double* part) {
     if (real_k) {

@@ -7,7 +7,9 @@
 //                        (complex k: one thread or one warp per pair);
 //   * singular pairs  -- one CTA per (coincident | adjacent pair, job), the
 //                        n_c x n_c Duffy-mapped composite points (x2 for adjacent)
-//                        split over the CTA and reduced in shared memory;
+//                        split over the CTA and reduced in shared memory; small meshes
+//                        at real k: one warp, 16 nodes with k-independent weights
+//                        (singular_rows.cuh);
 //   * gather          -- one thread per output entry: sums the four panel-pair
 //                        contributions of a P1 dof pair and forms T(k) blocks.
 // A "job" is one (wavenumber, refraction index) pair, so the two media of a
@@ -55,7 +57,8 @@ struct DevMesh {
     long long ngen = 0;                  // general (neither coincident nor adjacent) pairs
     const unsigned* gpairs = nullptr;    // [ngen] i << 16 | j (i > j) in order of the panels' distance
     const HkEntry* hk = nullptr;         // the Hankel table (hankel_u.cuh)
-    const double* sgeo = nullptr;   // [ntasks][2][kSGeoFields][nc*nc] singular-pair point data, or null
+    const double* sgeo = nullptr;   // [ntasks][2][kSGeoFields][nc*nc] singular-pair point data (complex k), or null
+    const double* snode = nullptr;  // [ntasks][kSNodeStride] singular-pair node table (real k), or null
 };
 
 // k-independent data of one composite quadrature point of a singular pair:

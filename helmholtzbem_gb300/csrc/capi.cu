@@ -31,8 +31,14 @@ size_t singular_part_bytes(int ntasks, int njobs, int d, bool curved);
 cudaError_t launch_gather_T(int N, int d, const cplx* loc, const double* Mmass, int nk, int sp, cplx* T,
                             cudaStream_t st);
 cudaError_t launch_local_multi(const MultiMesh* meshes, const MultiJob* jobs, int njobs, const long long* gstart,
-                               long long gblocks, const long long* sstart, long long sblocks, int max_nc, int min_p,
-                               bool curved, int d, cplx* loc, cudaStream_t st);
+                               long long gblocks, const long long* sstart, long long sblocks,
+                               const long long* nstart, long long nblocks, int max_nc, int min_p, bool curved, int d,
+                               cplx* loc, cudaStream_t st);
+size_t snode_bytes(int ntasks);
+size_t snode_scratch_bytes(int ntasks);
+double snode_limit();
+cudaError_t launch_snode(const DevMesh& M, const SingularTask* tasks, int ntasks, double* nodes, double* scratch,
+                         cudaStream_t st);
 cudaError_t launch_gather_layers(int N, int d, int layers, const cplx* loc, int job, int sp, cplx* out,
                                  cudaStream_t st);
 cudaError_t launch_gather_layers_sub(int N, int d, int layers, const cplx* loc, int job, int row, int rows, int col,
@@ -150,6 +156,11 @@ int g_plain_spec_async = 2;   // ... speculating while at most this many candida
 int g_plain_spec_deep = 2;    // ... two bisection levels deep while at most this many are
 int g_singular_table = 1;     // singular pairs read their k-independent point data from a table
 const size_t kSingularTableMax = (size_t)256 << 20;
+// The node table of the singular pairs costs about 900 FP64 instructions per quadrature
+// point, made once per builder, where one job (a wavenumber and medium) costs 40 (T) to 75
+// (T, T', T'') without it: calls with at least this many wavenumbers make and use it (and
+// the searches, which evaluate hundreds); smaller calls take the points themselves.
+const int kSNodeMinK = 12;
 
 int fail(int code, const std::string& msg) {
     g_err = msg;
@@ -359,25 +370,30 @@ int tuned_layout(const DevMesh& M, const SingularTask* tasks, int ntasks, const 
 }
 
 // part: scratch of singular_part_bytes for the split singular launch of few jobs (or
-// null: one CTA per pair and job)
+// null: one CTA per pair and job); rows: some singular pair is beyond the node table
 cudaError_t local_assembly(const DevMesh& M, const SingularTask* tasks, int ntasks, int ncoinc, const Job* jobs,
-                           int njobs, bool real_k, int d, cplx* loc, cudaStream_t st, double* part = nullptr) {
+                           int njobs, bool real_k, bool rows, int d, cplx* loc, cudaStream_t st,
+                           double* part = nullptr) {
     const int layout = (g_autotune && M.n > 1) ? tuned_layout(M, tasks, ntasks, jobs, njobs, real_k, d, loc, st)
                                                : kLayoutAuto;
     cudaEvent_t e0 = nullptr;
     const bool timed = g_timing != 0;
     if (timed) timing_begin(&e0, st);
-    cudaError_t e = launch_local(M, tasks, ntasks, jobs, njobs, real_k, d, loc, st, layout, 3, part);
-    g_launches += (M.n > 1 ? 1 : 0) + (ntasks > 0 ? 1 : 0) + (part && singular_parts(ntasks, njobs) > 0 ? 1 : 0);
+    cudaError_t e = launch_local(M, tasks, ntasks, jobs, njobs, real_k, d, loc, st, layout, rows ? 7 : 3, part);
+    const bool nodes = real_k && M.snode && ntasks > 0, points = ntasks > 0 && (!nodes || rows);
+    g_launches += (M.ngen > 0 ? 1 : 0) + (nodes ? 1 : 0) + (points ? 1 : 0) +
+                  (points && part && singular_parts(ntasks, njobs) > 0 ? 1 : 0);
     if (timed) {
         timing_end(e0, st);
         g_asm_launches += 1;
         long long nc2 = (long long)M.nc * M.nc;
         long long nadj = ntasks - ncoinc;
         long long gen = (long long)M.n * (M.n + 1) / 2 - ntasks;
-        g_asm_points += (long long)njobs * (ncoinc * nc2 + nadj * 2 * nc2 + gen * (long long)M.p * M.p);
+        // a launch that the node table serves evaluates 16 nodes per singular pair
+        const long long sing = points ? ncoinc * nc2 + nadj * 2 * nc2 : 16LL * ntasks;
+        g_asm_points += (long long)njobs * (sing + gen * (long long)M.p * M.p);
         g_asm_split[d] += (long long)njobs * gen * M.p * M.p;
-        g_asm_split[(M.sgeo ? 3 : 6) + d] += (long long)njobs * (ncoinc * nc2 + nadj * 2 * nc2);
+        g_asm_split[(!points || (!real_k && M.sgeo) ? 3 : 6) + d] += (long long)njobs * sing;
     }
     return e;
 }
@@ -400,7 +416,10 @@ struct hbem_builder_s {
     cudaStream_t st = nullptr;
     DBuf d_kind, d_par, d_xg, d_wg, d_xc, d_wc, d_gpt, d_gtan, d_gtn, d_ends, d_flags, d_tasks;
     DBuf d_loc, d_jobs, d_layers;
-    DBuf d_sgeo;   // k-independent point data of the singular pairs (when within kSingularTableMax)
+    DBuf d_sgeo;   // k-independent point data of the singular pairs (complex k; when within kSingularTableMax)
+    DBuf d_snode;  // node table of the singular pairs (real k; made by the first call that uses it)
+    double snode_dmax = 0.;   // largest distance bound of its pairs
+    std::mutex table_mu;      // the two tables above are made on first use
     DBuf d_gpairs; // general pairs (i << 16 | j) sorted by panel-midpoint distance
     long long ngen = 0;
     const HkEntry* hk = nullptr;
@@ -410,7 +429,8 @@ struct hbem_builder_s {
     // the gather's space bits: 1 test space P0, 2 trial space P0
     int sp() const { return (qtest == HBEM_SPACE_P0 ? 1 : 0) | (qtrial == HBEM_SPACE_P0 ? 2 : 0); }
     bool p1p1() const { return qtest == HBEM_SPACE_P1 && qtrial == HBEM_SPACE_P1; }
-    DevMesh view() const {
+    // nodes: the launch reads the node table of the singular pairs
+    DevMesh view(bool nodes = false) const {
         DevMesh M;
         M.n = n; M.p = p; M.nc = nc; M.lines = lines;
         M.kind = d_kind.as<int>(); M.par = d_par.as<double>();
@@ -419,10 +439,60 @@ struct hbem_builder_s {
         M.gpt = d_gpt.as<cplx>(); M.gtan = d_gtan.as<cplx>(); M.gtn = d_gtn.as<double>();
         M.ends = d_ends.as<cplx>(); M.flags = d_flags.as<uint8_t>();
         M.sgeo = g_singular_table ? d_sgeo.as<double>() : nullptr;
+        M.snode = nodes ? d_snode.as<double>() : nullptr;
         M.gpairs = d_gpairs.as<unsigned>();
         M.ngen = ngen;
         M.hk = hk;
         return M;
+    }
+    // whether some singular pair of these jobs is beyond the node table
+    bool beyond_nodes(const std::vector<Job>& jobs) const {
+        for (const Job& J : jobs)
+            if (!(J.kre * std::sqrt(J.c) * snode_dmax <= snode_limit() * (1. - 1e-6))) return true;
+        return false;
+    }
+    // The node table of the singular pairs, made by the first call that uses it
+    cudaError_t ensure_snode() {
+        std::lock_guard<std::mutex> lk(table_mu);
+        if (d_snode.p) return cudaSuccess;
+        const int ntasks = (int)tasks.size();
+        auto len = [&](int i) {
+            const double* P = &par[5 * (size_t)i];
+            return kind[i] == HBEM_PANEL_LINE ? std::hypot(P[2] - P[0], P[3] - P[1]) : std::fabs(P[2] * (P[4] - P[3]));
+        };
+        double dmax = 0.;
+        for (const SingularTask& T : tasks)
+            dmax = std::max(dmax, (T.kind == PK_ADJ ? len(T.i) + len(T.j) : len(T.i)) * (1. + 2e-9));
+        DBuf scratch, nodes;
+        cudaError_t e = scratch.ensure(snode_scratch_bytes(ntasks));
+        if (e == cudaSuccess) e = nodes.ensure(snode_bytes(ntasks));
+        if (e == cudaSuccess)
+            e = launch_snode(view(), d_tasks.as<SingularTask>(), ntasks, nodes.as<double>(), scratch.as<double>(), st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);   // complete before another stream reads it
+        scratch.release();
+        if (e != cudaSuccess) {
+            nodes.release();
+            return e;
+        }
+        g_launches += 2;
+        snode_dmax = dmax;
+        d_snode = nodes;
+        return cudaSuccess;
+    }
+    // The point table that complex wavenumbers read, made before their first assembly.
+    cudaError_t ensure_sgeo() {
+        std::lock_guard<std::mutex> lk(table_mu);
+        const size_t bytes = singular_geo_bytes(nc, (int)tasks.size());
+        if (!g_singular_table || d_sgeo.p || bytes == 0 || bytes > kSingularTableMax) return cudaSuccess;
+        cudaError_t e = d_sgeo.ensure(bytes);
+        if (e == cudaSuccess) {
+            DevMesh M = view();
+            M.sgeo = nullptr;
+            e = launch_singular_geo(M, d_tasks.as<SingularTask>(), (int)tasks.size(), d_sgeo.as<double>(), st);
+        }
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);   // complete before another stream reads it
+        if (e != cudaSuccess) d_sgeo.release();
+        return e;
     }
     // BuilderData::is_adjacent (galerkin_builder.cpp:189-201)
     bool adjacent(int i, int j, bool& swap) const {
@@ -433,7 +503,7 @@ struct hbem_builder_s {
     }
     ~hbem_builder_s() {
         for (DBuf* b : {&d_kind, &d_par, &d_xg, &d_wg, &d_xc, &d_wc, &d_gpt, &d_gtan, &d_gtn, &d_ends, &d_flags,
-                        &d_tasks, &d_loc, &d_jobs, &d_layers, &d_sgeo, &d_gpairs})
+                        &d_tasks, &d_loc, &d_jobs, &d_layers, &d_sgeo, &d_snode, &d_gpairs})
             b->release();
         if (st) cudaStreamDestroy(st);
     }
@@ -738,36 +808,42 @@ int hbem_builder_create(int npanels, const int* kinds, const double* params, int
     if (e == cudaSuccess) e = upload(b->d_tasks, b->tasks, b->st);
     if (e == cudaSuccess) e = launch_flags(b->view(), b->d_tasks.as<SingularTask>(), (int)b->tasks.size(),
                                            b->d_flags.as<uint8_t>(), b->st);
-    // general pairs in order of the distance between their panels' middle Gauss points
-    // (ties by index): a warp's points then lie in neighbouring intervals of the Hankel table
+    // general pairs in order of the distance between their panels' middle Gauss points (to
+    // a part in 2000; ties by index): a warp's points then lie in neighbouring intervals of the Hankel table
     if (e == cudaSuccess && n <= 65536) {
-        std::vector<std::pair<float, unsigned>> ord;
-        ord.reserve((size_t)b->npair());
-        for (int i = 1; i < n; ++i)
+        // counting sort by the leading bits of the squared distance (11 bits of mantissa)
+        std::vector<unsigned> key, raw;
+        key.reserve((size_t)b->npair());
+        raw.reserve((size_t)b->npair());
+        unsigned lo = ~0u, hi = 0;
+        for (int i = 1; i < n; ++i) {
+            const cplx a = gpt[(size_t)i * p + p / 2];
             for (int j = 0; j < i; ++j) {
                 if (flags[tri_index(i, j)]) continue;
-                const cplx a = gpt[(size_t)i * p + p / 2], c = gpt[(size_t)j * p + p / 2];
+                const cplx c = gpt[(size_t)j * p + p / 2];
                 const double dx = a.re - c.re, dy = a.im - c.im;
-                ord.emplace_back((float)(dx * dx + dy * dy), (unsigned)i << 16 | (unsigned)j);
+                const float d2 = (float)(dx * dx + dy * dy);
+                unsigned k;
+                std::memcpy(&k, &d2, sizeof k);
+                k >>= 12;
+                lo = std::min(lo, k);
+                hi = std::max(hi, k);
+                key.push_back(k);
+                raw.push_back((unsigned)i << 16 | (unsigned)j);
             }
-        std::sort(ord.begin(), ord.end());
-        std::vector<unsigned> pairs(ord.size());
-        for (size_t q = 0; q < ord.size(); ++q) pairs[q] = ord[q].second;
+        }
+        std::vector<unsigned> pairs(raw.size());
+        if (!raw.empty()) {
+            std::vector<size_t> at((size_t)(hi - lo) + 2, 0);
+            for (unsigned k : key) ++at[k - lo + 1];
+            for (size_t q = 1; q < at.size(); ++q) at[q] += at[q - 1];
+            for (size_t q = 0; q < raw.size(); ++q) pairs[at[key[q] - lo]++] = raw[q];
+        }
         b->ngen = (long long)pairs.size();
         e = upload(b->d_gpairs, pairs, b->st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(b->st);   // the host copy ends here
     }
     if (e == cudaSuccess) b->hk = hankel_table(&e);
-    const size_t geo_bytes = singular_geo_bytes(b->nc, (int)b->tasks.size());
-    if (e == cudaSuccess && geo_bytes > 0 && geo_bytes <= kSingularTableMax) {
-        e = b->d_sgeo.ensure(geo_bytes);
-        if (e == cudaSuccess) {
-            DevMesh M = b->view();
-            M.sgeo = nullptr;
-            e = launch_singular_geo(M, b->d_tasks.as<SingularTask>(), (int)b->tasks.size(), b->d_sgeo.as<double>(),
-                                    b->st);
-        }
-    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->st);
     if (e != cudaSuccess) {
         std::string msg = cudaGetErrorString(e);
@@ -831,8 +907,9 @@ int hbem_assemble_dense_sub(hbem_builder b, double k_re, double k_im, double c, 
     int nl = ((layers & 1) != 0) + ((layers & 2) != 0) + ((layers & 4) != 0);
     HB_CK(b->d_layers.ensure((size_t)nl * (d + 1) * rows * cols * sizeof(cplx)));
     bool real_k = (k_im == 0. && k_re > 0.);
+    if (!real_k) HB_CK(b->ensure_sgeo());
     HB_CK(local_assembly(b->view(), b->d_tasks.as<SingularTask>(), (int)b->tasks.size(), b->n, b->d_jobs.as<Job>(), 1,
-                         real_k, (int)d, b->d_loc.as<cplx>(), b->st));
+                         real_k, false, (int)d, b->d_loc.as<cplx>(), b->st));
     if (rows == (unsigned)b->n && cols == (unsigned)b->n)
         HB_CK(launch_gather_layers(b->n, (int)d, (int)layers, b->d_loc.as<cplx>(), 0, b->sp(), b->d_layers.as<cplx>(),
                                    b->st));
@@ -978,16 +1055,17 @@ int hbem_mass_matrix(hbem_solop s, double* host_out) {
 // T(k) (+ derivatives) for nk wavenumbers into T_dev [nk][d+1][2N][2N]; k_host may be complex
 // (interleaved) when kim_host != NULL.
 static int gen_T_batch_ws(hbem_solop s, const double* k_host, const double* kim_host, int nk, double c_o, double c_i,
-                          unsigned d, cplx* T_dev, DBuf& d_jobs, DBuf& d_loc, cudaStream_t st);
+                          unsigned d, cplx* T_dev, DBuf& d_jobs, DBuf& d_loc, cudaStream_t st, bool many);
 
+// many: the call is one of at least kSNodeMinK evaluations (node table of the singular pairs)
 static int gen_T_batch(hbem_solop s, const double* k_host, const double* kim_host, int nk, double c_o, double c_i,
-                       unsigned d, cplx* T_dev) {
-    return gen_T_batch_ws(s, k_host, kim_host, nk, c_o, c_i, d, T_dev, s->b->d_jobs, s->b->d_loc, s->b->st);
+                       unsigned d, cplx* T_dev, bool many) {
+    return gen_T_batch_ws(s, k_host, kim_host, nk, c_o, c_i, d, T_dev, s->b->d_jobs, s->b->d_loc, s->b->st, many);
 }
 
 // T(k) batch with the job table and pair-block scratch given, on stream st
 static int gen_T_batch_ws(hbem_solop s, const double* k_host, const double* kim_host, int nk, double c_o, double c_i,
-                          unsigned d, cplx* T_dev, DBuf& d_jobs, DBuf& d_loc, cudaStream_t st) {
+                          unsigned d, cplx* T_dev, DBuf& d_jobs, DBuf& d_loc, cudaStream_t st, bool many) {
     hbem_builder b = s->b;
     const int N = b->n;
     const long long np = b->npair();
@@ -1014,8 +1092,11 @@ static int gen_T_batch_ws(hbem_solop s, const double* k_host, const double* kim_
                                                 : 0;
         HB_CK(d_loc.ensure(per_job * 2 * kn + part_bytes));
         double* part = part_bytes ? reinterpret_cast<double*>(d_loc.as<char>() + per_job * 2 * kn) : nullptr;
-        HB_CK(local_assembly(b->view(), b->d_tasks.as<SingularTask>(), (int)b->tasks.size(), b->n, d_jobs.as<Job>(),
-                             2 * kn, real_k, (int)d, d_loc.as<cplx>(), st, part));
+        const bool nodes = many && real_k && g_singular_table;
+        if (!real_k) HB_CK(b->ensure_sgeo());
+        if (nodes) HB_CK(b->ensure_snode());
+        HB_CK(local_assembly(b->view(nodes), b->d_tasks.as<SingularTask>(), (int)b->tasks.size(), b->n,
+                             d_jobs.as<Job>(), 2 * kn, real_k, nodes && b->beyond_nodes(jobs), (int)d, d_loc.as<cplx>(), st, part));
         cplx* Tk = T_dev + (size_t)k0 * (d + 1) * mat;
         HB_CK(launch_gather_T(N, (int)d, d_loc.as<cplx>(), s->d_M.as<double>(), kn, b->sp(), Tk, st));
         g_launches += 1;
@@ -1035,7 +1116,7 @@ int hbem_gen_sol_op(hbem_solop s, double k_re, double k_im, double c_o, double c
     HB_CK(cudaSetDevice(b->device));
     const size_t mat = 4ULL * b->n * b->n;
     HB_CK(s->d_T.ensure((d + 1) * mat * sizeof(cplx)));
-    if (int r = gen_T_batch(s, &k_re, &k_im, 1, c_o, c_i, d, s->d_T.as<cplx>())) return r;
+    if (int r = gen_T_batch(s, &k_re, &k_im, 1, c_o, c_i, d, s->d_T.as<cplx>(), false)) return r;
     HB_CK(cudaMemcpyAsync(T_host, s->d_T.p, (d + 1) * mat * sizeof(cplx), cudaMemcpyDeviceToHost, b->st));
     HB_CK(cudaStreamSynchronize(b->st));
     return HBEM_OK;
@@ -1046,7 +1127,7 @@ int hbem_gen_sol_op_batch_device(hbem_solop s, const double* k_host, int nk, dou
     if (!s || !k_host || !T_dev || nk < 1) return fail(HBEM_ERR_INVALID, "bad argument");
     if (d > 2) return fail(HBEM_ERR_INVALID, "Invalid order of derivative");
     HB_CK(cudaSetDevice(s->b->device));
-    if (int r = gen_T_batch(s, k_host, nullptr, nk, c_o, c_i, d, static_cast<cplx*>(T_dev))) return r;
+    if (int r = gen_T_batch(s, k_host, nullptr, nk, c_o, c_i, d, static_cast<cplx*>(T_dev), nk >= kSNodeMinK)) return r;
     HB_CK(cudaStreamSynchronize(s->b->st));
     return HBEM_OK;
 }
@@ -1086,7 +1167,9 @@ int hbem_gen_sol_op_multi_device(const hbem_solop* ops, int nops, const int* cou
     std::vector<MultiMesh> meshes(nops);
     int max_nc = 0, min_p = 32;
     for (int i = 0; i < nops; ++i) {
-        meshes[i] = MultiMesh{ops[i]->b->view(), ops[i]->b->d_tasks.as<SingularTask>(), (int)ops[i]->b->tasks.size()};
+        const bool nodes = counts[i] >= kSNodeMinK && g_singular_table;
+        if (nodes) HB_CK(ops[i]->b->ensure_snode());
+        meshes[i] = MultiMesh{ops[i]->b->view(nodes), ops[i]->b->d_tasks.as<SingularTask>(), (int)ops[i]->b->tasks.size()};
         max_nc = std::max(max_nc, ops[i]->b->nc);
         min_p = std::min(min_p, ops[i]->b->p);
     }
@@ -1104,8 +1187,9 @@ int hbem_gen_sol_op_multi_device(const hbem_solop* ops, int nops, const int* cou
         if (per_k == 0) continue;
         const size_t chunk = std::max<size_t>(1, budget / per_k);
         for (size_t q0 = 0; q0 < kmax; q0 += chunk) {
+            const bool timed_points = g_timing != 0;
             std::vector<MultiJob> jobs;
-            std::vector<long long> gstart{0}, sstart{0};
+            std::vector<long long> gstart{0}, sstart{0}, nstart{0};
             std::vector<size_t> first(nops, 0), nk(nops, 0);
             long long off = 0;
             for (int i = 0; i < nops; ++i) {
@@ -1119,7 +1203,19 @@ int hbem_gen_sol_op_multi_device(const hbem_solop* ops, int nops, const int* cou
                         jobs.push_back(MultiJob{Job{k, 0., c}, i, off});
                         off += (long long)(b->npair() * per_pair);
                         gstart.push_back(gstart.back() + (b->ngen + 128 / b->p - 1) / (128 / b->p));
-                        sstart.push_back(sstart.back() + (long long)b->tasks.size());
+                        const bool nodes = meshes[i].M.snode != nullptr;
+                        const bool rows = !nodes || b->beyond_nodes({jobs.back().job});
+                        const long long nt = (long long)b->tasks.size();
+                        sstart.push_back(sstart.back() + (rows ? nt : 0));
+                        nstart.push_back(nstart.back() + (nodes ? (nt + 3) / 4 : 0));
+                        if (timed_points) {
+                            const long long nc2 = (long long)b->nc * b->nc;
+                            const long long sing = rows ? (2 * nt - b->n) * nc2 : 16 * nt;
+                            const long long gen = (b->npair() - nt) * b->p * b->p;
+                            g_asm_points += sing + gen;
+                            g_asm_split[d] += gen;
+                            g_asm_split[(rows ? 6 : 3) + d] += sing;
+                        }
                     }
                 }
             }
@@ -1127,6 +1223,7 @@ int hbem_gen_sol_op_multi_device(const hbem_solop* ops, int nops, const int* cou
             const int njobs = (int)jobs.size();
             std::vector<long long> starts(gstart);
             starts.insert(starts.end(), sstart.begin(), sstart.end());
+            starts.insert(starts.end(), nstart.begin(), nstart.end());
             HB_CK(upload(d_jobs, jobs, st));
             HB_CK(upload(d_start, starts, st));
             HB_CK(d_loc.ensure((size_t)off * sizeof(cplx)));
@@ -1134,23 +1231,13 @@ int hbem_gen_sol_op_multi_device(const hbem_solop* ops, int nops, const int* cou
             const bool timed = g_timing != 0;
             if (timed) timing_begin(&e0, st);
             HB_CK(launch_local_multi(d_meshes.as<MultiMesh>(), d_jobs.as<MultiJob>(), njobs, d_start.as<long long>(),
-                                     gstart.back(), d_start.as<long long>() + gstart.size(), sstart.back(), max_nc,
+                                     gstart.back(), d_start.as<long long>() + gstart.size(), sstart.back(),
+                                     d_start.as<long long>() + gstart.size() + sstart.size(), nstart.back(), max_nc,
                                      min_p, curved == 1, (int)d, d_loc.as<cplx>(), st));
-            g_launches += (gstart.back() > 0 ? 1 : 0) + (sstart.back() > 0 ? 1 : 0);
+            g_launches += (gstart.back() > 0 ? 1 : 0) + (sstart.back() > 0 ? 1 : 0) + (nstart.back() > 0 ? 1 : 0);
             if (timed) {
                 timing_end(e0, st);
                 g_asm_launches += 1;
-                for (int i = 0; i < nops; ++i) {
-                    if (!nk[i]) continue;
-                    const hbem_builder b = ops[i]->b;
-                    const long long nc2 = (long long)b->nc * b->nc, ntasks = (long long)b->tasks.size();
-                    const long long ncoinc = b->n, nadj = ntasks - ncoinc;
-                    const long long gen = b->npair() - ntasks;
-                    const long long nj = 2LL * (long long)nk[i];
-                    g_asm_points += nj * (ncoinc * nc2 + nadj * 2 * nc2 + gen * (long long)b->p * b->p);
-                    g_asm_split[d] += nj * gen * b->p * b->p;
-                    g_asm_split[(b->d_sgeo.p && g_singular_table ? 3 : 6) + d] += nj * (ncoinc * nc2 + nadj * 2 * nc2);
-                }
             }
             for (int i = 0; i < nops; ++i) {
                 if (!nk[i]) continue;
@@ -1477,7 +1564,7 @@ int hbem_sigma_rsvd_sweep(hbem_solop s, const double* k_host, int nk, double c_o
     HB_CK(s->d_T.ensure((size_t)chunk * mat * sizeof(cplx)));
     for (int k0 = 0; k0 < nk; k0 += chunk) {
         const int kn = std::min(chunk, nk - k0);
-        if (int r = gen_T_batch(s, k_host + k0, nullptr, kn, c_o, c_i, 0, s->d_T.as<cplx>())) return r;
+        if (int r = gen_T_batch(s, k_host + k0, nullptr, kn, c_o, c_i, 0, s->d_T.as<cplx>(), nk >= kSNodeMinK)) return r;
         HB_CK(cudaStreamSynchronize(b->st));
         if (int r = hbem_rsvd_sv_batch_device_ex(n, kn, 0, s->d_T.p, (long long)mat, (long long)mat, R.p, sketch, q,
                                                  precision, 3, sigma_out + k0))
@@ -1497,7 +1584,7 @@ int hbem_sweep_sigma(hbem_solop s, const double* k_host, int nk, double c_o, dou
     HB_CK(s->d_T.ensure((size_t)chunk * (d + 1) * mat * sizeof(cplx)));
     for (int k0 = 0; k0 < nk; k0 += chunk) {
         int kn = std::min(chunk, nk - k0);
-        if (int r = gen_T_batch(s, k_host + k0, nullptr, kn, c_o, c_i, d, s->d_T.as<cplx>())) return r;
+        if (int r = gen_T_batch(s, k_host + k0, nullptr, kn, c_o, c_i, d, s->d_T.as<cplx>(), nk >= kSNodeMinK)) return r;
         if (int r = sv_batch(b->st, n, kn, d, s->d_T.as<cplx>(), (long long)(d + 1) * mat, (long long)mat, s->d_svdA,
                              s->d_svdV, s->d_out, s->d_status, nullptr, out_host + 3LL * k0, nullptr))
             return r;
@@ -1552,7 +1639,8 @@ int hbem_sweep_sigma_multi(const hbem_solop* ops, int nops, const int* counts, c
             HB_CK(s->d_T.ensure((size_t)kn * (d + 1) * mat * sizeof(cplx)));
             HB_CK(s->d_out.ensure((size_t)kn * 3 * sizeof(double)));
             HB_CK(s->d_status.ensure((size_t)kn * sizeof(int)));
-            if (int r = gen_T_batch(s, k_host + off, nullptr, kn, c_o, c_i_host[i], d, s->d_T.as<cplx>())) return r;
+            if (int r = gen_T_batch(s, k_host + off, nullptr, kn, c_o, c_i_host[i], d, s->d_T.as<cplx>(),
+                                    kn >= kSNodeMinK)) return r;
             HB_CK(launch_svd_fast(n, kn, (int)d, s->d_T.as<cplx>(), (long long)(d + 1) * mat, (long long)mat,
                                   s->d_out.as<double>(), s->d_status.as<int>(), b->st));
             g_launches += 1;
@@ -1603,7 +1691,7 @@ int solop_mesh(hbem_solop s, int* n, const int** kinds, const double** par, int*
 
 // T(k) of the operator (projected or not, as created) into T_dev (2N x 2N), synchronised
 int solop_gen_T(hbem_solop s, double k_re, double k_im, double c_o, double c_i, void* T_dev) {
-    if (int r = gen_T_batch(s, &k_re, &k_im, 1, c_o, c_i, 0, static_cast<cplx*>(T_dev))) return r;
+    if (int r = gen_T_batch(s, &k_re, &k_im, 1, c_o, c_i, 0, static_cast<cplx*>(T_dev), false)) return r;
     HB_CK(cudaStreamSynchronize(s->b->st));
     return HBEM_OK;
 }
@@ -1711,7 +1799,7 @@ int lane_launch(hbem_solop s, int lane, const double* k_host, int npts, double c
     HB_CK(L.T.ensure((size_t)npts * (d + 1) * mat * sizeof(cplx)));
     HB_CK(L.out.ensure(3 * kLaneMaxPts * sizeof(double)));
     HB_CK(L.status.ensure(kLaneMaxPts * sizeof(int)));
-    if (int r = gen_T_batch_ws(s, k_host, nullptr, npts, c_o, c_i, d, L.T.as<cplx>(), L.jobs, L.loc, L.st)) return r;
+    if (int r = gen_T_batch_ws(s, k_host, nullptr, npts, c_o, c_i, d, L.T.as<cplx>(), L.jobs, L.loc, L.st, true)) return r;
     HB_CK(launch_svd_fast(n, npts, (int)d, L.T.as<cplx>(), (long long)(d + 1) * (long long)mat, (long long)mat, L.out.as<double>(),
                           L.status.as<int>(), L.st, s->d_vpool.as<cplxf>(), L.slots.as<int>(), L.slots.as<int>() + npts,
                           nullptr));
@@ -1838,7 +1926,7 @@ int lane_launch_grid(hbem_solop s, int lane, const double* k_host, int npts, int
     HB_CK(L.out.ensure(3 * kLaneMaxPts * sizeof(double)));
     HB_CK(L.status.ensure(kLaneMaxPts * sizeof(int)));
     if (after >= 0) HB_CK(cudaStreamWaitEvent(L.st, lanes[after]->asm_done, 0));
-    if (int r = gen_T_batch_ws(s, k_host, nullptr, npts, c_o, c_i, 0, L.T.as<cplx>(), L.jobs, L.loc, L.st)) return r;
+    if (int r = gen_T_batch_ws(s, k_host, nullptr, npts, c_o, c_i, 0, L.T.as<cplx>(), L.jobs, L.loc, L.st, true)) return r;
     HB_CK(cudaEventRecord(L.asm_done, L.st));
     HB_CK(launch_svd_fast(n, npts, 0, L.T.as<cplx>(), (long long)mat, (long long)mat, L.out.as<double>(),
                           L.status.as<int>(), L.st, s->d_vpool.as<cplxf>(), L.slots.as<int>(), L.slots.as<int>() + npts,
@@ -1870,7 +1958,7 @@ int lane_launch_ends(hbem_solop s, int lane, const double* k_host, const int* gi
     HB_CK(upload(L.slots, id, L.st));
     HB_CK(L.T.ensure(2 * 2 * mat * sizeof(cplx)));
     HB_CK(L.out.ensure(3 * kLaneMaxPts * sizeof(double)));
-    if (int r = gen_T_batch_ws(s, k_host, nullptr, 2, c_o, c_i, 1, L.T.as<cplx>(), L.jobs, L.loc, L.st)) return r;
+    if (int r = gen_T_batch_ws(s, k_host, nullptr, 2, c_o, c_i, 1, L.T.as<cplx>(), L.jobs, L.loc, L.st, true)) return r;
     HB_CK(launch_sigma1_uv(n, 2, L.T.as<cplx>() + mat, (long long)(2 * mat), s->d_uv.as<cplx>(), L.slots.as<int>(),
                            L.out.as<double>(), L.st));
     g_launches += 1;
@@ -1946,7 +2034,7 @@ int sweep_sigma_warm(hbem_solop s, const double* k_host, int nk, double c_o, dou
     std::copy(out_slot, out_slot + nk, slots.begin() + nk);
     HB_CK(upload(s->d_slots, slots, b->st));
     HB_CK(s->d_T.ensure((size_t)nk * (d + 1) * mat * sizeof(cplx)));
-    if (int r = gen_T_batch(s, k_host, nullptr, nk, c_o, c_i, d, s->d_T.as<cplx>())) return r;
+    if (int r = gen_T_batch(s, k_host, nullptr, nk, c_o, c_i, d, s->d_T.as<cplx>(), true)) return r;
     if (keep_uv) {
         s->uv_count = 0;
         HB_CK(s->d_uv.ensure((size_t)nk * 2 * n * sizeof(cplx)));
@@ -1976,7 +2064,7 @@ int sigma1_from_kept(hbem_solop s, const double* k_host, const int* idx, int ne,
     const int n = 2 * b->n;
     const size_t mat = (size_t)n * n;
     HB_CK(s->d_T.ensure((size_t)ne * 2 * mat * sizeof(cplx)));
-    if (int r = gen_T_batch(s, k_host, nullptr, ne, c_o, c_i, 1, s->d_T.as<cplx>())) return r;
+    if (int r = gen_T_batch(s, k_host, nullptr, ne, c_o, c_i, 1, s->d_T.as<cplx>(), true)) return r;
     std::vector<int> id(idx, idx + ne);
     HB_CK(upload(s->d_slots, id, b->st));
     HB_CK(s->d_d1.ensure((size_t)ne * sizeof(double)));

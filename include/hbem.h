@@ -69,20 +69,23 @@ int hbem_set_device(int device);
  *   bit-identical to the one-CTA form; 0 never pairs.
  *   "arnoldi_maxit" (default 1000, >= 1): iteration cap of hbem_arnoldi_sv_batch*.
  *   "mlp_tensor_cores" (default 1): the MLP's BF16 products on tcgen05; 0 uses FP32 FMA.
- *   "singular_table" (default 1): coincident / adjacent panel pairs read the
- *   k-independent data of their composite quadrature points (distance, tangent and
- *   normal products, weights) from a table the builder makes once (up to 256 MB);
- *   0 computes it in the kernel for every wavenumber and medium.
+ *   "singular_table" (default 1): real wavenumbers: calls of at least 12 wavenumbers, and
+ *   the searches, sum each coincident / adjacent pair over 16 interpolation nodes whose
+ *   k-independent weights a table holds (made once per builder, by the first such call;
+ *   pairs with ks x panel lengths above 8 take the quadrature points).  Complex
+ *   wavenumbers read the k-independent data of the points (distance, tangent and normal
+ *   products, weights) from a table the builder makes once (up to 256 MB).  0: the
+ *   quadrature points, computed in the kernel for every wavenumber and medium.
  *   "singular_split" (default 1): assembly launches of few wavenumbers (coincident /
- *   adjacent pairs x media below four CTAs per SM) split every such pair over several
- *   CTAs of equal work and add the parts in a second launch: lower latency for one
- *   T(k); sums in another order (results agree to ~1e-15).  The pipelined plain search
- *   does not split (its launches share the GPU).
+ *   adjacent pairs x media below four CTAs per SM) that sum the points split every such
+ *   pair over several CTAs of equal work and add the parts in a second launch: lower
+ *   latency for one T(k); sums in another order (results agree to ~1e-15).  The
+ *   pipelined plain search does not split (its launches share the GPU).
  *   "plain_speculate" (default 1): speculative bisection points in the plain
  *   search's small Newton rounds (hbem_find_resonances_plain).
  *   "autotune" (default 0): the panel-pair assembly times each layout of its general
- *   pairs (a thread per pair, or a warp per pair with 1-16 pairs per warp) on the
- *   first launch of every (panels, order, jobs rounded up to a power of two,
+ *   pairs (complex wavenumbers: a thread per pair, or a warp per pair with 1-16 pairs per
+ *   warp; real ones have a single layout, number 0) on the first launch of every (panels, order, jobs rounded up to a power of two,
  *   derivative order, real k, panel kind) and uses the fastest from then on; the
  *   choices persist in the file the environment variable HBEM_TUNE_CACHE names, if
  *   any.  Results of different layouts agree to rounding (~1e-15).
