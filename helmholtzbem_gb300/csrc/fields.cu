@@ -11,7 +11,8 @@
 //   u(x) = s sum_{panels, Gauss nodes} w |gamma'| [H0(kappa r) t_N - kappa H1(kappa r) t_D (x - y).n / r],
 // s = i/4 inside and -i/4 outside, kappa = k sqrt(c_i) or k sqrt(c_o), with the
 // outside traces minus the incoming wave, is summed on the GPU (one thread per grid
-// point, boundary nodes staged through shared memory).  Grid points on the boundary
+// point, boundary nodes staged through shared memory; H0 and H1 as functions of r^2 from
+// the table of hankel_u.cuh at real k).  Grid points on the boundary
 // take the Dirichlet trace; for panels within 1e-2 / |kappa| of the point the
 // panel's Gauss sum is replaced by a geometrically graded composite Gauss rule
 // around the nearest point (one warp per such pair).
@@ -28,7 +29,7 @@
 #include <vector>
 
 #include "../../include/hbem.h"
-#include "hbem_device.cuh"
+#include "hankel_u.cuh"
 #include "waves.cuh"
 
 namespace hbem {
@@ -56,6 +57,21 @@ constexpr double kMachEpsF = 2.220446049250313e-16;
 struct FNode {
     double yx, yy, nx, ny, D, pad;
     cplx tdi, tni, tdo, tno;          // Dirichlet / Neumann traces, inside and outside
+};
+
+// a node as the grid kernel reads it at real k: the weight and the factors of the kernel
+// are in the traces, [0] outside, [1] inside
+struct GNode {
+    double yx, yy, nx, ny;
+    cplx tD[2], tN[2];                // D tN, -kappa^2 D tD
+};
+
+// A panel as the grid kernel's FP32 look at it: centre of its chord, squared radii around
+// it outside of which a point is certainly neither near the panel (rin2, rout2: inside /
+// outside wavenumber) nor in an arc's segment (rseg2), and the y range of its chord with a
+// margin.  An FP64 comparison costs 76 cycles a warp, an FP32 one 1.
+struct PanelPre {
+    float cx, cy, rin2, rout2, ylo, yhi, rseg2, pad;
 };
 
 struct NearEntry {
@@ -214,6 +230,9 @@ struct FieldJob {
     const double* waves;
     const double* g21;
     const FNode* nodes;                    // npan x nq
+    const GNode* gnodes;                   // the same for the grid kernel at real k
+    const PanelPre* pre;                   // npan
+    const HkEntry* hk;
     cplx* acc;                             // per grid point: the Green sum (unscaled)
     int* flag;                             // 0 outside, 1 inside, 2 | 4 x panel on the boundary
     double* bnd_t;
@@ -239,7 +258,7 @@ __device__ __forceinline__ void hankel_pair(bool real_k, double kre, double kim,
 
 // Green quadrature nodes: points, normals, weights x |gamma'|, splined traces and the
 // outside traces (minus the incoming wave) -- in_solve, solvers.cpp:198-223
-__global__ void k_field_nodes(FieldJob J, const double* xg, const double* wg, FNode* out) {
+__global__ void k_field_nodes(FieldJob J, const double* xg, const double* wg, FNode* out, GNode* gout) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= J.npan * J.nq) return;
     const int i = q / J.nq, j = q % J.nq;
@@ -259,13 +278,30 @@ __global__ void k_field_nodes(FieldJob J, const double* xg, const double* wg, FN
     n.tdo = n.tdi - u;
     n.tno = n.tni - (n.nx * ux + n.ny * uy);
     out[q] = n;
+    if (!J.real_k) return;
+    GNode g;
+    g.yx = n.yx;
+    g.yy = n.yy;
+    g.nx = n.nx;
+    g.ny = n.ny;
+    g.tN[0] = n.D * n.tno;
+    g.tN[1] = n.D * n.tni;
+    g.tD[0] = (-J.kore * J.kore * n.D) * n.tdo;
+    g.tD[1] = (-J.kire * J.kire * n.D) * n.tdi;
+    gout[q] = g;
 }
 
 // 32 grid points per CTA, one per lane; the CTA's four warps split the panels for the
 // inside / boundary / near tests and the boundary nodes of every shared-memory tile
 // for the Green sum, then combine through shared memory.
+//
+// Bound by the FP64 pipe: at real k 34 instructions per (point, node) -- |x - y|^2, u, the
+// Hankel table (hankel_u.cuh), the normal projection and two complex multiply-adds -- and
+// the tests of a panel, ten times that in FP64, only where an FP32 look says that they
+// can matter.
+template <bool RK>
 __global__ void __launch_bounds__(kFieldThreads) k_field_grid(FieldJob J) {
-    __shared__ FNode tile[kNodeTile];
+    __shared__ __align__(16) unsigned char tile_raw[kNodeTile * (RK ? sizeof(GNode) : sizeof(FNode))];
     __shared__ int s_cross[kFieldSlices][32], s_seg[kFieldSlices][32], s_onb[kFieldSlices][32];
     __shared__ double s_bt[kFieldSlices][32];
     __shared__ cplx s_part[kFieldSlices][32];
@@ -274,9 +310,15 @@ __global__ void __launch_bounds__(kFieldThreads) k_field_grid(FieldJob J) {
     double x = 0., y = 0.;
     int cross = 0, seg = 0, onb = 0x7fffffff;
     double bt = 0.;
+    float xf = 0.f, yf = 0.f;
     if (g < G) {
         grid_xy(J, g, x, y);
+        xf = (float)x;
+        yf = (float)y;
         for (int i = w; i < J.npan; i += kFieldSlices) {
+            const PanelPre q = J.pre[i];
+            const float dx = xf - q.cx, dy = yf - q.cy;
+            if (!(yf >= q.ylo && yf <= q.yhi) && !(dx * dx + dy * dy <= q.rseg2)) continue;
             int c, sg;
             inside_share(J.par + 5 * i, J.kind[i], x, y, c, sg);
             cross ^= c;
@@ -295,6 +337,9 @@ __global__ void __launch_bounds__(kFieldThreads) k_field_grid(FieldJob J) {
     if (g < G) {
         const double akap = inside ? J.abs_ki : J.abs_ko;
         for (int i = w; i < J.npan; i += kFieldSlices) {
+            const PanelPre q = J.pre[i];
+            const float dx = xf - q.cx, dy = yf - q.cy;
+            if (!(dx * dx + dy * dy <= (inside ? q.rin2 : q.rout2))) continue;
             double t;
             const double d = fpan_dist(J.par + 5 * i, J.kind[i], x, y, t);
             if (d < 1e2 * kMachEpsF) {            // on the boundary: the Dirichlet trace
@@ -321,31 +366,52 @@ __global__ void __launch_bounds__(kFieldThreads) k_field_grid(FieldJob J) {
         J.flag[g] = onb != 0x7fffffff ? (2 | (onb << 2)) : (inside ? 1 : 0);
         if (onb != 0x7fffffff) J.bnd_t[g] = bt;
     }
-    const double kr = inside ? J.kire : J.kore, ki = inside ? J.kiim : J.koim;
-    const double ikr = kr > 0. ? 1.0 / kr : 0.;
+    const double kr = inside ? J.kire : J.kore, ki = inside ? J.kiim : J.koim, k2 = kr * kr;
     cplx sum = mk(0.);
-    const int M = J.npan * J.nq;
+    const int M = J.npan * J.nq, in = inside ? 1 : 0;
     constexpr int kPerWarp = kNodeTile / kFieldSlices;
     for (int base = 0; base < M; base += kNodeTile) {
         const int cnt = min(kNodeTile, M - base);
         __syncthreads();
-        for (int e = threadIdx.x; e < cnt; e += kFieldThreads) tile[e] = J.nodes[base + e];
+        {   // 16-byte copies
+            const size_t bytes = (RK ? sizeof(GNode) : sizeof(FNode));
+            const float4* src = reinterpret_cast<const float4*>(
+                RK ? reinterpret_cast<const unsigned char*>(J.gnodes + base)
+                   : reinterpret_cast<const unsigned char*>(J.nodes + base));
+            float4* dst = reinterpret_cast<float4*>(tile_raw);
+            for (int e = threadIdx.x; e < (int)(cnt * bytes / 16); e += kFieldThreads) dst[e] = src[e];
+        }
         __syncthreads();
         if (!active) continue;
         const int e1 = min(cnt, (w + 1) * kPerWarp);
         for (int e = w * kPerWarp; e < e1; ++e) {
-            const FNode& nd = tile[e];
-            const double zx = x - nd.yx, zy = y - nd.yy, r2 = zx * zx + zy * zy;
-            if (!(r2 > 0.)) continue;
-            // 1/r once: the normal projection and (real k) the Hankel pair's 1/x use it
-            const double ir = rsqrt(r2), r = r2 * ir;
-            cplx h0, h1;
-            if (J.real_k) hankel01_real_ix(kr * r, ikr * ir, h0, h1);
-            else hankel01_cplx(kr * r, ki * r, h0, h1);
-            const double zn = (zx * nd.nx + zy * nd.ny) * ir;
-            const cplx tD = inside ? nd.tdi : nd.tdo, tN = inside ? nd.tni : nd.tno;
-            cplx term = h0 * tN - (mk(kr, ki) * zn) * (h1 * tD);
-            sum += nd.D * term;
+            if (RK) {
+                const GNode& nd = reinterpret_cast<const GNode*>(tile_raw)[e];
+                const double zx = x - nd.yx, zy = y - nd.yy, r2 = fma(zx, zx, zy * zy), u = k2 * r2;
+                cplx f, gg;
+                if (hk_inside(u)) {
+                    hk_eval(J.hk, u, f, gg);
+                } else {
+                    if (!(r2 > 0.)) continue;
+                    hk_slow(u, f, gg);
+                }
+                // h0 tN - kappa h1 (n . z / r) tD = f tN - kappa^2 (n . z) g tD
+                const double zn = fma(zx, nd.nx, zy * nd.ny);
+                const cplx tN = nd.tN[in], tD = nd.tD[in];
+                cfma(sum, f, tN);
+                cfma(sum, zn * gg, tD);
+            } else {
+                const FNode& nd = reinterpret_cast<const FNode*>(tile_raw)[e];
+                const double zx = x - nd.yx, zy = y - nd.yy, r2 = zx * zx + zy * zy;
+                if (!(r2 > 0.)) continue;
+                const double ir = rsqrt(r2), r = r2 * ir;
+                cplx h0, h1;
+                hankel01_cplx(kr * r, ki * r, h0, h1);
+                const double zn = (zx * nd.nx + zy * nd.ny) * ir;
+                const cplx tD = inside ? nd.tdi : nd.tdo, tN = inside ? nd.tni : nd.tno;
+                cplx term = h0 * tN - (mk(kr, ki) * zn) * (h1 * tD);
+                sum += nd.D * term;
+            }
         }
     }
     s_part[w][lane] = sum;
@@ -597,7 +663,7 @@ int check_waves(const double* waves, int nw, double k_im) {
 
 struct FieldState {
     Buf waves, g21, T, piv, perm, info, uD, uN, rhs, M, flagbuf;
-    Buf kind, par, csum, plen, knots, spl, nodes, xg, wg, acc, flag, bndt, near, nearcnt, xq, wq, nearout, addidx,
+    Buf kind, par, csum, plen, knots, spl, nodes, gnodes, pre, xg, wg, acc, flag, bndt, near, nearcnt, xq, wq, nearout, addidx,
         addval, S;
     double last_grid_ms = 0.;
     long long last_units = 0, last_near = 0;
@@ -841,6 +907,7 @@ int hbem_tp_field_grid(hbem_solop s, const double* waves, int nwaves, double k_r
     const long long G = (long long)nx * ny;
     const int M = N * (int)order_green;
     FD_CK(F.nodes.ensure((size_t)M * sizeof(FNode)));
+    FD_CK(F.gnodes.ensure((size_t)M * sizeof(GNode)));
     FD_CK(F.acc.ensure(G * sizeof(cplx)));
     FD_CK(F.flag.ensure(G * sizeof(int)));
     FD_CK(F.bndt.ensure(G * sizeof(double)));
@@ -881,8 +948,54 @@ int hbem_tp_field_grid(hbem_solop s, const double* waves, int nwaves, double k_r
     J.flag = F.flag.as<int>();
     J.bnd_t = F.bndt.as<double>();
     J.near_count = F.nearcnt.as<int>();
+    J.gnodes = F.gnodes.as<GNode>();
+    cudaError_t hk_err = cudaSuccess;
+    J.hk = hankel_table(&hk_err);
+    FD_CK(hk_err);
+    // the grid kernel's FP32 look at the panels: coordinates round by 6e-8 of the largest,
+    // so a margin of 4e-6 of it covers the differences and squares taken there; coordinates
+    // beyond FP32's squares send every panel to the FP64 tests
+    double big = std::max(std::max(std::fabs(ll_x), std::fabs(ur_x)), std::max(std::fabs(ll_y), std::fabs(ur_y)));
+    for (int i = 0; i < N; ++i) {
+        const double* P = par + 5 * (size_t)i;
+        if (kinds[i] == HBEM_PANEL_LINE) for (int q = 0; q < 4; ++q) big = std::max(big, std::fabs(P[q]));
+        else big = std::max(big, std::max(std::fabs(P[0]), std::fabs(P[1])) + std::fabs(P[2]));
+    }
+    const double margin = 4e-6 * big;
+    std::vector<PanelPre> pre(N);
+    for (int i = 0; i < N; ++i) {
+        const double* P = par + 5 * (size_t)i;
+        const bool line = kinds[i] == HBEM_PANEL_LINE;
+        double x1 = P[0], y1 = P[1], x2 = P[2], y2 = P[3];
+        if (!line) {
+            x1 = P[0] + P[2] * std::cos(P[3]);
+            y1 = P[1] + P[2] * std::sin(P[3]);
+            x2 = P[0] + P[2] * std::cos(P[4]);
+            y2 = P[1] + P[2] * std::sin(P[4]);
+        }
+        const double len = std::fabs(plen[i]), ext = line ? 0.5 * len : len;   // the panel lies this near its chord's centre
+        auto r2 = [&](double r) { return (float)((r + margin) * (r + margin) * 1.0001); };
+        PanelPre& q = pre[i];
+        q.cx = (float)(0.5 * (x1 + x2));
+        q.cy = (float)(0.5 * (y1 + y2));
+        q.rin2 = r2(ext + 1e-2 / J.abs_ki + 1e3 * kMachEpsF);
+        q.rout2 = r2(ext + 1e-2 / J.abs_ko + 1e3 * kMachEpsF);
+        q.ylo = (float)(std::min(y1, y2) - margin);
+        q.yhi = (float)(std::max(y1, y2) + margin);
+        q.rseg2 = line ? -1.f : r2(2.5 * len);
+        q.pad = 0.f;
+        if (!(big < 1e15)) {
+            q.rin2 = q.rout2 = q.rseg2 = INFINITY;
+            q.cx = q.cy = 0.f;
+            q.ylo = -INFINITY;
+            q.yhi = INFINITY;
+        }
+    }
+    FD_CK(put(F.pre, pre.data(), pre.size()));
+    J.pre = F.pre.as<PanelPre>();
 
-    k_field_nodes<<<(M + 127) / 128, 128>>>(J, F.xg.as<double>(), F.wg.as<double>(), F.nodes.as<FNode>());
+    k_field_nodes<<<(M + 127) / 128, 128>>>(J, F.xg.as<double>(), F.wg.as<double>(), F.nodes.as<FNode>(),
+                                            F.gnodes.as<GNode>());
     FD_CK(cudaGetLastError());
     int cap = (int)std::max<long long>(4096, G / 8);
     int nnear = 0;
@@ -895,7 +1008,8 @@ int hbem_tp_field_grid(hbem_solop s, const double* waves, int nwaves, double k_r
         J.near_cap = cap;
         FD_CK(cudaMemset(F.nearcnt.p, 0, sizeof(int)));
         cudaEventRecord(e0, 0);
-        k_field_grid<<<(unsigned)((G + 31) / 32), kFieldThreads>>>(J);
+        if (J.real_k) k_field_grid<true><<<(unsigned)((G + 31) / 32), kFieldThreads>>>(J);
+        else k_field_grid<false><<<(unsigned)((G + 31) / 32), kFieldThreads>>>(J);
         cudaEventRecord(e1, 0);
         FD_CK(cudaGetLastError());
         FD_CK(cudaMemcpy(&nnear, F.nearcnt.p, sizeof(int), cudaMemcpyDeviceToHost));
