@@ -34,7 +34,7 @@ constexpr int kArnThreads = 256;
 constexpr int kArnMaxP = 32;
 
 struct Sv2Work {
-    cplx *B = nullptr, *ub = nullptr, *ud = nullptr, *rhs = nullptr, *tb = nullptr;
+    cplx *B = nullptr, *ub = nullptr, *ud = nullptr, *rhs = nullptr, *tb = nullptr, *dinv2 = nullptr;
     int *piv2 = nullptr, *perm2 = nullptr, *info2 = nullptr, *mcol = nullptr;
 };
 cudaError_t sv_der_from_vectors(int n, int nvec, int per, int D, const cplx* T, long long mat_stride,
@@ -46,8 +46,10 @@ cudaError_t copy_mats_batched(long long nn, int nmat, const cplx* src, long long
                               long long dstride, cudaStream_t st);
 cudaError_t lu_factor_batched(int n, int nmat, cplx* A, long long stride, int* piv, int* perm, int* info,
                               cudaStream_t st, long long* launches);
-cudaError_t lu_solve_batched(int n, int nmat, int trans, const cplx* LU, long long stride, const int* perm, int s,
-                             cplx* X, long long xstride, cudaStream_t st);
+cudaError_t lu_solve_batched(int n, int nmat, int trans, const cplx* LU, long long stride, const int* perm,
+                             const cplx* dinv, int s, cplx* X, long long xstride, cudaStream_t st);
+cudaError_t lu_diag_inv_batched(int n, int nmat, const cplx* LU, long long stride, cplx* dinv, cudaStream_t st);
+size_t lu_dinv_elems(int n);
 bool lu_solve_supported(int n);
 
 // Start block entry (r, c): real and imaginary parts uniform in [-1/2, 1/2) from a
@@ -309,7 +311,7 @@ __global__ void __launch_bounds__(kArnThreads) k_arn_check(ArnJob J, const cplx*
 // ------------------------------------------------------------------ orchestration
 
 struct ArnWork {
-    cplx *A = nullptr, *X = nullptr, *Y = nullptr, *Rf = nullptr, *Wg = nullptr, *uv = nullptr;
+    cplx *A = nullptr, *X = nullptr, *Y = nullptr, *Rf = nullptr, *Wg = nullptr, *uv = nullptr, *dinv = nullptr;
     double* nrm = nullptr;
     int *piv = nullptr, *perm = nullptr, *info = nullptr, *ord = nullptr, *done = nullptr, *ndone = nullptr;
     int *status = nullptr, *iters = nullptr;
@@ -343,6 +345,7 @@ size_t arnoldi_carve(int n, int nmat, int count, int D, char* base, ArnWork& w) 
     w.iters = (int*)take(nm * ii);
     if (!arnoldi_small_fits(n, p)) {
         w.A = (cplx*)take(nm * n * n * c);
+        w.dinv = (cplx*)take(nm * lu_dinv_elems(n) * c);
         w.X = (cplx*)take(nm * n * p * c);
         w.Y = (cplx*)take(nm * n * p * c);
         w.Rf = (cplx*)take(nm * p * p * c);
@@ -394,23 +397,24 @@ cudaError_t arnoldi_batched(int n, int nmat, int count, int D, double tol, int m
         const long long nn = (long long)n * n, ns = (long long)n * p;
         AR_CK(copy_mats_batched(nn, nmat, T, mat_stride, w.A, nn, st));
         AR_CK(lu_factor_batched(n, nmat, w.A, nn, w.piv, w.perm, w.info, st, &nl));
+        AR_CK(lu_diag_inv_batched(n, nmat, w.A, nn, w.dinv, st));
         AR_CK(cudaMemsetAsync(w.ndone, 0, sizeof(int), st));
         k_arn_init<<<nmat, 32, 0, st>>>(J, w.info, w.done, w.ndone);
         dim3 g((unsigned)std::min<long long>((ns + 255) / 256, 1024), (unsigned)nmat);
         k_arn_start<<<g, 256, 0, st>>>(n, p, seed, w.X, ns);
         nl += 3;
         AR_CK(cudaGetLastError());
-        AR_CK(lu_solve_batched(n, nmat, 0, w.A, nn, w.perm, p, w.X, ns, st));
+        AR_CK(lu_solve_batched(n, nmat, 0, w.A, nn, w.perm, w.dinv, p, w.X, ns, st));
         AR_CK(qr_global_batched(n, nmat, p, w.X, ns, nullptr, st));
         nl += 2;
         cplx *X = w.X, *Y = w.Y;
         for (int it = 1;; ++it) {
             const int last = it >= maxit;
             AR_CK(cudaMemcpyAsync(Y, X, (size_t)nmat * ns * sizeof(cplx), cudaMemcpyDeviceToDevice, st));
-            AR_CK(lu_solve_batched(n, nmat, 1, w.A, nn, w.perm, p, Y, ns, st));
+            AR_CK(lu_solve_batched(n, nmat, 1, w.A, nn, w.perm, w.dinv, p, Y, ns, st));
             AR_CK(qr_global_batched(n, nmat, p, Y, ns, w.Rf, st));
             k_arn_ritz<<<nmat, 32, 0, st>>>(p, count, w.Rf, w.Wg, w.nrm, w.ord, w.done);
-            AR_CK(lu_solve_batched(n, nmat, 0, w.A, nn, w.perm, p, Y, ns, st));
+            AR_CK(lu_solve_batched(n, nmat, 0, w.A, nn, w.perm, w.dinv, p, Y, ns, st));
             k_arn_check<<<nmat, kArnThreads, 0, st>>>(J, X, Y, ns, w.Rf, w.Wg, w.nrm, w.ord, w.done, w.ndone, it,
                                                       last);
             nl += 5;

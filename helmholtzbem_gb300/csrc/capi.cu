@@ -62,8 +62,11 @@ cudaError_t lu_factor_batched(int n, int nmat, cplx* A, long long stride, int* p
                               cudaStream_t st, long long* launches);
 cudaError_t lu_factor_batched_f32(int n, int nmat, cplxf* A, long long stride, int* piv, int* perm, int* info,
                                   cudaStream_t st, long long* launches, int* tc_err);
-cudaError_t lu_solve_batched(int n, int nmat, int trans, const cplx* LU, long long stride, const int* perm, int s,
-                             cplx* X, long long xstride, cudaStream_t st);
+cudaError_t lu_solve_batched(int n, int nmat, int trans, const cplx* LU, long long stride, const int* perm,
+                             const cplx* dinv, int s, cplx* X, long long xstride, cudaStream_t st);
+cudaError_t lu_diag_inv_batched(int n, int nmat, const cplx* LU, long long stride, cplx* dinv, cudaStream_t st);
+size_t lu_dinv_elems(int n);
+bool lu_solve_in_steps(int n, int nmat, int s);
 cudaError_t lu_perm_from_piv(int n, int nmat, const int* piv, int* perm, cudaStream_t st);
 bool lu_solve_supported(int n);
 void lu_set_cluster_panels(int on);
@@ -1529,10 +1532,17 @@ int hbem_lu_solve_batch_device(int n, int nmat, int trans, const void* LU_dev, l
         return fail(HBEM_ERR_INVALID, "lu_solve_batch: bad argument");
     if (!lu_solve_supported(n)) return fail(HBEM_ERR_UNSUPPORTED, "lu_solve_batch: n too large");
     HB_CK(cudaSetDevice(g_device));
-    static thread_local DBuf perm;
+    static thread_local DBuf perm, dinv;
     HB_CK(perm.ensure((size_t)nmat * n * sizeof(int)));
     HB_CK(lu_perm_from_piv(n, nmat, piv_dev, perm.as<int>(), 0));
-    HB_CK(lu_solve_batched(n, nmat, trans, static_cast<const cplx*>(LU_dev), stride, perm.as<int>(), nrhs,
+    const cplx* LU = static_cast<const cplx*>(LU_dev);
+    const bool steps = lu_solve_in_steps(n, nmat, nrhs);
+    if (steps) {
+        HB_CK(dinv.ensure((size_t)nmat * lu_dinv_elems(n) * sizeof(cplx)));
+        HB_CK(lu_diag_inv_batched(n, nmat, LU, stride, dinv.as<cplx>(), 0));
+        g_launches += 1;
+    }
+    HB_CK(lu_solve_batched(n, nmat, trans, LU, stride, perm.as<int>(), steps ? dinv.as<cplx>() : nullptr, nrhs,
                            static_cast<cplx*>(X_dev), xstride, 0));
     g_launches += 2;
     HB_CK(cudaStreamSynchronize(0));

@@ -42,8 +42,10 @@ void gauss_rule(double a, double b, int n, double* x, double* w);
 void count_launches(long long n);
 cudaError_t lu_factor_batched(int n, int nmat, cplx* A, long long stride, int* piv, int* perm, int* info,
                               cudaStream_t st, long long* launches);
-cudaError_t lu_solve_batched(int n, int nmat, int trans, const cplx* LU, long long stride, const int* perm, int s,
-                             cplx* X, long long xstride, cudaStream_t st);
+cudaError_t lu_solve_batched(int n, int nmat, int trans, const cplx* LU, long long stride, const int* perm,
+                             const cplx* dinv, int s, cplx* X, long long xstride, cudaStream_t st);
+cudaError_t lu_diag_inv_batched(int n, int nmat, const cplx* LU, long long stride, cplx* dinv, cudaStream_t st);
+size_t lu_dinv_elems(int n);
 
 namespace {
 
@@ -662,7 +664,7 @@ int check_waves(const double* waves, int nw, double k_im) {
 }
 
 struct FieldState {
-    Buf waves, g21, T, piv, perm, info, uD, uN, rhs, M, flagbuf;
+    Buf waves, g21, T, dinv, piv, perm, info, uD, uN, rhs, M, flagbuf;
     Buf kind, par, csum, plen, knots, spl, nodes, gnodes, pre, xg, wg, acc, flag, bndt, near, nearcnt, xq, wq, nearout, addidx,
         addval, S;
     double last_grid_ms = 0.;
@@ -741,7 +743,9 @@ int tp_solve_device(hbem_solop s, const double* waves, int nw, double k_re, doub
     int info = 0;
     FD_CK(cudaMemcpy(&info, F.info.p, sizeof(int), cudaMemcpyDeviceToHost));
     if (info) return set_error(HBEM_ERR_SINGULAR, "zgesv: LU is singular");
-    FD_CK(lu_solve_batched((int)n2, 1, 0, F.T.as<cplx>(), (long long)(n2 * n2), F.perm.as<int>(), 1, F.rhs.as<cplx>(),
+    FD_CK(F.dinv.ensure(lu_dinv_elems((int)n2) * sizeof(cplx)));
+    FD_CK(lu_diag_inv_batched((int)n2, 1, F.T.as<cplx>(), (long long)(n2 * n2), F.dinv.as<cplx>(), 0));
+    FD_CK(lu_solve_batched((int)n2, 1, 0, F.T.as<cplx>(), (long long)(n2 * n2), F.perm.as<int>(), F.dinv.as<cplx>(), 1, F.rhs.as<cplx>(),
                            (long long)n2, 0));
     count_launches(nl + 1);
     FD_CK(cudaDeviceSynchronize());

@@ -604,6 +604,155 @@ __global__ void __launch_bounds__(kLuSolveThreads) k_lu_solve(int n, int s, int 
     else lu_solve_n<E, CH>(M, pm, n, Xm, cs, sm);
 }
 
+// ---- few matrices or columns: one launch per 32-row block over all SMs
+//
+// k_lu_solve keeps a column group on one CTA, which reads all the factors by itself: a
+// single matrix of order 3000 (complex64, 16 columns) took 4.4 ms that way, order 802
+// (six matrices, 12 columns, complex128) 1.54 ms.  Here launch b of a triangular sweep
+// subtracts the solved block b from the rows left (a CTA per 32 rows, CPC columns and
+// matrix, its four warps splitting the block's columns), and the CTAs that hold the next
+// block's rows multiply them at once by the inverse of its triangle.  The 32 x 32 inverses
+// are made once per factorisation (k_diag_inv): substitution there, 32 dependent steps of
+// FP64 FMAs and shuffles on one warp, was two thirds of a launch (14.8 us; 6 with them).
+enum SolveSweep { kSweepL = 0, kSweepU = 1, kSweepUH = 2, kSweepLH = 3 };   // L y = b, U x = y; U^H y = b, L^H x = y
+
+size_t lu_dinv_elems(int n) { return (size_t)((n + kLuNB - 1) / kLuNB) * kLuNB * kLuNB; }
+
+// Inverses of the diagonal blocks of L (unit: strictly lower part stored) and U (upper
+// part) of every matrix: dinv[matrix][block][column][row].  grid (blocks, nmat, 4): a warp
+// per column, eight columns a CTA, by substitution.
+template <class E>
+__global__ void __launch_bounds__(256) k_diag_inv(int n, const E* LU, long long stride, E* dinv) {
+    __shared__ E W[kLuNB][kLuNB + 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r0 = blockIdx.x * kLuNB, nr = min(kLuNB, n - r0);
+    const E* M = LU + (long long)blockIdx.y * stride;
+    E* out = dinv + ((long long)blockIdx.y * gridDim.x + blockIdx.x) * kLuNB * kLuNB;
+    for (int e = threadIdx.x; e < kLuNB * kLuNB; e += blockDim.x) {   // beyond the matrix: the unit matrix
+        const int r = e % kLuNB, k = e / kLuNB;
+        W[r][k] = (r < nr && k < nr) ? M[(r0 + r) + (long long)(r0 + k) * n] : r == k ? Elem<E>::one() : Elem<E>::zero();
+    }
+    __syncthreads();
+    const int c = blockIdx.z * 8 + warp;
+    E v = lane == c ? Elem<E>::one() : Elem<E>::zero();               // L x = e_c
+    for (int k = c; k < kLuNB; ++k) {
+        E vk;
+        vk.re = __shfl_sync(0xffffffffu, v.re, k);
+        vk.im = __shfl_sync(0xffffffffu, v.im, k);
+        if (lane > k) cfms(v, W[lane][k], vk);
+    }
+    const E lower = v;
+    const E id = cdiv(Elem<E>::one(), W[lane][lane]);
+    v = lane == c ? Elem<E>::one() : Elem<E>::zero();                 // U x = e_c
+    for (int k = c; k >= 0; --k) {
+        if (lane == k) v = v * id;
+        E vk;
+        vk.re = __shfl_sync(0xffffffffu, v.re, k);
+        vk.im = __shfl_sync(0xffffffffu, v.im, k);
+        if (lane < k) cfms(v, W[lane][k], vk);
+    }
+    out[c * kLuNB + lane] = lane > c ? lower : v;
+}
+
+template <class E, int SWEEP, int CPC>
+__global__ void __launch_bounds__(128) k_solve_step(int n, int s, int cur, const E* LU, long long stride,
+                                                    const E* dinv, E* X, long long xstride) {
+    constexpr bool ASC = SWEEP == kSweepL || SWEEP == kSweepUH, HERM = SWEEP >= 2;
+    __shared__ E W[kLuNB][kLuNB + 1], D[kLuNB][kLuNB + 1];   // D[k][r]: entry (r, k) of the inverse as applied
+    __shared__ E xs[CPC][kLuNB], part[4][CPC][kLuNB];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = blockIdx.x;
+    const int nb = (n + kLuNB - 1) / kLuNB;
+    const int blk = ASC ? cur + 1 + t : cur - 1 - t;               // this CTA's rows
+    const int c0 = blockIdx.y * CPC, cs = min(CPC, s - c0);
+    const E* M = LU + (long long)blockIdx.z * stride;
+    E* Xm = X + (long long)blockIdx.z * xstride + (long long)c0 * n;
+    const int r0 = blk * kLuNB, nr = min(kLuNB, n - r0);
+    if (t == 0) {
+        const E* Db = dinv + ((long long)blockIdx.z * nb + blk) * kLuNB * kLuNB;
+        for (int c = warp; c < kLuNB; c += 4) {                    // (row lane, column c) of the stored inverses
+            const E z = Db[c * kLuNB + lane];
+            const bool low = lane > c;
+            const E o = (SWEEP == kSweepL || SWEEP == kSweepLH) ? (low ? z : lane == c ? Elem<E>::one() : Elem<E>::zero())
+                                                                : (low ? Elem<E>::zero() : z);
+            if (HERM) D[lane][c] = conj(o);
+            else D[c][lane] = o;
+        }
+    }
+    const bool update = ASC ? cur >= 0 : cur < nb;
+    E yold[CPC];
+#pragma unroll
+    for (int c = 0; c < CPC; ++c) yold[c] = (warp == 0 && c < cs && lane < nr) ? Xm[(long long)c * n + r0 + lane] : Elem<E>::zero();
+    if (update) {
+        const int k0 = cur * kLuNB, nk = min(kLuNB, n - k0);
+        for (int e = threadIdx.x; e < CPC * kLuNB; e += 128) {
+            const int c = e / kLuNB, k = e - c * kLuNB;
+            xs[c][k] = (c < cs && k < nk) ? Xm[(long long)c * n + k0 + k] : Elem<E>::zero();
+        }
+        E w[8];
+        if (HERM) {   // conj(M[k, r]): columns r of the factor, contiguous in k
+            for (int r = warp; r < kLuNB; r += 4)
+                W[lane][r] = (lane < nk && r < nr) ? conj(M[(k0 + lane) + (long long)(r0 + r) * n]) : Elem<E>::zero();
+        } else {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int k = 8 * warp + q;
+                w[q] = (lane < nr && k < nk) ? M[(r0 + lane) + (long long)(k0 + k) * n] : Elem<E>::zero();
+            }
+        }
+        __syncthreads();
+        E acc[CPC];
+#pragma unroll
+        for (int c = 0; c < CPC; ++c) acc[c] = Elem<E>::zero();
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int k = 8 * warp + q;
+            if (HERM) w[q] = W[k][lane];
+#pragma unroll
+            for (int c = 0; c < CPC; ++c) cfma(acc[c], w[q], xs[c][k]);
+        }
+#pragma unroll
+        for (int c = 0; c < CPC; ++c) part[warp][c][lane] = acc[c];
+        __syncthreads();
+        if (warp == 0) {
+#pragma unroll
+            for (int c = 0; c < CPC; ++c) {
+                yold[c] = yold[c] - ((part[0][c][lane] + part[1][c][lane]) + (part[2][c][lane] + part[3][c][lane]));
+                if (t > 0 && c < cs && lane < nr) Xm[(long long)c * n + r0 + lane] = yold[c];
+            }
+        }
+    }
+    if (t > 0) return;
+    // the next block: times the inverse of its triangle
+    if (warp == 0)
+#pragma unroll
+        for (int c = 0; c < CPC; ++c) xs[c][lane] = yold[c];
+    __syncthreads();
+    E acc[CPC];
+#pragma unroll
+    for (int c = 0; c < CPC; ++c) acc[c] = Elem<E>::zero();
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int k = 8 * warp + q;
+        const E w = D[k][lane];
+#pragma unroll
+        for (int c = 0; c < CPC; ++c) cfma(acc[c], w, xs[c][k]);
+    }
+#pragma unroll
+    for (int c = 0; c < CPC; ++c) part[warp][c][lane] = acc[c];
+    __syncthreads();
+    for (int c = warp; c < cs; c += 4)
+        if (lane < nr)
+            Xm[(long long)c * n + r0 + lane] =
+                (part[0][c][lane] + part[1][c][lane]) + (part[2][c][lane] + part[3][c][lane]);
+}
+
+// X <- P X (inverse: P^T X), a CTA per column
+template <class E>
+__global__ void __launch_bounds__(256) k_permute_rows(int n, const int* perm, E* X, long long xstride, int inverse) {
+    extern __shared__ double perm_sm[];
+    permute_rows(X + (long long)blockIdx.y * xstride + (long long)blockIdx.x * n, n, 1,
+                 perm + (long long)blockIdx.y * n, reinterpret_cast<E*>(perm_sm), inverse != 0);
+}
+
 constexpr size_t kLuSmemLimit = 220 * 1024;
 
 bool lu_solve_supported(int n) { return lu_solve_smem_bytes(n, sizeof(cplx)) <= kLuSmemLimit; }
@@ -804,11 +953,57 @@ cudaError_t lu_factor_impl(int n, int nmat, E* A, long long stride, int* piv, in
     return cudaGetLastError();
 }
 
+template <class E, int CPC>
+cudaError_t lu_solve_steps(int n, int nmat, int trans, const E* LU, long long stride, const int* perm, const E* dinv,
+                           int s, E* X, long long xstride, cudaStream_t st) {
+    const size_t psm = (size_t)n * sizeof(E);
+    if (cudaError_t e = cudaFuncSetAttribute(k_permute_rows<E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)kLuSmemLimit);
+        e != cudaSuccess)
+        return e;
+    const int nb = (n + kLuNB - 1) / kLuNB, cg = (s + CPC - 1) / CPC;
+    auto sweep = [&](auto kernel, bool asc) {
+        for (int q = -1; q < nb - 1; ++q) {
+            const int cur = asc ? q : nb - 1 - q, tiles = q < 0 ? 1 : nb - 1 - q;
+            kernel<<<dim3(tiles, cg, nmat), 128, 0, st>>>(n, s, cur, LU, stride, dinv, X, xstride);
+        }
+    };
+    if (trans) {
+        sweep(k_solve_step<E, kSweepUH, CPC>, true);
+        sweep(k_solve_step<E, kSweepLH, CPC>, false);
+        k_permute_rows<E><<<dim3(s, nmat), 256, psm, st>>>(n, perm, X, xstride, 1);
+    } else {
+        k_permute_rows<E><<<dim3(s, nmat), 256, psm, st>>>(n, perm, X, xstride, 0);
+        sweep(k_solve_step<E, kSweepL, CPC>, true);
+        sweep(k_solve_step<E, kSweepU, CPC>, false);
+    }
+    return cudaGetLastError();
+}
+
+// Whether a solve takes the launches per block: few columns in all (below four per SM a CTA
+// per column group leaves SMs idle, and its time is one CTA's).  Measured, T^-1 X with 12
+// columns a matrix, ms, a CTA per column group -> launches per block: order 128, 1 matrix
+// 0.177 -> 0.112; 512, 1: 0.766 -> 0.320; 802, 6: 1.54 -> 1.00; 1600, 16: 6.69 -> 4.92; 64 matrices:
+// order 256 0.678 -> 0.820, order 512 2.21 -> 2.31.
+bool lu_solve_in_steps(int n, int nmat, int s) { return n >= 128 && (long long)nmat * s < 608; }
+
 template <class E>
-cudaError_t lu_solve_impl(int n, int nmat, int trans, const E* LU, long long stride, const int* perm, int s, E* X,
-                          long long xstride, cudaStream_t st) {
+cudaError_t lu_diag_inv(int n, int nmat, const E* LU, long long stride, E* dinv, cudaStream_t st) {
+    k_diag_inv<E><<<dim3((n + kLuNB - 1) / kLuNB, nmat, 4), 256, 0, st>>>(n, LU, stride, dinv);
+    return cudaGetLastError();
+}
+
+// dinv: the factors' lu_diag_inv (nmat x lu_dinv_elems(n)), or null (a CTA per column group)
+template <class E>
+cudaError_t lu_solve_impl(int n, int nmat, int trans, const E* LU, long long stride, const int* perm, const E* dinv,
+                          int s, E* X, long long xstride, cudaStream_t st) {
     const size_t smem = lu_solve_smem_bytes(n, sizeof(E));
     if (n < 1 || nmat < 1 || nmat > 65535 || s < 1 || smem > kLuSmemLimit) return cudaErrorInvalidValue;
+    if (dinv && lu_solve_in_steps(n, nmat, s)) {
+        if ((long long)nmat * s <= 32)
+            return lu_solve_steps<E, 1>(n, nmat, trans, LU, stride, perm, dinv, s, X, xstride, st);
+        return lu_solve_steps<E, 2>(n, nmat, trans, LU, stride, perm, dinv, s, X, xstride, st);
+    }
     // columns per CTA: a power of two <= 16 (the register chunk is exactly that wide,
     // so no lane computes for absent columns), the widest that still gives about two
     // CTAs per SM of the 152, which re-reads the factors least
@@ -843,13 +1038,19 @@ cudaError_t lu_factor_batched_f32(int n, int nmat, cplxf* A, long long stride, i
                                   cudaStream_t st, long long* launches, int* tc_err) {
     return lu_factor_impl<cplxf>(n, nmat, A, stride, piv, perm, info, st, launches, tc_err);
 }
-cudaError_t lu_solve_batched(int n, int nmat, int trans, const cplx* LU, long long stride, const int* perm, int s,
-                             cplx* X, long long xstride, cudaStream_t st) {
-    return lu_solve_impl<cplx>(n, nmat, trans, LU, stride, perm, s, X, xstride, st);
+cudaError_t lu_solve_batched(int n, int nmat, int trans, const cplx* LU, long long stride, const int* perm,
+                             const cplx* dinv, int s, cplx* X, long long xstride, cudaStream_t st) {
+    return lu_solve_impl<cplx>(n, nmat, trans, LU, stride, perm, dinv, s, X, xstride, st);
 }
 cudaError_t lu_solve_batched_f32(int n, int nmat, int trans, const cplxf* LU, long long stride, const int* perm,
-                                 int s, cplxf* X, long long xstride, cudaStream_t st) {
-    return lu_solve_impl<cplxf>(n, nmat, trans, LU, stride, perm, s, X, xstride, st);
+                                 const cplxf* dinv, int s, cplxf* X, long long xstride, cudaStream_t st) {
+    return lu_solve_impl<cplxf>(n, nmat, trans, LU, stride, perm, dinv, s, X, xstride, st);
+}
+cudaError_t lu_diag_inv_batched(int n, int nmat, const cplx* LU, long long stride, cplx* dinv, cudaStream_t st) {
+    return lu_diag_inv<cplx>(n, nmat, LU, stride, dinv, st);
+}
+cudaError_t lu_diag_inv_batched_f32(int n, int nmat, const cplxf* LU, long long stride, cplxf* dinv, cudaStream_t st) {
+    return lu_diag_inv<cplxf>(n, nmat, LU, stride, dinv, st);
 }
 
 }  // namespace hbem

@@ -11,8 +11,12 @@
 // QR; the Ritz vectors are that null vector to the accuracy of the sketch.)
 #include <algorithm>
 
+#include <cooperative_groups.h>
+
 #include "hbem_device.cuh"
 #include "smem_linalg.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace hbem {
 
@@ -131,8 +135,10 @@ cudaError_t launch_rsvd_small(int n, int nmat, int s, int q, int D, const cplx* 
 
 cudaError_t lu_factor_batched(int n, int nmat, cplx* A, long long stride, int* piv, int* perm, int* info,
                               cudaStream_t st, long long* launches);
-cudaError_t lu_solve_batched(int n, int nmat, int trans, const cplx* LU, long long stride, const int* perm, int s,
-                             cplx* X, long long xstride, cudaStream_t st);
+cudaError_t lu_solve_batched(int n, int nmat, int trans, const cplx* LU, long long stride, const int* perm,
+                             const cplx* dinv, int s, cplx* X, long long xstride, cudaStream_t st);
+cudaError_t lu_diag_inv_batched(int n, int nmat, const cplx* LU, long long stride, cplx* dinv, cudaStream_t st);
+size_t lu_dinv_elems(int n);
 bool lu_solve_supported(int n);
 
 __global__ void k_copy_mats(int nn, const cplx* src, long long sstride, cplx* dst, long long dstride) {
@@ -148,6 +154,107 @@ __global__ void __launch_bounds__(kRsvdThreads) k_qr_global(int n, int s, cplx* 
     qr_cgs2(X + (long long)blockIdx.x * xstride, n, s, coef, red, Rf ? Rf + (long long)blockIdx.x * s * s : nullptr);
 }
 
+// The same orthonormalisation (classical Gram-Schmidt, twice per column) on a cluster of
+// CTAs, each holding its rows in shared memory: one CTA reads X through one SM and has
+// 1/152 of the FP64 rate (n = 3000, 16 columns: 2.08 ms).  Per column three cluster-wide
+// sums -- the coefficients of both passes and the norm -- through distributed shared
+// memory; the partial sums alternate between two buffers, so one barrier each is enough.
+__global__ void __launch_bounds__(kRsvdThreads) k_qr_cluster(int n, int s, int rows, cplx* X, long long xstride,
+                                                             cplx* Rf) {
+    cg::cluster_group cl = cg::this_cluster();
+    const int ncta = (int)cl.num_blocks(), rank = (int)cl.block_rank(), mat = blockIdx.x / ncta;
+    extern __shared__ __align__(16) double qr_sm[];
+    cplx* P = reinterpret_cast<cplx*>(qr_sm);             // [column][row], leading dimension rows
+    __shared__ cplx part[2][kRsvdMaxS], coef[kRsvdMaxS];
+    __shared__ double red[128];
+    cplx* Xm = X + (long long)mat * xstride;
+    const int r0 = rank * rows, nr = max(0, min(rows, n - r0));
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int c = warp; c < s; c += nw)
+        for (int r = lane; r < nr; r += 32) P[c * rows + r] = Xm[r0 + r + (long long)c * n];
+    __syncthreads();
+    int buf = 0;
+    for (int j = 0; j < s; ++j) {
+        cplx* xj = P + j * rows;
+        for (int pass = 0; pass < 2 && j > 0; ++pass, buf ^= 1) {
+            for (int i = warp; i < j; i += nw) {
+                const cplx* qi = P + i * rows;
+                cplx a = mk(0.);
+                for (int r = lane; r < nr; r += 32) cfma_c(a, qi[r], xj[r]);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    a.re += __shfl_xor_sync(0xffffffffu, a.re, o);
+                    a.im += __shfl_xor_sync(0xffffffffu, a.im, o);
+                }
+                if (lane == 0) part[buf][i] = a;
+            }
+            cl.sync();
+            for (int i = threadIdx.x; i < j; i += blockDim.x) {
+                cplx a = mk(0.);
+                for (int q = 0; q < ncta; ++q) a += cl.map_shared_rank(part[buf], q)[i];
+                coef[i] = a;
+                if (Rf && rank == 0) {
+                    cplx* R = Rf + (long long)mat * s * s + i + j * s;
+                    *R = pass ? *R + a : a;
+                }
+            }
+            __syncthreads();
+            for (int r = threadIdx.x; r < nr; r += blockDim.x) {
+                cplx v = xj[r];
+                for (int i = 0; i < j; ++i) cfms(v, P[i * rows + r], coef[i]);
+                xj[r] = v;
+            }
+            __syncthreads();
+        }
+        double nn = 0.;
+        for (int r = threadIdx.x; r < nr; r += blockDim.x) nn += norm2(xj[r]);
+        const double mine = bsum(nn, red);
+        if (threadIdx.x == 0) part[buf][0] = mk(mine);
+        cl.sync();
+        double tot = 0.;
+        for (int q = 0; q < ncta; ++q) tot += cl.map_shared_rank(part[buf], q)[0].re;
+        buf ^= 1;
+        const double nrm = sqrt(tot), inv = nrm > 0. ? 1. / nrm : 0.;
+        if (Rf && rank == 0) {
+            cplx* R = Rf + (long long)mat * s * s + j * s;
+            if (threadIdx.x == 0) R[j] = mk(nrm);
+            for (int i = j + 1 + threadIdx.x; i < s; i += blockDim.x) R[i] = mk(0.);
+        }
+        for (int r = threadIdx.x; r < nr; r += blockDim.x) xj[r] = inv * xj[r];
+        __syncthreads();
+    }
+    for (int c = warp; c < s; c += nw)
+        for (int r = lane; r < nr; r += 32) Xm[r0 + r + (long long)c * n] = P[c * rows + r];
+    cl.sync();   // no CTA leaves while another may still read its partial sums
+}
+
+// QR of the s columns of nmat blocks: on clusters of eight CTAs while those are few
+// (below four per SM in all) and the rows fit, else a CTA per block.
+static cudaError_t launch_qr(int n, int nmat, int s, cplx* X, long long xstride, cplx* Rf, cudaStream_t st) {
+    constexpr int CS = 8;
+    const int rows = (n + CS - 1) / CS;
+    const size_t smem = (size_t)rows * s * sizeof(cplx);
+    if (n >= 256 && (long long)nmat * CS <= 4 * 152 && smem <= 200 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(k_qr_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        if (e != cudaSuccess) return e;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(nmat * CS));
+        cfg.blockDim = dim3(kRsvdThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = CS;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, k_qr_cluster, n, s, rows, X, xstride, Rf);
+    }
+    k_qr_global<<<nmat, kRsvdThreads, 0, st>>>(n, s, X, xstride, Rf);
+    return cudaGetLastError();
+}
+
 // sigma from the triangular factor Rf of B = T^-H Q = Q_B Rf: sigma_max(B) =
 // sigma_max(Rf).  D >= 1: the right Ritz vector v = Q w (w the top right singular
 // vector of Rf) into the v half of uv.
@@ -157,16 +264,22 @@ __global__ void __launch_bounds__(kRsvdThreads) k_rsvd_tail(int n, int s, int D,
                                                              const int* info, double* out, int* status, cplx* uv,
                                                              const int* tc_err) {
     __shared__ cplx Rs[kRsvdMaxS * kRsvdMaxS], W[kRsvdMaxS * kRsvdMaxS], tw[kRsvdMaxS];
+    __shared__ double cn[kRsvdMaxS];
+    __shared__ int rot;
     const int mat = blockIdx.x, os = D + 1;
     for (int e = threadIdx.x; e < s * s; e += blockDim.x) Rs[e] = Rf[(long long)mat * s * s + e];
     __syncthreads();
-    if (threadIdx.x < 32) jacobi_warp(Rs, s, W);
-    __syncthreads();
+    jacobi_cta(Rs, s, W, &rot);   // a warp per column pair (one warp for all of them: 3.4 ms at s = 16)
     double best = -1.;
     int bj = 0;
-    for (int j = 0; j < s; ++j) {
+    if (threadIdx.x < s) {
         double nb = 0.;
-        for (int r = 0; r < s; ++r) nb += norm2(Rs[j * s + r]);
+        for (int r = 0; r < s; ++r) nb += norm2(Rs[threadIdx.x * s + r]);
+        cn[threadIdx.x] = nb;
+    }
+    __syncthreads();
+    for (int j = 0; j < s; ++j) {
+        const double nb = cn[j];
         if (nb > best) { best = nb; bj = j; }
     }
     const double smax = sqrt(best), isn = smax > 0. ? 1. / smax : 0.;
@@ -357,7 +470,8 @@ __global__ void k_sv2_out(int n, int nmat, const cplx* sol, const int* mcol, con
 cudaError_t lu_factor_batched_f32(int n, int nmat, cplxf* A, long long stride, int* piv, int* perm, int* info,
                                   cudaStream_t st, long long* launches, int* tc_err);
 cudaError_t lu_solve_batched_f32(int n, int nmat, int trans, const cplxf* LU, long long stride, const int* perm,
-                                 int s, cplxf* X, long long xstride, cudaStream_t st);
+                                 const cplxf* dinv, int s, cplxf* X, long long xstride, cudaStream_t st);
+cudaError_t lu_diag_inv_batched_f32(int n, int nmat, const cplxf* LU, long long stride, cplxf* dinv, cudaStream_t st);
 bool lu_solve_supported_f32(int n);
 
 __global__ void k_to_f32(long long len, const cplx* src, long long sstride, cplxf* dst, long long dstride) {
@@ -442,6 +556,7 @@ __global__ void __launch_bounds__(256) k_resid_h(int n, int s, const cplx* T, lo
 struct MixedBufs {
     const cplxf* LU32;
     const int* perm;
+    const cplxf* dinv;
     cplx* Bsave;
     cplx* Rres;
     cplxf* X32;
@@ -463,7 +578,7 @@ cudaError_t solve_mixed(int n, int nmat, int trans, const MixedBufs& mb, const c
         ++nl;
     }
     k_to_f32<<<g, 256, 0, st>>>(len, X, xs, mb.X32, len);
-    RS_CK(lu_solve_batched_f32(n, nmat, trans, mb.LU32, nn, mb.perm, ncol, mb.X32, len, st));
+    RS_CK(lu_solve_batched_f32(n, nmat, trans, mb.LU32, nn, mb.perm, mb.dinv, ncol, mb.X32, len, st));
     k_acc_f64<<<g, 256, 0, st>>>(len, mb.X32, len, X, xs, 1);
     nl += 3;
     for (int it = 1; it < iters; ++it) {
@@ -473,7 +588,7 @@ cudaError_t solve_mixed(int n, int nmat, int trans, const MixedBufs& mb, const c
             k_resid_n<<<dim3((n + 255) / 256, nmat), 256, 0, st>>>(n, ncol, T, mat_stride, X, xs, mb.Bsave, len, mb.Rres,
                                                                   len);
         k_to_f32<<<g, 256, 0, st>>>(len, mb.Rres, len, mb.X32, len);
-        RS_CK(lu_solve_batched_f32(n, nmat, trans, mb.LU32, nn, mb.perm, ncol, mb.X32, len, st));
+        RS_CK(lu_solve_batched_f32(n, nmat, trans, mb.LU32, nn, mb.perm, mb.dinv, ncol, mb.X32, len, st));
         k_acc_f64<<<g, 256, 0, st>>>(len, mb.X32, len, X, xs, 0);
         nl += 4;
     }
@@ -483,7 +598,7 @@ cudaError_t solve_mixed(int n, int nmat, int trans, const MixedBufs& mb, const c
 // ------------------------------------------------------------------ orchestration
 
 struct Sv2Work {
-    cplx *B = nullptr, *ub = nullptr, *ud = nullptr, *rhs = nullptr, *tb = nullptr;
+    cplx *B = nullptr, *ub = nullptr, *ud = nullptr, *rhs = nullptr, *tb = nullptr, *dinv2 = nullptr;
     int *piv2 = nullptr, *perm2 = nullptr, *info2 = nullptr, *mcol = nullptr;
 };
 cudaError_t sv_der_from_vectors(int n, int nvec, int per, int D, const cplx* T, long long mat_stride,
@@ -491,9 +606,9 @@ cudaError_t sv_der_from_vectors(int n, int nvec, int per, int D, const cplx* T, 
                                 long long& nl);
 
 struct RsvdWork {
-    cplx *A = nullptr, *X = nullptr, *Y = nullptr, *Rf = nullptr, *uv = nullptr;
+    cplx *A = nullptr, *X = nullptr, *Y = nullptr, *Rf = nullptr, *uv = nullptr, *dinv = nullptr, *dinv2 = nullptr;
     int *piv = nullptr, *perm = nullptr, *info = nullptr;
-    cplxf *A32 = nullptr, *X32 = nullptr;
+    cplxf *A32 = nullptr, *X32 = nullptr, *dinv32 = nullptr;
     int* tc_err = nullptr;
     cplx *Bsave = nullptr, *Rres = nullptr;
     cplx *B = nullptr, *ub = nullptr, *ud = nullptr, *rhs = nullptr, *tb = nullptr;
@@ -502,7 +617,7 @@ struct RsvdWork {
 
 static Sv2Work sv2_work(const RsvdWork& w) {
     Sv2Work v;
-    v.B = w.B; v.ub = w.ub; v.ud = w.ud; v.rhs = w.rhs; v.tb = w.tb;
+    v.B = w.B; v.ub = w.ub; v.ud = w.ud; v.rhs = w.rhs; v.tb = w.tb; v.dinv2 = w.dinv2;
     v.piv2 = w.piv2; v.perm2 = w.perm2; v.info2 = w.info2; v.mcol = w.mcol;
     return v;
 }
@@ -519,12 +634,14 @@ size_t rsvd_carve(int n, int nmat, int s, int D, bool small, bool mixed, char* b
     if (!small) {
         if (mixed) {
             w.A32 = (cplxf*)take(nm * nn * cf);
+            w.dinv32 = (cplxf*)take(nm * lu_dinv_elems(n) * cf);
             w.tc_err = (int*)take(sizeof(int));
             w.X32 = (cplxf*)take(nm * n * s * cf);
             w.Bsave = (cplx*)take(nm * n * s * c);
             w.Rres = (cplx*)take(nm * n * s * c);
         } else {
             w.A = (cplx*)take(nm * nn * c);
+            w.dinv = (cplx*)take(nm * lu_dinv_elems(n) * c);
         }
         w.piv = (int*)take(nm * n * ii);
         w.perm = (int*)take(nm * n * ii);
@@ -536,6 +653,7 @@ size_t rsvd_carve(int n, int nmat, int s, int D, bool small, bool mixed, char* b
     if (D >= 1) w.uv = (cplx*)take(nm * 2 * n * c);
     if (D == 2) {
         w.B = (cplx*)take(nm * 4 * nn * c);
+        w.dinv2 = (cplx*)take(nm * lu_dinv_elems(2 * n) * c);
         w.piv2 = (int*)take(nm * 2 * n * ii);
         w.perm2 = (int*)take(nm * 2 * n * ii);
         w.info2 = (int*)take(nm * ii);
@@ -582,12 +700,12 @@ cudaError_t rsvd_batched(int n, int nmat, int s, int q, int D, int precision, in
         ++nl;
     } else {
         const long long nn = (long long)n * n, ns = (long long)n * s;
-        const MixedBufs mb{w.A32, w.perm, w.Bsave, w.Rres, w.X32};
+        const MixedBufs mb{w.A32, w.perm, w.dinv32, w.Bsave, w.Rres, w.X32};
         // op(T)^-1 on ncol columns: FP64 factors, or FP32 factors with `iters` refinement passes
         auto solve = [&](int trans, cplx* X, int ncol, long long xs, int iters) -> cudaError_t {
             if (!mixed) {
                 ++nl;
-                return lu_solve_batched(n, nmat, trans, w.A, nn, w.perm, ncol, X, xs, st);
+                return lu_solve_batched(n, nmat, trans, w.A, nn, w.perm, w.dinv, ncol, X, xs, st);
             }
             return solve_mixed(n, nmat, trans, mb, T, mat_stride, X, ncol, xs, iters, st, nl);
         };
@@ -595,25 +713,27 @@ cudaError_t rsvd_batched(int n, int nmat, int s, int q, int D, int precision, in
             k_to_f32<<<grid_len(nn, nmat), 256, 0, st>>>(nn, T, mat_stride, w.A32, nn);
             RS_CK(cudaMemsetAsync(w.tc_err, 0, sizeof(int), st));
             RS_CK(lu_factor_batched_f32(n, nmat, w.A32, nn, w.piv, w.perm, w.info, st, &nl, w.tc_err));
+            RS_CK(lu_diag_inv_batched_f32(n, nmat, w.A32, nn, w.dinv32, st));
         } else {
             k_copy_mats<<<grid_len(nn, nmat), 256, 0, st>>>((int)nn, T, mat_stride, w.A, nn);
             RS_CK(lu_factor_batched(n, nmat, w.A, nn, w.piv, w.perm, w.info, st, &nl));
+            RS_CK(lu_diag_inv_batched(n, nmat, w.A, nn, w.dinv, st));
         }
         k_copy_mats<<<grid_len(ns, nmat), 256, 0, st>>>((int)ns, R, 0, w.X, ns);
-        nl += 2;
+        nl += 3;
         RS_CK(solve(0, w.X, s, ns, 1));
-        k_qr_global<<<nmat, kRsvdThreads, 0, st>>>(n, s, w.X, ns, nullptr);
+        RS_CK(launch_qr(n, nmat, s, w.X, ns, nullptr, st));
         ++nl;
         for (int it = 0; it < q; ++it) {
             RS_CK(solve(1, w.X, s, ns, 1));
-            k_qr_global<<<nmat, kRsvdThreads, 0, st>>>(n, s, w.X, ns, nullptr);
+            RS_CK(launch_qr(n, nmat, s, w.X, ns, nullptr, st));
             RS_CK(solve(0, w.X, s, ns, 1));
-            k_qr_global<<<nmat, kRsvdThreads, 0, st>>>(n, s, w.X, ns, nullptr);
+            RS_CK(launch_qr(n, nmat, s, w.X, ns, nullptr, st));
             nl += 2;
         }
         RS_CK(cudaMemcpyAsync(w.Y, w.X, (size_t)nmat * ns * sizeof(cplx), cudaMemcpyDeviceToDevice, st));
         RS_CK(solve(1, w.Y, s, ns, refine));
-        k_qr_global<<<nmat, kRsvdThreads, 0, st>>>(n, s, w.Y, ns, w.Rf);
+        RS_CK(launch_qr(n, nmat, s, w.Y, ns, w.Rf, st));
         k_rsvd_tail<<<nmat, kRsvdThreads, 0, st>>>(n, s, D, w.X, w.Y, ns, w.Rf, T, mat_stride, der_stride, w.info,
                                                     out, status, w.uv, w.tc_err);
         nl += 2;
@@ -645,15 +765,16 @@ cudaError_t sv_der_from_vectors(int n, int nvec, int per, int D, const cplx* T, 
     k_sv2_prep<<<nvec, 256, 0, st>>>(n, uv, w.ub, w.mcol);
     k_build_bordered<<<grid_len(nn2, nvec), 256, 0, st>>>(n, T, mat_stride, per, out, 3, w.ub, w.mcol, w.B);
     RS_CK(lu_factor_batched(n2, nvec, w.B, nn2, w.piv2, w.perm2, w.info2, st, &nl));
+    RS_CK(lu_diag_inv_batched(n2, nvec, w.B, nn2, w.dinv2, st));
     k_wapply<<<nvec, 256, 0, st>>>(n, T + der_stride, mat_stride, per, w.ub, w.ud, -1., 0);
-    RS_CK(lu_solve_batched(n2, nvec, 0, w.B, nn2, w.perm2, 1, w.ud, n2, st));
+    RS_CK(lu_solve_batched(n2, nvec, 0, w.B, nn2, w.perm2, w.dinv2, 1, w.ud, n2, st));
     k_sv2_extract<<<(nvec + 127) / 128, 128, 0, st>>>(n, nvec, w.ud, w.mcol, w.tb);
     k_wapply<<<nvec, 256, 0, st>>>(n, T + 2 * der_stride, mat_stride, per, w.ub, w.rhs, 1., 0);
     k_wapply<<<nvec, 256, 0, st>>>(n, T + der_stride, mat_stride, per, w.ud, w.rhs, 2., 1);
     k_sv2_axpy<<<nvec, 256, 0, st>>>(n, w.rhs, w.ud, w.tb);
-    RS_CK(lu_solve_batched(n2, nvec, 0, w.B, nn2, w.perm2, 1, w.rhs, n2, st));
+    RS_CK(lu_solve_batched(n2, nvec, 0, w.B, nn2, w.perm2, w.dinv2, 1, w.rhs, n2, st));
     k_sv2_out<<<(nvec + 127) / 128, 128, 0, st>>>(n, nvec, w.rhs, w.mcol, w.info2, out);
-    nl += 10;
+    nl += 11;
     return cudaGetLastError();
 }
 
@@ -668,6 +789,7 @@ size_t sv2_carve(int n, int nvec, int D, char* base, Sv2Work& w) {
     if (D < 2) return 0;
     const size_t nv = (size_t)nvec, nn = (size_t)n * n, c = sizeof(cplx), ii = sizeof(int);
     w.B = (cplx*)take(nv * 4 * nn * c);
+    w.dinv2 = (cplx*)take(nv * lu_dinv_elems(2 * n) * c);
     w.piv2 = (int*)take(nv * 2 * n * ii);
     w.perm2 = (int*)take(nv * 2 * n * ii);
     w.info2 = (int*)take(nv * ii);
@@ -682,8 +804,7 @@ size_t sv2_carve(int n, int nvec, int D, char* base, Sv2Work& w) {
 // Launchers shared with the block iteration of arnoldi.cu
 cudaError_t qr_global_batched(int n, int nmat, int s, cplx* X, long long xstride, cplx* Rf, cudaStream_t st) {
     if (s < 1 || s > kRsvdMaxS) return cudaErrorInvalidValue;
-    k_qr_global<<<nmat, kRsvdThreads, 0, st>>>(n, s, X, xstride, Rf);
-    return cudaGetLastError();
+    return launch_qr(n, nmat, s, X, xstride, Rf, st);
 }
 
 cudaError_t copy_mats_batched(long long nn, int nmat, const cplx* src, long long sstride, cplx* dst,
