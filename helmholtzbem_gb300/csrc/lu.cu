@@ -28,72 +28,115 @@ constexpr int kLuTile = 64;
 constexpr int kLuSolveThreads = 512;
 constexpr int kLuSolveChunk = 16;      // right-hand sides held in registers at a time
 
-// Unblocked LU of the panel rows [k0, n) x columns [k0, k0 + nb).  STAGED: the
-// panel is copied to shared memory (column-major, leading dimension n - k0), factored
-// there and written back; otherwise it is factored in place in global memory (L2).
+// Pivot candidates as integers: |x|^2 >= 0, so its bits order like its value, and an integer
+// comparison costs 2 cycles a warp where an FP64 one costs 76 (the comparisons of the search
+// were a third of a panel's time).  NaN counts as smaller than everything, as in a > best.
+struct PivotKey {
+    unsigned long long v;   // 0: no candidate; else 1 + the bits of |x|^2
+    int i;
+};
+__device__ __forceinline__ unsigned long long pivot_key(cplx z) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(norm2(z));
+    return b > 0x7ff0000000000000ull ? 0ull : b + 1;
+}
+__device__ __forceinline__ unsigned long long pivot_key(cplxf z) {
+    const unsigned b = __float_as_uint(norm2(z));
+    return b > 0x7f800000u ? 0ull : (unsigned long long)b + 1;
+}
+__device__ __forceinline__ void pivot_max(PivotKey& a, unsigned long long v, int i) {   // ties: the smaller index
+    if (v > a.v || (v == a.v && i < a.i)) { a.v = v; a.i = i; }
+}
+__device__ __forceinline__ PivotKey pivot_warp_max(PivotKey a) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long ov = __shfl_xor_sync(0xffffffffu, a.v, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, a.i, o);
+        pivot_max(a, ov, oi);
+    }
+    return a;
+}
+
+// Row i of the rank-1 update of a panel step, shared over the CTA: threads take (row, every
+// fourth column).  lcol: the scaled column.  rows [i0, i1) of the panel storage P (leading
+// dimension ld), columns j + 1 .. nb - 1.
+template <class E>
+__device__ __forceinline__ void panel_rank1(E* P, int ld, int i0, int i1, int j, int nb, const E* lcol, const E* prow) {
+    const int tr = threadIdx.x & 127, cg = threadIdx.x >> 7;
+    for (int i = i0 + tr; i < i1; i += 128) {
+        const E l = lcol[i];
+        for (int cc = j + 1 + cg; cc < nb; cc += kLuPanelThreads / 128) cfms(P[i + (long long)cc * ld], l, prow[cc]);
+    }
+}
+
+// Unblocked LU of the panel rows [k0, n) x columns [k0, k0 + nb), one CTA per matrix.
+// STAGED: the panel is copied to shared memory (column-major, leading dimension n - k0, the
+// scaled column behind it), factored there and written back; otherwise it is factored in
+// place in global memory (L2).
 template <class E, bool STAGED>
 __global__ void __launch_bounds__(kLuPanelThreads) k_lu_panel(int n, int k0, int nb, E* A, long long stride,
                                                               int* piv, int* info) {
     extern __shared__ double panel_sm[];
-    E* P = reinterpret_cast<E*>(panel_sm);
     E* M = A + (long long)blockIdx.x * stride;
     int* pv = piv + (long long)blockIdx.x * n;
     const int m = n - k0;
-    __shared__ double rv[32];
-    __shared__ int ri[32];
-    __shared__ E prow[kLuNB];
+    E* P = STAGED ? reinterpret_cast<E*>(panel_sm) : M + k0 + (long long)k0 * n;
+    const int ld = STAGED ? m : n;
+    E* lcol = STAGED ? P + (long long)m * nb : nullptr;
+    __shared__ PivotKey cand[kLuPanelThreads / 32];
+    __shared__ E prow[kLuNB], s_id;
     __shared__ int s_p;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    // element (row i, panel column cc)
-    auto at = [&](int i, int cc) -> E& {
-        return STAGED ? P[(i - k0) + cc * m] : M[i + (long long)(k0 + cc) * n];
-    };
     if (STAGED) {
         for (int e = threadIdx.x; e < m * nb; e += blockDim.x) P[e] = M[(k0 + e % m) + (long long)(k0 + e / m) * n];
         __syncthreads();
     }
     for (int j = 0; j < nb; ++j) {
-        const int c = k0 + j;
-        double best = -1.;
-        int bi = c;
-        for (int i = c + threadIdx.x; i < n; i += blockDim.x) {
-            const double a = norm2(at(i, j));
-            if (a > best) { best = a; bi = i; }
+        PivotKey best{0ull, j};
+        for (int i = j + threadIdx.x; i < m; i += blockDim.x) {
+            const unsigned long long a = pivot_key(P[i + (long long)j * ld]);
+            if (a > best.v) { best.v = a; best.i = i; }
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-        }
-        if (lane == 0) { rv[warp] = best; ri[warp] = bi; }
+        best = pivot_warp_max(best);
+        if (lane == 0) cand[warp] = best;
         __syncthreads();
-        if (threadIdx.x == 0) {
-            double b = rv[0];
-            int p = ri[0];
-            for (int w = 1; w < nw; ++w)
-                if (rv[w] > b || (rv[w] == b && ri[w] < p)) { b = rv[w]; p = ri[w]; }
-            s_p = p;
-            pv[c] = p;
-            if (b == 0. && info[blockIdx.x] == 0) info[blockIdx.x] = c + 1;
-        }
-        __syncthreads();
-        const int p = s_p;
-        if (threadIdx.x < nb) {
-            E& xa = at(c, threadIdx.x);
-            E& ya = at(p, threadIdx.x);
-            const E x = xa, y = ya;
-            if (p != c) { xa = y; ya = x; }
-            prow[threadIdx.x] = (p != c) ? y : x;
+        if (warp == 0) {
+            best = lane < nw ? cand[lane] : PivotKey{0ull, m};
+            best = pivot_warp_max(best);
+            if (lane == 0) {
+                if (best.v == 0ull) best.i = j;
+                s_p = best.i;
+                pv[k0 + j] = k0 + best.i;
+                if (best.v == 1ull && info[blockIdx.x] == 0) info[blockIdx.x] = k0 + j + 1;
+            }
+            __syncwarp();
+            const int p = s_p;
+            E y = Elem<E>::zero();
+            if (lane < nb) {
+                E& xa = P[j + (long long)lane * ld];
+                E& ya = P[p + (long long)lane * ld];
+                const E x = xa;
+                y = ya;
+                if (p != j) { xa = y; ya = x; }
+                prow[lane] = y;
+            }
+            if (lane == j) s_id = norm2(y) > 0 ? cdiv(Elem<E>::one(), y) : Elem<E>::one();   // zero pivot: unscaled
         }
         __syncthreads();
-        const E d = prow[j];
-        const bool nz = norm2(d) > 0;
-        const E id = nz ? cdiv(Elem<E>::one(), d) : Elem<E>::zero();
-        for (int i = c + 1 + threadIdx.x; i < n; i += blockDim.x) {
-            E l = at(i, j);
-            if (nz) { l = l * id; at(i, j) = l; }
-            for (int cc = j + 1; cc < nb; ++cc) cfms(at(i, cc), l, prow[cc]);
+        const E id = s_id;
+        if (STAGED) {
+            for (int i = j + 1 + threadIdx.x; i < m; i += blockDim.x) {
+                const E l = P[i + j * m] * id;
+                P[i + j * m] = l;
+                lcol[i] = l;
+            }
+            __syncthreads();
+            panel_rank1(P, m, j + 1, m, j, nb, lcol, prow);
+        } else {
+            for (int i = j + 1 + threadIdx.x; i < m; i += blockDim.x) {
+                const E l = P[i + (long long)j * ld] * id;
+                P[i + (long long)j * ld] = l;
+                for (int cc = j + 1; cc < nb; ++cc) cfms(P[i + (long long)cc * ld], l, prow[cc]);
+            }
         }
         __syncthreads();
     }
@@ -101,13 +144,13 @@ __global__ void __launch_bounds__(kLuPanelThreads) k_lu_panel(int n, int k0, int
         for (int e = threadIdx.x; e < m * nb; e += blockDim.x) M[(k0 + e % m) + (long long)(k0 + e / m) * n] = P[e];
 }
 
-// Panels too tall for one CTA's shared memory: a cluster of CS CTAs per matrix (grid
-// nmat * CS), CTA r holding panel rows [k0 + r R, k0 + (r + 1) R) in its shared memory
-// (column-major, leading dimension R).  Per column: every CTA posts its pivot
-// candidate, all read all candidates through distributed shared memory (cluster
-// barrier 1), every CTA copies the pivot row, the owner of the pivot row copies the
-// row it will receive (barrier 2), the two owners write the exchanged rows, and each
-// CTA applies the rank-1 update to its own rows.
+// The same on a cluster of CS CTAs per matrix (grid nmat * CS), CTA r holding panel rows
+// [k0 + r R, k0 + (r + 1) R) in its shared memory (column-major, leading dimension R): for
+// panels too tall for one CTA, and for few matrices because the FP64 rate of one SM bounds
+// the rank-1 updates.  Per column: every CTA posts its pivot candidate, all read all
+// candidates through distributed shared memory (cluster barrier 1), every CTA copies the
+// pivot row, the owner of the pivot row copies the row it will receive (barrier 2), the two
+// owners write the exchanged rows, and each CTA applies the rank-1 update to its own rows.
 template <class E>
 __global__ void __launch_bounds__(kLuPanelThreads) k_lu_panel_cluster(int n, int k0, int nb, int R, E* A,
                                                                       long long stride, int* piv, int* info) {
@@ -116,11 +159,9 @@ __global__ void __launch_bounds__(kLuPanelThreads) k_lu_panel_cluster(int n, int
     const int mat = blockIdx.x / ncta;
     extern __shared__ double panel_sm[];
     E* P = reinterpret_cast<E*>(panel_sm);
-    __shared__ double cand_v;
-    __shared__ int cand_i;
-    __shared__ double rv[32];
-    __shared__ int ri[32];
-    __shared__ E prow[kLuNB], tmp[kLuNB];
+    E* lcol = P + (long long)R * nb;
+    __shared__ PivotKey post, cand[kLuPanelThreads / 32];
+    __shared__ E prow[kLuNB], tmp[kLuNB], s_id;
     __shared__ int s_p;
     E* M = A + (long long)mat * stride;
     int* pv = piv + (long long)mat * n;
@@ -130,69 +171,58 @@ __global__ void __launch_bounds__(kLuPanelThreads) k_lu_panel_cluster(int n, int
         P[(e % rows) + (e / rows) * R] = M[(r0 + e % rows) + (long long)(k0 + e / rows) * n];
     __syncthreads();
     for (int j = 0; j < nb; ++j) {
-        const int c = k0 + j;
-        double best = -1.;
-        int bi = n;
-        for (int i = max(c, r0) + threadIdx.x; i < r1; i += blockDim.x) {
-            const double a = norm2(P[(i - r0) + j * R]);
-            if (a > best) { best = a; bi = i; }
+        const int c = k0 + j, first = max(c, r0) - r0;      // local index of the first row left
+        PivotKey best{0ull, n};
+        for (int i = first + threadIdx.x; i < rows; i += blockDim.x) {
+            const unsigned long long a = pivot_key(P[i + j * R]);
+            if (a > best.v) { best.v = a; best.i = r0 + i; }
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-        }
-        if (lane == 0) { rv[warp] = best; ri[warp] = bi; }
+        best = pivot_warp_max(best);
+        if (lane == 0) cand[warp] = best;
         __syncthreads();
-        if (threadIdx.x == 0) {
-            double b = rv[0];
-            int p = ri[0];
-            for (int w = 1; w < nw; ++w)
-                if (rv[w] > b || (rv[w] == b && ri[w] < p)) { b = rv[w]; p = ri[w]; }
-            cand_v = b;
-            cand_i = p;
+        if (warp == 0) {
+            best = lane < nw ? cand[lane] : PivotKey{0ull, n};
+            best = pivot_warp_max(best);
+            if (lane == 0) post = best;
         }
         cl.sync();                                                   // (1) candidates posted
-        if (threadIdx.x == 0) {
-            double b = -1.;
-            int p = n;
-            for (int q = 0; q < ncta; ++q) {
-                const double v = *cl.map_shared_rank(&cand_v, q);
-                const int i = *cl.map_shared_rank(&cand_i, q);
-                if (v > b || (v == b && i < p)) { b = v; p = i; }
+        if (warp == 0) {
+            best = lane < ncta ? *cl.map_shared_rank(&post, lane) : PivotKey{0ull, n};
+            best = pivot_warp_max(best);
+            if (best.v == 0ull) best.i = c;
+            const int p = best.i;
+            if (lane == 0) {
+                s_p = p;
+                if (rank == 0) {
+                    pv[c] = p;
+                    if (best.v == 1ull && info[mat] == 0) info[mat] = c + 1;
+                }
             }
-            s_p = p;
-            if (rank == 0) {
-                pv[c] = p;
-                if (b == 0. && info[mat] == 0) info[mat] = c + 1;
+            const int rp = (p - k0) / R, rc = (c - k0) / R;
+            E y = Elem<E>::zero();
+            if (lane < nb) {
+                y = cl.map_shared_rank(P, rp)[(p - (k0 + rp * R)) + lane * R];
+                prow[lane] = y;
+                if (rank == rp && p != c) tmp[lane] = cl.map_shared_rank(P, rc)[(c - (k0 + rc * R)) + lane * R];
             }
-        }
-        __syncthreads();
-        const int p = s_p;
-        const int rp = (p - k0) / R, rc = (c - k0) / R;
-        if (threadIdx.x < nb) {
-            const E* Pp = cl.map_shared_rank(P, rp);
-            prow[threadIdx.x] = Pp[(p - (k0 + rp * R)) + threadIdx.x * R];
-            if (rank == rp && p != c) {
-                const E* Pc = cl.map_shared_rank(P, rc);
-                tmp[threadIdx.x] = Pc[(c - (k0 + rc * R)) + threadIdx.x * R];
-            }
+            if (lane == j) s_id = norm2(y) > 0 ? cdiv(Elem<E>::one(), y) : Elem<E>::one();   // zero pivot: unscaled
         }
         cl.sync();                                                   // (2) rows c and p read
+        const int p = s_p, rp = (p - k0) / R, rc = (c - k0) / R;
         if (threadIdx.x < nb && p != c) {
             if (rank == rc) P[(c - r0) + threadIdx.x * R] = prow[threadIdx.x];
             if (rank == rp) P[(p - r0) + threadIdx.x * R] = tmp[threadIdx.x];
         }
         __syncthreads();
-        const E d = prow[j];
-        const bool nz = norm2(d) > 0;
-        const E id = nz ? cdiv(Elem<E>::one(), d) : Elem<E>::zero();
-        for (int i = max(c + 1, r0) + threadIdx.x; i < r1; i += blockDim.x) {
-            E l = P[(i - r0) + j * R];
-            if (nz) { l = l * id; P[(i - r0) + j * R] = l; }
-            for (int cc = j + 1; cc < nb; ++cc) cfms(P[(i - r0) + cc * R], l, prow[cc]);
+        const E id = s_id;
+        const int i0 = max(c + 1, r0) - r0;
+        for (int i = i0 + threadIdx.x; i < rows; i += blockDim.x) {
+            const E l = P[i + j * R] * id;
+            P[i + j * R] = l;
+            lcol[i] = l;
         }
+        __syncthreads();
+        panel_rank1(P, R, i0, rows, j, nb, lcol, prow);
         __syncthreads();
     }
     for (int e = threadIdx.x; e < rows * nb; e += blockDim.x)
@@ -781,11 +811,25 @@ cudaError_t launch_cgemm_f32(int m, int n, int k, const cplxf* A, long long lda,
                              long long ldb, long long sb, cplxf* C, long long ldc, long long sc, int nmat,
                              int use_tc, int* err, cudaStream_t st);
 
-// Cluster launch of the panel factorisation when the panel is too tall for one CTA.
-// Returns with *launched = false (nothing launched) when no cluster size up to 16
-// holds the panel or the device cannot co-schedule such a cluster.
+size_t panel_smem(int rows, int nb, size_t esz) { return (size_t)rows * (nb + 1) * esz; }
+
+// CTAs per matrix that a panel of m rows is best split over when nmat matrices share the
+// 152 SMs: as long as a CTA keeps enough rows that its share of the rank-1 updates is not
+// less than the two cluster barriers of a column (about 2 us; complex128: 64 rows, 16 columns
+// on average, 4 FMAs at two lanes a cycle: 2 us; complex64 is latency bound at any size).
 template <class E>
-cudaError_t launch_panel_cluster(int n, int k0, int nb, int nmat, E* A, long long stride, int* piv, int* info,
+int panel_split(int m, int nmat) {
+    const int least = std::is_same<E, cplx>::value ? 64 : 384;
+    int cs = 1;
+    while (cs < 16 && 2LL * cs * nmat <= 152 && m / (2 * cs) >= least) cs *= 2;
+    return cs;
+}
+
+// Cluster launch of the panel factorisation: when the panel is too tall for one CTA, or to
+// split it over `want` CTAs.  Returns with *launched = false (nothing launched) when no
+// cluster size up to 16 holds the panel or the device cannot co-schedule such a cluster.
+template <class E>
+cudaError_t launch_panel_cluster(int n, int k0, int nb, int nmat, E* A, long long stride, int* piv, int* info, int want,
                                  cudaStream_t st, bool* launched) {
     *launched = false;
     const int m = n - k0;
@@ -793,8 +837,8 @@ cudaError_t launch_panel_cluster(int n, int k0, int nb, int nmat, E* A, long lon
     size_t R = 0, smem = 0;
     for (; cs <= 16; cs *= 2, ++ci) {
         R = (m + cs - 1) / cs;
-        smem = R * nb * sizeof(E);
-        if (smem <= kPanelClusterSmem) break;
+        smem = panel_smem((int)R, nb, sizeof(E));
+        if (smem <= kPanelClusterSmem && cs >= want) break;
     }
     if (cs > 16 || (long long)nmat * cs > 0x7fffffffLL) return cudaSuccess;
     static int ok[4] = {-1, -1, -1, -1};     // per cluster size 2, 4, 8, 16: unknown / no / yes
@@ -848,19 +892,23 @@ cudaError_t lu_factor_impl(int n, int nmat, E* A, long long stride, int* piv, in
     const int ncb = (n + kLuNB - 1) / kLuNB;
     // one 32-column panel: factor, exchange and solve the columns below cmax, update
     // the trailing columns below cend
-    auto panel_step = [&](int k0, int nb, int cmax, int cend) -> cudaError_t {
-        const size_t psm = (size_t)(n - k0) * nb * sizeof(E);
-        if (psm <= kLuSmemLimit) {
-            k_lu_panel<E, true><<<nmat, kLuPanelThreads, psm, st>>>(n, k0, nb, A, stride, piv, info);
-        } else {
-            bool launched = false;
-            if (g_lu_cluster_panels) {
-                cudaError_t e2 = launch_panel_cluster<E>(n, k0, nb, nmat, A, stride, piv, info, st, &launched);
+    auto panel = [&](int k0, int nb) -> cudaError_t {
+        const size_t psm = panel_smem(n - k0, nb, sizeof(E));
+        const bool fits = psm <= kLuSmemLimit;
+        bool launched = false;
+        if (g_lu_cluster_panels)
+            for (int want = panel_split<E>(n - k0, nmat); !launched && (want > 1 || !fits); want /= 2) {
+                cudaError_t e2 = launch_panel_cluster<E>(n, k0, nb, nmat, A, stride, piv, info, want, st, &launched);
                 if (e2 != cudaSuccess) return e2;
+                if (want <= 1) break;
             }
-            if (!launched) k_lu_panel<E, false><<<nmat, kLuPanelThreads, 0, st>>>(n, k0, nb, A, stride, piv, info);
-        }
+        if (!launched && fits) k_lu_panel<E, true><<<nmat, kLuPanelThreads, psm, st>>>(n, k0, nb, A, stride, piv, info);
+        else if (!launched) k_lu_panel<E, false><<<nmat, kLuPanelThreads, 0, st>>>(n, k0, nb, A, stride, piv, info);
         ++nl;
+        return cudaGetLastError();
+    };
+    auto panel_step = [&](int k0, int nb, int cmax, int cend) -> cudaError_t {
+        if (cudaError_t e2 = panel(k0, nb); e2 != cudaSuccess) return e2;
         if (ncb > 1) {
             k_lu_swap_trsm<E><<<dim3(ncb, nmat), 256, 0, st>>>(n, k0, nb, A, stride, piv, cmax);
             ++nl;
@@ -908,18 +956,8 @@ cudaError_t lu_factor_impl(int n, int nmat, E* A, long long stride, int* piv, in
     } else {
         for (int k0 = 0; k0 < n; k0 += kLuNB) {
             const int nb = min(kLuNB, n - k0);
-            const size_t psm = (size_t)(n - k0) * nb * sizeof(E);
-            if (psm <= kLuSmemLimit) {
-                k_lu_panel<E, true><<<nmat, kLuPanelThreads, psm, st>>>(n, k0, nb, A, stride, piv, info);
-            } else {
-                bool launched = false;
-                if (g_lu_cluster_panels) {
-                    e = launch_panel_cluster<E>(n, k0, nb, nmat, A, stride, piv, info, st, &launched);
-                    if (e != cudaSuccess) return e;
-                }
-                if (!launched) k_lu_panel<E, false><<<nmat, kLuPanelThreads, 0, st>>>(n, k0, nb, A, stride, piv, info);
-            }
-            ++nl;
+            e = panel(k0, nb);
+            if (e != cudaSuccess) return e;
             if (ncb > 1) {
                 k_lu_swap_trsm<E><<<dim3(ncb, nmat), 256, 0, st>>>(n, k0, nb, A, stride, piv, n);
                 ++nl;
