@@ -13,7 +13,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "_lib")
 LIB = os.path.join(OUT_DIR, "libhbem.so")
-SOURCES = ["assemble.cu", "hankel_u.cu", "solop.cu", "dense.cu", "lu.cu", "tc_gemm.cu", "rsvd.cu", "arnoldi.cu", "capi.cu", "roots.cu",
+SOURCES = ["assemble.cu", "hankel_u.cu", "solop.cu", "dense.cu", "lu.cu", "tc_gemm.cu", "zgemm_tc.cu", "rsvd.cu", "arnoldi.cu", "capi.cu", "roots.cu",
            "scatterer.cpp", "fields.cu", "mlp.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 # Host code: no floating-point contraction, so that x86-64 and aarch64 hosts (where

@@ -25,6 +25,7 @@ namespace hbem {
 constexpr int kLuNB = 32;
 constexpr int kLuPanelThreads = 512;
 constexpr int kLuTile = 64;
+constexpr int kLuTcMin = 128;            // smallest trailing order the complex128 tensor-core update takes
 constexpr int kLuSolveThreads = 512;
 constexpr int kLuSolveChunk = 16;      // right-hand sides held in registers at a time
 
@@ -825,6 +826,9 @@ int panel_split(int m, int nmat) {
     return cs;
 }
 
+cudaError_t launch_zgemm_tc(int m, int n, int k, const cplx* A, long long lda, long long sa, const cplx* B, long long ldb,
+                            long long sb, cplx* C, long long ldc, long long sc, int nmat, cudaStream_t st);
+
 // Cluster launch of the panel factorisation: when the panel is too tall for one CTA, or to
 // split it over `want` CTAs.  Returns with *launched = false (nothing launched) when no
 // cluster size up to 16 holds the panel or the device cannot co-schedule such a cluster.
@@ -972,6 +976,16 @@ cudaError_t lu_factor_impl(int n, int nmat, E* A, long long stride, int* piv, in
                         const int t0 = k0 + nb;
                         e = launch_cgemm_f32(m, m, nb, A + t0 + (long long)k0 * n, n, stride, A + k0 + (long long)t0 * n,
                                              n, stride, A + t0 + (long long)t0 * n, n, stride, nmat, 1, tc_err, st);
+                        if (e != cudaSuccess) return e;
+                        done = true;
+                    }
+                }
+                if constexpr (std::is_same<E, cplx>::value) {
+                    // complex128: the same as exact BF16 digit products (zgemm_tc.cu)
+                    if (g_lu_tensor_cores && m >= kLuTcMin) {
+                        const int t0 = k0 + nb;
+                        e = launch_zgemm_tc(m, m, nb, A + t0 + (long long)k0 * n, n, stride, A + k0 + (long long)t0 * n, n,
+                                            stride, A + t0 + (long long)t0 * n, n, stride, nmat, st);
                         if (e != cudaSuccess) return e;
                         done = true;
                     }
