@@ -377,8 +377,9 @@ __global__ void k_flags_singular(DevMesh M, const SingularTask* tasks, uint8_t* 
 //   * every kernel value is f, g, |v|^2 f or |v|^2 g up to factors of the job, and along b
 //     only two moments of each are needed (weights w_b and w_b y_b); the powers of x_a and
 //     the factors of node a enter once per row.  On straight panels v x tau_j does not
-//     depend on b, so the double layer shares the sums of the single layer.
-// At order 2 that is 58 FP64 instructions on lines and 84 on arcs where a thread per pair
+//     depend on b and tau_i x v is linear in y_b, so both double layers come from the plain
+//     sums, with a third moment in y.
+// At order 2 that is 48 FP64 instructions on lines and 84 on arcs where a thread per pair
 // with the four moments per kernel value, the distance and the branches of
 // hankel01_real took about 230 and 300.
 // The rows' sums are then combined through shared memory: 2 p instructions per value.
@@ -474,13 +475,18 @@ __device__ __forceinline__ void general_rows(const DevMesh& M, const KConst& K, 
         const cplx* ptj = M.gpt + j * p;
         const cplx* tgj = M.gtan + j * p;
         const double* tnj = M.gtn + j * p;
-        cplx S[F][2], L[CURVED ? F : 1][2], T[F][2], W[CURVED ? F : 1][2];
+        // S, T, L, W: row sums of the sets (curved: two powers of y each).  Straight panels:
+        // tau_i x v is linear in y, so T comes from S and G (g) with a third power of y.
+        constexpr int P = CURVED ? 2 : 3;
+        cplx S[F][P], Gs[P], L[CURVED ? F : 1][2], T[CURVED ? F : 1][2], W[CURVED ? F : 1][2];
 #pragma unroll
-        for (int t = 0; t < F; ++t) {
-            S[t][0] = S[t][1] = T[t][0] = T[t][1] = mk(0.);
-            if (CURVED || t == 0) L[CURVED ? t : 0][0] = L[CURVED ? t : 0][1] = mk(0.);
-            if (CURVED) W[CURVED ? t : 0][0] = W[CURVED ? t : 0][1] = mk(0.);
+        for (int h = 0; h < P; ++h) {
+            Gs[h] = mk(0.);
+#pragma unroll
+            for (int t = 0; t < F; ++t) S[t][h] = mk(0.);
         }
+#pragma unroll
+        for (int t = 0; t < (CURVED ? F : 1); ++t) L[t][0] = L[t][1] = T[t][0] = T[t][1] = W[t][0] = W[t][1] = mk(0.);
         for (int b = 0; b < p; ++b) {
             const cplx v = xi - ptj[b];
             const double v2 = norm2(v);
@@ -489,24 +495,28 @@ __device__ __forceinline__ void general_rows(const DevMesh& M, const KConst& K, 
             const double w = sw[b], y = sx[b], wy = sw[p + b];   // sw[p + b] = w_b y_b
             const cplx vg = D > 0 ? v2 * g : mk(0.), vf = D > 1 ? v2 * f : mk(0.);
             const cplx ks[3] = {f, vg, vf}, kd[3] = {g, f, vg};
-#pragma unroll
-            for (int t = 0; t < F; ++t) row_add(S[t], w, wy, ks[t]);
-            const double ct = v.im * ti.re - v.re * ti.im;       // tau_i x v
-            if (CURVED) {
+            if constexpr (CURVED) {
                 const cplx tj = tgj[b];
-                const double wt = w * tnj[b] * ct, wd = w * (v.re * tj.im - v.im * tj.re);
-                const double wc = w * (ti.im * tj.im + ti.re * tj.re);
+                const double wt = w * tnj[b] * (v.im * ti.re - v.re * ti.im);   // tau_i x v
+                const double wd = w * (v.re * tj.im - v.im * tj.re), wc = w * (ti.im * tj.im + ti.re * tj.re);
 #pragma unroll
                 for (int t = 0; t < F; ++t) {
+                    row_add(S[t], w, wy, ks[t]);
                     row_add(T[t], wt, wt * y, kd[t]);
-                    row_add(L[CURVED ? t : 0], wd, wd * y, kd[t]);
-                    row_add(W[CURVED ? t : 0], wc, wc * y, ks[t]);
+                    row_add(L[t], wd, wd * y, kd[t]);
+                    row_add(W[t], wc, wc * y, ks[t]);
                 }
             } else {
-                const double wt = w * ct, wty = wy * ct;
+                const double wy2 = sw[2 * p + b];            // w_b y_b^2
 #pragma unroll
-                for (int t = 0; t < F; ++t) row_add(T[t], wt, wty, kd[t]);
-                row_add(L[0], w, wy, g);
+                for (int t = 0; t < F; ++t) {
+                    axpy(S[t][0], w, ks[t]);
+                    axpy(S[t][1], wy, ks[t]);
+                    if (t < 2) axpy(S[t][P - 1], wy2, ks[t]);   // v2 f is not in the double layers
+                }
+                axpy(Gs[0], w, g);
+                axpy(Gs[1], wy, g);
+                axpy(Gs[P - 1], wy2, g);
             }
         }
         // the factors of node a; a pair whose geometric factor vanishes at every point (the
@@ -516,6 +526,9 @@ __device__ __forceinline__ void general_rows(const DevMesh& M, const KConst& K, 
         const double fd = (fl & PF_DL0_ZERO) ? 0. : CURVED ? wa * tin : wa * tin * (v0.re * t0j.im - v0.im * t0j.re);
         const double ft = (fl & PF_DLT0_ZERO) ? 0. : CURVED ? wa : wa * tnj[0];
         const double fw = (fl & PF_TDT0_ZERO) ? 0. : 2. * wa;
+        // straight: tau_i x v = c0 + c1 y, y = gamma_j(0) + y tau_j
+        const double c1 = ft * (t0j.re * ti.im - t0j.im * ti.re);
+        const double c0 = fma(-c1, sx[0], ft * (v0.im * ti.re - v0.re * ti.im));
         cplx* r = rows + threadIdx.x;
 #pragma unroll
         for (int t = 0; t < F; ++t)
@@ -523,25 +536,34 @@ __device__ __forceinline__ void general_rows(const DevMesh& M, const KConst& K, 
             for (int h = 0; h < 2; ++h) {
                 const int e = 2 * t + h;
                 r[e * G::THREADS] = wa * S[t][h];
-                r[(2 * F + e) * G::THREADS] = fd * (CURVED ? L[CURVED ? t : 0][h] : t == 0 ? L[0][h] : S[t > 0 ? t - 1 : 0][h]);
-                r[(4 * F + e) * G::THREADS] = ft * T[t][h];
-                if (CURVED) r[(6 * F + e) * G::THREADS] = fw * W[CURVED ? t : 0][h];
+                if constexpr (CURVED) {
+                    r[(2 * F + e) * G::THREADS] = fd * L[t][h];
+                    r[(4 * F + e) * G::THREADS] = ft * T[t][h];
+                    r[(6 * F + e) * G::THREADS] = fw * W[t][h];
+                } else {
+                    const cplx* k = t == 0 ? Gs : S[t > 0 ? t - 1 : 0];
+                    r[(2 * F + e) * G::THREADS] = fd * k[h];
+                    cplx z = c0 * k[h];
+                    axpy(z, c1, k[h + 1]);
+                    r[(4 * F + e) * G::THREADS] = z;
+                }
             }
     }
     __syncthreads();
     const int npairs = (int)(M.ngen - q0 < ppc ? M.ngen - q0 : ppc);
-    for (int it = threadIdx.x; it < npairs * G::NV; it += G::THREADS) {
-        const int e = it / npairs, l = it - e * npairs;
-        const cplx* r = rows + e * G::THREADS + l * p;
-        cplx m0 = mk(0.), m1 = mk(0.);
-        for (int c = 0; c < p; ++c) {
-            const cplx z = r[c];
+    // a thread per (value, pair, real or imaginary part): even rounds of the CTA
+    for (int it = threadIdx.x; it < npairs * G::NV * 2; it += G::THREADS) {
+        const int c = it & 1, el = it >> 1, e = el / npairs, l = el - e * npairs;
+        const double* r = reinterpret_cast<const double*>(rows + e * G::THREADS + l * p) + c;
+        double m0 = 0., m1 = 0.;
+        for (int q = 0; q < p; ++q) {
+            const double z = r[2 * q];
             m0 += z;
-            axpy(m1, sx[c], z);
+            m1 = fma(sx[q], z, m1);
         }
-        cplx* m = mom + ((long long)l * (G::NV / 2) + (e >> 1)) * 4 + 2 * (e & 1);
+        double* m = reinterpret_cast<double*>(mom + ((long long)l * (G::NV / 2) + (e >> 1)) * 4 + 2 * (e & 1)) + c;
         m[0] = m0;
-        m[1] = m1;
+        m[2] = m1;
     }
     __syncthreads();
     // the pair's blocks: 4 kinds x 4 shape-function pairs, the kind slowest so that a warp
@@ -558,20 +580,21 @@ __device__ __forceinline__ void general_rows(const DevMesh& M, const KConst& K, 
     }
 }
 
-// the Gauss nodes sx[p] and weights sw[p], w_b x_b behind the weights
+// the Gauss nodes sx[p] and weights sw[p], w_b x_b and w_b x_b^2 behind the weights
 __device__ __forceinline__ void load_rule(const DevMesh& M, double* sx, double* sw) {
     for (int t = threadIdx.x; t < M.p; t += blockDim.x) {
         const double x = M.xg[t], w = M.wg[t];
         sx[t] = x;
         sw[t] = w;
         sw[M.p + t] = w * x;
+        sw[2 * M.p + t] = w * x * x;
     }
 }
 
 template <int D, bool CURVED>
 __global__ void __launch_bounds__(128, 2) k_general(DevMesh M, const Job* jobs, cplx* loc, long long npair) {
     extern __shared__ __align__(16) unsigned char gsm[];
-    __shared__ double sx[32], sw[64];
+    __shared__ double sx[32], sw[96];
     load_rule(M, sx, sw);
     __syncthreads();
     const int job = blockIdx.y;
@@ -975,7 +998,7 @@ __global__ void __launch_bounds__(128, 2) k_general_multi(const MultiMesh* meshe
                                                           const long long* start, int njobs, cplx* loc) {
     extern __shared__ __align__(16) unsigned char gsm[];
     __shared__ DevMesh sM;
-    __shared__ double sx[32], sw[64];
+    __shared__ double sx[32], sw[96];
     __shared__ int sjob;
     if (threadIdx.x == 0) {
         sjob = job_of_block(start, njobs, blockIdx.x);
@@ -1010,13 +1033,14 @@ __global__ void __launch_bounds__(128, 2) k_singular_multi(const MultiMesh* mesh
     cplx* mom = acc + R::NA * 128;
     double* sxc = reinterpret_cast<double*>(mom + R::NA);
     double* swc = sxc + sM.nc;
+    double* sz = swc + sM.nc;
     const MultiJob J = jobs[sjob];
     const KConst K = make_kconst(J.job);
     const SingularTask T = sT;
     if (nodes_serve(sM, (int)(blockIdx.x - start[sjob]), K)) return;   // whole CTA
-    load_composite(sM, sxc, swc);
+    load_composite(sM, T.kind == PK_COINC, sxc, swc, sz);
     __syncthreads();
-    singular_moments<D, CURVED>(sM, T, K, 0, 1, sxc, swc, acc, mom);
+    singular_moments<D, CURVED>(sM, T, K, 0, 1, sxc, swc, sz, acc, mom);
     singular_store<D, CURVED>(sM, T, K, mom, threadIdx.x, 128,
                               loc + J.loc + tri_index(T.i, T.j) * (D + 1) * kLocPerD);
 }
@@ -1253,7 +1277,7 @@ static cudaError_t launch_local_c(const DevMesh& M, const SingularTask* tasks, i
     const int q = (part && (which & 2)) ? singular_parts(ntasks, njobs) : 0;
     const bool rows = (which & 2) && ntasks > 0 && (!RK || !M.snode || (which & 4));
     constexpr int NV = (int)(sizeof(Acc<D, CURVED>) / sizeof(double));
-    const size_t ssmem = RK ? RowDims<D, CURVED>::kSmem + 2 * (size_t)M.nc * sizeof(double)
+    const size_t ssmem = RK ? RowDims<D, CURVED>::kSmem + 3 * (size_t)M.nc * sizeof(double)
                             : (2 * (size_t)M.nc + 4 * NV) * sizeof(double);
     if (rows && RK) {
         if (cudaError_t e = allow_smem(k_singular_rows<D, CURVED>, ssmem); e != cudaSuccess) return e;
@@ -1355,7 +1379,7 @@ static cudaError_t launch_multi_c(const MultiMesh* meshes, const MultiJob* jobs,
         k_general_multi<D, CURVED><<<(unsigned)gblocks, 128, smem, st>>>(meshes, jobs, gstart, njobs, loc);
     }
     if (sblocks > 0) {
-        const size_t smem = RowDims<D, CURVED>::kSmem + 2 * (size_t)max_nc * sizeof(double);
+        const size_t smem = RowDims<D, CURVED>::kSmem + 3 * (size_t)max_nc * sizeof(double);
         if (cudaError_t e = allow_smem(k_singular_multi<D, CURVED>, smem); e != cudaSuccess) return e;
         k_singular_multi<D, CURVED><<<(unsigned)sblocks, 128, smem, st>>>(meshes, jobs, sstart, njobs, loc);
     }

@@ -15,9 +15,9 @@
 //   against the nodes' Lagrange polynomials, plain and times log(|v|/s) -- do not depend on the
 //   wavenumber: they are made once per builder (k_snode_part, k_snode_join).  Order 11: 16
 //   node values instead of 4225 or 8450 points.
-// * k_singular_rows, for everything else: the points themselves.  A thread takes a
-//   contiguous part of the points in rows of one outer node; f and g come from the Hankel
-//   table, and along a row two moments per kernel value are enough (see k_general).
+// * k_singular_rows, for everything else: the points themselves.  A thread takes pieces of
+//   the rows of one outer node; f and g come from the Hankel table, and along a row two
+//   moments per kernel value are enough (see k_general).
 #pragma once
 
 namespace hbem {
@@ -113,15 +113,30 @@ struct RowDims {
     static constexpr size_t kSmem = ((size_t)NA * 128 + NA) * sizeof(cplx);
 };
 
-// Moments of part `sub` of `nparts` equal parts of a pair's points, reduced over the CTA
-// (128 threads) into mom[NA] (shared memory).  acc: NA x 128 entries.
+// Pieces a row of nc inner nodes is cut into so that `rows` rows fill rounds of 128 threads:
+// the threads of a warp take pieces of equal length (a run of points per thread, whose rows
+// ended at different steps in every lane, left a warp idle 40 % of its issue slots).  A
+// piece costs its points (about 45 FP64 instructions) and one fold (about 50).
+__device__ __forceinline__ int row_pieces(int rows, int nc) {
+    int best = 1, cost = 0x7fffffff;
+    for (int c = 1; c <= 16 && c <= nc; ++c) {
+        const int t = (rows * c + 127) / 128 * ((nc + c - 1) / c * 45 + 50);
+        if (t < cost) { cost = t; best = c; }
+    }
+    return best;
+}
+
+// Moments of part `sub` of `nparts` equal parts of a pair's rows, reduced over the CTA
+// (128 threads) into mom[NA] (shared memory).  acc: NA x 128 entries; sz: the composite nodes z
+// (adjacent pairs) or 1 - z (coincident ones).
 template <int D, bool CURVED>
 __device__ __forceinline__ void singular_moments(const DevMesh& M, const SingularTask& T, const KConst& K, int sub,
-                                                 int nparts, const double* sxc, const double* swc, cplx* acc,
-                                                 cplx* mom) {
+                                                 int nparts, const double* sxc, const double* swc, const double* sz,
+                                                 cplx* acc, cplx* mom) {
     typedef RowDims<D, CURVED> R;
     constexpr int F = R::F;
-    const int nc = M.nc, tot = nc * nc, nset = T.kind == PK_COINC ? 1 : 2;
+    const bool coinc = T.kind == PK_COINC;
+    const int nc = M.nc, nrows = (coinc ? 1 : 2) * nc;
     const uint8_t fl = M.flags[tri_index(T.i, T.j)];
     const double ks2 = K.ks.re * K.ks.re;
     PMap mi, mj;
@@ -129,16 +144,11 @@ __device__ __forceinline__ void singular_moments(const DevMesh& M, const Singula
     cplx* A = acc + threadIdx.x;
 #pragma unroll
     for (int e = 0; e < R::NA; ++e) A[e * 128] = mk(0.);
-    const long long W = (long long)nset * tot, c0 = W * sub / nparts, c1 = W * (sub + 1) / nparts;
-    int w = (int)(c0 + (c1 - c0) * threadIdx.x / 128);
-    const int w1 = (int)(c0 + (c1 - c0) * (threadIdx.x + 1) / 128);
-    while (w < w1) {
-        const int row = w / nc, K0 = row >= nc ? 1 : 0, a = row - K0 * nc;
-        int z = w - row * nc;
-        const int z1 = min(nc, z + (w1 - w));
-        w += z1 - z;
+    const int ra = nrows * sub / nparts, rb = nrows * (sub + 1) / nparts, pieces = row_pieces(rb - ra, nc);
+    for (int it = ra * pieces + threadIdx.x; it < rb * pieces; it += 128) {
+        const int row = it / pieces, piece = it - row * pieces, K0 = row >= nc ? 1 : 0, a = row - K0 * nc;
+        const int z0 = nc * piece / pieces, z1 = nc * (piece + 1) / pieces;
         const double t = sxc[a], wt = t * swc[a];
-        const bool coinc = T.kind == PK_COINC;
         // coincident: x = s moves on panel i, y = t; adjacent set 0 likewise, set 1: x = t, y = s
         const bool move_i = coinc || K0 == 0;
         const PMap& mm = move_i ? mi : mj;
@@ -153,12 +163,10 @@ __device__ __forceinline__ void singular_moments(const DevMesh& M, const Singula
             S[q][0] = S[q][1] = L[q][0] = L[q][1] = B[q][0] = B[q][1] = mk(0.);
             if (CURVED) Wc[CURVED ? q : 0][0] = Wc[CURVED ? q : 0][1] = mk(0.);
         }
-        for (; z < z1; ++z) {
-            const double xz = sxc[z], wz = swc[z], s = coinc ? t * (1. - xz) : t * xz, ws = wz * s;
+        for (int z = z0; z < z1; ++z) {
+            const double wz = swc[z], s = t * sz[z], ws = wz * s;
             cplx tm;
-            const cplx pm = pmap_at(mm, s, tm);
-            const cplx v = move_i ? pm - pfix : pfix - pm;
-            const cplx ti = move_i ? tm : tfix, tj = move_i ? tfix : tm;
+            const cplx v = pmap_at(mm, s, tm) - pfix;          // minus gamma_i - gamma_j when panel j moves
             const double v2 = norm2(v);
             cplx f, g;
             hk_pair(M.hk, ks2 * v2, f, g);
@@ -167,23 +175,27 @@ __device__ __forceinline__ void singular_moments(const DevMesh& M, const Singula
 #pragma unroll
             for (int q = 0; q < F; ++q) row_add(S[q], wz, ws, kf[q]);
             if (uw) {
-                const double d = ti.im * tj.im + ti.re * tj.re;
+                const double d = tm.im * tfix.im + tm.re * tfix.re;
 #pragma unroll
                 for (int q = 0; q < F; ++q) row_add(Wc[CURVED ? q : 0], wz * d, ws * d, kf[q]);
             }
+            // with v as it is here: L collects v x (fixed or moving tangent of panel j), B the
+            // tangent of panel i x v; the sign of v goes into the fold
             if (ua) {
+                const cplx tj = move_i ? tfix : tm;
                 const double d = v.re * tj.im - v.im * tj.re;
 #pragma unroll
                 for (int q = 0; q < F; ++q) row_add(L[q], wz * d, ws * d, kd[q]);
             }
             if (ub) {
+                const cplx ti = move_i ? tm : tfix;
                 const double d = v.im * ti.re - v.re * ti.im;
 #pragma unroll
                 for (int q = 0; q < F; ++q) row_add(B[q], wz * d, ws * d, kd[q]);
             }
         }
         // the row's two moments into the four of the pair (moments 1, x, y, xy)
-        const double tin = mi.tn, tjn = mj.tn;
+        const double sg = move_i ? wt : -wt, tin = sg * mi.tn, tjn = sg * mj.tn;
         auto fold = [&](int set, int q, const cplx (&r)[2], double c, bool s_is_x) {
             cplx* m = A + ((set * F + q) * 4) * 128;
             const cplx r0 = c * r[0], r1 = c * r[1];
@@ -200,8 +212,8 @@ __device__ __forceinline__ void singular_moments(const DevMesh& M, const Singula
                 fold(CURVED ? 3 : 0, q, Wc[CURVED ? q : 0], 2. * wt, K0 == 0);
                 if (coinc) fold(CURVED ? 3 : 0, q, Wc[CURVED ? q : 0], 2. * wt, false);
             }
-            if (ua) fold(1, q, L[q], wt * tin, K0 == 0);
-            if (ub) fold(coinc ? 1 : 2, q, B[q], wt * tjn, !coinc && K0 == 0);
+            if (ua) fold(1, q, L[q], tin, K0 == 0);
+            if (ub) fold(coinc ? 1 : 2, q, B[q], tjn, !coinc && K0 == 0);
         }
     }
     __syncthreads();
@@ -233,10 +245,12 @@ __device__ __forceinline__ bool nodes_serve(const DevMesh& M, int ti, const KCon
     return K.ks.re * K.ks.re * d2 <= kSNodeX * kSNodeX;
 }
 
-__device__ __forceinline__ void load_composite(const DevMesh& M, double* sxc, double* swc) {
+__device__ __forceinline__ void load_composite(const DevMesh& M, bool coinc, double* sxc, double* swc, double* sz) {
     for (int t = threadIdx.x; t < M.nc; t += blockDim.x) {
-        sxc[t] = M.xc[t];
+        const double x = M.xc[t];
+        sxc[t] = x;
         swc[t] = M.wc[t];
+        sz[t] = coinc ? 1. - x : x;
     }
 }
 
@@ -251,15 +265,16 @@ __global__ void __launch_bounds__(128, 2) k_singular_rows(DevMesh M, const Singu
     cplx* mom = acc + R::NA * 128;
     double* sxc = reinterpret_cast<double*>(mom + R::NA);
     double* swc = sxc + M.nc;
+    double* sz = swc + M.nc;
     const int job = blockIdx.y;
     const int task = q ? blockIdx.x / (2 * q) : blockIdx.x, sub = q ? blockIdx.x - task * 2 * q : 0;
     const SingularTask T = tasks[task];
     const int nparts = q ? (T.kind == PK_COINC ? q : 2 * q) : 1;
     const KConst K = make_kconst(jobs[job]);
     if (sub >= nparts || nodes_serve(M, task, K)) return;   // whole CTA, before any barrier
-    load_composite(M, sxc, swc);
+    load_composite(M, T.kind == PK_COINC, sxc, swc, sz);
     __syncthreads();
-    singular_moments<D, CURVED>(M, T, K, sub, nparts, sxc, swc, acc, mom);
+    singular_moments<D, CURVED>(M, T, K, sub, nparts, sxc, swc, sz, acc, mom);
     if (q) {
         cplx* dst = reinterpret_cast<cplx*>(part) + ((long long)job * gridDim.x + blockIdx.x) * R::NA;
         for (int e = threadIdx.x; e < R::NA; e += 128) dst[e] = mom[e];
