@@ -188,28 +188,26 @@ __global__ void __launch_bounds__(kArnThreads) k_arn_small(ArnJob J) {
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) A[e] = T0[e];
     for (int e = threadIdx.x; e < n * p; e += blockDim.x) X[e] = arn_start(J.seed, e % n, e / n);
     __syncthreads();
-    lu_smem(A, n, piv, &s_sing, buf);
+    lu_smem(A, n, piv, &s_sing);
     __syncthreads();
     if (s_sing) {
         arn_fail(J, mat, 5);
         return;
     }
     perm_from_piv(piv, n, perm);
-    // U's diagonal replaced by its reciprocals: the solves multiply
-    for (int k = threadIdx.x; k < n; k += blockDim.x) A[k + (long long)k * n] = cdiv(mk(1.), A[k + (long long)k * n]);
-    __syncthreads();
-    solve_lu_blk(A, perm, n, X, p, buf, nullptr, true);
+    lu_inv_diag(A, n);
+    solve_lu_blk(A, perm, n, X, p, buf);
     qr_cgs2(X, n, p, coef, red);
     int it = 1;
     bool conv = false;
     for (;; ++it) {
         for (int e = threadIdx.x; e < n * p; e += blockDim.x) Y[e] = X[e];
         __syncthreads();
-        solve_lu_h_blk(A, perm, n, Y, p, buf, nullptr, true);
+        solve_lu_h_blk(A, perm, n, Y, p, buf);
         qr_cgs2(Y, n, p, coef, red, Rs);
         __syncthreads();
         arn_ritz(Rs, W, p, J.count, nrm, ord, &s_rot);
-        solve_lu_blk(A, perm, n, Y, p, buf, nullptr, true);
+        solve_lu_blk(A, perm, n, Y, p, buf);
         __syncthreads();
         conv = arn_converged(X, Y, n, p, Rs, W, nrm, ord, J.count, J.tol, red);
         if (conv || it >= J.maxit) break;

@@ -60,26 +60,36 @@ __device__ __forceinline__ float warp_sumf(float x) {
     return x;
 }
 
-// Stage 1 of the mixed-precision path: one-sided Jacobi of T in FP32 (A32 and V32
-// both in shared memory), to the FP32 noise level.  Only V32 is used afterwards.
-// Each column pair of a round-robin step is handled by a group of G lanes (G = 8 for
-// n <= 128: the 64 groups of a 512-thread CTA take a whole step at once, with
-// 3-level shuffle reductions), G = 32 for larger n.
+// Stage 1 of the mixed-precision paths: one-sided Jacobi of T in FP32 (A32 and V32, leading
+// dimension ld, both in shared memory), to the FP32 noise level; n <= 8 NQ.  Each column pair
+// of a round-robin step is handled by a group of 8 lanes (the 64 groups of a 512-thread CTA
+// take a whole step at once, with 3-level shuffle reductions).  A step moves both columns of
+// every pair through shared memory and that bounds it (n = 100: 320 KB, 2500 cycles of an SM's
+// 128 B a cycle), so the columns are read once, into registers, for the inner products and the
+// rotation, and ld keeps the groups of a warp on different banks.  With the FP64 stage's shorter
+// chains (one warp per norm, look-ahead LU, half-warps in the Ritz step's rotations) k_svd_fast
+// went from 7.80 to 5.70 ms for 100 matrices of n = 96 and from 2.24 to 1.79 ms for n = 50;
+// every operation and its order are as they were.  (Sweeps on the triangular factor of a
+// pivoted QR instead take half the time of this stage, but leave other FP32 noise in the start
+// block, which reaches sigma' and sigma'' at nearly degenerate matrices, where the inverse
+// iterations' count is capped: 1.25 times the error on average.)
 //
 // Warm start (Vw != null, n x n unitary to FP32 working precision, typically the V32
 // of a nearby wavenumber): the sweeps start from A = T Vw, V = Vw instead of A = T,
 // V = I.  The stopping rule is the same, so the result has the cold start's accuracy;
 // when T Vw is nearly column-orthogonal far fewer sweeps are needed.  rowbuf: one row
 // of n entries per warp (shared memory).
-template <int G>
-__device__ void jacobi_fp32_g(const cplx* T0, int n, cpf* A32, cpf* V32, int* s_rot, const cpf* Vw, cpf* rowbuf) {
+template <int NQ>
+__device__ void jacobi_fp32_q(const cplx* T0, int n, int ld, cpf* A32, cpf* V32, int* s_rot, const cpf* Vw,
+                              cpf* rowbuf) {
     const int np = n + (n & 1), m = np - 1;
-    const int gl = threadIdx.x % G, grp = threadIdx.x / G, ngrp = blockDim.x / G;
-    const unsigned gmask = (G == 32) ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1)));
+    const int gl = threadIdx.x & 7, grp = threadIdx.x >> 3, ngrp = blockDim.x >> 3;
+    const unsigned gmask = 0xffu << (threadIdx.x & 24);
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        cplx t = T0[e];
-        A32[e] = mkf((float)t.re, (float)t.im);
-        V32[e] = Vw ? Vw[e] : mkf((e % n) == (e / n) ? 1.f : 0.f, 0.f);
+        const int i = e % n, j = e / n;
+        const cplx t = T0[e];
+        A32[i + j * ld] = mkf((float)t.re, (float)t.im);
+        V32[i + j * ld] = Vw ? Vw[e] : mkf(i == j ? 1.f : 0.f, 0.f);
     }
     __syncthreads();
     if (Vw) {
@@ -88,17 +98,17 @@ __device__ void jacobi_fp32_g(const cplx* T0, int n, cpf* A32, cpf* V32, int* s_
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
         cpf* rb = rowbuf + (long long)warp * n;
         for (int i = warp; i < n; i += nw) {
-            for (int c = lane; c < n; c += 32) rb[c] = A32[i + (long long)c * n];
+            for (int c = lane; c < n; c += 32) rb[c] = A32[i + c * ld];
             __syncwarp();
             for (int j = lane; j < n; j += 32) {
-                const cpf* vj = V32 + (long long)j * n;
+                const cpf* vj = V32 + j * ld;
                 float ar = 0.f, ai = 0.f;
                 for (int c = 0; c < n; ++c) {
                     const cpf a = rb[c], v = vj[c];
                     ar = fmaf(a.re, v.re, fmaf(-a.im, v.im, ar));
                     ai = fmaf(a.re, v.im, fmaf(a.im, v.re, ai));
                 }
-                A32[i + (long long)j * n] = mkf(ar, ai);
+                A32[i + j * ld] = mkf(ar, ai);
             }
             __syncwarp();
         }
@@ -110,22 +120,33 @@ __device__ void jacobi_fp32_g(const cplx* T0, int n, cpf* A32, cpf* V32, int* s_
         __syncthreads();
         for (int r = 0; r < m; ++r) {
             for (int k = grp; k < np / 2; k += ngrp) {
-                int p, q;
-                rr_pair(r, k, m, p, q);
+                int p = 0, q = r + 1;   // rr_pair without its remainders
+                if (k) {
+                    p = r + k < m ? r + k + 1 : r + k - m + 1;
+                    q = r >= k ? r - k + 1 : r - k + m + 1;
+                }
                 if (p >= n || q >= n) continue;
                 if (p > q) { int t = p; p = q; q = t; }
-                cpf* ap = A32 + p * n;
-                cpf* aq = A32 + q * n;
+                cpf* ap = A32 + p * ld + gl;
+                cpf* aq = A32 + q * ld + gl;
+                cpf xs[NQ], ys[NQ];
+#pragma unroll
+                for (int u = 0; u < NQ; ++u) {
+                    const bool in = gl + 8 * u < n;
+                    xs[u] = in ? ap[8 * u] : mkf(0.f, 0.f);
+                    ys[u] = in ? aq[8 * u] : mkf(0.f, 0.f);
+                }
                 float al = 0.f, be = 0.f, gr = 0.f, gi = 0.f;
-                for (int i = gl; i < n; i += G) {
-                    cpf x = ap[i], y = aq[i];
+#pragma unroll
+                for (int u = 0; u < NQ; ++u) {
+                    const cpf x = xs[u], y = ys[u];
                     al = fmaf(x.re, x.re, fmaf(x.im, x.im, al));
                     be = fmaf(y.re, y.re, fmaf(y.im, y.im, be));
                     gr = fmaf(x.re, y.re, fmaf(x.im, y.im, gr));
                     gi = fmaf(x.re, y.im, fmaf(-x.im, y.re, gi));
                 }
 #pragma unroll
-                for (int o = G / 2; o > 0; o >>= 1) {
+                for (int o = 4; o > 0; o >>= 1) {
                     al += __shfl_xor_sync(gmask, al, o);
                     be += __shfl_xor_sync(gmask, be, o);
                     gr += __shfl_xor_sync(gmask, gr, o);
@@ -138,17 +159,19 @@ __device__ void jacobi_fp32_g(const cplx* T0, int n, cpf* A32, cpf* V32, int* s_
                 float t = (zeta >= 0.f ? 1.f : -1.f) / (fabsf(zeta) + sqrtf(1.f + zeta * zeta));
                 float c = 1.f / sqrtf(1.f + t * t), s = c * t;
                 float er = gr / g, ei = -gi / g;
-                cpf* vp = V32 + p * n;
-                cpf* vq = V32 + q * n;
-                for (int i = gl; i < n; i += G) {
-                    cpf x = ap[i], y0 = aq[i];
+                cpf* vp = V32 + p * ld + gl;
+                cpf* vq = V32 + q * ld + gl;
+#pragma unroll
+                for (int u = 0; u < NQ; ++u) {
+                    if (gl + 8 * u >= n) continue;
+                    cpf x = xs[u], y0 = ys[u];
                     cpf y = mkf(er * y0.re - ei * y0.im, er * y0.im + ei * y0.re);
-                    ap[i] = mkf(c * x.re - s * y.re, c * x.im - s * y.im);
-                    aq[i] = mkf(s * x.re + c * y.re, s * x.im + c * y.im);
-                    cpf xv = vp[i], yv0 = vq[i];
+                    ap[8 * u] = mkf(c * x.re - s * y.re, c * x.im - s * y.im);
+                    aq[8 * u] = mkf(s * x.re + c * y.re, s * x.im + c * y.im);
+                    cpf xv = vp[8 * u], yv0 = vq[8 * u];
                     cpf yv = mkf(er * yv0.re - ei * yv0.im, er * yv0.im + ei * yv0.re);
-                    vp[i] = mkf(c * xv.re - s * yv.re, c * xv.im - s * yv.im);
-                    vq[i] = mkf(s * xv.re + c * yv.re, s * xv.im + c * yv.im);
+                    vp[8 * u] = mkf(c * xv.re - s * yv.re, c * xv.im - s * yv.im);
+                    vq[8 * u] = mkf(s * xv.re + c * yv.re, s * xv.im + c * yv.im);
                 }
             }
             __syncthreads();
@@ -158,10 +181,12 @@ __device__ void jacobi_fp32_g(const cplx* T0, int n, cpf* A32, cpf* V32, int* s_
     }
 }
 
-__device__ void jacobi_fp32(const cplx* T0, int n, cpf* A32, cpf* V32, int* s_rot, const cpf* Vw = nullptr,
+// n <= 120: what fits into shared memory in the kernels that call it
+__device__ void jacobi_fp32(const cplx* T0, int n, int ld, cpf* A32, cpf* V32, int* s_rot, const cpf* Vw = nullptr,
                             cpf* rowbuf = nullptr) {
-    if (n <= 128) jacobi_fp32_g<8>(T0, n, A32, V32, s_rot, Vw, rowbuf);
-    else jacobi_fp32_g<32>(T0, n, A32, V32, s_rot, Vw, rowbuf);
+    if (n <= 56) jacobi_fp32_q<7>(T0, n, ld, A32, V32, s_rot, Vw, rowbuf);
+    else if (n <= 104) jacobi_fp32_q<13>(T0, n, ld, A32, V32, s_rot, Vw, rowbuf);
+    else jacobi_fp32_q<15>(T0, n, ld, A32, V32, s_rot, Vw, rowbuf);
 }
 
 // Stage 2: V = orthonormalised columns of V32 in FP64 (classical Gram-Schmidt; one
@@ -238,7 +263,7 @@ __global__ void __launch_bounds__(kSvdThreads) k_svd_jacobi(SvdJob J) {
         // V orthonormalised in FP64; the FP64 sweeps below only polish (A must be in
         // shared memory: the FP32 stage uses the same space)
         cpf* A32 = reinterpret_cast<cpf*>(sbase);
-        jacobi_fp32(T0, n, A32, A32 + (long long)n * n, &s_rot);
+        jacobi_fp32(T0, n, n, A32, A32 + (long long)n * n, &s_rot);
         orthonormalise_fp64(A32 + (long long)n * n, n, V, uy, uz, red);
         product_fp64(T0, V, n, A);
     } else {
@@ -460,6 +485,8 @@ cudaError_t launch_svd_mixed(int n, int nmat, int D, int which, const cplx* T, l
 // (measured: 142.8 -> 138.0 ms per bench step; 139.7 ms with 10).  At least 8: the
 // block's storage doubles as the Jacobi warm start's row buffer (16 warps x n).
 constexpr int kFastKmax = 8;
+constexpr int kFastNmax = 112;   // no larger matrix fits into shared memory
+constexpr int kNearPer = (kFastNmax * kFastKmax + kSvdThreads - 1) / kSvdThreads;   // entries of the block per thread
 constexpr int kFastInvIter = 4;
 constexpr int kFastNeumannMax = 200;   // preconditioned CG iteration cap
 // launches of at most this many matrices run the paired (two-CTA cluster) form
@@ -532,20 +559,21 @@ static __device__ void gemv_n(const cplx* A, int n, const cplx* x, cplx* y) {
     __syncthreads();
 }
 
-// y = A^H x (warp per column)
+// y = A^H x: eight consecutive lanes per column (a warp per column spends more on its
+// five-level sums than on the products)
 static __device__ void gemv_h(const cplx* A, int n, const cplx* x, cplx* y) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int c = warp; c < n; c += nw) {
+    const int sub = threadIdx.x & 7;
+    const unsigned gmask = 0xFFu << (threadIdx.x & 24);
+    for (int c = threadIdx.x >> 3; c < n; c += blockDim.x >> 3) {
         const cplx* col = A + (long long)c * n;
-        double sr = 0., si = 0.;
-        for (int r = lane; r < n; r += 32) {
-            const cplx a = conj(col[r]), b = x[r];
-            sr = fma(a.re, b.re, fma(-a.im, b.im, sr));
-            si = fma(a.re, b.im, fma(a.im, b.re, si));
+        cplx a = mk(0.);
+        for (int r = sub; r < n; r += 8) cfma_c(a, col[r], x[r]);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) {
+            a.re += __shfl_xor_sync(gmask, a.re, o);
+            a.im += __shfl_xor_sync(gmask, a.im, o);
         }
-        sr = warp_sum(sr);
-        si = warp_sum(si);
-        if (lane == 0) y[c] = mk(sr, si);
+        if (sub == 0) y[c] = a;
     }
     __syncthreads();
 }
@@ -584,26 +612,29 @@ static __device__ double dot_re(const cplx* a, const cplx* b, int n, double* red
     return bsum(part, red);
 }
 
-// Rows of B (n x kb) times the kb x kb matrix M, in place, row by row.
+// Rows of B (n x kb) times the kb x kb matrix M in place, a thread per entry.
 static __device__ void rows_times(cplx* B, int n, int kb, const cplx* M) {
-    for (int r = threadIdx.x; r < n; r += blockDim.x) {
-        cplx row[kFastKmax], outr[kFastKmax];
+    cplx o[kNearPer];
 #pragma unroll
-        for (int j = 0; j < kFastKmax; ++j) row[j] = j < kb ? B[r + (long long)j * n] : mk(0.);
+    for (int u = 0; u < kNearPer; ++u) {
+        const int e = threadIdx.x + u * kSvdThreads, r = e % n, j = e / n;
+        o[u] = mk(0.);
+        if (j < kb)
+            for (int l = 0; l < kb; ++l) cfma(o[u], B[r + (long long)l * n], M[l + j * kb]);
+    }
+    __syncthreads();
 #pragma unroll
-        for (int j = 0; j < kFastKmax; ++j) {
-            cplx a = mk(0.);
-#pragma unroll
-            for (int l = 0; l < kFastKmax; ++l)
-                if (l < kb) cfma(a, row[l], M[l + j * kb]);
-            outr[j] = a;
-        }
-#pragma unroll
-        for (int j = 0; j < kFastKmax; ++j)
-            if (j < kb) B[r + (long long)j * n] = outr[j];
+    for (int u = 0; u < kNearPer; ++u) {
+        const int e = threadIdx.x + u * kSvdThreads;
+        if (e < n * kb) B[e] = o[u];
     }
     __syncthreads();
 }
+
+// Leading dimension of the FP32 stage: the two column pairs that a half-warp's 8-byte accesses
+// take lie 16 banks apart.  At most n + 15: A32 and V32 end before the block W (fast_layout's
+// x and y are free in that stage).
+__host__ __device__ inline int jac_ld(int n) { return n < 16 ? n : (n + 7) / 16 * 16 + 8; }
 
 // PAIR: a cluster of two CTAs per matrix (blocks 2m, 2m + 1), for launches of a few
 // matrices where the latency of one matrix matters.  CTA 0 runs stage 1 (FP32 Jacobi,
@@ -625,7 +656,8 @@ __global__ void __launch_bounds__(kSvdThreads) k_svd_fast(SvdFastJob J) {
     const FastSmem L = fast_layout(n);
     cplx* T64 = reinterpret_cast<cplx*>(sb + L.r0);
     cpf* A32 = reinterpret_cast<cpf*>(sb + L.r0);
-    cpf* V32 = A32 + (long long)n * n;
+    const int ld32 = jac_ld(n);
+    cpf* V32 = A32 + n * ld32;
     cplx* X = reinterpret_cast<cplx*>(sb + L.x);
     cplx* Y = reinterpret_cast<cplx*>(sb + L.y);
     cplx* W = reinterpret_cast<cplx*>(sb + L.w);
@@ -642,7 +674,6 @@ __global__ void __launch_bounds__(kSvdThreads) k_svd_fast(SvdFastJob J) {
     cplx *F = vec, *G = vec + n, *f1 = vec + 2 * n, *f2 = vec + 3 * n, *rr = vec + 4 * n, *acc = vec + 5 * n,
          *term = vec + 6 * n, *z2 = vec + 7 * n, *sbuf = vec + 8 * n;
     __shared__ int s_rot, s_kb, s_im, s_sing, s_conv, s_iters, s_next;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const cplx* T0 = J.T + (long long)mat * J.mat_stride;
     double* out = J.out + 3LL * mat;
 
@@ -651,17 +682,21 @@ __global__ void __launch_bounds__(kSvdThreads) k_svd_fast(SvdFastJob J) {
     // 1. FP32 Jacobi, from the pool's V set of a nearby wavenumber when given
     const int wslot = (J.vpool && J.warm_slot) ? J.warm_slot[mat] : -1;
     const int oslot = (J.vpool && J.out_slot) ? J.out_slot[mat] : -1;
-    jacobi_fp32(T0, n, A32, V32, &s_rot, wslot >= 0 ? J.vpool + wslot * nn : nullptr, reinterpret_cast<cpf*>(X));
+    jacobi_fp32(T0, n, ld32, A32, V32, &s_rot, wslot >= 0 ? J.vpool + wslot * nn : nullptr,
+                reinterpret_cast<cpf*>(vec));
     if (oslot >= 0) {
         cpf* dst = J.vpool + oslot * nn;
-        for (long long e = threadIdx.x; e < nn; e += blockDim.x) dst[e] = V32[e];
+        for (int e = threadIdx.x; e < nn; e += blockDim.x) dst[e] = V32[e / n * ld32 + e % n];
     }
-    for (int j = warp; j < n; j += nw) {
-        float s2 = 0.f;
-        for (int i = lane; i < n; i += 32) s2 = fmaf(A32[j * n + i].re, A32[j * n + i].re,
-                                                     fmaf(A32[j * n + i].im, A32[j * n + i].im, s2));
-        s2 = warp_sumf(s2);
-        if (lane == 0) sig32[j] = sqrtf(s2);
+    {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+        for (int j = warp; j < n; j += nw) {
+            const cpf* a = A32 + j * ld32;
+            float s2 = 0.f;
+            for (int i = lane; i < n; i += 32) s2 = fmaf(a[i].re, a[i].re, fmaf(a[i].im, a[i].im, s2));
+            s2 = warp_sumf(s2);
+            if (lane == 0) sig32[j] = sqrtf(s2);
+        }
     }
     __syncthreads();
     // 2. near block: the kb smallest FP32 singular values (ascending, ties by index):
@@ -713,9 +748,17 @@ __global__ void __launch_bounds__(kSvdThreads) k_svd_fast(SvdFastJob J) {
     __syncthreads();
     {
         const int kb = s_kb;
-        for (int e = threadIdx.x; e < n * kb; e += blockDim.x) {
-            const cpf v = V32[idx[e / n] * n + e % n];
-            X[e] = mk((double)v.re, (double)v.im);
+        cpf v[kNearPer];   // V32 reaches into X
+#pragma unroll
+        for (int u = 0; u < kNearPer; ++u) {
+            const int e = threadIdx.x + u * kSvdThreads;
+            if (e < n * kb) v[u] = V32[idx[e / n] * ld32 + e % n];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < kNearPer; ++u) {
+            const int e = threadIdx.x + u * kSvdThreads;
+            if (e < n * kb) X[e] = mk((double)v[u].re, (double)v[u].im);
         }
         __syncthreads();
         if constexpr (PAIR) {   // the start block and its two counts to CTA 1
@@ -734,14 +777,9 @@ __global__ void __launch_bounds__(kSvdThreads) k_svd_fast(SvdFastJob J) {
         if (threadIdx.x == 0) s_sing = 0;
         for (int e = threadIdx.x; e < n * n; e += blockDim.x) T64[e] = T0[e];
         __syncthreads();
-        lu_smem(T64, n, piv, &s_sing, sbuf);
+        lu_smem(T64, n, piv, &s_sing);
         perm_from_piv(piv, n, perm);
-        // U's diagonal replaced by its reciprocals: the solves below multiply
-        for (int k = threadIdx.x; k < n; k += blockDim.x) {
-            const cplx d = T64[k + (long long)k * n];
-            T64[k + (long long)k * n] = norm2(d) > 0. ? cdiv(mk(1.), d) : mk(0.);
-        }
-        __syncthreads();
+        lu_inv_diag(T64, n);
     }
     if constexpr (PAIR) {
         cg::cluster_group cl = cg::this_cluster();
@@ -766,8 +804,8 @@ __global__ void __launch_bounds__(kSvdThreads) k_svd_fast(SvdFastJob J) {
     cplx* Xc = X + (long long)col0 * n;
     const int inv_iters = s_iters;
     for (int it = 0; it < inv_iters; ++it) {   // Y is free until the Rayleigh-Ritz step
-        solve_lu_h_blk(T64, perm, n, Xc, cnt, sbuf, Y, true);
-        solve_lu_blk(T64, perm, n, Xc, cnt, sbuf, Y, true);
+        solve_lu_h_blk(T64, perm, n, Xc, cnt, sbuf, Y);
+        solve_lu_blk(T64, perm, n, Xc, cnt, sbuf, Y);
         if constexpr (PAIR) {   // each CTA's columns to the other, then both orthonormalise all
             cg::cluster_group cl = cg::this_cluster();
             cl.sync();   // the other CTA has finished reading its block (the last QR)
@@ -918,8 +956,8 @@ __global__ void __launch_bounds__(kSvdThreads) k_svd_fast(SvdFastJob J) {
     const double s2 = sg * sg;
     for (int r = threadIdx.x; r < n; r += blockDim.x) { yv[r] = mk(0.); zv[r] = rr[r]; }
     __syncthreads();
-    solve_lu_blk(T64, perm, n, zv, 1, sbuf, nullptr, true);                 // z = T^-H T^-1 res
-    solve_lu_h_blk(T64, perm, n, zv, 1, sbuf, nullptr, true);
+    solve_lu_blk(T64, perm, n, zv, 1, sbuf);                 // z = T^-H T^-1 res
+    solve_lu_h_blk(T64, perm, n, zv, 1, sbuf);
     dots_h(Y, n, nd, zv, coef);
     sub_span(Y, n, nd, coef, zv);
     for (int r = threadIdx.x; r < n; r += blockDim.x) pv[r] = zv[r];
@@ -943,8 +981,8 @@ __global__ void __launch_bounds__(kSvdThreads) k_svd_fast(SvdFastJob J) {
             zv[r] = rr[r];
         }
         __syncthreads();
-        solve_lu_blk(T64, perm, n, zv, 1, sbuf, nullptr, true);
-        solve_lu_h_blk(T64, perm, n, zv, 1, sbuf, nullptr, true);
+        solve_lu_blk(T64, perm, n, zv, 1, sbuf);
+        solve_lu_h_blk(T64, perm, n, zv, 1, sbuf);
         dots_h(Y, n, nd, zv, coef);
         sub_span(Y, n, nd, coef, zv);
         const double rz1 = dot_re(rr, zv, n, red + 64);
@@ -997,7 +1035,7 @@ cudaError_t launch_svd_fast(int n, int nmat, int D, const cplx* T, long long mat
                             double* out, int* status, cudaStream_t st, cplxf* vpool, const int* warm_slot,
                             const int* out_slot, cplx* uv) {
     const size_t limit = 220 * 1024, smem = svd_fast_smem_bytes(n);
-    if (smem > limit || n < 2) return cudaErrorInvalidValue;
+    if (smem > limit || n < 2 || n > kFastNmax) return cudaErrorInvalidValue;
     SvdFastJob J{n, nmat, D, T, mat_stride, der_stride, out, status, vpool, warm_slot, out_slot, uv};
     if (t_svd_pair_hold || nmat > g_svd_pair_max.load(std::memory_order_relaxed)) {
         cudaError_t e = cudaFuncSetAttribute(k_svd_fast<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);

@@ -53,27 +53,23 @@ __global__ void __launch_bounds__(kRsvdThreads) k_rsvd_small(RsvdJob J) {
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) A[e] = T0[e];
     for (int e = threadIdx.x; e < n * s; e += blockDim.x) X[e] = J.R[e];
     __syncthreads();
-    lu_smem(A, n, piv, &s_sing, vb);
-    // blocked solves: rows permuted once, U's diagonal replaced by its reciprocals
+    lu_smem(A, n, piv, &s_sing);
+    // blocked solves: rows permuted once
     perm_from_piv(piv, n, perm);
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        const cplx d = A[k + (long long)k * n];
-        A[k + (long long)k * n] = norm2(d) > 0. ? cdiv(mk(1.), d) : mk(0.);
-    }
-    __syncthreads();
+    lu_inv_diag(A, n);
     // Q = qr(T^-1 R)
-    solve_lu_blk(A, perm, n, X, s, vb, nullptr, true);
+    solve_lu_blk(A, perm, n, X, s, vb);
     qr_cgs2(X, n, s, coef, red);
     for (int it = 0; it < J.q; ++it) {
-        solve_lu_h_blk(A, perm, n, X, s, vb, nullptr, true);
+        solve_lu_h_blk(A, perm, n, X, s, vb);
         qr_cgs2(X, n, s, coef, red);
-        solve_lu_blk(A, perm, n, X, s, vb, nullptr, true);
+        solve_lu_blk(A, perm, n, X, s, vb);
         qr_cgs2(X, n, s, coef, red);
     }
     // B = T^-H Q (keep Q in X, B in Y)
     for (int e = threadIdx.x; e < n * s; e += blockDim.x) Y[e] = X[e];
     __syncthreads();
-    solve_lu_h_blk(A, perm, n, Y, s, vb, nullptr, true);
+    solve_lu_h_blk(A, perm, n, Y, s, vb);
     jacobi_thin(Y, n, s, W, red);
     // largest column of B W
     double best = -1.;
@@ -103,8 +99,8 @@ __global__ void __launch_bounds__(kRsvdThreads) k_rsvd_small(RsvdJob J) {
     }
     __syncthreads();
     for (int it = 0; it < kRitzRefine; ++it) {   // Y is free now: row-permutation scratch
-        solve_lu_h_blk(A, perm, n, vb, 1, Y, nullptr, true);
-        solve_lu_blk(A, perm, n, vb, 1, Y, nullptr, true);
+        solve_lu_h_blk(A, perm, n, vb, 1, Y);
+        solve_lu_blk(A, perm, n, vb, 1, Y);
     }
     for (int r = threadIdx.x; r < n; r += blockDim.x) J.uv[2LL * n * mat + n + r] = vb[r];
 }

@@ -7,129 +7,136 @@
 
 namespace hbem {
 
-static __device__ __forceinline__ double bsum(double x, double* red) {
+// (An FP64 instruction of one warp holds its SM sub-partition for 64 cycles, so what every
+// warp repeats -- adding up the warps' sums, a square root, a division -- costs more than the
+// work it follows: one warp does those here and below.)  At most 16 warps.
+static __device__ __forceinline__ double bsum(double x, double* red) {   // red: 32 entries
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
     __syncthreads();
     if (lane == 0) red[warp] = x;
     __syncthreads();
-    double s = 0.;
-    for (int w = 0; w < nw; ++w) s += red[w];
-    return s;
+    if (warp == 0) {
+        double s = 0.;
+        for (int w = 0; w < nw; ++w) s += red[w];
+        if (lane == 0) red[31] = s;
+    }
+    __syncthreads();
+    return red[31];
 }
 
-// LU with partial pivoting of the n x n column-major matrix A (shared memory).
-// piv[k] = row exchanged with row k at step k.  Returns via *sing a zero-pivot flag.
-// Per step: warp 0 finds the pivot (largest |A[i,k]|^2, i >= k, ties to the smallest
-// i), exchanges the two rows and scales column k into lbuf (n entries of scratch) and
-// A; after one barrier all warps update the trailing matrix, a warp per column and
-// its lanes over the rows; a second barrier ends the step.
-static __device__ void lu_smem(cplx* A, int n, int* piv, int* sing, cplx* lbuf) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int k = 0; k < n; ++k) {
-        if (warp == 0) {
-            double best = -1.;
-            int bi = k;
-            for (int i = k + lane; i < n; i += 32) {
-                const double a = norm2(A[i + (long long)k * n]);
-                if (a > best) { best = a; bi = i; }
-            }
+// LU with partial pivoting of the n x n column-major matrix A (shared memory), n <= 128, by a
+// CTA of at least two warps.
+// piv[k] = row exchanged with row k at step k (largest |A[i,k]|^2, i >= k, ties to the
+// smallest i).  Returns via *sing a zero-pivot flag.  Step k finds column k exchanged and
+// scaled already; the other columns' exchange is one thread each, then warp 0 updates column
+// k + 1, finds its pivot, exchanges and scales it, while the other warps share the entries of
+// the rest -- the pivot's chain of dependent work stays off the other warps' way.  Pivot
+// candidates are compared as integers (|x|^2 >= 0 orders like its bits; an FP64 comparison
+// is as slow as an FMA).
+static __device__ void lu_smem(cplx* A, int n, int* piv, int* sing) {
+    __shared__ int s_piv;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // warp 0: column k from its updated entries v (rows k + lane + 32 q): pivot, exchange, scaling
+    auto finish = [&](int k, cplx (&v)[4]) {
+        unsigned long long best = 0ull;
+        int bi = k;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
+        for (int q = 0; q < 4; ++q) {
+            const int i = k + lane + 32 * q;
+            if (i < n) {
+                const unsigned long long b = (unsigned long long)__double_as_longlong(norm2(v[q]));
+                const unsigned long long key = b > 0x7ff0000000000000ull ? 0ull : b + 1;
+                if (key > best) { best = key; bi = i; }
             }
-            const int p = bi;   // the same on every lane
-            if (lane == 0) {
-                piv[k] = p;
-                if (best == 0.) *sing = 1;
-            }
-            if (p != k)
-                for (int j = lane; j < n; j += 32) {
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long ob = __shfl_xor_sync(0xffffffffu, best, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+            if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
+        }
+        const int p = best ? bi : k, pl = (p - k) & 31, pq = (p - k) >> 5;
+        cplx d = mk(0.);                    // the pivot, from the lane that holds it
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (q == pq) d = v[q];
+        d.re = __shfl_sync(0xffffffffu, d.re, pl);
+        d.im = __shfl_sync(0xffffffffu, d.im, pl);
+        cplx top;                           // row k's entry goes to row p
+        top.re = __shfl_sync(0xffffffffu, v[0].re, 0);
+        top.im = __shfl_sync(0xffffffffu, v[0].im, 0);
+        const bool nz = best > 1ull;
+        const cplx id = nz ? cdiv(mk(1.), d) : mk(1.);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int i = k + lane + 32 * q;
+            if (i >= n) continue;
+            cplx x = i == p ? top : v[q];
+            A[i + (long long)k * n] = i == k ? d : x * id;
+        }
+        if (lane == 0) {
+            piv[k] = p;
+            s_piv = p;
+            if (best <= 1ull) *sing = 1;
+        }
+    };
+    if (warp == 0) {
+        cplx v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = lane + 32 * q < n ? A[lane + 32 * q] : mk(0.);
+        finish(0, v);
+    }
+    __syncthreads();
+    for (int k = 0; k < n; ++k) {
+        const int p = s_piv;
+        if (p != k)
+            for (int j = threadIdx.x; j < n; j += blockDim.x)
+                if (j != k) {
                     const cplx t = A[k + (long long)j * n];
                     A[k + (long long)j * n] = A[p + (long long)j * n];
                     A[p + (long long)j * n] = t;
                 }
-            __syncwarp();
-            const cplx d = A[k + (long long)k * n];
-            const bool nz = norm2(d) > 0.;
-            const cplx id = nz ? cdiv(mk(1.), d) : mk(0.);
-            for (int i = k + 1 + lane; i < n; i += 32) {
-                cplx l = A[i + (long long)k * n];
-                if (nz) l = l * id;
-                A[i + (long long)k * n] = l;
-                lbuf[i] = l;
-            }
-        }
         __syncthreads();
-        for (int j = k + 1 + warp; j < n; j += nw) {
-            const cplx u = A[k + (long long)j * n];
-            for (int i = k + 1 + lane; i < n; i += 32) cfms(A[i + (long long)j * n], lbuf[i], u);
+        const int m = n - k - 1;
+        if (warp == 0) {
+            if (m > 0) {
+                const cplx u = A[k + (long long)(k + 1) * n];
+                cplx v[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int i = k + 1 + lane + 32 * q;
+                    v[q] = mk(0.);
+                    if (i < n) {
+                        v[q] = A[i + (long long)(k + 1) * n];
+                        cfms(v[q], A[i + (long long)k * n], u);
+                    }
+                }
+                finish(k + 1, v);
+            }
+        } else {
+            const int tot = m * (m - 1);
+            for (int e = threadIdx.x - 32; e < tot; e += blockDim.x - 32) {
+                const int j = e / m, i = k + 1 + e - j * m;
+                cplx* a = A + i + (long long)(k + 2 + j) * n;
+                cplx z = *a;
+                cfms(z, A[i + (long long)k * n], A[k + (long long)(k + 2 + j) * n]);
+                *a = z;
+            }
         }
         __syncthreads();
     }
 }
 
-// X <- T^-1 X  (s columns, leading dimension n), with P T = L U in A
-static __device__ void solve_lu(const cplx* A, const int* piv, int n, cplx* X, int s) {
-    for (int k = 0; k < n; ++k) {          // row exchanges in order
-        const int p = piv[k];
-        if (p != k)
-            for (int c = threadIdx.x; c < s; c += blockDim.x) {
-                cplx t = X[k + c * n];
-                X[k + c * n] = X[p + c * n];
-                X[p + c * n] = t;
-            }
-        __syncthreads();
+// After lu_smem: U's diagonal replaced by its reciprocals (0 for a zero pivot), by which the
+// blocked solves below multiply.
+static __device__ void lu_inv_diag(cplx* A, int n) {
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+        const cplx d = A[k + (long long)k * n];
+        A[k + (long long)k * n] = norm2(d) > 0. ? cdiv(mk(1.), d) : mk(0.);
     }
-    for (int k = 0; k < n; ++k) {          // L y = P b (unit diagonal)
-        for (int e = threadIdx.x; e < (n - k - 1) * s; e += blockDim.x) {
-            const int i = k + 1 + e % (n - k - 1), c = e / (n - k - 1);
-            cfms(X[i + c * n], A[i + (long long)k * n], X[k + c * n]);
-        }
-        __syncthreads();
-    }
-    for (int k = n - 1; k >= 0; --k) {     // U x = y
-        for (int c = threadIdx.x; c < s; c += blockDim.x) X[k + c * n] = cdiv(X[k + c * n], A[k + (long long)k * n]);
-        __syncthreads();
-        for (int e = threadIdx.x; e < k * s; e += blockDim.x) {
-            const int i = e % k, c = e / k;
-            cfms(X[i + c * n], A[i + (long long)k * n], X[k + c * n]);
-        }
-        __syncthreads();
-    }
-}
-
-// X <- T^-H X:  T^H = U^H L^H P  =>  x = P^T L^-H U^-H b
-static __device__ void solve_lu_h(const cplx* A, const int* piv, int n, cplx* X, int s) {
-    for (int k = 0; k < n; ++k) {          // U^H y = b (lower triangular, diagonal conj(u_kk))
-        for (int c = threadIdx.x; c < s; c += blockDim.x) X[k + c * n] = cdiv(X[k + c * n], conj(A[k + (long long)k * n]));
-        __syncthreads();
-        for (int e = threadIdx.x; e < (n - k - 1) * s; e += blockDim.x) {
-            const int i = k + 1 + e % (n - k - 1), c = e / (n - k - 1);
-            cfms_c(X[i + c * n], A[k + (long long)i * n], X[k + c * n]);
-        }
-        __syncthreads();
-    }
-    for (int k = n - 1; k >= 0; --k) {     // L^H z = y (unit upper triangular)
-        for (int e = threadIdx.x; e < k * s; e += blockDim.x) {
-            const int i = e % k, c = e / k;
-            cfms_c(X[i + c * n], A[k + (long long)i * n], X[k + c * n]);
-        }
-        __syncthreads();
-    }
-    for (int k = n - 1; k >= 0; --k) {     // x = P^T z (exchanges in reverse order)
-        const int p = piv[k];
-        if (p != k)
-            for (int c = threadIdx.x; c < s; c += blockDim.x) {
-                cplx t = X[k + c * n];
-                X[k + c * n] = X[p + c * n];
-                X[p + c * n] = t;
-            }
-        __syncthreads();
-    }
+    __syncthreads();
 }
 
 // Orthonormalise the s columns of X (n x s) in place: classical Gram-Schmidt,
@@ -169,9 +176,21 @@ static __device__ void qr_cgs2(cplx* X, int n, int s, cplx* coef, double* red, c
         }
         double part = 0.;
         for (int r = threadIdx.x; r < n; r += blockDim.x) part += norm2(xj[r]);
-        const double nrm = sqrt(bsum(part, red));
-        if (Rf && threadIdx.x == 0) Rf[j + j * s] = mk(nrm);
-        const double inv = nrm > 0. ? 1. / nrm : 0.;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+        if (lane == 0) red[warp] = part;
+        __syncthreads();
+        if (warp == 0) {
+            double t = 0.;
+            for (int w = 0; w < nw; ++w) t += red[w];
+            const double nrm = sqrt(t);
+            if (lane == 0) {
+                if (Rf) Rf[j + j * s] = mk(nrm);
+                red[31] = nrm > 0. ? 1. / nrm : 0.;
+            }
+        }
+        __syncthreads();
+        const double inv = red[31];
         for (int r = threadIdx.x; r < n; r += blockDim.x) xj[r] = inv * xj[r];
         __syncthreads();
     }
@@ -296,37 +315,71 @@ static __device__ void jacobi_cta(cplx* B, int s, cplx* W, int* flag) {
                 else { p = (r + k) % m + 1; q = (r - k + m) % m + 1; }
                 if (p >= s || q >= s) continue;
                 if (p > q) { const int t = p; p = q; q = t; }
-                const cplx x = lane < s ? B[p * s + lane] : mk(0.), y = lane < s ? B[q * s + lane] : mk(0.);
-                double al = norm2(x), be = norm2(y);
-                double gr = fma(x.re, y.re, x.im * y.im), gi = fma(x.re, y.im, -x.im * y.re);
-                // rows >= s hold zeros: for s <= 16 the lower half-warp has the sums
-                for (int o = s <= 16 ? 8 : 16; o > 0; o >>= 1) {
-                    al += __shfl_xor_sync(0xffffffffu, al, o);
-                    be += __shfl_xor_sync(0xffffffffu, be, o);
-                    gr += __shfl_xor_sync(0xffffffffu, gr, o);
-                    gi += __shfl_xor_sync(0xffffffffu, gi, o);
+                // s <= 16: the half-warps share the pair -- the lower forms |x|^2 and Re x^H y and
+                // rotates column p, the upper |y|^2, Im x^H y and column q
+                const bool halves = s <= 16;
+                const int row = halves ? lane & 15 : lane;
+                const bool up = halves && lane >= 16;
+                const cplx x = row < s ? B[p * s + row] : mk(0.), y = row < s ? B[q * s + row] : mk(0.);
+                double al, be, gr, gi;
+                if (halves) {
+                    const cplx z = up ? y : x;
+                    double nz = norm2(z);
+                    double g = up ? fma(x.re, y.im, -x.im * y.re) : fma(x.re, y.re, x.im * y.im);
+#pragma unroll
+                    for (int o = 8; o > 0; o >>= 1) {
+                        nz += __shfl_xor_sync(0xffffffffu, nz, o);
+                        g += __shfl_xor_sync(0xffffffffu, g, o);
+                    }
+                    al = __shfl_sync(0xffffffffu, nz, 0);
+                    be = __shfl_sync(0xffffffffu, nz, 16);
+                    gr = __shfl_sync(0xffffffffu, g, 0);
+                    gi = __shfl_sync(0xffffffffu, g, 16);
+                } else {
+                    al = norm2(x);
+                    be = norm2(y);
+                    gr = fma(x.re, y.re, x.im * y.im);
+                    gi = fma(x.re, y.im, -x.im * y.re);
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) {
+                        al += __shfl_xor_sync(0xffffffffu, al, o);
+                        be += __shfl_xor_sync(0xffffffffu, be, o);
+                        gr += __shfl_xor_sync(0xffffffffu, gr, o);
+                        gi += __shfl_xor_sync(0xffffffffu, gi, o);
+                    }
+                    al = __shfl_sync(0xffffffffu, al, 0);
+                    be = __shfl_sync(0xffffffffu, be, 0);
+                    gr = __shfl_sync(0xffffffffu, gr, 0);
+                    gi = __shfl_sync(0xffffffffu, gi, 0);
                 }
-                al = __shfl_sync(0xffffffffu, al, 0);
-                be = __shfl_sync(0xffffffffu, be, 0);
-                gr = __shfl_sync(0xffffffffu, gr, 0);
-                gi = __shfl_sync(0xffffffffu, gi, 0);
-                // rotation from |g|^2 and one reciprocal square root: shorter dependent
-                // chain than hypot and the divisions by |g|
                 const double g2 = fma(gr, gr, gi * gi);
                 if (g2 == 0. || g2 <= (tol * tol) * (al * be)) continue;
                 if (lane == 0) *flag = 1;
+                // The tangent, root of t^2 + 2 zeta t - 1, from FP32 and one Newton step in FP64
+                // with an FP32 slope (to about 1e-14): no FP64 square root and division.  The
+                // rotation's unit length and phase from FP64 reciprocal square roots.
                 const double ig = rsqrt(g2);
-                const double zeta = (be - al) * (0.5 * ig);
-                const double t = (zeta >= 0. ? 1. : -1.) / (fabs(zeta) + sqrt(fma(zeta, zeta, 1.)));
+                const double zd = (be - al) * (0.5 * ig);
+                const float zeta = (float)zd;
+                const float az = fabsf(zeta);
+                const float tf = copysignf(1.f, zeta) / (az + (az > 1e8f ? az : sqrtf(fmaf(az, az, 1.f))));
+                double t = (double)tf;
+                t = fma(-fma(t, fma(2., zd, t), -1.), (double)(0.5f / (tf + zeta)), t);
                 const double c = rsqrt(fma(t, t, 1.)), sn = c * t;
                 const cplx eph = mk(gr * ig, -gi * ig);
-                if (lane < s) {
-                    const cplx ey = eph * y;
-                    B[p * s + lane] = c * x - sn * ey;
-                    B[q * s + lane] = sn * x + c * ey;
-                    const cplx wx = W[p * s + lane], wy = eph * W[q * s + lane];
-                    W[p * s + lane] = c * wx - sn * wy;
-                    W[q * s + lane] = sn * wx + c * wy;
+                // p' = c x - s e y, q' = s x + c e y
+                auto turn = [&](cplx* M, cplx mx, cplx my) {
+                    const cplx ey = eph * my;
+                    const double f = up ? sn : c, h = up ? c : -sn;
+                    const cplx z = mk(fma(f, mx.re, h * ey.re), fma(f, mx.im, h * ey.im));
+                    M[(up ? q : p) * s + row] = z;
+                    if (!halves) M[q * s + row] = mk(fma(sn, mx.re, c * ey.re), fma(sn, mx.im, c * ey.im));
+                };
+                const cplx wx = row < s ? W[p * s + row] : mk(0.), wy = row < s ? W[q * s + row] : mk(0.);
+                __syncwarp();   // the other half has read this half's columns
+                if (row < s) {
+                    turn(B, x, y);
+                    turn(W, wx, wy);
                 }
             }
             __syncthreads();
@@ -385,7 +438,7 @@ static __device__ void permute_cols(cplx* X, int n, int s, const int* perm, cplx
 // X <- T^-1 X.  wide (optional): n x s scratch for a one-pass row permutation;
 // inv_diag: A's diagonal holds 1 / u_kk (multiplications instead of divisions).
 static __device__ void solve_lu_blk(const cplx* A, const int* perm, int n, cplx* X, int s, cplx* buf,
-                                    cplx* wide = nullptr, bool inv_diag = false) {
+                                    cplx* wide = nullptr) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     permute_cols(X, n, s, perm, buf, false, wide);
     for (int b0 = 0; b0 < n; b0 += 32) {                       // L y = P b, L unit lower
@@ -420,7 +473,7 @@ static __device__ void solve_lu_blk(const cplx* A, const int* perm, int n, cplx*
             for (int k = bs - 1; k >= 0; --k) {
                 if (lane == k) {
                     const cplx d = A[(b0 + k) + (long long)(b0 + k) * n];
-                    v = inv_diag ? v * d : cdiv(v, d);
+                    v = v * d;
                 }
                 cplx vk;
                 vk.re = __shfl_sync(0xffffffffu, v.re, k);
@@ -441,9 +494,9 @@ static __device__ void solve_lu_blk(const cplx* A, const int* perm, int n, cplx*
     }
 }
 
-// X <- T^-H X:  T^H = U^H L^H P, x = P^T L^-H U^-H b (wide, inv_diag as in solve_lu_blk)
+// X <- T^-H X:  T^H = U^H L^H P, x = P^T L^-H U^-H b (wide as in solve_lu_blk)
 static __device__ void solve_lu_h_blk(const cplx* A, const int* perm, int n, cplx* X, int s, cplx* buf,
-                                      cplx* wide = nullptr, bool inv_diag = false) {
+                                      cplx* wide = nullptr) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int b0 = 0; b0 < n; b0 += 32) {                       // U^H y = b (lower, diagonal conj(u_kk))
         const int bs = min(32, n - b0);
@@ -453,7 +506,7 @@ static __device__ void solve_lu_h_blk(const cplx* A, const int* perm, int n, cpl
             for (int k = 0; k < bs; ++k) {
                 if (lane == k) {
                     const cplx d = conj(A[(b0 + k) + (long long)(b0 + k) * n]);
-                    v = inv_diag ? v * d : cdiv(v, d);
+                    v = v * d;
                 }
                 cplx vk;
                 vk.re = __shfl_sync(0xffffffffu, v.re, k);

@@ -1,0 +1,32 @@
+"""The dense kernel's FP32 stage at the edges of its column layouts: orders below, at and past
+a change of the leading dimension or of the columns' register count, and the largest that fits.
+
+T = U diag(s) V^H with s known: sigma_min = 0.1, the others in [0.4, 1].  Tolerances: sigma is
+a Ritz value, off by rounding (n eps |T| times a few) and by the square of the vectors' error.
+The vectors: the FP32 stage leaves at most n eps32 |T| / gap = 106 * 6e-8 / 0.3 = 2e-5 outside
+the near block, which the inverse iterations take down by a factor of 3^-8 = 1.5e-4 at least,
+to 3e-9; sigma' = Re u^H T' v with |T'| about 2 is first order in that."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+from helmholtzbem_gb300 import api  # noqa: E402
+
+
+@pytest.mark.parametrize("nmat", [3, 17])   # a pair of CTAs per matrix, one CTA per matrix
+@pytest.mark.parametrize("n", [2, 9, 15, 16, 24, 25, 56, 57, 104])
+def test_known_singular_values(n, nmat):
+    rng = np.random.default_rng(100 * n + nmat)
+    mats, ref = [], []
+    for _ in range(nmat):
+        z = rng.standard_normal((4, n, n)) + 1j * rng.standard_normal((4, n, n))
+        U, V = np.linalg.qr(z[0])[0], np.linalg.qr(z[1])[0]
+        s = rng.permutation(np.concatenate([[0.1], np.linspace(0.4, 1.0, n - 1)]))
+        T1 = z[2] / np.sqrt(2.0 * n)
+        i = int(np.argmin(s))
+        mats.append([(U * s) @ V.conj().T, T1])
+        ref.append([0.1, (U[:, i].conj() @ T1 @ V[:, i]).real])
+    got, ref = np.array(api.sv_dense(mats, d=1)), np.array(ref)
+    assert np.abs(got[:, 0] - ref[:, 0]).max() <= 16 * n * np.finfo(float).eps
+    assert np.abs(got[:, 1] - ref[:, 1]).max() <= 1e-7
