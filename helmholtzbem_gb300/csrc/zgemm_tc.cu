@@ -20,11 +20,14 @@
 // kernel's (tests/test_gpu_zgemm.py).
 //
 // Complex product as one real GEMM, as in tc_gemm.cu: A' = [A_r | A_i] (128 x 64),
-// B' = [[B_r, B_i], [-B_i, B_r]] (64 x 64 for 32 complex columns), C' = [re | im].
-// A CTA takes 128 rows and a run of 32-column tiles: A's digits are cut once (112 KB of
-// 128-byte-swizzled K-major shared memory), B's per tile (56 KB).  Tensor memory: the eight
-// sums, 64 columns each, all 512.  Per tile 34 digit products of four K = 16 steps; the FP64
-// pipe does two instructions per real entry (a conversion and an FMA) instead of 128.
+// B' = [[B_r, B_i], [-B_i, B_r]] (64 x 32 for 16 complex columns), C' = [re | im].
+// A CTA takes 128 rows and a run of 16-column tiles: A's digits are cut once (112 KB of
+// 128-byte-swizzled K-major shared memory), B's per tile (28 KB, two buffers).  Tensor memory:
+// the eight sums of a tile are 256 columns, so two tiles fit, and a tile's products run while
+// the sums of the one before are read, joined and subtracted.  That epilogue is what bounds the
+// kernel: per real entry eight 32-bit conversions and two FP64 instructions (a conversion and an
+// FMA) instead of 128.  The first update of four matrices of order 1500 takes 196 us; with
+// tiles of 32 columns in one buffer, C read in the epilogue and a product per digit pair, 362.
 #include <algorithm>
 #include <cstdint>
 
@@ -35,17 +38,18 @@ namespace hbem {
 namespace {
 
 constexpr int kZM = 128;                   // rows per CTA
-constexpr int kZNc = 32;                   // complex columns per tile
+constexpr int kZNc = 16;                   // complex columns per tile
 constexpr int kZN = 2 * kZNc;              // MMA N
 constexpr int kZK = 32;                    // complex depth
 constexpr int kZDig = 7, kZSums = 8;
 constexpr int kZThreads = 256;
 constexpr uint32_t kZABytes = kZM * 128u, kZBBytes = kZN * 128u;   // a digit of each operand: rows of 64 BF16
-constexpr size_t kZSmem = kZDig * (size_t)(kZABytes + kZBBytes) + 1024;
+constexpr size_t kZSmem = kZDig * (size_t)(kZABytes + 2 * kZBBytes) + 1024;
 constexpr long long kZSpinCap = 1LL << 24;
 // instruction descriptor, kind::f16: D FP32, A and B BF16, K-major, N >> 3, M >> 4
-constexpr uint32_t kZIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kZN >> 3) << 17) |
-                             ((uint32_t)(kZM >> 4) << 24);
+__device__ constexpr uint32_t z_idesc(int n) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kZM >> 4) << 24);
+}
 
 __device__ __forceinline__ uint32_t z_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -123,13 +127,27 @@ __device__ __forceinline__ void z_ld4(uint32_t addr, uint32_t (&r)[4]) {
                  : "r"(addr));
 }
 
+// the sums (exact integers in FP32) of one real entry as one integer in units of 2^16 of the last
+// sum's: neighbours fit 32 bits (sum s has at most s + 1 digit pairs of 64 x 2^14)
+__device__ __forceinline__ int z_int(float f, bool small) {   // small: |f| <= 2^22
+    return small ? __float_as_int(f + 12582912.f) - 0x4B400000 : __float2int_rn(f);
+}
+__device__ __forceinline__ long long z_join(const uint32_t (&d)[kZSums][4], int jj) {
+    int p[4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+        p[s] = z_int(__uint_as_float(d[2 * s][jj]), 2 * s < 3) * 256 + z_int(__uint_as_float(d[2 * s + 1][jj]), 2 * s + 1 < 3);
+    const long long hi = (long long)p[0] * 65536 + p[1], lo = (long long)p[2] * 65536 + p[3];
+    return hi * 65536 + ((lo + 0x8000) >> 16);
+}
+
 __global__ void __launch_bounds__(kZThreads, 1) k_zgemm_tc(ZJob J) {
     extern __shared__ uint8_t z_raw[];
     uint8_t* As = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(z_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* Bs = As + kZDig * kZABytes;
-    __shared__ __align__(8) uint64_t mbar;
+    __shared__ __align__(8) uint64_t mbar[2];
     __shared__ uint32_t tmem_slot;
-    __shared__ int s_fail, s_ea[2][kZM], s_eb[kZNc];
+    __shared__ int s_ea[2][kZM], s_eb[3][kZNc];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int r0 = blockIdx.x * kZM;
     const cplx* A = J.A + (long long)blockIdx.z * J.sa;
@@ -141,10 +159,21 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zgemm_tc(ZJob J) {
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {
-        s_fail = 0;
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(z_smem(&mbar)), "r"(1));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(z_smem(&mbar[0])), "r"(1));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(z_smem(&mbar[1])), "r"(1));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    const int tile0 = blockIdx.y * J.tiles, ntiles = (J.n + kZNc - 1) / kZNc, tile1 = min(ntiles, tile0 + J.tiles);
+    // B of the next tile and the entries of C that a tile updates are read ahead, into registers:
+    // one CTA fits an SM, so nothing else covers their latency
+    cplx b[2];   // thread (column tid >> 4, two depths)
+    auto load_b = [&](int t) {
+        const int col = t * kZNc + (tid >> 4), k0 = (tid & 15) * 2;
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+            b[q] = (t < tile1 && col < J.n && k0 + q < J.k) ? B[(k0 + q) + (long long)col * J.ldb] : mk(0.);
+    };
+    load_b(tile0);
     {   // A: thread (row tid & 127, half of the depth)
         const int r = tid & 127, kh = tid >> 7;
         cplx a[16];
@@ -176,82 +205,105 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zgemm_tc(ZJob J) {
                 }
             }
     }
-    const uint32_t mbar_addr = z_smem(&mbar);
-    const int tile0 = blockIdx.y * J.tiles, ntiles = (J.n + kZNc - 1) / kZNc, tile1 = min(ntiles, tile0 + J.tiles);
-    for (int t = tile0; t < tile1; ++t) {
-        const int c0 = t * kZNc;
-        {   // B: thread (column tid >> 3, four depths); columns j (re) and 32 + j (im) of C' take
-            // [B_r | -B_i] and [B_i | B_r]
-            const int j = tid >> 3, k0 = (tid & 7) * 4;
-            cplx b[4];
-            int E = 0;
+    // the loaded tile's digits into buffer u, its columns' exponents into s_eb[e]: columns j (re) and 16 + j (im) of C' take [B_r | -B_i]
+    // and [B_i | B_r]
+    auto cut_b = [&](int u, int e) {
+        const int j = tid >> 4, k0 = (tid & 15) * 2;
+        int E = 0;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                b[q] = (c0 + j < J.n && k0 + q < J.k) ? B[(k0 + q) + (long long)(c0 + j) * J.ldb] : mk(0.);
-                E = max(E, max(z_exp(b[q].re), z_exp(b[q].im)));
+        for (int q = 0; q < 2; ++q) E = max(E, max(z_exp(b[q].re), z_exp(b[q].im)));
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) E = max(E, __shfl_xor_sync(0xffffffffu, E, o));
+        if ((tid & 15) == 0) s_eb[e][j] = E;
+        long long vr[2], vi[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            vr[q] = z_fixed(b[q].re, E);
+            vi[q] = z_fixed(b[q].im, E);
+        }
+        const int ch = k0 >> 3, sub = (k0 & 7) * 2;               // chunk and byte within it
+        const uint32_t o00 = z_chunk(j, ch) + sub, o01 = z_chunk(j, 4 + ch) + sub;
+        const uint32_t o10 = z_chunk(kZNc + j, ch) + sub, o11 = z_chunk(kZNc + j, 4 + ch) + sub;
+#pragma unroll
+        for (int dgt = kZDig - 1; dgt >= 0; --dgt) {
+            int dr[2], di[2];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                dr[q] = dgt ? z_digit(vr[q]) : (int)vr[q];
+                di[q] = dgt ? z_digit(vi[q]) : (int)vi[q];
             }
-#pragma unroll
-            for (int o = 4; o > 0; o >>= 1) E = max(E, __shfl_xor_sync(0xffffffffu, E, o));
-            if ((tid & 7) == 0) s_eb[j] = E;
-            long long vr[4], vi[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                vr[q] = z_fixed(b[q].re, E);
-                vi[q] = z_fixed(b[q].im, E);
-            }
-            const int ch = k0 >> 3, sub = (k0 & 4) << 1;          // chunk and byte of its half
-            const uint32_t o00 = z_chunk(j, ch) + sub, o01 = z_chunk(j, 4 + ch) + sub;
-            const uint32_t o10 = z_chunk(kZNc + j, ch) + sub, o11 = z_chunk(kZNc + j, 4 + ch) + sub;
-#pragma unroll
-            for (int dgt = kZDig - 1; dgt >= 0; --dgt) {
-                int dr[4], di[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    dr[q] = dgt ? z_digit(vr[q]) : (int)vr[q];
-                    di[q] = dgt ? z_digit(vi[q]) : (int)vi[q];
-                }
-                uint8_t* S = Bs + dgt * kZBBytes;
-                const uint2 re = make_uint2(z_pack(dr[0], dr[1]), z_pack(dr[2], dr[3]));
-                const uint2 im = make_uint2(z_pack(di[0], di[1]), z_pack(di[2], di[3]));
-                const uint2 ng = make_uint2(z_pack(-di[0], -di[1]), z_pack(-di[2], -di[3]));
-                *reinterpret_cast<uint2*>(S + o00) = re;
-                *reinterpret_cast<uint2*>(S + o01) = ng;
-                *reinterpret_cast<uint2*>(S + o10) = im;
-                *reinterpret_cast<uint2*>(S + o11) = re;
-            }
+            uint8_t* S = Bs + (u * kZDig + dgt) * kZBBytes;
+            const uint32_t re = z_pack(dr[0], dr[1]);
+            *reinterpret_cast<uint32_t*>(S + o00) = re;
+            *reinterpret_cast<uint32_t*>(S + o01) = z_pack(-di[0], -di[1]);
+            *reinterpret_cast<uint32_t*>(S + o10) = z_pack(di[0], di[1]);
+            *reinterpret_cast<uint32_t*>(S + o11) = re;
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the tensor core reads what was written
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t taddr = tmem_slot;
-        if (tid == 0) {
-            for (int s = 0; s < kZSums; ++s) {
-                uint32_t acc = 0u;
-                for (int a = max(0, s - kZDig + 1); a <= min(s, kZDig - 1); ++a)
-                    for (int kk = 0; kk < 4; ++kk) {
-                        const uint64_t ad = z_desc(z_smem(As) + a * kZABytes + kk * 32u);
-                        const uint64_t bd = z_desc(z_smem(Bs) + (s - a) * kZBBytes + kk * 32u);
-                        asm volatile(
-                            "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-                            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(taddr + s * kZN),
-                            "l"(ad), "l"(bd), "r"(kZIdesc), "r"(acc));
-                        acc = 1u;
-                    }
-            }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar_addr)
-                         : "memory");
+    };
+    // one thread: the digit products of buffer u into its half of the tensor memory.  Digit a of A
+    // times digits 0 .. of B is one product: B's digits lie one behind the other, 32 rows each, and
+    // so do the sums a + b.  29 products of up to 224 columns, where digit by digit 136 products of
+    // 32 columns took 75 ns each whatever their width.
+    auto products = [&](int u) {
+        const uint32_t taddr = tmem_slot + u * kZSums * kZN;
+        const uint64_t ad = z_desc(z_smem(As)), bd = z_desc(z_smem(Bs) + u * kZDig * kZBBytes);
+        auto mma = [&](int a, int b0, int nb, int kk, uint32_t acc) {
+            asm volatile(
+                "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(taddr + (a + b0) * kZN),
+                "l"(ad + (a * kZABytes + kk * 32) / 16), "l"(bd + (b0 * kZBBytes + kk * 32) / 16),
+                "r"(z_idesc(nb * kZN)), "r"(acc));
+        };
+#pragma unroll
+        for (int a = 0; a < kZDig; ++a) {
+            const int nb = min(kZDig, kZSums - a);
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+                if (a == 1 && kk == 0) {   // the last sum begins here
+                    mma(a, nb - 1, 1, kk, 0u);
+                    mma(a, 0, nb - 1, kk, 1u);
+                } else
+                    mma(a, 0, nb, kk, a > 0 || kk > 0 ? 1u : 0u);
         }
-        // the entries to update, while the products run
-        const int row = r0 + (warp & 3) * 32 + lane, half = warp >> 2;
-        if (!z_wait(mbar_addr, (uint32_t)((t - tile0) & 1))) s_fail = 1;
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(z_smem(&mbar[u]))
+                     : "memory");
+    };
+    const int ra = (warp & 3) * 32 + lane, row = r0 + ra, half = warp >> 2;   // half: which 8 columns of a tile
+    bool fail = false;   // a wait ran out (warp-uniform)
+    cut_b(0, 0);
+    load_b(tile0 + 1);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (tid == 0 && tile0 < tile1) products(0);
+    for (int t = tile0; t < tile1; ++t) {
+        const int u = (t - tile0) & 1, c0 = t * kZNc;
+        cplx cc[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int col = c0 + half * 8 + q;
+            cc[q] = row < J.m && col < J.n ? C[row + (long long)col * J.ldc] : mk(0.);
+        }
+        // the next tile's digits go where those of the tile before this one were, whose products
+        // this thread has waited for; its exponents do not, slower warps may still read them (three
+        // rounds: the barrier below has every warp past the tile before that one)
+        if (t + 1 < tile1) cut_b(u ^ 1, (t + 1 - tile0) % 3);
+        load_b(t + 2);
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        if (__syncthreads_or(fail)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const bool bad = __syncthreads_or(s_fail);
-        const int Er = max(s_ea[0][(warp & 3) * 32 + lane], s_ea[1][(warp & 3) * 32 + lane]);
-        const uint32_t lane_base = taddr + ((uint32_t)((warp & 3) * 32) << 16);
-        for (int j0 = half * 16; j0 < half * 16 + 16; j0 += 4) {
+        if (tid == 0 && t + 1 < tile1) products(u ^ 1);
+        __syncwarp();
+        fail = __any_sync(0xffffffffu, !z_wait(z_smem(&mbar[u]), (uint32_t)(((t - tile0) >> 1) & 1)));
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const int Er = max(s_ea[0][ra], s_ea[1][ra]);
+        const uint32_t lane_base = tmem_slot + u * kZSums * kZN + ((uint32_t)((warp & 3) * 32) << 16);
+#pragma unroll
+        for (int jq = 0; jq < 2; ++jq) {
+            const int j0 = half * 8 + 4 * jq;
             uint32_t re[kZSums][4], im[kZSums][4];
-            if (!bad) {
+            if (!fail) {
 #pragma unroll
                 for (int s = 0; s < kZSums; ++s) {
                     z_ld4(lane_base + s * kZN + j0, re[s]);
@@ -264,32 +316,20 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zgemm_tc(ZJob J) {
                 for (int jj = 0; jj < 4; ++jj) {
                     const int col = c0 + j0 + jj;
                     if (col >= J.n) continue;
-                    // sums 0..3 and 4..7 as integers of weight 2^32 and 1, together in units of 2^16
-                    auto join = [&](const uint32_t (&d)[kZSums][4]) {
-                        long long hi = 0, lo = 0;
-#pragma unroll
-                        for (int s = 0; s < 4; ++s) {
-                            hi = (hi << 8) + (long long)__float2int_rn(__uint_as_float(d[s][jj]));
-                            lo = (lo << 8) + (long long)__float2int_rn(__uint_as_float(d[4 + s][jj]));
-                        }
-                        return (hi << 16) + ((lo + 0x8000) >> 16);
-                    };
-                    const double sc = bad ? CUDART_NAN : z_scale(Er, s_eb[j0 + jj]);   // a wait that ran out shows
-                    cplx* p = C + row + (long long)col * J.ldc;
-                    const cplx c = *p;
-                    *p = mk(fma(-sc, (double)join(re), c.re), fma(-sc, (double)join(im), c.im));
+                    const double sc = fail ? CUDART_NAN : z_scale(Er, s_eb[(t - tile0) % 3][j0 + jj]);   // a wait that ran out shows
+                    const cplx c = cc[4 * jq + jj];
+                    C[row + (long long)col * J.ldc] =
+                        mk(fma(-sc, (double)z_join(re, jj), c.re), fma(-sc, (double)z_join(im, jj), c.im));
                 }
             }
         }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();   // B's digits, the sums and s_eb are free
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (bad) {   // another bounded chance for the products before the memory is given back
-            z_wait(mbar_addr, (uint32_t)((t - tile0) & 1));
-            break;
-        }
     }
-    __syncthreads();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    if (__syncthreads_or(fail)) {   // another bounded chance for the products before the memory is given back
+        for (int u = 0; u < 2; ++u)
+            for (uint32_t par = 0; par < 2; ++par) z_wait(z_smem(&mbar[u]), par);
+        __syncthreads();
+    }
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_slot), "r"(512u));
 }
