@@ -4,10 +4,15 @@
 // T(k)) and :205 (the bordered Wielandt system of sv_der2).
 //
 // Right-looking blocked factorisation, panel width 32, three launches per panel:
-//   k_lu_panel      one CTA per matrix: unblocked LU of the n-k0 x 32 panel
-//   k_lu_swap_trsm  row exchanges on every column block outside the panel and
-//                   U12 = L11^-1 A12 on the blocks right of it
-//   k_lu_gemm       A22 -= L21 U12, 64 x 64 tiles, all matrices in one grid
+//   k_lu_panel      unblocked LU of the n-k0 x 32 panel, one CTA per matrix, or
+//                   k_lu_panel_cluster, a cluster of up to 16
+//   k_lu_swap_trsm  row exchanges on every column outside the panel and
+//                   U12 = L11^-1 A12 on the columns right of it
+//   k_lu_gemm       A22 -= L21 U12, 64 x 64 tiles, all matrices in one grid; large ones
+//                   on the tensor cores (zgemm_tc.cu, tc_gemm.cu)
+// Four complex128 matrices of order 1500: 43 panels on clusters 5.4 ms, exchanges and
+// triangular solves 1.5 (71 us a launch with serial exchanges, 31 now: its FP64 steps), updates
+// 3.6 (6.0 before the second tile buffer of zgemm_tc.cu).
 // Matrices are column-major with leading dimension n (Eigen's layout); matrix m
 // starts at A + m * stride.  piv[m*n + k] = row exchanged with row k at step k
 // (LAPACK's ipiv, 0-based); perm[m*n + i] = source row of row i of P A.
@@ -24,6 +29,7 @@ namespace hbem {
 
 constexpr int kLuNB = 32;
 constexpr int kLuPanelThreads = 512;
+constexpr int kLuClusterThreads = 512;   // a multiple of 128
 constexpr int kLuTile = 64;
 constexpr int kLuTcMin = 128;            // smallest trailing order the complex128 tensor-core update takes
 constexpr int kLuSolveThreads = 512;
@@ -44,17 +50,12 @@ __device__ __forceinline__ unsigned long long pivot_key(cplxf z) {
     const unsigned b = __float_as_uint(norm2(z));
     return b > 0x7f800000u ? 0ull : (unsigned long long)b + 1;
 }
-__device__ __forceinline__ void pivot_max(PivotKey& a, unsigned long long v, int i) {   // ties: the smaller index
-    if (v > a.v || (v == a.v && i < a.i)) { a.v = v; a.i = i; }
-}
+// the largest of a warp's candidates; ties: the smaller index
 __device__ __forceinline__ PivotKey pivot_warp_max(PivotKey a) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long ov = __shfl_xor_sync(0xffffffffu, a.v, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, a.i, o);
-        pivot_max(a, ov, oi);
-    }
-    return a;
+    const unsigned hi = (unsigned)(a.v >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)a.v : 0u);
+    const unsigned long long v = ((unsigned long long)mh << 32) | ml;
+    return PivotKey{v, (int)__reduce_min_sync(0xffffffffu, a.v == v ? (unsigned)a.i : 0xffffffffu)};
 }
 
 // Row i of the rank-1 update of a panel step, shared over the CTA: threads take (row, every
@@ -148,12 +149,16 @@ __global__ void __launch_bounds__(kLuPanelThreads) k_lu_panel(int n, int k0, int
 // The same on a cluster of CS CTAs per matrix (grid nmat * CS), CTA r holding panel rows
 // [k0 + r R, k0 + (r + 1) R) in its shared memory (column-major, leading dimension R): for
 // panels too tall for one CTA, and for few matrices because the FP64 rate of one SM bounds
-// the rank-1 updates.  Per column: every CTA posts its pivot candidate, all read all
-// candidates through distributed shared memory (cluster barrier 1), every CTA copies the
-// pivot row, the owner of the pivot row copies the row it will receive (barrier 2), the two
-// owners write the exchanged rows, and each CTA applies the rank-1 update to its own rows.
+// the rank-1 updates.  What is left is a chain of dependent steps per column, kept to one
+// cluster barrier: before it every CTA writes its candidate into all the others' shared memory
+// and posts that whole row in its own, and row c's owner posts row c; after it all read the
+// winner's posted row through distributed shared memory, and the two owners write the exchanged
+// rows.  The posts alternate between two buffers: a buffer is written again two columns on, past
+// a barrier that every reader reached after its reads.  The next column's candidates come out of
+// the rank-1 update, and the pivots go to global memory at the end (the barrier would wait for
+// the write).
 template <class E>
-__global__ void __launch_bounds__(kLuPanelThreads) k_lu_panel_cluster(int n, int k0, int nb, int R, E* A,
+__global__ void __launch_bounds__(kLuClusterThreads) k_lu_panel_cluster(int n, int k0, int nb, int R, E* A,
                                                                       long long stride, int* piv, int* info) {
     cg::cluster_group cl = cg::this_cluster();
     const int ncta = (int)cl.num_blocks(), rank = (int)cl.block_rank();
@@ -161,58 +166,57 @@ __global__ void __launch_bounds__(kLuPanelThreads) k_lu_panel_cluster(int n, int
     extern __shared__ double panel_sm[];
     E* P = reinterpret_cast<E*>(panel_sm);
     E* lcol = P + (long long)R * nb;
-    __shared__ PivotKey post, cand[kLuPanelThreads / 32];
-    __shared__ E prow[kLuNB], tmp[kLuNB], s_id;
-    __shared__ int s_p;
+    __shared__ PivotKey post[2][16], cand[kLuClusterThreads / 32];
+    __shared__ int s_piv[kLuNB], s_info;
+    __shared__ E post_row[2][kLuNB], post_c[2][kLuNB], prow[kLuNB], s_id;
     E* M = A + (long long)mat * stride;
     int* pv = piv + (long long)mat * n;
     const int r0 = k0 + rank * R, r1 = min(n, r0 + R), rows = max(0, r1 - r0);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int tr = threadIdx.x & 127, part = threadIdx.x >> 7;   // a row and every so many columns
     for (int e = threadIdx.x; e < rows * nb; e += blockDim.x)
         P[(e % rows) + (e / rows) * R] = M[(r0 + e % rows) + (long long)(k0 + e / rows) * n];
-    __syncthreads();
-    for (int j = 0; j < nb; ++j) {
-        const int c = k0 + j, first = max(c, r0) - r0;      // local index of the first row left
+    if (threadIdx.x == 0) s_info = 0;
+    cl.sync();   // every CTA runs before another writes into it
+    {
         PivotKey best{0ull, n};
-        for (int i = first + threadIdx.x; i < rows; i += blockDim.x) {
-            const unsigned long long a = pivot_key(P[i + j * R]);
+        for (int i = threadIdx.x; i < rows; i += blockDim.x) {
+            const unsigned long long a = pivot_key(P[i]);
             if (a > best.v) { best.v = a; best.i = r0 + i; }
         }
         best = pivot_warp_max(best);
         if (lane == 0) cand[warp] = best;
-        __syncthreads();
+    }
+    __syncthreads();
+    for (int j = 0; j < nb; ++j) {
+        const int c = k0 + j, rc = j / R, b = j & 1;
         if (warp == 0) {
-            best = lane < nw ? cand[lane] : PivotKey{0ull, n};
-            best = pivot_warp_max(best);
-            if (lane == 0) post = best;
-        }
-        cl.sync();                                                   // (1) candidates posted
-        if (warp == 0) {
-            best = lane < ncta ? *cl.map_shared_rank(&post, lane) : PivotKey{0ull, n};
-            best = pivot_warp_max(best);
-            if (best.v == 0ull) best.i = c;
-            const int p = best.i;
-            if (lane == 0) {
-                s_p = p;
-                if (rank == 0) {
-                    pv[c] = p;
-                    if (best.v == 1ull && info[mat] == 0) info[mat] = c + 1;
-                }
+            const PivotKey mine = pivot_warp_max(lane < nw ? cand[lane] : PivotKey{0ull, n});
+            if (lane < ncta) *cl.map_shared_rank(&post[b][rank], lane) = mine;
+            if (lane < nb) {
+                if (mine.v) post_row[b][lane] = P[(mine.i - r0) + lane * R];
+                if (rank == rc) post_c[b][lane] = P[(c - r0) + lane * R];
             }
-            const int rp = (p - k0) / R, rc = (c - k0) / R;
+        }
+        cl.sync();
+        if (warp == 0) {
+            PivotKey best = pivot_warp_max(lane < ncta ? post[b][lane] : PivotKey{0ull, n});
+            if (best.v == 0ull) best.i = c;
+            const int p = best.i, rp = (p - k0) / R;
+            if (lane == 0) {
+                s_piv[j] = p;
+                if (best.v == 1ull && s_info == 0) s_info = c + 1;
+            }
             E y = Elem<E>::zero();
             if (lane < nb) {
-                y = cl.map_shared_rank(P, rp)[(p - (k0 + rp * R)) + lane * R];
+                y = p == c ? cl.map_shared_rank(&post_c[b][0], rc)[lane] : cl.map_shared_rank(&post_row[b][0], rp)[lane];
                 prow[lane] = y;
-                if (rank == rp && p != c) tmp[lane] = cl.map_shared_rank(P, rc)[(c - (k0 + rc * R)) + lane * R];
+                if (p != c) {
+                    if (rank == rc) P[(c - r0) + lane * R] = y;
+                    if (rank == rp) P[(p - r0) + lane * R] = cl.map_shared_rank(&post_c[b][0], rc)[lane];
+                }
             }
             if (lane == j) s_id = norm2(y) > 0 ? cdiv(Elem<E>::one(), y) : Elem<E>::one();   // zero pivot: unscaled
-        }
-        cl.sync();                                                   // (2) rows c and p read
-        const int p = s_p, rp = (p - k0) / R, rc = (c - k0) / R;
-        if (threadIdx.x < nb && p != c) {
-            if (rank == rc) P[(c - r0) + threadIdx.x * R] = prow[threadIdx.x];
-            if (rank == rp) P[(p - r0) + threadIdx.x * R] = tmp[threadIdx.x];
         }
         __syncthreads();
         const E id = s_id;
@@ -223,58 +227,115 @@ __global__ void __launch_bounds__(kLuPanelThreads) k_lu_panel_cluster(int n, int
             lcol[i] = l;
         }
         __syncthreads();
-        panel_rank1(P, R, i0, rows, j, nb, lcol, prow);
+        PivotKey best{0ull, n};
+        for (int i = i0 + tr; i < rows; i += 128) {
+            const E l = lcol[i];
+            // complex64: four loads, then four updates (latency; 129 -> 89 us a panel of order 3000
+            // with the finer split).  complex128: the FP64 pipe is what waits, and alternates better
+            // one by one (126 us; 150 in fours, order 1500)
+            constexpr int kStep = kLuClusterThreads / 128, kBatch = std::is_same<E, cplxf>::value ? 4 : 1;
+            for (int cc = j + 1 + part; cc < nb; cc += kBatch * kStep) {
+                E z[kBatch];
+#pragma unroll
+                for (int q = 0; q < kBatch; ++q)
+                    if (cc + q * kStep < nb) z[q] = P[i + (cc + q * kStep) * R];
+#pragma unroll
+                for (int q = 0; q < kBatch; ++q)
+                    if (cc + q * kStep < nb) {
+                        cfms(z[q], l, prow[cc + q * kStep]);
+                        P[i + (cc + q * kStep) * R] = z[q];
+                    }
+                if (cc == j + 1) {
+                    const unsigned long long a = pivot_key(z[0]);
+                    if (a > best.v) { best.v = a; best.i = r0 + i; }
+                }
+            }
+        }
+        best = pivot_warp_max(best);
+        if (lane == 0) cand[warp] = best;
         __syncthreads();
     }
     for (int e = threadIdx.x; e < rows * nb; e += blockDim.x)
         M[(r0 + e % rows) + (long long)(k0 + e / rows) * n] = P[(e % rows) + (e / rows) * R];
+    if (rank == 0) {
+        if (threadIdx.x < nb) pv[k0 + threadIdx.x] = s_piv[threadIdx.x];
+        if (threadIdx.x == 0 && s_info && info[mat] == 0) info[mat] = s_info;
+    }
     cl.sync();   // no CTA leaves while another may still read its shared memory
 }
 
-// grid (ceil(n/32), nmat): column block b covers columns [32 b, 32 b + 32).  Columns
-// from cmax on are left alone (the two-level factorisation exchanges and solves them
+// Row exchanges of a panel's nb <= 32 columns on every column outside the panel, and
+// U12 = L11^-1 A12 on the columns right of it.  grid (ceil(n / 16), nmat), 16 columns a CTA;
+// columns from cmax on are left alone (the two-level factorisation exchanges and solves them
 // once per 128-column block, k_lu_swap_trsm_block).
+// The exchanges are composed into one gather over the at most 64 rows they touch (slot x < 32:
+// row k0 + x; slot 32 + j: the pivot of step j where it lies below the panel), so that a column
+// waits for memory once and not 32 times.  Eight lanes to a column, lane r holding rows r, r + 8,
+// r + 16, r + 24: the substitution takes 80 FP64 steps for four columns where a warp per column,
+// half idle, takes 128 for one.
+constexpr int kLuSwapCols = 16;
 template <class E>
-__global__ void __launch_bounds__(256) k_lu_swap_trsm(int n, int k0, int nb, E* A, long long stride,
-                                                      const int* piv, int cmax) {
-    const int col0 = blockIdx.x * kLuNB;
-    if (col0 == k0 || col0 >= cmax) return;            // the panel itself, or deferred
+__global__ void __launch_bounds__(kLuSwapCols * 8) k_lu_swap_trsm(int n, int k0, int nb, E* A, long long stride,
+                                                                  const int* piv, int cmax) {
+    const int col0 = blockIdx.x * kLuSwapCols;
+    if ((col0 >= k0 && col0 < k0 + nb) || col0 >= cmax) return;   // the panel itself, or deferred
     E* M = A + (long long)blockIdx.y * stride;
     const int* pv = piv + (long long)blockIdx.y * n;
-    const int ncols = min(kLuNB, n - col0);
-    __shared__ int sp[kLuNB];
-    __shared__ E L11[kLuNB][kLuNB + 1];
-    if (threadIdx.x < nb) sp[threadIdx.x] = pv[k0 + threadIdx.x];
-    __syncthreads();
-    if (threadIdx.x < ncols) {
-        E* a = M + (long long)(col0 + threadIdx.x) * n;
-        for (int j = 0; j < nb; ++j) {
-            const int p = sp[j];
-            if (p != k0 + j) {
-                const E t = a[k0 + j];
-                a[k0 + j] = a[p];
-                a[p] = t;
-            }
-        }
-    }
-    if (col0 < k0) return;                             // left of the panel: exchanges only
-    for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-        const int r = e % nb, k = e / nb;
-        L11[r][k] = M[(k0 + r) + (long long)(k0 + k) * n];
-    }
-    __syncthreads();
+    __shared__ int pos[64], from[64];       // the slot's row (-1: none), the row its entry comes from
+    __shared__ E L11[kLuNB][kLuNB + 1];     // [k][r]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int cc = warp; cc < ncols; cc += (blockDim.x >> 5)) {
-        E* a = M + (long long)(col0 + cc) * n + k0;
-        E x = lane < nb ? a[lane] : Elem<E>::zero();
-        for (int k = 0; k < nb; ++k) {
-            E xk;
-            xk.re = __shfl_sync(0xffffffffu, x.re, k);
-            xk.im = __shfl_sync(0xffffffffu, x.im, k);
-            if (lane > k && lane < nb) cfms(x, L11[lane][k], xk);
+    if (warp == 0) {
+        const int p = lane < nb ? pv[k0 + lane] : -1 - lane;
+        const int first = __ffs(__match_any_sync(0xffffffffu, p)) - 1;
+        const bool below = lane < nb && p >= k0 + nb;
+        const int slot = lane >= nb ? lane : below ? 32 + first : p - k0;
+        pos[lane] = lane < nb ? k0 + lane : -1;
+        pos[32 + lane] = below && first == lane ? p : -1;
+        int x = lane, y = 32 + lane;        // where the final entries of slots lane, 32 + lane were
+        for (int j = nb - 1; j >= 0; --j) {
+            const int s = __shfl_sync(0xffffffffu, slot, j);
+            x = x == j ? s : x == s ? j : x;
+            y = y == j ? s : y == s ? j : y;
         }
-        if (lane < nb) a[lane] = x;
+        __syncwarp();
+        from[lane] = pos[x];
+        from[32 + lane] = pos[y];
     }
+    if (col0 > k0)
+        for (int e = threadIdx.x; e < kLuNB * kLuNB; e += blockDim.x) {
+            const int r = e % kLuNB, k = e / kLuNB;
+            L11[k][r] = r < nb && k < nb ? M[(k0 + r) + (long long)(k0 + k) * n] : Elem<E>::zero();
+        }
+    __syncthreads();
+    const int col = col0 + (threadIdx.x >> 3), r = lane & 7;
+    const bool in = col < min(n, cmax);
+    E* a = M + (long long)(in ? col : col0) * n;
+    E v[4], w[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int s = r + 8 * q;
+        v[q] = in && pos[s] >= 0 ? a[from[s]] : Elem<E>::zero();
+        w[q] = in && pos[32 + s] >= 0 ? a[from[32 + s]] : Elem<E>::zero();
+    }
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        if (in && pos[32 + r + 8 * q] >= 0) a[pos[32 + r + 8 * q]] = w[q];
+    if (col0 > k0) {
+#pragma unroll
+        for (int k = 0; k < kLuNB; ++k) {
+            if (k >= nb) break;
+            E xk;
+            xk.re = __shfl_sync(0xffffffffu, v[k >> 3].re, (lane & 24) + (k & 7));
+            xk.im = __shfl_sync(0xffffffffu, v[k >> 3].im, (lane & 24) + (k & 7));
+#pragma unroll
+            for (int q = k >> 3; q < 4; ++q)
+                if (q > (k >> 3) || r > (k & 7)) cfms(v[q], L11[k][r + 8 * q], xk);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        if (in && pos[r + 8 * q] >= 0) a[pos[r + 8 * q]] = v[q];
 }
 
 // Two-level factorisation, after the kb (<= 128) columns from K0 are factored: the
@@ -645,6 +706,9 @@ __global__ void __launch_bounds__(kLuSolveThreads) k_lu_solve(int n, int s, int 
 // block's rows multiply them at once by the inverse of its triangle.  The 32 x 32 inverses
 // are made once per factorisation (k_diag_inv): substitution there, 32 dependent steps of
 // FP64 FMAs and shuffles on one warp, was two thirds of a launch (14.8 us; 6 with them).
+// The launches of a sweep are programmatic dependents of one another: a launch comes up and
+// reads its part of the factors, which no launch of the sweep writes, while the one before it
+// still runs, and waits for that one's end before it touches X.
 enum SolveSweep { kSweepL = 0, kSweepU = 1, kSweepUH = 2, kSweepLH = 3 };   // L y = b, U x = y; U^H y = b, L^H x = y
 
 size_t lu_dinv_elems(int n) { return (size_t)((n + kLuNB - 1) / kLuNB) * kLuNB * kLuNB; }
@@ -697,6 +761,7 @@ __global__ void __launch_bounds__(128) k_solve_step(int n, int s, int cur, const
     const E* M = LU + (long long)blockIdx.z * stride;
     E* Xm = X + (long long)blockIdx.z * xstride + (long long)c0 * n;
     const int r0 = blk * kLuNB, nr = min(kLuNB, n - r0);
+    asm volatile("griddepcontrol.launch_dependents;");
     if (t == 0) {
         const E* Db = dinv + ((long long)blockIdx.z * nb + blk) * kLuNB * kLuNB;
         for (int c = warp; c < kLuNB; c += 4) {                    // (row lane, column c) of the stored inverses
@@ -709,25 +774,31 @@ __global__ void __launch_bounds__(128) k_solve_step(int n, int s, int cur, const
         }
     }
     const bool update = ASC ? cur >= 0 : cur < nb;
-    E yold[CPC];
-#pragma unroll
-    for (int c = 0; c < CPC; ++c) yold[c] = (warp == 0 && c < cs && lane < nr) ? Xm[(long long)c * n + r0 + lane] : Elem<E>::zero();
+    const int k0 = cur * kLuNB, nk = min(kLuNB, n - k0);
+    E w[8];
     if (update) {
-        const int k0 = cur * kLuNB, nk = min(kLuNB, n - k0);
-        for (int e = threadIdx.x; e < CPC * kLuNB; e += 128) {
-            const int c = e / kLuNB, k = e - c * kLuNB;
-            xs[c][k] = (c < cs && k < nk) ? Xm[(long long)c * n + k0 + k] : Elem<E>::zero();
-        }
-        E w[8];
         if (HERM) {   // conj(M[k, r]): columns r of the factor, contiguous in k
-            for (int r = warp; r < kLuNB; r += 4)
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int r = warp + 4 * q;
                 W[lane][r] = (lane < nk && r < nr) ? conj(M[(k0 + lane) + (long long)(r0 + r) * n]) : Elem<E>::zero();
+            }
         } else {
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
                 const int k = 8 * warp + q;
                 w[q] = (lane < nr && k < nk) ? M[(r0 + lane) + (long long)(k0 + k) * n] : Elem<E>::zero();
             }
+        }
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // X from here on
+    E yold[CPC];
+#pragma unroll
+    for (int c = 0; c < CPC; ++c) yold[c] = (warp == 0 && c < cs && lane < nr) ? Xm[(long long)c * n + r0 + lane] : Elem<E>::zero();
+    if (update) {
+        for (int e = threadIdx.x; e < CPC * kLuNB; e += 128) {
+            const int c = e / kLuNB, k = e - c * kLuNB;
+            xs[c][k] = (c < cs && k < nk) ? Xm[(long long)c * n + k0 + k] : Elem<E>::zero();
         }
         __syncthreads();
         E acc[CPC];
@@ -815,12 +886,13 @@ cudaError_t launch_cgemm_f32(int m, int n, int k, const cplxf* A, long long lda,
 size_t panel_smem(int rows, int nb, size_t esz) { return (size_t)rows * (nb + 1) * esz; }
 
 // CTAs per matrix that a panel of m rows is best split over when nmat matrices share the
-// 152 SMs: as long as a CTA keeps enough rows that its share of the rank-1 updates is not
-// less than the two cluster barriers of a column (about 2 us; complex128: 64 rows, 16 columns
-// on average, 4 FMAs at two lanes a cycle: 2 us; complex64 is latency bound at any size).
+// 152 SMs: as long as a CTA keeps enough rows that its share of a column's work is not less
+// than the column's cluster barrier (about a microsecond; complex128: 64 rows, 16 columns on
+// average, 4 FMAs at two lanes a cycle: 2 us; complex64, 96 rows: order 3000 takes 89 us a panel
+// on 16 CTAs, 129 on 8).
 template <class E>
 int panel_split(int m, int nmat) {
-    const int least = std::is_same<E, cplx>::value ? 64 : 384;
+    const int least = std::is_same<E, cplx>::value ? 64 : 96;
     int cs = 1;
     while (cs < 16 && 2LL * cs * nmat <= 152 && m / (2 * cs) >= least) cs *= 2;
     return cs;
@@ -858,7 +930,7 @@ cudaError_t launch_panel_cluster(int n, int k0, int nb, int nmat, E* A, long lon
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(nmat * cs));
-    cfg.blockDim = dim3(kLuPanelThreads);
+    cfg.blockDim = dim3(kLuClusterThreads);
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -914,7 +986,7 @@ cudaError_t lu_factor_impl(int n, int nmat, E* A, long long stride, int* piv, in
     auto panel_step = [&](int k0, int nb, int cmax, int cend) -> cudaError_t {
         if (cudaError_t e2 = panel(k0, nb); e2 != cudaSuccess) return e2;
         if (ncb > 1) {
-            k_lu_swap_trsm<E><<<dim3(ncb, nmat), 256, 0, st>>>(n, k0, nb, A, stride, piv, cmax);
+            k_lu_swap_trsm<E><<<dim3((n + kLuSwapCols - 1) / kLuSwapCols, nmat), kLuSwapCols * 8, 0, st>>>(n, k0, nb, A, stride, piv, cmax);
             ++nl;
         }
         const int t0 = k0 + nb;
@@ -963,7 +1035,7 @@ cudaError_t lu_factor_impl(int n, int nmat, E* A, long long stride, int* piv, in
             e = panel(k0, nb);
             if (e != cudaSuccess) return e;
             if (ncb > 1) {
-                k_lu_swap_trsm<E><<<dim3(ncb, nmat), 256, 0, st>>>(n, k0, nb, A, stride, piv, n);
+                k_lu_swap_trsm<E><<<dim3((n + kLuSwapCols - 1) / kLuSwapCols, nmat), kLuSwapCols * 8, 0, st>>>(n, k0, nb, A, stride, piv, n);
                 ++nl;
             }
             const int m = n - k0 - nb;
@@ -1014,10 +1086,21 @@ cudaError_t lu_solve_steps(int n, int nmat, int trans, const E* LU, long long st
         e != cudaSuccess)
         return e;
     const int nb = (n + kLuNB - 1) / kLuNB, cg = (s + CPC - 1) / CPC;
+    // the first launch of a sweep waits for all before it, the others only where they say so
+    cudaError_t e = cudaSuccess;
     auto sweep = [&](auto kernel, bool asc) {
-        for (int q = -1; q < nb - 1; ++q) {
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.blockDim = dim3(128);
+        cfg.stream = st;
+        cfg.attrs = at;
+        for (int q = -1; q < nb - 1 && e == cudaSuccess; ++q) {
             const int cur = asc ? q : nb - 1 - q, tiles = q < 0 ? 1 : nb - 1 - q;
-            kernel<<<dim3(tiles, cg, nmat), 128, 0, st>>>(n, s, cur, LU, stride, dinv, X, xstride);
+            cfg.gridDim = dim3(tiles, cg, nmat);
+            cfg.numAttrs = q < 0 ? 0 : 1;
+            e = cudaLaunchKernelEx(&cfg, kernel, n, s, cur, LU, stride, dinv, X, xstride);
         }
     };
     if (trans) {
@@ -1029,6 +1112,7 @@ cudaError_t lu_solve_steps(int n, int nmat, int trans, const E* LU, long long st
         sweep(k_solve_step<E, kSweepL, CPC>, true);
         sweep(k_solve_step<E, kSweepU, CPC>, false);
     }
+    if (e != cudaSuccess) return e;
     return cudaGetLastError();
 }
 
