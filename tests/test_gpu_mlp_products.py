@@ -16,7 +16,8 @@ from helmholtzbem_gb300 import _capi as C  # noqa: E402
 
 
 @pytest.mark.parametrize("M,N,K", [(128, 128, 64), (128, 256, 512), (256, 128, 576), (384, 128, 1088),
-                                   (1920, 1280, 448), (2432, 1024, 384), (2432, 1024, 64)])
+                                   (1920, 1280, 448), (2432, 1024, 384), (2432, 1024, 64),
+                                   (256, 2432, 448), (384, 1664, 384), (384, 1664, 64)])
 def test_products(M, N, K):
     g = torch.Generator().manual_seed(M + N + K)
     A = torch.randn((M, K), generator=g).to(torch.bfloat16).cuda()
