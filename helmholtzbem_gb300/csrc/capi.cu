@@ -904,7 +904,12 @@ int hbem_assemble_dense_sub(hbem_builder b, double k_re, double k_im, double c, 
     HB_CK(cudaSetDevice(b->device));
     const long long np = b->npair();
     const size_t loc_bytes = (size_t)np * (d + 1) * kLocPerD * sizeof(cplx);
-    HB_CK(b->d_loc.ensure(loc_bytes));
+    // behind the pair blocks the partial sums of a split singular launch (one medium: a pair per
+    // CTA leaves most of the GPU idle; 24 panels, order 7: 67 -> 46 us, caches cold)
+    const size_t part_bytes =
+        (g_singular_split && !t_split_hold) ? singular_part_bytes((int)b->tasks.size(), 1, (int)d, !b->lines) : 0;
+    HB_CK(b->d_loc.ensure(loc_bytes + part_bytes));
+    double* part = part_bytes ? reinterpret_cast<double*>(b->d_loc.as<char>() + loc_bytes) : nullptr;
     std::vector<Job> jobs{Job{k_re, k_im, c}};
     HB_CK(upload(b->d_jobs, jobs, b->st));
     int nl = ((layers & 1) != 0) + ((layers & 2) != 0) + ((layers & 4) != 0);
@@ -912,7 +917,7 @@ int hbem_assemble_dense_sub(hbem_builder b, double k_re, double k_im, double c, 
     bool real_k = (k_im == 0. && k_re > 0.);
     if (!real_k) HB_CK(b->ensure_sgeo());
     HB_CK(local_assembly(b->view(), b->d_tasks.as<SingularTask>(), (int)b->tasks.size(), b->n, b->d_jobs.as<Job>(), 1,
-                         real_k, false, (int)d, b->d_loc.as<cplx>(), b->st));
+                         real_k, false, (int)d, b->d_loc.as<cplx>(), b->st, part));
     if (rows == (unsigned)b->n && cols == (unsigned)b->n)
         HB_CK(launch_gather_layers(b->n, (int)d, (int)layers, b->d_loc.as<cplx>(), 0, b->sp(), b->d_layers.as<cplx>(),
                                    b->st));
