@@ -601,6 +601,9 @@ __global__ void __launch_bounds__(128, 2) k_general(DevMesh M, const Job* jobs, 
     const KConst K = make_kconst(jobs[job]);
     general_rows<D, CURVED>(M, K, blockIdx.x * (long long)(128 / M.p), sx, sw, reinterpret_cast<cplx*>(gsm),
                             loc + (long long)job * npair * (D + 1) * kLocPerD);
+    // Launched as a programmatic dependent of the singular pairs' kernel, which it needs nothing
+    // of: it fills the SMs that kernel leaves idle, and ends after it for those who read both.
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // Complex wavenumbers: general pair number q of mesh M (in the builder's order by
@@ -1291,8 +1294,18 @@ static cudaError_t launch_local_c(const DevMesh& M, const SingularTask* tasks, i
             const size_t smem = GenDims<D, CURVED>::smem(M.p);
             if (cudaError_t e = allow_smem(k_general<D, CURVED>, smem); e != cudaSuccess) return e;
             const int ppc = 128 / M.p;
-            k_general<D, CURVED><<<dim3((unsigned)((M.ngen + ppc - 1) / ppc), njobs), 128, smem, st>>>(M, jobs, loc,
-                                                                                                     npair);
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            at[0].val.programmaticStreamSerializationAllowed = 1;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)((M.ngen + ppc - 1) / ppc), njobs);
+            cfg.blockDim = dim3(128);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = st;
+            cfg.attrs = at;
+            cfg.numAttrs = rows ? 1 : 0;   // behind k_singular_rows
+            if (cudaError_t e = cudaLaunchKernelEx(&cfg, k_general<D, CURVED>, M, jobs, loc, npair); e != cudaSuccess)
+                return e;
         } else {
             int ppw = layout;
             if (layout == kLayoutAuto) {

@@ -261,6 +261,7 @@ __global__ void __launch_bounds__(128, 2) k_singular_rows(DevMesh M, const Singu
                                                           int q, double* part, cplx* loc, long long npair) {
     typedef RowDims<D, CURVED> R;
     extern __shared__ __align__(16) unsigned char ssm[];
+    asm volatile("griddepcontrol.launch_dependents;");   // the general pairs' kernel may fill in behind
     cplx* acc = reinterpret_cast<cplx*>(ssm);
     cplx* mom = acc + R::NA * 128;
     double* sxc = reinterpret_cast<double*>(mom + R::NA);
