@@ -25,12 +25,15 @@
 #include <cmath>
 #include <vector>
 
+#include <cooperative_groups.h>
+
 #include "hbem_device.cuh"
 #include "smem_linalg.cuh"
 
 namespace hbem {
 
-constexpr int kArnThreads = 256;
+constexpr int kArnThreads = 512;
+constexpr int kArnSmemLimit = 220 * 1024;
 constexpr int kArnMaxP = 32;
 
 struct Sv2Work {
@@ -167,9 +170,16 @@ size_t arn_smem_bytes(int n, int p) {
            (128 + kArnMaxP) * sizeof(double) + (2 * (size_t)n + kArnMaxP + 32) * sizeof(int);
 }
 
+// PAIR: a cluster of two CTAs per matrix for launches that leave half the SMs idle otherwise.  An
+// iteration is mostly the two triangular solves, bound by the FP64 rate of one SM and the chains of
+// its columns: each CTA solves half of the block's columns and reads the other half from the other
+// CTA; everything else both compute alike (the same operations on the same numbers), so both
+// forms give the same bits.
+template <bool PAIR>
 __global__ void __launch_bounds__(kArnThreads) k_arn_small(ArnJob J) {
     extern __shared__ double smraw[];
-    const int n = J.n, p = J.p, mat = blockIdx.x;
+    const int n = J.n, p = J.p, mat = PAIR ? blockIdx.x >> 1 : blockIdx.x, rank = PAIR ? blockIdx.x & 1 : 0;
+    const int half = (p + 1) / 2, c0 = rank ? half : 0, cnt = !PAIR ? p : rank ? p - half : half;
     cplx* A = reinterpret_cast<cplx*>(smraw);        // n x n: T, then its LU
     cplx* X = A + (long long)n * n;                  // n x p: Q
     cplx* Y = X + (long long)n * p;                  // n x p: QB, then T^-1 QB
@@ -191,23 +201,35 @@ __global__ void __launch_bounds__(kArnThreads) k_arn_small(ArnJob J) {
     lu_smem(A, n, piv, &s_sing);
     __syncthreads();
     if (s_sing) {
-        arn_fail(J, mat, 5);
+        if (rank == 0) arn_fail(J, mat, 5);
         return;
     }
     perm_from_piv(piv, n, perm);
     lu_inv_diag(A, n);
-    solve_lu_blk(A, perm, n, X, p, buf);
+    auto solve = [&](cplx* Z, bool herm) {
+        if (herm) solve_lu_h_blk(A, perm, n, Z + c0 * n, cnt, buf);
+        else solve_lu_blk(A, perm, n, Z + c0 * n, cnt, buf);
+        if constexpr (PAIR) {
+            cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+            cl.sync();   // both halves are solved
+            const cplx* Zr = cl.map_shared_rank(Z, rank ^ 1);
+            const int o0 = rank ? 0 : half * n, o1 = rank ? half * n : p * n;
+            for (int e = o0 + threadIdx.x; e < o1; e += blockDim.x) Z[e] = Zr[e];
+            cl.sync();   // and read
+        }
+    };
+    solve(X, false);
     qr_cgs2(X, n, p, coef, red);
     int it = 1;
     bool conv = false;
     for (;; ++it) {
         for (int e = threadIdx.x; e < n * p; e += blockDim.x) Y[e] = X[e];
         __syncthreads();
-        solve_lu_h_blk(A, perm, n, Y, p, buf);
+        solve(Y, true);
         qr_cgs2(Y, n, p, coef, red, Rs);
         __syncthreads();
         arn_ritz(Rs, W, p, J.count, nrm, ord, &s_rot);
-        solve_lu_blk(A, perm, n, Y, p, buf);
+        solve(Y, false);
         __syncthreads();
         conv = arn_converged(X, Y, n, p, Rs, W, nrm, ord, J.count, J.tol, red);
         if (conv || it >= J.maxit) break;
@@ -216,6 +238,7 @@ __global__ void __launch_bounds__(kArnThreads) k_arn_small(ArnJob J) {
         X = Y;
         Y = t;
     }
+    if (rank) return;
     arn_write(J, mat, X, W, nrm, ord);
     if (threadIdx.x == 0) {
         J.status[mat] = conv ? 0 : 6;
@@ -318,7 +341,7 @@ struct ArnWork {
 
 int arnoldi_block(int n, int count) { return std::min(std::min(n, kArnMaxP), std::max(12, 2 * count)); }
 
-bool arnoldi_small_fits(int n, int p) { return arn_smem_bytes(n, p) <= 220 * 1024; }
+bool arnoldi_small_fits(int n, int p) { return arn_smem_bytes(n, p) <= kArnSmemLimit; }
 
 // The block must hold the count wanted vectors plus a margin of 4 for the
 // convergence ratio sigma_count / sigma_(p+1), unless it spans the whole space.
@@ -387,8 +410,27 @@ cudaError_t arnoldi_batched(int n, int nmat, int count, int D, double tol, int m
     long long nl = 0;
     if (arnoldi_small_fits(n, p)) {
         const size_t smem = arn_smem_bytes(n, p);
-        AR_CK(cudaFuncSetAttribute(k_arn_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_arn_small<<<nmat, kArnThreads, smem, st>>>(J);
+        // two CTAs a matrix while both fit the 152 SMs (one CTA fills an SM's shared memory from
+        // order 80 or so).  64 matrices of order 100:
+        // 14.5 -> 11.3 ms a call, one 8.0 -> 6.2; 76 of order 32 7.2 -> 6.6
+        if (2 * nmat <= 152) {
+            AR_CK(cudaFuncSetAttribute(k_arn_small<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kArnSmemLimit));
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = 2;
+            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(2 * nmat);
+            cfg.blockDim = dim3(kArnThreads);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = st;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            AR_CK(cudaLaunchKernelEx(&cfg, k_arn_small<true>, J));
+        } else {
+            AR_CK(cudaFuncSetAttribute(k_arn_small<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kArnSmemLimit));
+            k_arn_small<false><<<nmat, kArnThreads, smem, st>>>(J);
+        }
         ++nl;
         AR_CK(cudaGetLastError());
     } else {

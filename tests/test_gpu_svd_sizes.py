@@ -30,3 +30,13 @@ def test_known_singular_values(n, nmat):
     got, ref = np.array(api.sv_dense(mats, d=1)), np.array(ref)
     assert np.abs(got[:, 0] - ref[:, 0]).max() <= 16 * n * np.finfo(float).eps
     assert np.abs(got[:, 1] - ref[:, 1]).max() <= 1e-7
+
+
+@pytest.mark.parametrize("n", [2, 13, 33, 64, 97])
+def test_arnoldi_pairs_of_ctas_give_the_same_bits(n):
+    """76 matrices run on pairs of CTAs, 77 on one CTA each."""
+    rng = np.random.default_rng(n)
+    mats = [[rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))] for _ in range(77)]
+    a, b = api.arnoldi_sv(mats[:76], 1, return_status=True), api.arnoldi_sv(mats, 1, return_status=True)
+    for x, y in zip(a, b):
+        assert np.array_equal(np.asarray(x)[:76], np.asarray(y)[:76], equal_nan=True)
