@@ -927,14 +927,13 @@ def run_gpu(args):
     peak = fp64_peak_tflops()
     roofline = {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                 "frac": achieved / peak if peak else None,
-                # DRAM bytes (read + write) per assembly launch, averaged over the 24
-                # k_singular / k_general(_w) launches of one plain search of this workload
-                # (ncu dram__bytes_read.sum + dram__bytes_write.sum, caches flushed
-                # between launches): the singular launches read the 68 MB point table,
-                # the grid's general launch writes 63 MB of pair blocks
-                "traffic": 3.0e7, "traffic_unit": "bytes per launch",
+                # DRAM bytes (read + write) per assembly launch, averaged over the 150
+                # k_general / k_singular_nodes launches of one plain search of this workload
+                # (ncu dram__bytes_read.sum + dram__bytes_write.sum): the Hankel table, the
+                # node table and the pair blocks stay in L2
+                "traffic": 4.6e5, "traffic_unit": "bytes per launch",
                 "peak_source": "measured: cuBLAS DGEMM 8192^3 on this GPU (MEASURED_PEAKS.json has no FP64 entry)",
-                "kernel": "k_general + k_singular (panel-pair assembly)", "launches": asm_l.value,
+                "kernel": "k_general + k_singular_nodes (panel-pair assembly)", "launches": asm_l.value,
                 "measured_on": "one search of the workload, Newton candidates in lock step (non-overlapping launches)",
                 "avg_launch_ms": asm_ms.value / max(1, asm_l.value),
                 # nominal FP64 peak: 2 DFMA per cycle per SM x 152 SMs at the sampled SM clock
@@ -943,8 +942,8 @@ def run_gpu(args):
                 # x SM clock), from profiles/assembly_kernels_circle_N50_p11_d2.md; the
                 # algorithmic count above uses the reference's per-point work, which this
                 # build's Hankel pair undercuts, so the algorithmic rate reads above these
-                "ncu_executed_fp64_tflops": {"k_general<0> grid": 0.79, "k_singular<0> grid": 0.66,
-                                             "k_singular<2> Newton": 0.77}}
+                "ncu_executed_fp64_tflops": {"k_general<0> grid": 0.83, "k_singular_nodes<0> grid": 0.35,
+                                             "k_general<1> Newton": 0.79}}
 
     scale = assembly_at_scale(torch, C, api, geometry, lib, peak)
     tail = dense_tail_at_scale(torch, C, api, geometry, lib, peak)

@@ -1,4 +1,4 @@
-"""The dense kernel's FP32 stage at the edges of its column layouts: orders below, at and past
+"""Small-matrix kernels.  The dense kernel's FP32 stage at the edges of its column layouts: orders below, at and past
 a change of the leading dimension or of the columns' register count, and the largest that fits.
 
 T = U diag(s) V^H with s known: sigma_min = 0.1, the others in [0.4, 1].  Tolerances: sigma is
@@ -40,3 +40,18 @@ def test_arnoldi_pairs_of_ctas_give_the_same_bits(n):
     a, b = api.arnoldi_sv(mats[:76], 1, return_status=True), api.arnoldi_sv(mats, 1, return_status=True)
     for x, y in zip(a, b):
         assert np.array_equal(np.asarray(x)[:76], np.asarray(y)[:76], equal_nan=True)
+
+
+@pytest.mark.parametrize("count", [6, 8, 9, 14])
+def test_arnoldi_block_widths(count):
+    """Blocks of 12, 16, 18 and 28 columns: the Ritz step's rotations on half-warps up to 16, on
+    whole warps beyond.  Ritz values at a relative residual of 1e-9 are off by its square, and
+    by rounding: n eps |T|^2 / sigma^2 times a few, 60 * 2.2e-16 * 100 * 4 = 5e-12."""
+    n, rng = 60, np.random.default_rng(count)
+    s = np.linspace(0.1, 1.0, n)
+    mats = []
+    for _ in range(3):
+        z = rng.standard_normal((2, n, n)) + 1j * rng.standard_normal((2, n, n))
+        mats.append([(np.linalg.qr(z[0])[0] * s) @ np.linalg.qr(z[1])[0].conj().T])
+    got = api.arnoldi_sv(mats, count, acc=1e-9)[:, :, 0]
+    assert np.abs(got / s[:count] - 1).max() <= 5e-12
