@@ -273,10 +273,15 @@ __global__ void __launch_bounds__(kLuClusterThreads) k_lu_panel_cluster(int n, i
 // waits for memory once and not 32 times.  Eight lanes to a column, lane r holding rows r, r + 8,
 // r + 16, r + 24: the substitution takes 80 FP64 steps for four columns where a warp per column,
 // half idle, takes 128 for one.
+// ek (complex128, or null): per matrix n integers, zero before, that take the biased exponents of
+// the largest entries of U's rows right of their panel (the digit products' scales, zgemm_tc.cu).
 constexpr int kLuSwapCols = 16;
+__device__ __forceinline__ int abs_high(cplx z) {   // high words order like the sizes
+    return max(__double2hiint(z.re) & 0x7fffffff, __double2hiint(z.im) & 0x7fffffff);
+}
 template <class E>
 __global__ void __launch_bounds__(kLuSwapCols * 8) k_lu_swap_trsm(int n, int k0, int nb, E* A, long long stride,
-                                                                  const int* piv, int cmax) {
+                                                                  const int* piv, int cmax, int* ek) {
     const int col0 = blockIdx.x * kLuSwapCols;
     if ((col0 >= k0 && col0 < k0 + nb) || col0 >= cmax) return;   // the panel itself, or deferred
     E* M = A + (long long)blockIdx.y * stride;
@@ -336,6 +341,21 @@ __global__ void __launch_bounds__(kLuSwapCols * 8) k_lu_swap_trsm(int n, int k0,
 #pragma unroll
     for (int q = 0; q < 4; ++q)
         if (in && pos[r + 8 * q] >= 0) a[pos[r + 8 * q]] = v[q];
+    if constexpr (std::is_same<E, cplx>::value) {
+        if (!ek || col0 < k0) return;   // whole CTA
+        __shared__ int high[kLuNB];
+        if (threadIdx.x < kLuNB) high[threadIdx.x] = 0;
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            int h = in ? abs_high(v[q]) : 0;
+            h = max(h, __shfl_xor_sync(0xffffffffu, h, 8));
+            h = max(h, __shfl_xor_sync(0xffffffffu, h, 16));
+            if (lane < 8) atomicMax(&high[r + 8 * q], h);
+        }
+        __syncthreads();
+        if (threadIdx.x < nb) atomicMax(ek + (long long)blockIdx.y * n + k0 + threadIdx.x, high[threadIdx.x] >> 20);
+    }
 }
 
 // Two-level factorisation, after the kb (<= 128) columns from K0 are factored: the
@@ -872,7 +892,7 @@ cudaError_t lu_perm_from_piv(int n, int nmat, const int* piv, int* perm, cudaStr
 
 constexpr size_t kPanelClusterSmem = 200 * 1024;
 int g_lu_cluster_panels = 1;   // 0: tall panels in global memory (kept for comparison tests)
-int g_lu_tensor_cores = 1;     // complex64 trailing updates on the tensor cores
+int g_lu_tensor_cores = 1;     // trailing updates on the tensor cores (complex64 and complex128)
 
 void lu_set_cluster_panels(int on) { g_lu_cluster_panels = on ? 1 : 0; }
 void lu_set_tensor_cores(int on) { g_lu_tensor_cores = on ? 1 : 0; }
@@ -899,7 +919,8 @@ int panel_split(int m, int nmat) {
 }
 
 cudaError_t launch_zgemm_tc(int m, int n, int k, const cplx* A, long long lda, long long sa, const cplx* B, long long ldb,
-                            long long sb, cplx* C, long long ldc, long long sc, int nmat, cudaStream_t st);
+                            long long sb, cplx* C, long long ldc, long long sc, const int* ek, long long se, int nmat,
+                            cudaStream_t st);
 
 // Cluster launch of the panel factorisation: when the panel is too tall for one CTA, or to
 // split it over `want` CTAs.  Returns with *launched = false (nothing launched) when no
@@ -986,7 +1007,8 @@ cudaError_t lu_factor_impl(int n, int nmat, E* A, long long stride, int* piv, in
     auto panel_step = [&](int k0, int nb, int cmax, int cend) -> cudaError_t {
         if (cudaError_t e2 = panel(k0, nb); e2 != cudaSuccess) return e2;
         if (ncb > 1) {
-            k_lu_swap_trsm<E><<<dim3((n + kLuSwapCols - 1) / kLuSwapCols, nmat), kLuSwapCols * 8, 0, st>>>(n, k0, nb, A, stride, piv, cmax);
+            k_lu_swap_trsm<E><<<dim3((n + kLuSwapCols - 1) / kLuSwapCols, nmat), kLuSwapCols * 8, 0, st>>>(
+                n, k0, nb, A, stride, piv, cmax, nullptr);
             ++nl;
         }
         const int t0 = k0 + nb;
@@ -1030,12 +1052,19 @@ cudaError_t lu_factor_impl(int n, int nmat, E* A, long long stride, int* piv, in
             }
         }
     } else {
+        int* ek = nullptr;   // exponents of U's rows, in perm, which is written last
+        if (std::is_same<E, cplx>::value && g_lu_tensor_cores && n >= kLuTcMin + kLuNB) {
+            ek = perm;
+            e = cudaMemsetAsync(ek, 0, (size_t)nmat * n * sizeof(int), st);
+            if (e != cudaSuccess) return e;
+        }
         for (int k0 = 0; k0 < n; k0 += kLuNB) {
             const int nb = min(kLuNB, n - k0);
             e = panel(k0, nb);
             if (e != cudaSuccess) return e;
             if (ncb > 1) {
-                k_lu_swap_trsm<E><<<dim3((n + kLuSwapCols - 1) / kLuSwapCols, nmat), kLuSwapCols * 8, 0, st>>>(n, k0, nb, A, stride, piv, n);
+                k_lu_swap_trsm<E><<<dim3((n + kLuSwapCols - 1) / kLuSwapCols, nmat), kLuSwapCols * 8, 0, st>>>(
+                    n, k0, nb, A, stride, piv, n, n - k0 - nb >= kLuTcMin ? ek : nullptr);
                 ++nl;
             }
             const int m = n - k0 - nb;
@@ -1054,10 +1083,10 @@ cudaError_t lu_factor_impl(int n, int nmat, E* A, long long stride, int* piv, in
                 }
                 if constexpr (std::is_same<E, cplx>::value) {
                     // complex128: the same as exact BF16 digit products (zgemm_tc.cu)
-                    if (g_lu_tensor_cores && m >= kLuTcMin) {
+                    if (ek && m >= kLuTcMin) {
                         const int t0 = k0 + nb;
                         e = launch_zgemm_tc(m, m, nb, A + t0 + (long long)k0 * n, n, stride, A + k0 + (long long)t0 * n, n,
-                                            stride, A + t0 + (long long)t0 * n, n, stride, nmat, st);
+                                            stride, A + t0 + (long long)t0 * n, n, stride, ek + k0, n, nmat, st);
                         if (e != cudaSuccess) return e;
                         done = true;
                     }

@@ -6,18 +6,29 @@
 // cores have no FP64 of use here either.  Instead the operands become integers and their
 // products exact BF16 ones (the scheme of Ootomo, Ozaki and Yokota for integer units, here
 // with BF16 digits and FP32 accumulation):
-//   * a row of A (a column of B) is scaled by the power of two above its largest entry and
-//     rounded to 56-bit integers X (error 2^-56 of the largest entry, where an FP64 entry
-//     itself has 2^-53 of its own size), cut into seven balanced base-256 digits, each of at
-//     most 128 in size and so exact in BF16;
+//   * where B's rows differ in size by 2^5 or more, column k of A is multiplied and row k of B divided
+//     by the power of two of that row's largest entry over all columns (integer additions on
+//     exponents): with rows of different size, partial pivoting leaves A growing and B falling along
+//     the depth, and the large entries of the one then meet the small ones of the other (random
+//     matrices' rows differ by up to 2^2, those of T(k), orders 192 to 800, mostly by 2^1 to 2^4);
+//   * a row of A (a column of B) so scaled is rounded to 56-bit integers X in units of the power
+//     of two above its largest entry (error 2^-56 of that entry, where an FP64 entry itself has
+//     2^-53 of its own size), cut into seven balanced base-256 digits, each of at most 128 in
+//     size and so exact in BF16;
 //   * digits a of A and b of B are multiplied for a + b = s <= 7, the products of one s summed
 //     in one FP32 accumulator: at most 7 x 64 terms of at most 2^14, below 2^23, hence exact in
 //     any order; what is left out (s >= 8) is below 2^-60 of row times column maximum;
 //   * the eight sums of an entry make one 64-bit integer (error 2^-54 of row times column
 //     maximum), converted and subtracted from C in FP64: one rounding for the whole depth,
 //     where 64 FMAs round 64 times.
-// Measured against 64-bit products of random and of LU operands the error is below the FMA
-// kernel's (tests/test_gpu_zgemm.py).
+// The error is relative to (row maximum x column maximum), an FMA's to the terms themselves, so
+// the first must not exceed the second by much.  Every row and column carries masks of the depths
+// at which it is within 0, 3, 6 and 9 powers of two of its maximum; an entry for which no depth has
+// the two distances adding up to 9 is formed by FMAs from A and B instead (z_direct).  So an
+// entry's error stays below 2^-38 of its sum |a||b| at worst, whatever the matrix's scaling; over the
+// rows of random, graded and T(k) operands it is the FMA kernel's (0.9 to 2.2 times).  Of the
+// entries of T(k), orders 300 to 800, at most 2e-4 go the direct way, in 2e-3 of the warps (masks
+// of 0 and 6 or less alone: up to 3e-2), of random operands none.
 //
 // Complex product as one real GEMM, as in tc_gemm.cu: A' = [A_r | A_i] (128 x 64),
 // B' = [[B_r, B_i], [-B_i, B_r]] (64 x 32 for 16 complex columns), C' = [re | im].
@@ -26,8 +37,10 @@
 // the eight sums of a tile are 256 columns, so two tiles fit, and a tile's products run while
 // the sums of the one before are read, joined and subtracted.  That epilogue is what bounds the
 // kernel: per real entry eight 32-bit conversions and two FP64 instructions (a conversion and an
-// FMA) instead of 128.  The first update of four matrices of order 1500 takes 196 us; with
-// tiles of 32 columns in one buffer, C read in the epilogue and a product per digit pair, 362.
+// FMA) instead of 128.  The first update of four matrices of order 1500 takes 174 us (with
+// the masks of every column loaded and tested by every thread 189, by warp reductions of half
+// warps 215; without masks 171); with tiles of 32 columns in one buffer, C read in the epilogue and
+// a product per digit pair, 362.
 #include <algorithm>
 #include <cstdint>
 
@@ -67,16 +80,33 @@ __device__ __forceinline__ uint64_t z_desc(uint32_t saddr) {
     return d;
 }
 
-// biased exponent (zero and subnormals: 0)
-__device__ __forceinline__ int z_exp(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+// Exponents here are biased ones plus a depth's shift s, as plain integers; of zeros kZNone, of
+// Inf and NaN kZBad.  Subnormals have the exponent of the smallest normal number.
+constexpr int kZNone = -(1 << 20), kZBad = 1 << 20;
+constexpr int kZNear = 3, kZLevels = 4;   // the masks' step and number
+constexpr int kZEven = 5;                 // rows of B within fewer powers of two are not scaled
 
-// x as an integer in units of 2^-55 of the power of two above the row's (column's) largest
-// entry, E its biased exponent: |result| <= 2^55
-__device__ __forceinline__ long long z_fixed(double x, int E) {
+__device__ __forceinline__ int z_exp(cplx z, int s) {
+    const int m = max(__double2hiint(z.re) & 0x7fffffff, __double2hiint(z.im) & 0x7fffffff), e = m >> 20;
+    return (m | __double2loint(z.re) | __double2loint(z.im)) == 0 ? kZNone : e == 0x7ff ? kZBad : max(e, 1) + s;
+}
+
+// The shifts of the depths, lane k that of depth k; a whole warp.  ek: the biased exponents of the
+// largest entries of B's k rows (0: nothing known).
+__device__ __forceinline__ int z_shift(const int* ek, int k) {
+    const int lane = threadIdx.x & 31, e = lane < k ? ek[lane] : 0;
+    const bool in = e > 0 && e < 0x7ff;
+    const int hi = __reduce_max_sync(0xffffffffu, in ? e : 0), lo = __reduce_min_sync(0xffffffffu, in ? e : 0x7ff);
+    return in && hi - lo >= kZEven ? e - 1023 : 0;
+}
+
+// x times 2^s as an integer in units of 2^-55 of the power of two above the row's (column's)
+// largest entry, E its exponent: |result| <= 2^55
+__device__ __forceinline__ long long z_fixed(double x, int s, int E) {
     const long long b = __double_as_longlong(x);
-    const int e = (int)((b >> 52) & 0x7ff), d = min(60, E - e);
-    long long v = ((b & 0xfffffffffffffll) | 0x10000000000000ll) << 2;
-    v = e ? (v + ((1ll << d) >> 1)) >> d : 0;
+    const int e = (int)((b >> 52) & 0x7ff), d = max(0, min(60, E - max(e, 1) - s));
+    long long v = ((b & 0xfffffffffffffll) | (e ? 0x10000000000000ll : 0)) << 2;
+    v = (v + ((1ll << d) >> 1)) >> d;
     return b < 0 ? -v : v;
 }
 
@@ -93,22 +123,22 @@ __device__ __forceinline__ uint32_t z_pack(int a, int b) {
     return __byte_perm(__float_as_uint(fa), __float_as_uint(fb), 0x7632);
 }
 
-// 2^(E + F - 1022 - 1022 - 54) for the largest entries' biased exponents; NaN where either is Inf or NaN
-__device__ __forceinline__ double z_scale(int E, int F) {
-    if (E == 0x7ff || F == 0x7ff) return CUDART_NAN;
-    const int e = E + F - 1022 - 1022 - 54 + 1023;
-    if (E == 0 || F == 0 || e < 1) return 0.;
-    if (e > 2046) return CUDART_INF;
-    return __hiloint2double(e << 20, 0);
-}
-
 struct ZJob {
-    int m, n, k, tiles;           // tiles: 32-column tiles per CTA
+    int m, n, k, tiles;           // tiles: tiles of kZNc columns per CTA
     const cplx* A;
     const cplx* B;
     cplx* C;
     long long lda, ldb, ldc, sa, sb, sc;
+    const int* ek;                // per matrix k exponents of B's rows (z_shift)
+    long long se;
 };
+
+// An entry of C by FMAs from its row of A and column of B, as k_lu_gemm forms it
+__device__ __forceinline__ cplx z_direct(const cplx* a, long long lda, const cplx* b, int k, cplx c) {
+#pragma unroll 1
+    for (int q = 0; q < k; ++q) cfms(c, a[q * lda], b[q]);
+    return c;
+}
 
 __device__ __forceinline__ bool z_wait(uint32_t mbar, uint32_t parity) {
     uint32_t done = 0;
@@ -148,11 +178,14 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zgemm_tc(ZJob J) {
     __shared__ __align__(8) uint64_t mbar[2];
     __shared__ uint32_t tmem_slot;
     __shared__ int s_ea[2][kZM], s_eb[3][kZNc];
+    // depths near the maximum, a bit each (all: nothing but zeros): bit k / 2 for an even depth k, 16 + k / 2 for an odd one
+    __shared__ uint4 s_ma[2][kZM], s_mb[3][kZNc];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int r0 = blockIdx.x * kZM;
     const cplx* A = J.A + (long long)blockIdx.z * J.sa;
     const cplx* B = J.B + (long long)blockIdx.z * J.sb;
     cplx* C = J.C + (long long)blockIdx.z * J.sc;
+    const int shift = z_shift(J.ek + (long long)blockIdx.z * J.se, J.k);
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(z_smem(&tmem_slot)),
                      "r"(512u));
@@ -167,6 +200,9 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zgemm_tc(ZJob J) {
     // B of the next tile and the entries of C that a tile updates are read ahead, into registers:
     // one CTA fits an SM, so nothing else covers their latency
     cplx b[2];   // thread (column tid >> 4, two depths)
+    int bs[2];   // and the shifts of those
+#pragma unroll
+    for (int q = 0; q < 2; ++q) bs[q] = -__shfl_sync(0xffffffffu, shift, (tid & 15) * 2 + q);
     auto load_b = [&](int t) {
         const int col = t * kZNc + (tid >> 4), k0 = (tid & 15) * 2;
 #pragma unroll
@@ -177,23 +213,32 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zgemm_tc(ZJob J) {
     {   // A: thread (row tid & 127, half of the depth)
         const int r = tid & 127, kh = tid >> 7;
         cplx a[16];
-        int E = 0;
+        int as[16], E = kZNone;
 #pragma unroll
         for (int q = 0; q < 16; ++q) {
             const int k = 16 * kh + q;
             a[q] = (r0 + r < J.m && k < J.k) ? A[(r0 + r) + (long long)k * J.lda] : mk(0.);
-            E = max(E, max(z_exp(a[q].re), z_exp(a[q].im)));
+            as[q] = __shfl_sync(0xffffffffu, shift, k);
+            E = max(E, z_exp(a[q], as[q]));
         }
         s_ea[kh][r] = E;
         __syncthreads();
         E = max(s_ea[0][r], s_ea[1][r]);
+        unsigned near[kZLevels] = {};
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            const int d = E - z_exp(a[q], as[q]);
+#pragma unroll
+            for (int l = 0; l < kZLevels; ++l) near[l] |= (d <= kZNear * l ? 1u : 0u) << ((q & 1) * 16 + (q >> 1));
+        }
+        s_ma[kh][r] = make_uint4(near[0] << 8 * kh, near[1] << 8 * kh, near[2] << 8 * kh, near[3] << 8 * kh);
 #pragma unroll
         for (int part = 0; part < 2; ++part)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {      // 8 depths: a 16-byte chunk
                 long long v[8];
 #pragma unroll
-                for (int q = 0; q < 8; ++q) v[q] = z_fixed(part ? a[8 * h + q].im : a[8 * h + q].re, E);
+                for (int q = 0; q < 8; ++q) v[q] = z_fixed(part ? a[8 * h + q].im : a[8 * h + q].re, as[8 * h + q], E);
                 const uint32_t off = z_chunk(r, part * 4 + kh * 2 + h);
 #pragma unroll
                 for (int dgt = kZDig - 1; dgt >= 0; --dgt) {   // digit 0 is the leading one
@@ -205,21 +250,29 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zgemm_tc(ZJob J) {
                 }
             }
     }
-    // the loaded tile's digits into buffer u, its columns' exponents into s_eb[e]: columns j (re) and 16 + j (im) of C' take [B_r | -B_i]
-    // and [B_i | B_r]
+    // the loaded tile's digits into buffer u, its columns' exponents and masks into s_eb[e], s_mb[e]:
+    // columns j (re) and 16 + j (im) of C' take [B_r | -B_i] and [B_i | B_r]
     auto cut_b = [&](int u, int e) {
         const int j = tid >> 4, k0 = (tid & 15) * 2;
-        int E = 0;
-#pragma unroll
-        for (int q = 0; q < 2; ++q) E = max(E, max(z_exp(b[q].re), z_exp(b[q].im)));
+        const int e0 = z_exp(b[0], bs[0]), e1 = z_exp(b[1], bs[1]);
+        int E = max(e0, e1);
 #pragma unroll
         for (int o = 8; o > 0; o >>= 1) E = max(E, __shfl_xor_sync(0xffffffffu, E, o));
-        if ((tid & 15) == 0) s_eb[e][j] = E;
+        unsigned near[kZLevels];
+#pragma unroll
+        for (int l = 0; l < kZLevels; ++l) {
+            const unsigned even = __ballot_sync(0xffffffffu, E - e0 <= kZNear * l), odd = __ballot_sync(0xffffffffu, E - e1 <= kZNear * l);
+            near[l] = __byte_perm(even, odd, lane < 16 ? 0x5410 : 0x7632);
+        }
+        if ((tid & 15) == 0) {
+            s_eb[e][j] = E;
+            s_mb[e][j] = make_uint4(near[3], near[2], near[1], near[0]);   // beside the row's levels
+        }
         long long vr[2], vi[2];
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-            vr[q] = z_fixed(b[q].re, E);
-            vi[q] = z_fixed(b[q].im, E);
+            vr[q] = z_fixed(b[q].re, bs[q], E);
+            vi[q] = z_fixed(b[q].im, bs[q], E);
         }
         const int ch = k0 >> 3, sub = (k0 & 7) * 2;               // chunk and byte within it
         const uint32_t o00 = z_chunk(j, ch) + sub, o01 = z_chunk(j, 4 + ch) + sub;
@@ -277,6 +330,8 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zgemm_tc(ZJob J) {
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (tid == 0 && tile0 < tile1) products(0);
+    const int Er = max(s_ea[0][ra], s_ea[1][ra]);
+    const uint4 m0 = s_ma[0][ra], m1 = s_ma[1][ra], mr = make_uint4(m0.x | m1.x, m0.y | m1.y, m0.z | m1.z, m0.w | m1.w);
     for (int t = tile0; t < tile1; ++t) {
         const int u = (t - tile0) & 1, c0 = t * kZNc;
         cplx cc[8];
@@ -284,6 +339,29 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zgemm_tc(ZJob J) {
         for (int q = 0; q < 8; ++q) {
             const int col = c0 + half * 8 + q;
             cc[q] = row < J.m && col < J.n ? C[row + (long long)col * J.ldc] : mk(0.);
+        }
+        // bits of the thread's columns: to write from the products; left to z_direct (no depth serves
+        // the entry, or its scale has no FP64 number).  Neither: a row or column of zeros.  First all
+        // eight at once, by the depths that serve each of them: 8 loads and tests less.
+        unsigned write = 0u, odd = 0u;
+        {
+            const int slot = (t - tile0) % 3;
+            const uint4 mb = s_mb[slot][half * 8 + (lane & 7)];
+            const int eb = s_eb[slot][half * 8 + (lane & 7)];
+            const unsigned meet = (mr.x & __reduce_and_sync(0xffffffffu, mb.x)) | (mr.y & __reduce_and_sync(0xffffffffu, mb.y)) |
+                                  (mr.z & __reduce_and_sync(0xffffffffu, mb.z)) | (mr.w & __reduce_and_sync(0xffffffffu, mb.w));
+            const int lo = Er - 1076 + __reduce_min_sync(0xffffffffu, eb), hi = Er - 1076 + __reduce_max_sync(0xffffffffu, eb);
+            if (meet && lo >= 0 && hi < 2046 && c0 + half * 8 + 8 <= J.n) {
+                write = row < J.m ? 0xffu : 0u;
+            } else {
+#pragma unroll 1
+                for (int q = 0; q < 8; ++q) {
+                    const int j = half * 8 + q, es = Er + s_eb[slot][j] - 1075;
+                    const uint4 m = s_mb[slot][j];
+                    const bool one = ((mr.x & m.x) | (mr.y & m.y) | (mr.z & m.z) | (mr.w & m.w)) != 0u;
+                    if (row < J.m && c0 + j < J.n && es > kZNone / 2) (one && (unsigned)(es - 1) < 2046u ? write : odd) |= 1u << q;
+                }
+            }
         }
         // the next tile's digits go where those of the tile before this one were, whose products
         // this thread has waited for; its exponents do not, slower warps may still read them (three
@@ -297,7 +375,6 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zgemm_tc(ZJob J) {
         __syncwarp();
         fail = __any_sync(0xffffffffu, !z_wait(z_smem(&mbar[u]), (uint32_t)(((t - tile0) >> 1) & 1)));
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int Er = max(s_ea[0][ra], s_ea[1][ra]);
         const uint32_t lane_base = tmem_slot + u * kZSums * kZN + ((uint32_t)((warp & 3) * 32) << 16);
 #pragma unroll
         for (int jq = 0; jq < 2; ++jq) {
@@ -311,17 +388,18 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zgemm_tc(ZJob J) {
                 }
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             }
-            if (row < J.m) {
 #pragma unroll
-                for (int jj = 0; jj < 4; ++jj) {
-                    const int col = c0 + j0 + jj;
-                    if (col >= J.n) continue;
-                    const double sc = fail ? CUDART_NAN : z_scale(Er, s_eb[(t - tile0) % 3][j0 + jj]);   // a wait that ran out shows
-                    const cplx c = cc[4 * jq + jj];
-                    C[row + (long long)col * J.ldc] =
-                        mk(fma(-sc, (double)z_join(re, jj), c.re), fma(-sc, (double)z_join(im, jj), c.im));
-                }
+            for (int jj = 0; jj < 4; ++jj) {
+                const int es = Er + s_eb[(t - tile0) % 3][j0 + jj] - 1075;
+                const double nsc = __hiloint2double(fail ? 0x7ff80000 : (es << 20) | 0x80000000, 0);   // a wait that ran out shows
+                const cplx c = cc[4 * jq + jj];
+                const cplx o = mk(fma(nsc, (double)z_join(re, jj), c.re), fma(nsc, (double)z_join(im, jj), c.im));
+                if ((write >> (4 * jq + jj)) & 1u) C[row + (long long)(c0 + j0 + jj) * J.ldc] = o;
             }
+        }
+        for (; odd; odd &= odd - 1) {
+            const long long col = c0 + half * 8 + __ffs(odd) - 1;
+            C[row + col * J.ldc] = z_direct(A + row, J.lda, B + col * J.ldb, J.k, C[row + col * J.ldc]);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -336,9 +414,11 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zgemm_tc(ZJob J) {
 
 }  // namespace
 
-// C_b -= A_b B_b for nmat matrices: m x n, depth k <= 32, column-major
+// C_b -= A_b B_b for nmat matrices: m x n, depth k <= 32, column-major.  ek + b se: the biased
+// exponents of the largest entries of B_b's k rows.
 cudaError_t launch_zgemm_tc(int m, int n, int k, const cplx* A, long long lda, long long sa, const cplx* B, long long ldb,
-                            long long sb, cplx* C, long long ldc, long long sc, int nmat, cudaStream_t st) {
+                            long long sb, cplx* C, long long ldc, long long sc, const int* ek, long long se, int nmat,
+                            cudaStream_t st) {
     if (m <= 0 || n <= 0 || k <= 0) return cudaSuccess;
     if (k > kZK || nmat < 1 || nmat > 65535) return cudaErrorInvalidValue;
     if (cudaError_t e = cudaFuncSetAttribute(k_zgemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kZSmem);
@@ -348,7 +428,7 @@ cudaError_t launch_zgemm_tc(int m, int n, int k, const cplx* A, long long lda, l
     // tiles per CTA: one CTA per SM at a time, so as many as spread all the tiles over the 152
     const long long total = (long long)rt * ct * nmat;
     const int tiles = (int)std::max<long long>(1, std::min<long long>(ct, (total + 151) / 152));
-    ZJob J{m, n, k, tiles, A, B, C, lda, ldb, ldc, sa, sb, sc};
+    ZJob J{m, n, k, tiles, A, B, C, lda, ldb, ldc, sa, sb, sc, ek, se};
     const dim3 grid(rt, (ct + tiles - 1) / tiles, nmat);
     k_zgemm_tc<<<grid, kZThreads, kZSmem, st>>>(J);
     return cudaGetLastError();

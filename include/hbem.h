@@ -56,8 +56,9 @@ int hbem_set_device(int device);
  *   memory; 0 factors them in global memory.
  *   "lu_tensor_cores" (default 1): the LU's trailing updates on the tensor cores:
  *   complex FP32 (the mixed-precision randomized SVD) with 3xTF32 products, complex128 with
- *   exact products of BF16 digits (56 bits of every row's and column's scale; residuals at
- *   or below the FMA form's); 0 uses FP32 and FP64 FMA.
+ *   exact products of BF16 digits (56 bits of every row's and column's scale, entries whose terms
+ *   lie 9 or more powers of two below it by FMA: an entry's error is at most 2^-38 of its sum of
+ *   absolute terms, a row's like the FMA form's); 0 uses FP32 and FP64 FMA.
  *   "svd_fast" (default 1): dense sigma_min / sigma' / sigma'' (direct::sv*) of matrices
  *   up to order 100 by FP32 Jacobi plus FP64 refinement of the near singular triplets
  *   (one FP64 LU per matrix); 0 always uses the FP64-polished Jacobi kernel.
