@@ -1545,7 +1545,7 @@ int hbem_lu_solve_batch_device(int n, int nmat, int trans, const void* LU_dev, l
     if (steps) {
         HB_CK(dinv.ensure((size_t)nmat * lu_dinv_elems(n) * sizeof(cplx)));
         HB_CK(lu_diag_inv_batched(n, nmat, LU, stride, dinv.as<cplx>(), 0));
-        g_launches += 1;
+        g_launches += 2;
     }
     HB_CK(lu_solve_batched(n, nmat, trans, LU, stride, perm.as<int>(), steps ? dinv.as<cplx>() : nullptr, nrhs,
                            static_cast<cplx*>(X_dev), xstride, 0));

@@ -747,7 +747,7 @@ int tp_solve_device(hbem_solop s, const double* waves, int nw, double k_re, doub
     FD_CK(lu_diag_inv_batched((int)n2, 1, F.T.as<cplx>(), (long long)(n2 * n2), F.dinv.as<cplx>(), 0));
     FD_CK(lu_solve_batched((int)n2, 1, 0, F.T.as<cplx>(), (long long)(n2 * n2), F.perm.as<int>(), F.dinv.as<cplx>(), 1, F.rhs.as<cplx>(),
                            (long long)n2, 0));
-    count_launches(nl + 1);
+    count_launches(nl + 3);
     FD_CK(cudaDeviceSynchronize());
     return HBEM_OK;
 }

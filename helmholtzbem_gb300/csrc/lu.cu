@@ -726,12 +726,24 @@ __global__ void __launch_bounds__(kLuSolveThreads) k_lu_solve(int n, int s, int 
 // block's rows multiply them at once by the inverse of its triangle.  The 32 x 32 inverses
 // are made once per factorisation (k_diag_inv): substitution there, 32 dependent steps of
 // FP64 FMAs and shuffles on one warp, was two thirds of a launch (14.8 us; 6 with them).
+// A multiplication by a rounded inverse D of a triangle B leaves a residual of |B| |D| |B| |x|
+// roundings where substitution leaves |B| |x|: with the nearly dependent columns of a smooth kernel
+// inside a block, 1e5 times more.  So k_diag_cond estimates the norm of |D| |B| for each triangle.
+// Up to kInvAlone the residuals are substitution's to a factor of about two (T(k), orders 160 to 240:
+// half of the blocks below 20 to 55, the largest 55 to 215); up to kInvRefined one step of
+// iterative refinement inside the block brings them there (its two products more); beyond, where
+// the refinement need not converge, the block is solved by substitution.
 // The launches of a sweep are programmatic dependents of one another: a launch comes up and
 // reads its part of the factors, which no launch of the sweep writes, while the one before it
 // still runs, and waits for that one's end before it touches X.
 enum SolveSweep { kSweepL = 0, kSweepU = 1, kSweepUH = 2, kSweepLH = 3 };   // L y = b, U x = y; U^H y = b, L^H x = y
 
-size_t lu_dinv_elems(int n) { return (size_t)((n + kLuNB - 1) / kLuNB) * kLuNB * kLuNB; }
+constexpr int kDinvBlock = kLuNB * kLuNB + 2;   // a block's inverses, then the estimates: L, U; L^H, U^H
+constexpr float kInvAlone = 64.f;
+template <class E>
+constexpr float kInvRefined = std::is_same<E, cplx>::value ? 16777216.f : 1024.f;
+
+size_t lu_dinv_elems(int n) { return (size_t)((n + kLuNB - 1) / kLuNB) * kDinvBlock; }
 
 // Inverses of the diagonal blocks of L (unit: strictly lower part stored) and U (upper
 // part) of every matrix: dinv[matrix][block][column][row].  grid (blocks, nmat, 4): a warp
@@ -741,7 +753,7 @@ __global__ void __launch_bounds__(256) k_diag_inv(int n, const E* LU, long long 
     __shared__ E W[kLuNB][kLuNB + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r0 = blockIdx.x * kLuNB, nr = min(kLuNB, n - r0);
     const E* M = LU + (long long)blockIdx.y * stride;
-    E* out = dinv + ((long long)blockIdx.y * gridDim.x + blockIdx.x) * kLuNB * kLuNB;
+    E* out = dinv + ((long long)blockIdx.y * gridDim.x + blockIdx.x) * kDinvBlock;
     for (int e = threadIdx.x; e < kLuNB * kLuNB; e += blockDim.x) {   // beyond the matrix: the unit matrix
         const int r = e % kLuNB, k = e / kLuNB;
         W[r][k] = (r < nr && k < nr) ? M[(r0 + r) + (long long)(r0 + k) * n] : r == k ? Elem<E>::one() : Elem<E>::zero();
@@ -768,6 +780,70 @@ __global__ void __launch_bounds__(256) k_diag_inv(int n, const E* LU, long long 
     out[c * kLuNB + lane] = lane > c ? lower : v;
 }
 
+// max(|re|, |im|) = f 2^e, 1 <= f < 2 (zero and subnormal: f = 0; Inf and NaN: f infinite)
+__device__ __forceinline__ int size_of(cplx z, float& f) {
+    const int m = max(__double2hiint(z.re) & 0x7fffffff, __double2hiint(z.im) & 0x7fffffff), e = m >> 20;
+    f = e == 0 ? 0.f : e == 0x7ff ? INFINITY : __int_as_float(0x3f800000 | (m & 0xfffff) << 3);
+    return e - 1023;
+}
+__device__ __forceinline__ int size_of(cplxf z, float& f) {
+    const int m = max(__float_as_int(z.re) & 0x7fffffff, __float_as_int(z.im) & 0x7fffffff), e = m >> 23;
+    f = e == 0 ? 0.f : e == 0xff ? INFINITY : __int_as_float(0x3f800000 | (m & 0x7fffff));
+    return e - 127;
+}
+__device__ __forceinline__ float scaled(float f, int e) { return f > 0.f ? ldexpf(f, max(-300, min(300, e))) : 0.f; }
+
+// The largest row sum of |D| |B| for the triangles B of a diagonal block as the sweeps apply them (L, U,
+// L^H, U^H: a warp each) and their inverses D, to a factor of two, in FP32; rows of B and then its
+// columns brought to the size of one by powers of two, so that the scaling of the matrix does not
+// count.  grid (blocks, nmat); lane r has row r.
+template <class E>
+__global__ void __launch_bounds__(128) k_diag_cond(int n, const E* LU, long long stride, E* dinv) {
+    const int lane = threadIdx.x & 31, up = (threadIdx.x >> 5) & 1, herm = threadIdx.x >> 6;
+    const int r0 = blockIdx.x * kLuNB, nr = min(kLuNB, n - r0);
+    const E* M = LU + (long long)blockIdx.y * stride;
+    E* D = dinv + ((long long)blockIdx.y * gridDim.x + blockIdx.x) * kDinvBlock;
+    float f[kLuNB];
+    int e[kLuNB], re = -(1 << 20);
+#pragma unroll
+    for (int k = 0; k < kLuNB; ++k) {
+        const int row = herm ? k : lane, col = herm ? lane : k;   // of the stored block
+        const bool in = row < nr && col < nr;
+        E z = in ? M[(r0 + row) + (long long)(r0 + col) * n] : Elem<E>::zero();
+        if (up ? row > col : row < col) z = Elem<E>::zero();
+        if (row == col && (!up || !in)) z = Elem<E>::one();
+        e[k] = size_of(z, f[k]);
+        if (f[k] > 0.f) re = max(re, e[k]);
+    }
+    int ce = 0;                    // column lane's exponent
+    float v = 0.f;
+#pragma unroll
+    for (int k = 0; k < kLuNB; ++k) {
+        const int c = __reduce_max_sync(0xffffffffu, f[k] > 0.f ? e[k] - re : -(1 << 20));
+        if (lane == k) ce = c;
+        v += scaled(f[k], e[k] - re - c);
+    }
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < kLuNB; ++k) {
+        const int row = herm ? k : lane, col = herm ? lane : k;
+        E z = D[col * kLuNB + row];
+        if (up ? row > col : row < col) z = Elem<E>::zero();
+        if (!up && row == col) z = Elem<E>::one();
+        const int rk = __shfl_sync(0xffffffffu, re, k);
+        const float vk = __shfl_sync(0xffffffffu, v, k);
+        float g;
+        const int q = size_of(z, g);
+        s = fmaf(scaled(g, q + ce + rk), vk, s);
+    }
+    s = s >= 0.f ? s : INFINITY;   // NaN: 0 times infinity
+    const float top = __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(s)));
+    if (lane == 0) {
+        E* est = D + kLuNB * kLuNB + herm;
+        (up ? est->im : est->re) = top;
+    }
+}
+
 template <class E, int SWEEP, int CPC>
 __global__ void __launch_bounds__(128) k_solve_step(int n, int s, int cur, const E* LU, long long stride,
                                                     const E* dinv, E* X, long long xstride) {
@@ -782,8 +858,11 @@ __global__ void __launch_bounds__(128) k_solve_step(int n, int s, int cur, const
     E* Xm = X + (long long)blockIdx.z * xstride + (long long)c0 * n;
     const int r0 = blk * kLuNB, nr = min(kLuNB, n - r0);
     asm volatile("griddepcontrol.launch_dependents;");
+    float cond = 0.f;
     if (t == 0) {
-        const E* Db = dinv + ((long long)blockIdx.z * nb + blk) * kLuNB * kLuNB;
+        const E* Db = dinv + ((long long)blockIdx.z * nb + blk) * kDinvBlock;
+        const E est = Db[kLuNB * kLuNB + (HERM ? 1 : 0)];
+        cond = (float)(SWEEP == kSweepL || SWEEP == kSweepLH ? est.re : est.im);
         for (int c = warp; c < kLuNB; c += 4) {                    // (row lane, column c) of the stored inverses
             const E z = Db[c * kLuNB + lane];
             const bool low = lane > c;
@@ -847,24 +926,64 @@ __global__ void __launch_bounds__(128) k_solve_step(int n, int s, int cur, const
     if (warp == 0)
 #pragma unroll
         for (int c = 0; c < CPC; ++c) xs[c][lane] = yold[c];
+    const bool exact = cond <= kInvAlone, refine = cond <= kInvRefined<E>;   // the CTA's
+    if (!exact)   // the block's triangle as applied: W[k][r]
+        for (int c = warp; c < kLuNB; c += 4) {
+            E z = lane < nr && c < nr ? M[(r0 + lane) + (long long)(r0 + c) * n] : Elem<E>::zero();
+            const bool low = lane > c, lower = SWEEP == kSweepL || SWEEP == kSweepLH;
+            if (lane != c && low != lower) z = Elem<E>::zero();
+            if (lane == c && (lower || lane >= nr)) z = Elem<E>::one();
+            if (HERM) W[lane][c] = conj(z);
+            else W[c][lane] = z;
+        }
     __syncthreads();
-    E acc[CPC];
+    // part <- a block (columns k, lane r row r) times xs
+    auto times = [&](const E (&B)[kLuNB][kLuNB + 1]) {
+        E acc[CPC];
 #pragma unroll
-    for (int c = 0; c < CPC; ++c) acc[c] = Elem<E>::zero();
+        for (int c = 0; c < CPC; ++c) acc[c] = Elem<E>::zero();
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const int k = 8 * warp + q;
-        const E w = D[k][lane];
+        for (int q = 0; q < 8; ++q) {
+            const int k = 8 * warp + q;
+            const E w = B[k][lane];
 #pragma unroll
-        for (int c = 0; c < CPC; ++c) cfma(acc[c], w, xs[c][k]);
+            for (int c = 0; c < CPC; ++c) cfma(acc[c], w, xs[c][k]);
+        }
+#pragma unroll
+        for (int c = 0; c < CPC; ++c) part[warp][c][lane] = acc[c];
+        __syncthreads();
+    };
+    auto sum = [&](int c) { return (part[0][c][lane] + part[1][c][lane]) + (part[2][c][lane] + part[3][c][lane]); };
+    if (!refine) {   // substitution, a warp per column
+        if (warp >= cs) return;
+        E v = xs[warp][lane];
+        for (int q = 0; q < kLuNB; ++q) {
+            const int k = ASC ? q : kLuNB - 1 - q;
+            if (lane == k) v = v * D[k][k];
+            E vk;
+            vk.re = __shfl_sync(0xffffffffu, v.re, k);
+            vk.im = __shfl_sync(0xffffffffu, v.im, k);
+            if (ASC ? lane > k : lane < k) cfms(v, W[k][lane], vk);
+        }
+        if (lane < nr) Xm[(long long)warp * n + r0 + lane] = v;
+        return;
     }
+    times(D);
+    if (!exact) {
+        E x = Elem<E>::zero();   // warps below CPC: the column's first solution
+        if (warp < CPC) xs[warp][lane] = x = sum(warp);
+        __syncthreads();
+        times(W);
+        if (warp == 0) {
 #pragma unroll
-    for (int c = 0; c < CPC; ++c) part[warp][c][lane] = acc[c];
-    __syncthreads();
-    for (int c = warp; c < cs; c += 4)
-        if (lane < nr)
-            Xm[(long long)c * n + r0 + lane] =
-                (part[0][c][lane] + part[1][c][lane]) + (part[2][c][lane] + part[3][c][lane]);
+            for (int c = 0; c < CPC; ++c) xs[c][lane] = yold[c] - sum(c);
+        }
+        __syncthreads();
+        times(D);
+        if (warp < cs && lane < nr) Xm[(long long)warp * n + r0 + lane] = x + sum(warp);
+        return;
+    }
+    if (warp < cs && lane < nr) Xm[(long long)warp * n + r0 + lane] = sum(warp);
 }
 
 // X <- P X (inverse: P^T X), a CTA per column
@@ -1155,6 +1274,7 @@ bool lu_solve_in_steps(int n, int nmat, int s) { return n >= 128 && (long long)n
 template <class E>
 cudaError_t lu_diag_inv(int n, int nmat, const E* LU, long long stride, E* dinv, cudaStream_t st) {
     k_diag_inv<E><<<dim3((n + kLuNB - 1) / kLuNB, nmat, 4), 256, 0, st>>>(n, LU, stride, dinv);
+    k_diag_cond<E><<<dim3((n + kLuNB - 1) / kLuNB, nmat), 128, 0, st>>>(n, LU, stride, dinv);
     return cudaGetLastError();
 }
 

@@ -716,7 +716,7 @@ cudaError_t rsvd_batched(int n, int nmat, int s, int q, int D, int precision, in
             RS_CK(lu_diag_inv_batched(n, nmat, w.A, nn, w.dinv, st));
         }
         k_copy_mats<<<grid_len(ns, nmat), 256, 0, st>>>((int)ns, R, 0, w.X, ns);
-        nl += 3;
+        nl += 4;
         RS_CK(solve(0, w.X, s, ns, 1));
         RS_CK(launch_qr(n, nmat, s, w.X, ns, nullptr, st));
         ++nl;
@@ -770,7 +770,7 @@ cudaError_t sv_der_from_vectors(int n, int nvec, int per, int D, const cplx* T, 
     k_sv2_axpy<<<nvec, 256, 0, st>>>(n, w.rhs, w.ud, w.tb);
     RS_CK(lu_solve_batched(n2, nvec, 0, w.B, nn2, w.perm2, w.dinv2, 1, w.rhs, n2, st));
     k_sv2_out<<<(nvec + 127) / 128, 128, 0, st>>>(n, nvec, w.rhs, w.mcol, w.info2, out);
-    nl += 11;
+    nl += 12;
     return cudaGetLastError();
 }
 
