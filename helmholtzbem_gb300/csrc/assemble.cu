@@ -1245,11 +1245,15 @@ cudaError_t launch_hankel01(int n, const cplx* z, int complex_arg, cplx* h0, cpl
 // wavenumbers have one layout (k_general).
 constexpr int kLayoutAuto = -1;
 
-// more than 48 KB of shared memory (with the static part) has to be asked for
+// More than 48 KB of shared memory (with the static part) has to be asked for.  The permission
+// is the kernel's and shared by all host threads, so it is always the same, above every launch's need
+// (order 2 or 32, arcs, derivative order 2: 110 KB): a smaller one, set by another thread between this
+// call and its launch, would fail the launch.
+constexpr int kAllowedSmem = 160 * 1024;
 template <class Kernel>
 static cudaError_t allow_smem(Kernel kernel, size_t bytes) {
     return bytes <= 40 * 1024 ? cudaSuccess
-                              : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+                              : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAllowedSmem);
 }
 
 // Parts per point set (q) of the split singular launch: about four CTAs per SM (152
