@@ -79,7 +79,7 @@ static __device__ void lu_smem(cplx* A, int n, int* piv, int* sing) {
         if (lane == 0) {
             piv[k] = p;
             s_piv = p;
-            if (best <= 1ull) *sing = 1;
+            if (best == 1ull) *sing = 1;   // a column of NaN is none
         }
     };
     if (warp == 0) {
