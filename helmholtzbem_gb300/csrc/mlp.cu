@@ -226,8 +226,9 @@ __device__ __forceinline__ float gelu_grad(float x) {
     return 0.5f * (1.f + erff(x * 0.70710678118654752f)) + x * 0.39894228040143268f * expf(-0.5f * x * x);
 }
 
-// The kernels around the products work on 32 x 32 tiles (block 32 x 8) of a padded
-// rows x cols matrix, so that they can write the transpose that a later product reads.
+// The kernels around the products work on 32 x 32 tiles (block 32 x 8; grid row tiles x column
+// tiles, a batch may have more than the 65,535 that y takes) of a padded rows x cols matrix, so that
+// they can write the transpose that a later product reads.
 
 // Z = C + bias (pre-activation, kept for the backward pass); H = act(Z) in BF16, HT its
 // transpose (each where not null)
@@ -236,7 +237,7 @@ __global__ void __launch_bounds__(256) k_bias_act(int rows, int cols, int cols_u
                                                   const float* bias, int act, float* Z, __nv_bfloat16* H,
                                                   __nv_bfloat16* HT) {
     __shared__ __nv_bfloat16 t[32][33];
-    const int c = blockIdx.x * 32 + threadIdx.x, r0 = blockIdx.y * 32;
+    const int c = blockIdx.y * 32 + threadIdx.x, r0 = blockIdx.x * 32;
     const float bc = c < cols_used ? bias[c] : 0.f;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -254,7 +255,7 @@ __global__ void __launch_bounds__(256) k_bias_act(int rows, int cols, int cols_u
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int tc = threadIdx.y + 8 * q;
-        HT[(long long)(blockIdx.x * 32 + tc) * rows + r0 + threadIdx.x] = t[threadIdx.x][tc];
+        HT[(long long)(blockIdx.y * 32 + tc) * rows + r0 + threadIdx.x] = t[threadIdx.x][tc];
     }
 }
 
@@ -264,7 +265,7 @@ __device__ __forceinline__ void grad_tile(int rows, int cols, const float (&g)[4
                                           float* part) {
     __shared__ __nv_bfloat16 t[32][33];
     __shared__ float cs[8][33];
-    const int c = blockIdx.x * 32 + threadIdx.x, r0 = blockIdx.y * 32;
+    const int c = blockIdx.y * 32 + threadIdx.x, r0 = blockIdx.x * 32;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const __nv_bfloat16 h = __float2bfloat16(g[q]);
@@ -276,13 +277,13 @@ __device__ __forceinline__ void grad_tile(int rows, int cols, const float (&g)[4
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int tc = threadIdx.y + 8 * q;
-        GT[(long long)(blockIdx.x * 32 + tc) * rows + r0 + threadIdx.x] = t[threadIdx.x][tc];
+        GT[(long long)(blockIdx.y * 32 + tc) * rows + r0 + threadIdx.x] = t[threadIdx.x][tc];
     }
     if (threadIdx.y == 0) {
         float s = 0.f;
 #pragma unroll
         for (int y = 0; y < 8; ++y) s += cs[y][threadIdx.x];
-        part[(long long)blockIdx.y * cols + c] = s;
+        part[(long long)blockIdx.x * cols + c] = s;
     }
 }
 
@@ -290,11 +291,11 @@ __device__ __forceinline__ void grad_tile(int rows, int cols, const float (&g)[4
 __global__ void __launch_bounds__(256) k_mse(int rows, int cols, int rows_used, int cols_used, const float* Y,
                                              const float* T, float inv_count, __nv_bfloat16* Gb, __nv_bfloat16* GT,
                                              float* part, float* loss) {
-    const int c = blockIdx.x * 32 + threadIdx.x;
+    const int c = blockIdx.y * 32 + threadIdx.x;
     float g[4], s = 0.f;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        const int r = blockIdx.y * 32 + threadIdx.y + 8 * q;
+        const int r = blockIdx.x * 32 + threadIdx.y + 8 * q;
         float d = 0.f;
         if (r < rows_used && c < cols_used) d = Y[(long long)r * cols + c] - T[(long long)r * cols_used + c];
         g[q] = 2.f * d * inv_count;
@@ -309,11 +310,11 @@ __global__ void __launch_bounds__(256) k_mse(int rows, int cols, int rows_used, 
 // dZ = dH * GELU'(Z)
 __global__ void __launch_bounds__(256) k_act_bwd(int rows, int cols, const float* Z, const float* dH, __nv_bfloat16* Gb,
                                                  __nv_bfloat16* GT, float* part) {
-    const int c = blockIdx.x * 32 + threadIdx.x;
+    const int c = blockIdx.y * 32 + threadIdx.x;
     float g[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        const long long e = (long long)(blockIdx.y * 32 + threadIdx.y + 8 * q) * cols + c;
+        const long long e = (long long)(blockIdx.x * 32 + threadIdx.y + 8 * q) * cols + c;
         g[q] = dH[e] * gelu_grad(Z[e]);
     }
     grad_tile(rows, cols, g, Gb, GT, part);
@@ -509,7 +510,7 @@ int forward(hbem_mlp m, int batch, int batch_p, bool transposes) {
         ML_CK(m->Z[l].ensure((size_t)batch_p * m->dout_p[l]));
         ML_CK(gemm_bf16(batch_p, m->dout_p[l], m->din_p[l], m->H[l].p, m->din_p[l], m->Wb[l].p, m->din_p[l], m->C.p,
                         m->dout_p[l], m->err.p, g_mlp_tensor_cores, 0));
-        const dim3 grid(m->dout_p[l] / 32, batch_p / 32), block(32, 8);
+        const dim3 grid(batch_p / 32, m->dout_p[l] / 32), block(32, 8);
         if (!last) {
             ML_CK(m->H[l + 1].ensure((size_t)batch_p * m->din_p[l + 1]));
             if (transposes) ML_CK(m->HT[l + 1].ensure((size_t)batch_p * m->din_p[l + 1]));
@@ -558,7 +559,7 @@ int backward(hbem_mlp m, const float* T_host, int batch, int batch_p) {
     }
     ML_CK(cudaMemsetAsync(m->loss(), 0, sizeof(float), 0));
     const int no = m->dout_p[L - 1];
-    k_mse<<<dim3(no / 32, rt), block>>>(batch_p, no, batch, m->n_out, m->Y.p, m->T.p,
+    k_mse<<<dim3(rt, no / 32), block>>>(batch_p, no, batch, m->n_out, m->Y.p, m->T.p,
                                         1.f / (float)((long long)batch * m->n_out), m->Gb.p, m->GT[L - 1].p,
                                         m->part[L - 1].p, m->loss());
     count_launches(1);
@@ -567,7 +568,7 @@ int backward(hbem_mlp m, const float* T_host, int batch, int batch_p) {
         // dH = dZ W: A = dZ (batch_p x op), B = W^T (ip x op)
         ML_CK(gemm_bf16(batch_p, ip, op, m->Gb.p, op, m->WTb[l].p, op, m->C.p, ip, m->err.p, g_mlp_tensor_cores, 0));
         // dZ_(l-1) = dH * GELU'(Z_(l-1)) (the padded columns stay zero: Z there is zero, dH too)
-        k_act_bwd<<<dim3(ip / 32, rt), block>>>(batch_p, ip, m->Z[l - 1].p, m->C.p, l > 1 ? m->Gb.p : nullptr,
+        k_act_bwd<<<dim3(rt, ip / 32), block>>>(batch_p, ip, m->Z[l - 1].p, m->C.p, l > 1 ? m->Gb.p : nullptr,
                                                 m->GT[l - 1].p, m->part[l - 1].p);
         count_launches(2);
         ML_CK(cudaGetLastError());
