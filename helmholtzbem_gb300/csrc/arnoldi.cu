@@ -263,7 +263,7 @@ __global__ void k_arn_start(int n, int p, unsigned long long seed, cplx* X, long
 __global__ void k_arn_init(ArnJob J, const int* info, int* done, int* ndone) {
     const int mat = blockIdx.x;
     const bool sing = info[mat] != 0;
-    if (sing) arn_fail(J, mat, 5);
+    if (sing) arn_fail(J, mat, info[mat] < 0 ? 4 : 5);
     if (threadIdx.x == 0) {
         done[mat] = sing ? 1 : 0;
         if (sing) atomicAdd(ndone, 1);

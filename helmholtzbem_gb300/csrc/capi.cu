@@ -1438,10 +1438,12 @@ int hbem_arnoldi_sv_batch_device(int n, int nmat, unsigned d, int count, double 
     if (iters_host) std::copy(iters.begin(), iters.end(), iters_host);
     int worst = 0;
     for (int m = 0; m < nmat; ++m) {
-        if (stat[m] == 5)
+        if (stat[m] == 4 || stat[m] == 5)
             for (size_t e = (size_t)m * count * os; e < (size_t)(m + 1) * count * os; ++e) out_host[e] = NAN;
         worst = std::max(worst, stat[m]);
     }
+    if (std::count(stat.begin(), stat.end(), 4))
+        return fail(HBEM_ERR_NOCONV, "arnoldi_sv_batch: a tensor-core completion wait timed out");
     if (worst == 5) return fail(HBEM_ERR_SINGULAR, "arnoldi_sv_batch: zero pivot in the LU of T");
     if (worst == 6) return fail(HBEM_ERR_NOCONV, "arnoldi_sv_batch: maximum number of iterations taken");
     return HBEM_OK;
@@ -1521,6 +1523,8 @@ int hbem_lu_factor_batch_device(int n, int nmat, void* A_dev, long long stride, 
     g_launches += nl;
     std::vector<int> inf(nmat);
     HB_CK(cudaMemcpy(inf.data(), info.p, (size_t)nmat * sizeof(int), cudaMemcpyDeviceToHost));
+    if (*std::min_element(inf.begin(), inf.end()) < 0)
+        return fail(HBEM_ERR_NOCONV, "lu_factor_batch: a tensor-core completion wait timed out");
     int first = 0;
     for (int m = 0; m < nmat; ++m) {
         if (info_host) info_host[m] = inf[m];

@@ -742,6 +742,7 @@ int tp_solve_device(hbem_solop s, const double* waves, int nw, double k_re, doub
                             F.info.as<int>(), 0, &nl));
     int info = 0;
     FD_CK(cudaMemcpy(&info, F.info.p, sizeof(int), cudaMemcpyDeviceToHost));
+    if (info < 0) return set_error(HBEM_ERR_NOCONV, "zgesv: a tensor-core completion wait timed out");
     if (info) return set_error(HBEM_ERR_SINGULAR, "zgesv: LU is singular");
     FD_CK(F.dinv.ensure(lu_dinv_elems((int)n2) * sizeof(cplx)));
     FD_CK(lu_diag_inv_batched((int)n2, 1, F.T.as<cplx>(), (long long)(n2 * n2), F.dinv.as<cplx>(), 0));

@@ -15,7 +15,8 @@
 // 3.6 (6.0 before the second tile buffer of zgemm_tc.cu).
 // Matrices are column-major with leading dimension n (Eigen's layout); matrix m
 // starts at A + m * stride.  piv[m*n + k] = row exchanged with row k at step k
-// (LAPACK's ipiv, 0-based); perm[m*n + i] = source row of row i of P A.
+// (LAPACK's ipiv, 0-based); perm[m*n + i] = source row of row i of P A; info[m]: 0, 1 + the first step
+// with a zero pivot, or -1 where a wait of the complex128 tensor-core update ran out.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -1039,7 +1040,7 @@ int panel_split(int m, int nmat) {
 
 cudaError_t launch_zgemm_tc(int m, int n, int k, const cplx* A, long long lda, long long sa, const cplx* B, long long ldb,
                             long long sb, cplx* C, long long ldc, long long sc, const int* ek, long long se, int nmat,
-                            cudaStream_t st);
+                            int* info, cudaStream_t st);
 
 // Cluster launch of the panel factorisation: when the panel is too tall for one CTA, or to
 // split it over `want` CTAs.  Returns with *launched = false (nothing launched) when no
@@ -1205,7 +1206,7 @@ cudaError_t lu_factor_impl(int n, int nmat, E* A, long long stride, int* piv, in
                     if (ek && m >= kLuTcMin) {
                         const int t0 = k0 + nb;
                         e = launch_zgemm_tc(m, m, nb, A + t0 + (long long)k0 * n, n, stride, A + k0 + (long long)t0 * n, n,
-                                            stride, A + t0 + (long long)t0 * n, n, stride, ek + k0, n, nmat, st);
+                                            stride, A + t0 + (long long)t0 * n, n, stride, ek + k0, n, nmat, info, st);
                         if (e != cudaSuccess) return e;
                         done = true;
                     }

@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(kRsvdThreads) k_rsvd_tail(int n, int s, int D,
     if (threadIdx.x == 0) {
         out[(long long)os * mat] = isn;
         for (int t = 1; t < os; ++t) out[(long long)os * mat + t] = 0.;
-        status[mat] = info[mat] ? 5 : ((tc_err && *tc_err) ? 4 : 0);
+        status[mat] = info[mat] < 0 || (tc_err && *tc_err) ? 4 : info[mat] ? 5 : 0;
     }
     if (D == 0) return;
     if (threadIdx.x < s) tw[threadIdx.x] = W[bj * s + threadIdx.x];   // w

@@ -58,7 +58,7 @@ constexpr int kZDig = 7, kZSums = 8;
 constexpr int kZThreads = 256;
 constexpr uint32_t kZABytes = kZM * 128u, kZBBytes = kZN * 128u;   // a digit of each operand: rows of 64 BF16
 constexpr size_t kZSmem = kZDig * (size_t)(kZABytes + 2 * kZBBytes) + 1024;
-constexpr long long kZSpinCap = 1LL << 24;
+constexpr int kZSpinCap = 1 << 18;         // tries, each suspended for a while: about a second; a tile's products take microseconds
 // instruction descriptor, kind::f16: D FP32, A and B BF16, K-major, N >> 3, M >> 4
 __device__ constexpr uint32_t z_idesc(int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kZM >> 4) << 24);
@@ -131,6 +131,7 @@ struct ZJob {
     long long lda, ldb, ldc, sa, sb, sc;
     const int* ek;                // per matrix k exponents of B's rows (z_shift)
     long long se;
+    int* info;                    // per matrix: -1 where a wait ran out
 };
 
 // An entry of C by FMAs from its row of A and column of B, as k_lu_gemm forms it
@@ -142,7 +143,7 @@ __device__ __forceinline__ cplx z_direct(const cplx* a, long long lda, const cpl
 
 __device__ __forceinline__ bool z_wait(uint32_t mbar, uint32_t parity) {
     uint32_t done = 0;
-    for (long long it = 0; it < kZSpinCap && !done; ++it)
+    for (int it = 0; it < kZSpinCap && !done; ++it)
         asm volatile(
             "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
             : "=r"(done)
@@ -330,6 +331,7 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zgemm_tc(ZJob J) {
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (tid == 0 && tile0 < tile1) products(0);
+    int issued = tile0 < tile1 ? 1 : 0;   // tiles, buffers in turn
     const int Er = max(s_ea[0][ra], s_ea[1][ra]);
     const uint4 m0 = s_ma[0][ra], m1 = s_ma[1][ra], mr = make_uint4(m0.x | m1.x, m0.y | m1.y, m0.z | m1.z, m0.w | m1.w);
     for (int t = tile0; t < tile1; ++t) {
@@ -371,7 +373,10 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zgemm_tc(ZJob J) {
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         if (__syncthreads_or(fail)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (tid == 0 && t + 1 < tile1) products(u ^ 1);
+        if (t + 1 < tile1) {
+            if (tid == 0) products(u ^ 1);
+            ++issued;
+        }
         __syncwarp();
         fail = __any_sync(0xffffffffu, !z_wait(z_smem(&mbar[u]), (uint32_t)(((t - tile0) >> 1) & 1)));
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -404,8 +409,9 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zgemm_tc(ZJob J) {
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     if (__syncthreads_or(fail)) {   // another bounded chance for the products before the memory is given back
+        if (tid == 0) atomicExch(J.info + blockIdx.z, -1);
         for (int u = 0; u < 2; ++u)
-            for (uint32_t par = 0; par < 2; ++par) z_wait(z_smem(&mbar[u]), par);
+            if (const int count = (issued + 1 - u) >> 1) z_wait(z_smem(&mbar[u]), (uint32_t)((count - 1) & 1));
         __syncthreads();
     }
     if (warp == 0)
@@ -415,10 +421,10 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zgemm_tc(ZJob J) {
 }  // namespace
 
 // C_b -= A_b B_b for nmat matrices: m x n, depth k <= 32, column-major.  ek + b se: the biased
-// exponents of the largest entries of B_b's k rows.
+// exponents of the largest entries of B_b's k rows.  info[b]: set to -1 where a tensor-core wait ran out.
 cudaError_t launch_zgemm_tc(int m, int n, int k, const cplx* A, long long lda, long long sa, const cplx* B, long long ldb,
                             long long sb, cplx* C, long long ldc, long long sc, const int* ek, long long se, int nmat,
-                            cudaStream_t st) {
+                            int* info, cudaStream_t st) {
     if (m <= 0 || n <= 0 || k <= 0) return cudaSuccess;
     if (k > kZK || nmat < 1 || nmat > 65535) return cudaErrorInvalidValue;
     if (cudaError_t e = cudaFuncSetAttribute(k_zgemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kZSmem);
@@ -428,7 +434,7 @@ cudaError_t launch_zgemm_tc(int m, int n, int k, const cplx* A, long long lda, l
     // tiles per CTA: one CTA per SM at a time, so as many as spread all the tiles over the 152
     const long long total = (long long)rt * ct * nmat;
     const int tiles = (int)std::max<long long>(1, std::min<long long>(ct, (total + 151) / 152));
-    ZJob J{m, n, k, tiles, A, B, C, lda, ldb, ldc, sa, sb, sc, ek, se};
+    ZJob J{m, n, k, tiles, A, B, C, lda, ldb, ldc, sa, sb, sc, ek, se, info};
     const dim3 grid(rt, (ct + tiles - 1) / tiles, nmat);
     k_zgemm_tc<<<grid, kZThreads, kZSmem, st>>>(J);
     return cudaGetLastError();

@@ -402,7 +402,8 @@ int hbem_rsvd_sv_batch_device_ex(int n, int nmat, unsigned d, const void* T_dev,
  * when n <= 32) runs the block iteration; larger counts with d = 0 take all n
  * singular values from the dense Jacobi kernel, larger counts with d > 0 give
  * HBEM_ERR_UNSUPPORTED.  status_host / iters_host (may be NULL): per matrix 0
- * converged, 5 zero pivot in the LU of T (results NaN), 6 iteration cap reached
+ * converged, 4 a tensor-core wait of the LU timed out (results NaN, HBEM_ERR_NOCONV),
+ * 5 zero pivot in the LU of T (results NaN), 6 iteration cap reached
  * (set_option "arnoldi_maxit", default 1000; results are the last iterate's) and the
  * number of block iterations.  Returns HBEM_ERR_SINGULAR / HBEM_ERR_NOCONV when any
  * matrix has status 5 / 6, with out_host filled either way.  T_host: nmat blocks
@@ -427,7 +428,8 @@ int hbem_cgemm_f32_batch_device(int m, int n, int k, const void* A, long long ld
  * source/utilities/randsvd.cpp:104,205): nmat column-major complex128 matrices of
  * order n at A_dev + m * stride (elements).  piv_dev[m n + k] = row exchanged with
  * row k at step k (0-based LAPACK ipiv).  info_host (may be NULL): per matrix 0 or
- * 1 + the first step with a zero pivot; any zero pivot -> HBEM_ERR_SINGULAR.     */
+ * 1 + the first step with a zero pivot; any zero pivot -> HBEM_ERR_SINGULAR.
+ * HBEM_ERR_NOCONV if a tensor-core completion wait timed out.                     */
 int hbem_lu_factor_batch_device(int n, int nmat, void* A_dev, long long stride, int* piv_dev, int* info_host);
 /* The same in complex FP32 (the factorisation behind the mixed-precision randomized
  * SVD): complex64 matrices; from order 256 on in 128-column blocks whose trailing
