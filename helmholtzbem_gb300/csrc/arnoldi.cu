@@ -413,7 +413,8 @@ cudaError_t arnoldi_batched(int n, int nmat, int count, int D, double tol, int m
         // two CTAs a matrix while both fit the 152 SMs (one CTA fills an SM's shared memory from
         // order 80 or so).  64 matrices of order 100:
         // 14.5 -> 11.3 ms a call, one 8.0 -> 6.2; 76 of order 32 7.2 -> 6.6
-        if (2 * nmat <= 152) {
+        bool pairs = 2 * nmat <= 152;
+        if (pairs) {
             AR_CK(cudaFuncSetAttribute(k_arn_small<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kArnSmemLimit));
             cudaLaunchAttribute at[1];
             at[0].id = cudaLaunchAttributeClusterDimension;
@@ -426,8 +427,11 @@ cudaError_t arnoldi_batched(int n, int nmat, int count, int D, double tol, int m
             cfg.stream = st;
             cfg.attrs = at;
             cfg.numAttrs = 1;
-            AR_CK(cudaLaunchKernelEx(&cfg, k_arn_small<true>, J));
-        } else {
+            static std::atomic<int> known[64];
+            pairs = cluster_runs(k_arn_small<true>, cfg, kArnSmemLimit, known);
+            if (pairs) AR_CK(cudaLaunchKernelEx(&cfg, k_arn_small<true>, J));
+        }
+        if (!pairs) {
             AR_CK(cudaFuncSetAttribute(k_arn_small<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kArnSmemLimit));
             k_arn_small<false><<<nmat, kArnThreads, smem, st>>>(J);
         }

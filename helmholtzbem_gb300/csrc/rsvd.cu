@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(kRsvdThreads) k_qr_cluster(int n, int s, int r
 }
 
 // QR of the s columns of nmat blocks: on clusters of eight CTAs while those are few
-// (below four per SM in all) and the rows fit, else a CTA per block.
+// (below four per SM in all), the rows fit and the device runs such clusters, else a CTA per block.
 static cudaError_t launch_qr(int n, int nmat, int s, cplx* X, long long xstride, cplx* Rf, cudaStream_t st) {
     constexpr int CS = 8;
     const int rows = (n + CS - 1) / CS;
@@ -245,7 +245,9 @@ static cudaError_t launch_qr(int n, int nmat, int s, cplx* X, long long xstride,
         at[0].val.clusterDim.z = 1;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, k_qr_cluster, n, s, rows, X, xstride, Rf);
+        static std::atomic<int> known[64];
+        if (cluster_runs(k_qr_cluster, cfg, 200 * 1024, known))
+            return cudaLaunchKernelEx(&cfg, k_qr_cluster, n, s, rows, X, xstride, Rf);
     }
     k_qr_global<<<nmat, kRsvdThreads, 0, st>>>(n, s, X, xstride, Rf);
     return cudaGetLastError();

@@ -3,9 +3,30 @@
 // QR (twice), and one-sided Jacobi for thin matrices.  Used by the randomized SVD
 // (rsvd.cu) and the dense singular-value kernels (dense.cu).
 #pragma once
+#include <atomic>
+
 #include "hbem_device.cuh"
 
 namespace hbem {
+
+// Whether the current device runs clusters of cfg's size of this kernel, with `smem` bytes each (the
+// most it is launched with): part of a GPU may have too few SMs side by side.  Asked once per kernel
+// and device.
+template <class Kernel>
+inline bool cluster_runs(Kernel kernel, cudaLaunchConfig_t cfg, size_t smem, std::atomic<int> (&known)[64]) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    int k = known[dev].load(std::memory_order_relaxed);
+    if (k == 0) {
+        cfg.dynamicSmemBytes = smem;
+        int ncl = 0;
+        const cudaError_t e = cudaOccupancyMaxActiveClusters(&ncl, kernel, &cfg);
+        if (e != cudaSuccess) cudaGetLastError();
+        k = e == cudaSuccess && ncl > 0 ? 1 : -1;
+        known[dev].store(k, std::memory_order_relaxed);
+    }
+    return k > 0;
+}
 
 // (An FP64 instruction of one warp holds its SM sub-partition for 64 cycles, so what every
 // warp repeats -- adding up the warps' sums, a square root, a division -- costs more than the
