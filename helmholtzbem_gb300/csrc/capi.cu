@@ -891,6 +891,11 @@ int hbem_assemble_dense(hbem_builder b, double k_re, double k_im, double c, unsi
     return hbem_assemble_dense_sub(b, k_re, k_im, c, layers, d, 0, 0, 0, 0);
 }
 
+// the general pairs' list has 16 bits per panel (the pair blocks of so many panels are 550 GB)
+static int check_panels(hbem_builder b) {
+    return b->n <= 65536 ? HBEM_OK : fail(HBEM_ERR_UNSUPPORTED, "assembly of more than 65,536 panels");
+}
+
 int hbem_assemble_dense_sub(hbem_builder b, double k_re, double k_im, double c, unsigned layers, unsigned d,
                             unsigned row, unsigned col, unsigned rows, unsigned cols) {
     if (!b) return fail(HBEM_ERR_INVALID, "null builder");
@@ -901,6 +906,7 @@ int hbem_assemble_dense_sub(hbem_builder b, double k_re, double k_im, double c, 
     if (int r = check_kc(k_im, c)) return r;
     if (d > 2) return fail(HBEM_ERR_INVALID, "Invalid order of derivative");
     if (layers == 0 || layers > 7) return fail(HBEM_ERR_INVALID, "bad layer mask");
+    if (int r = check_panels(b)) return r;
     HB_CK(cudaSetDevice(b->device));
     const long long np = b->npair();
     const size_t loc_bytes = (size_t)np * (d + 1) * kLocPerD * sizeof(cplx);
@@ -1075,6 +1081,7 @@ static int gen_T_batch(hbem_solop s, const double* k_host, const double* kim_hos
 static int gen_T_batch_ws(hbem_solop s, const double* k_host, const double* kim_host, int nk, double c_o, double c_i,
                           unsigned d, cplx* T_dev, DBuf& d_jobs, DBuf& d_loc, cudaStream_t st, bool many) {
     hbem_builder b = s->b;
+    if (int r = check_panels(b)) return r;
     const int N = b->n;
     const long long np = b->npair();
     const size_t per_job = (size_t)np * (d + 1) * kLocPerD * sizeof(cplx);
@@ -1154,6 +1161,7 @@ int hbem_gen_sol_op_multi_device(const hbem_solop* ops, int nops, const int* cou
         if (ops[i]->b->device != ops[0]->b->device)
             return fail(HBEM_ERR_INVALID, "gen_sol_op_multi: operators on different devices");
         if (int r = check_kc(0., c_i_host[i])) return r;
+        if (int r = check_panels(ops[i]->b)) return r;
     }
     if (int r = check_kc(0., c_o)) return r;
     std::vector<size_t> koff(nops + 1, 0);
