@@ -255,7 +255,8 @@ static cudaError_t launch_qr(int n, int nmat, int s, cplx* X, long long xstride,
 
 // sigma from the triangular factor Rf of B = T^-H Q = Q_B Rf: sigma_max(B) =
 // sigma_max(Rf).  D >= 1: the right Ritz vector v = Q w (w the top right singular
-// vector of Rf) into the v half of uv.
+// vector of Rf) into the v half of uv.  The rotations square inner products, so Rf is brought to
+// the size of one first, by a power of two: exact, and T may be of any size.
 __global__ void __launch_bounds__(kRsvdThreads) k_rsvd_tail(int n, int s, int D, const cplx* Q, const cplx* QB,
                                                              long long xstride, const cplx* Rf, const cplx* T,
                                                              long long mat_stride, long long der_stride,
@@ -263,9 +264,20 @@ __global__ void __launch_bounds__(kRsvdThreads) k_rsvd_tail(int n, int s, int D,
                                                              const int* tc_err) {
     __shared__ cplx Rs[kRsvdMaxS * kRsvdMaxS], W[kRsvdMaxS * kRsvdMaxS], tw[kRsvdMaxS];
     __shared__ double cn[kRsvdMaxS];
-    __shared__ int rot;
+    __shared__ int rot, top;
     const int mat = blockIdx.x, os = D + 1;
-    for (int e = threadIdx.x; e < s * s; e += blockDim.x) Rs[e] = Rf[(long long)mat * s * s + e];
+    if (threadIdx.x == 0) top = 0;
+    __syncthreads();
+    int hi = 0;
+    for (int e = threadIdx.x; e < s * s; e += blockDim.x) {
+        const cplx z = Rs[e] = Rf[(long long)mat * s * s + e];
+        hi = max(hi, max(__double2hiint(z.re) & 0x7fffffff, __double2hiint(z.im) & 0x7fffffff));
+    }
+    atomicMax(&top, hi);
+    __syncthreads();
+    const int ex = min(1000, max(-1000, (top >> 20) - 1023));   // of the largest entry (none: scaled all the same)
+    const double up = __hiloint2double((1023 + ex) << 20, 0), down = __hiloint2double((1023 - ex) << 20, 0);
+    for (int e = threadIdx.x; e < s * s; e += blockDim.x) Rs[e] = down * Rs[e];
     __syncthreads();
     jacobi_cta(Rs, s, W, &rot);   // a warp per column pair (one warp for all of them: 3.4 ms at s = 16)
     double best = -1.;
@@ -280,7 +292,7 @@ __global__ void __launch_bounds__(kRsvdThreads) k_rsvd_tail(int n, int s, int D,
         const double nb = cn[j];
         if (nb > best) { best = nb; bj = j; }
     }
-    const double smax = sqrt(best), isn = smax > 0. ? 1. / smax : 0.;
+    const double smax = sqrt(best) * up, isn = smax > 0. ? 1. / smax : 0.;
     if (threadIdx.x == 0) {
         out[(long long)os * mat] = isn;
         for (int t = 1; t < os; ++t) out[(long long)os * mat + t] = 0.;
