@@ -184,7 +184,6 @@ __device__ HkEntry g_hk_table[kHkEntries];
 
 std::mutex g_hk_mu;
 bool g_hk_made[64];
-const HkEntry* g_hk_ptr[64];
 
 }  // namespace
 
@@ -197,23 +196,22 @@ const HkEntry* hankel_table(cudaError_t* err) {
         return nullptr;
     }
     std::lock_guard<std::mutex> lk(g_hk_mu);
-    if (g_hk_made[dev]) {   // a device reset in between clears the array (its entries are never zero)
-        double first = 0.;
-        *err = cudaMemcpy(&first, g_hk_ptr[dev], sizeof(double), cudaMemcpyDeviceToHost);
-        if (*err == cudaSuccess && first != 0.) return g_hk_ptr[dev];
-        cudaGetLastError();
-        g_hk_made[dev] = false;
-    }
-    void* p = nullptr;
+    void* p = nullptr;   // asked for each time: a device reset may move the array
     *err = cudaGetSymbolAddress(&p, g_hk_table);
     if (*err != cudaSuccess) return nullptr;
+    if (g_hk_made[dev]) {   // a device reset in between clears it (its entries are never zero)
+        double first = 0.;
+        *err = cudaMemcpy(&first, p, sizeof(double), cudaMemcpyDeviceToHost);
+        if (*err != cudaSuccess) return nullptr;
+        if (first != 0.) return static_cast<const HkEntry*>(p);
+        g_hk_made[dev] = false;
+    }
     k_hankel_table<<<(kHkEntries + 63) / 64, 64>>>(static_cast<HkEntry*>(p));
     *err = cudaGetLastError();
     if (*err == cudaSuccess) *err = cudaStreamSynchronize(0);   // complete before any stream reads it
     if (*err != cudaSuccess) return nullptr;
-    g_hk_ptr[dev] = static_cast<const HkEntry*>(p);
     g_hk_made[dev] = true;
-    return g_hk_ptr[dev];
+    return static_cast<const HkEntry*>(p);
 }
 
 }  // namespace hbem
