@@ -17,7 +17,6 @@ namespace hbem {
 struct KConst {
     cplx k, ks, k2ch, ks_inv, ks_two;
     double c, sqrtc;
-    double ks_re_inv, lg_ks;   // real k: 1 / ks, log(ks / 2) + gamma
 };
 
 __device__ __forceinline__ KConst make_kconst(const Job& jb) {
@@ -29,8 +28,6 @@ __device__ __forceinline__ KConst make_kconst(const Job& jb) {
     K.k2ch = 0.5 * (K.ks * K.ks);
     K.ks_inv = cdiv(mk(1.), K.ks);
     K.ks_two = 2.0 * K.ks;
-    K.ks_re_inv = K.ks.re > 0. ? 1.0 / K.ks.re : 0.;
-    K.lg_ks = K.ks.re > 0. ? log(0.5 * K.ks.re) + kEulerGamma : 0.;
     return K;
 }
 
@@ -60,53 +57,26 @@ struct Acc {
     }
 };
 
-// H0, H1 at ks |v| with 1/|v| given (real k: no division for 1/x)
-template <bool RK>
-__device__ __forceinline__ void hankel_at_ix(const KConst& K, double vn, double ivn, cplx& h0, cplx& h1) {
-    if (RK) {
-        if (vn > 0.) hankel01_real_ix(K.ks.re * vn, K.ks_re_inv * ivn, h0, h1);
-        else hankel01_real(0., h0, h1);
-    } else {
-        hankel01_cplx(vn * K.ks.re, vn * K.ks.im, h0, h1);
-    }
-}
-
-// H0, H1 at ks |v| with 1/|v| and log|v| given (k-independent point data): for real k
-// the series branch needs neither a division nor a logarithm
-template <bool RK>
-__device__ __forceinline__ void hankel_at_pre(const KConst& K, double vn, double ivn, double lvn, cplx& h0,
-                                              cplx& h1) {
-    if (RK) {
-        if (vn > 0.) hankel01_real_pre(K.ks.re * vn, K.ks_re_inv * ivn, K.lg_ks + lvn, h0, h1);
-        else hankel01_real(0., h0, h1);
-    } else {
-        hankel01_cplx(vn * K.ks.re, vn * K.ks.im, h0, h1);
-    }
-}
-
-// complex scalar times complex, specialised for real ks
-template <bool RK>
-__device__ __forceinline__ cplx kmul(cplx a, cplx z) { return RK ? a.re * z : a * z; }
-
 // Kernel values of one quadrature point (see Acc).
-template <int D, bool RK>
+template <int D>
 struct KVals {
     cplx s[D + 1], d[D + 1];
 };
 
-template <int D, bool RK>
-__device__ __forceinline__ KVals<D, RK> kernel_values(const KConst& K, double vn, double vn2, double ivn, cplx h0,
-                                                      cplx h1) {
-    KVals<D, RK> kv;
+template <int D>
+__device__ __forceinline__ KVals<D> kernel_values(const KConst& K, double vn, double vn2, double ivn) {
+    cplx h0, h1;
+    hankel01_cplx(vn * K.ks.re, vn * K.ks.im, h0, h1);
+    KVals<D> kv;
     kv.s[0] = h0;
-    kv.d[0] = vn > 0. ? kmul<RK>(K.ks, ivn * h1) : mk(0.);
+    kv.d[0] = vn > 0. ? K.ks * (ivn * h1) : mk(0.);
     if (D > 0) {
         cplx hv = vn * h1;
         kv.s[1] = hv;
         kv.d[1] = h0;
         if (D > 1) {
-            kv.s[2] = vn2 * h0 - kmul<RK>(K.ks_inv, hv);
-            kv.d[2] = h0 - kmul<RK>(K.ks, hv);
+            kv.s[2] = vn2 * h0 - K.ks_inv * hv;
+            kv.d[2] = h0 - K.ks * hv;
         }
     }
     return kv;
@@ -118,8 +88,8 @@ __device__ __forceinline__ void moments4(cplx (&m)[4], const double wm[4], cplx 
 }
 
 // single layer / hypersingular moments (weights wm = {w, w x, w y, w x y})
-template <int D, bool RK, bool CURVED>
-__device__ __forceinline__ void acc_s(Acc<D, CURVED>& A, const double wm[4], const KVals<D, RK>& kv, double tdt,
+template <int D, bool CURVED>
+__device__ __forceinline__ void acc_s(Acc<D, CURVED>& A, const double wm[4], const KVals<D>& kv, double tdt,
                                       bool with_w) {
 #pragma unroll
     for (int t = 0; t <= D; ++t) moments4(A.s[t], wm, kv.s[t]);
@@ -129,14 +99,14 @@ __device__ __forceinline__ void acc_s(Acc<D, CURVED>& A, const double wm[4], con
     }
 }
 
-template <int D, bool RK, bool CURVED>
-__device__ __forceinline__ void acc_dl(Acc<D, CURVED>& A, const double wm[4], const KVals<D, RK>& kv, double vd) {
+template <int D, bool CURVED>
+__device__ __forceinline__ void acc_dl(Acc<D, CURVED>& A, const double wm[4], const KVals<D>& kv, double vd) {
 #pragma unroll
     for (int t = 0; t <= D; ++t) moments4(A.dl[t], wm, vd * kv.d[t]);
 }
 
-template <int D, bool RK, bool CURVED>
-__device__ __forceinline__ void acc_dlt(Acc<D, CURVED>& A, const double wm[4], const KVals<D, RK>& kv, double vdt) {
+template <int D, bool CURVED>
+__device__ __forceinline__ void acc_dlt(Acc<D, CURVED>& A, const double wm[4], const KVals<D>& kv, double vdt) {
 #pragma unroll
     for (int t = 0; t <= D; ++t) moments4(A.dlt[t], wm, vdt * kv.d[t]);
 }
@@ -612,7 +582,6 @@ __global__ void __launch_bounds__(128, 2) k_general(DevMesh M, const Job* jobs, 
 template <int D, bool CURVED>
 __device__ __forceinline__ void general_pair(const DevMesh& M, const KConst& K, long long q, const double* sx,
                                              const double* sw, cplx* locj) {
-    constexpr bool RK = false;
     // neighbouring threads take pairs of similar panel distance, so a warp's lanes
     // mostly follow the same Hankel branch and series length
     const unsigned pr = M.gpairs[q];
@@ -638,15 +607,13 @@ __device__ __forceinline__ void general_pair(const DevMesh& M, const KConst& K, 
             const cplx v = xi - yj;
             const double vn2 = norm2(v), vn = sqrt(vn2);
             const double ivn = vn > 0. ? 1.0 / vn : 0.;
-            cplx h0, h1;
-            hankel_at_ix<RK>(K, vn, ivn, h0, h1);
-            const KVals<D, RK> kv = kernel_values<D, RK>(K, vn, vn2, ivn, h0, h1);
+            const KVals<D> kv = kernel_values<D>(K, vn, vn2, ivn);
             double wm[4];
             mom_weights(wa * sw[b], s, sx[b], wm);
-            acc_s<D, RK, CURVED>(A, wm, kv, 2. * (ti.im * tj.im + ti.re * tj.re), !tz);
+            acc_s<D, CURVED>(A, wm, kv, 2. * (ti.im * tj.im + ti.re * tj.re), !tz);
             // general: zero test on v x tau_j before the norm (galerkin_builder.cpp:475-499)
-            if (use_dl) acc_dl<D, RK, CURVED>(A, wm, kv, (v.re * tj.im - v.im * tj.re) * tin);
-            if (use_dlt) acc_dlt<D, RK, CURVED>(A, wm, kv, (v.im * ti.re - v.re * ti.im) * tjn);
+            if (use_dl) acc_dl<D, CURVED>(A, wm, kv, (v.re * tj.im - v.im * tj.re) * tin);
+            if (use_dlt) acc_dlt<D, CURVED>(A, wm, kv, (v.im * ti.re - v.re * ti.im) * tjn);
         }
     }
     const cplx t0i = tgi[0], t0j = tgj[0];
@@ -676,7 +643,6 @@ __global__ void __launch_bounds__(128) k_general_zw(DevMesh M, const Job* jobs, 
     // launches with few pairs x media (the Newton rounds of a small scatterer) a thread
     // per pair leaves most of the GPU idle.  Each warp takes ppw consecutive pairs.
     const int lane = threadIdx.x & 31;
-    constexpr bool RK = false;
     const long long q0 = (blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5)) * ppw;
     if (q0 >= M.ngen) return;   // whole warp
     const int job = blockIdx.y;
@@ -705,15 +671,13 @@ __global__ void __launch_bounds__(128) k_general_zw(DevMesh M, const Job* jobs, 
             const cplx v = xi - yj;
             const double vn2 = norm2(v), vn = sqrt(vn2);
             const double ivn = vn > 0. ? 1.0 / vn : 0.;
-            cplx h0, h1;
-            hankel_at_ix<RK>(K, vn, ivn, h0, h1);
-            const KVals<D, RK> kv = kernel_values<D, RK>(K, vn, vn2, ivn, h0, h1);
+            const KVals<D> kv = kernel_values<D>(K, vn, vn2, ivn);
             double wm[4];
             mom_weights(wa * sw[b], s, sx[b], wm);
-            acc_s<D, RK, CURVED>(A, wm, kv, 2. * (ti.im * tj.im + ti.re * tj.re), !tz);
+            acc_s<D, CURVED>(A, wm, kv, 2. * (ti.im * tj.im + ti.re * tj.re), !tz);
             // general: zero test on v x tau_j before the norm (galerkin_builder.cpp:475-499)
-            if (use_dl) acc_dl<D, RK, CURVED>(A, wm, kv, (v.re * tj.im - v.im * tj.re) * tin);
-            if (use_dlt) acc_dlt<D, RK, CURVED>(A, wm, kv, (v.im * ti.re - v.re * ti.im) * tjn);
+            if (use_dl) acc_dl<D, CURVED>(A, wm, kv, (v.re * tj.im - v.im * tj.re) * tin);
+            if (use_dlt) acc_dlt<D, CURVED>(A, wm, kv, (v.im * ti.re - v.re * ti.im) * tjn);
         }
         constexpr int NV = (int)(sizeof(Acc<D, CURVED>) / sizeof(double));
         double* av = reinterpret_cast<double*>(&A);
@@ -775,7 +739,6 @@ __device__ __forceinline__ void singular_fields(const DevMesh& M, const Singular
     f[6] = P.x;
     f[7] = P.y;
     f[8] = f[1] > 0. ? 1.0 / f[1] : 0.;
-    f[9] = f[1] > 0. ? log(f[1]) : 0.;
 }
 
 // Tabulate singular_fields for every task, set and point: [task][set][field][point].
@@ -796,36 +759,34 @@ __global__ void __launch_bounds__(256) k_singular_geo(DevMesh M, const SingularT
 }
 
 // Kernel values and moment updates of one point of a singular pair from its fields.
-template <int D, bool RK, bool CURVED>
+template <int D, bool CURVED>
 __device__ __forceinline__ void singular_accumulate(Acc<D, CURVED>& A, const KConst& K, int kind, uint8_t fl,
                                                     int Kset, const double* f) {
     const double vn2 = f[0], vn = f[1];
-    cplx h0, h1;
-    hankel_at_pre<RK>(K, vn, f[8], f[9], h0, h1);
-    const KVals<D, RK> kv = kernel_values<D, RK>(K, vn, vn2, f[8], h0, h1);
+    const KVals<D> kv = kernel_values<D>(K, vn, vn2, f[8]);
     double wm[4];
     if (kind == PK_COINC) {
         // one point serves both triangles: set 0 has (x, y) = (s, t), set 1 (t, s);
         // V and W kernels are symmetric in s <-> t: both sets in one moment update
         const double w = f[5], s = f[6], t = f[7];
         const double wsym[4] = {2. * w, w * (s + t), w * (s + t), 2. * w * s * t};
-        acc_s<D, RK, CURVED>(A, wsym, kv, f[2], !(fl & PF_TDT0_ZERO));
+        acc_s<D, CURVED>(A, wsym, kv, f[2], !(fl & PF_TDT0_ZERO));
         if (!(fl & PF_DL0_ZERO)) {
             mom_weights(w, s, t, wm);
-            acc_dl<D, RK, CURVED>(A, wm, kv, f[3]);
+            acc_dl<D, CURVED>(A, wm, kv, f[3]);
         }
         if (!(fl & PF_DL1_ZERO)) {
             mom_weights(w, t, s, wm);
-            acc_dl<D, RK, CURVED>(A, wm, kv, f[4]);
+            acc_dl<D, CURVED>(A, wm, kv, f[4]);
         }
     } else {
         const uint8_t dlz = Kset == 0 ? PF_DL0_ZERO : PF_DL1_ZERO;
         const uint8_t dltz = Kset == 0 ? PF_DLT0_ZERO : PF_DLT1_ZERO;
         const uint8_t tdz = Kset == 0 ? PF_TDT0_ZERO : PF_TDT1_ZERO;
         mom_weights(f[5], f[6], f[7], wm);
-        acc_s<D, RK, CURVED>(A, wm, kv, f[2], !(fl & tdz));
-        if (!(fl & dlz)) acc_dl<D, RK, CURVED>(A, wm, kv, f[3]);
-        if (!(fl & dltz)) acc_dlt<D, RK, CURVED>(A, wm, kv, f[4]);
+        acc_s<D, CURVED>(A, wm, kv, f[2], !(fl & tdz));
+        if (!(fl & dlz)) acc_dl<D, CURVED>(A, wm, kv, f[3]);
+        if (!(fl & dltz)) acc_dlt<D, CURVED>(A, wm, kv, f[4]);
     }
 }
 
@@ -861,7 +822,7 @@ __global__ void __launch_bounds__(128) k_singular_z(DevMesh M, const SingularTas
             } else {
                 singular_fields(M, T, Kset, sxc[a], sxc[b], swc[a], swc[b], f);
             }
-            singular_accumulate<D, false, CURVED>(A, K, T.kind, fl, Kset, f);
+            singular_accumulate<D, CURVED>(A, K, T.kind, fl, Kset, f);
         }
     }
     block_reduce(A, red);
@@ -921,7 +882,7 @@ __global__ void __launch_bounds__(128) k_singular_part(DevMesh M, const Singular
             const int a = e % nc, b = e / nc;
             singular_fields(M, T, Kset, sxc[a], sxc[b], swc[a], swc[b], f);
         }
-        singular_accumulate<D, false, CURVED>(A, K, T.kind, fl, Kset, f);
+        singular_accumulate<D, CURVED>(A, K, T.kind, fl, Kset, f);
     }
     block_reduce(A, red);
     constexpr int NV = (int)(sizeof(Acc<D, CURVED>) / sizeof(double));
