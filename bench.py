@@ -294,7 +294,7 @@ def assembly_at_scale(torch, C, api, geometry, lib, peak):
     """Assembly-at-scale configuration: seeded star polygon (24 vertices, r = 1 + 0.3 u),
     N = 1000 line panels, Gauss order 16, c_i = 4, c_o = 1, k = 20: T, T', T'' (2000 x
     2000 complex128, both media, projected) on the device.  Reports T-sets/s and the
-    assembly kernels' algorithmic FP64 rate (CUDA events on their stream)."""
+    assembly kernels' executed FP64 rate (CUDA events on their stream)."""
     N, order, k = 1000, 16, 20.0
     data = api.BuilderData(geometry.polygon(*geometry.star_polygon(24, seed=2), N), order=order)
     so = api.SolutionsOperator(data)
@@ -322,7 +322,7 @@ def assembly_at_scale(torch, C, api, geometry, lib, peak):
                                         C.ctypes.c_longlong())
     lib.hbem_stats_read(C.ctypes.byref(launches), C.ctypes.byref(asm_ms), C.ctypes.byref(asm_l),
                         C.ctypes.byref(asm_pts))
-    achieved = assembly_flops(C, lib) / (asm_ms.value * 1e-3) / 1e12 if asm_ms.value > 0 else 0.0
+    achieved = assembly_flops(C, lib, False) / (asm_ms.value * 1e-3) / 1e12 if asm_ms.value > 0 else 0.0
     del T
     return {"workload": "star polygon 24 vertices (seed 2), N=1000 lines, order 16, k=20, c_i=4, c_o=1, "
                         "T/T'/T'' 2000x2000 c128 projected",
@@ -331,22 +331,27 @@ def assembly_at_scale(torch, C, api, geometry, lib, peak):
             "assembly_ms_per_T_set": asm_ms.value / reps,
             "assembly_fp64_tflops": achieved, "assembly_frac_of_measured_fp64": achieved / peak if peak else None,
             "assembly_frac_of_nominal_fp64": achieved / nominal_fp64_tflops(),
-            "note": "algorithmic flops (the reference's per-point work); a fraction above 1 means this build "
-                    "executes fewer FP64 instructions per point than that count credits, not a rate above the pipe's"}
+            "note": "FP64 operations executed per point, library functions' own not counted"}
 
 
-def assembly_flops(C, lib):
-    """Algorithmic FP64 flops of the timed assembly launches: per quadrature point and
-    medium F(d) = 130 (Hankel pair) + 50 (geometry and weights) + 100 (d + 1) (kernel
-    values and moment updates of orders 0..d); singular-pair points whose geometry
-    comes from the builder's k-independent table do not repeat the 50."""
+def assembly_flops(C, lib, arcs):
+    """FP64 operations (an FMA is two) that the real-wavenumber kernels execute at the points of the
+    timed assembly launches, by derivative order; what library functions do inside (sine and cosine on
+    arcs' singular points, logarithms of the node kernel) and the work per row or pair is not counted.
+      general pairs    36 for the distance and the two Hankel functions of u, the products with
+                       |v|^2, then two-point moments: on arcs 16 for the geometric factors and 32 per
+                       order, on lines 4 per moment (2 or 3 of each value);
+      singular points  42 likewise, then on arcs 24 and 32 per order, on lines 8 per order (the double
+                       layers of collinear neighbours vanish: theirs are not counted);
+      singular nodes   164 for the four entire functions, 24 per moment set and order."""
     split = (C.ctypes.c_longlong * 9)()
     lib.hbem_stats_read_points(split)
     f = 0.0
     for d in range(3):
-        f += split[d] * (180.0 + 100.0 * (d + 1))
-        f += split[3 + d] * (130.0 + 100.0 * (d + 1))
-        f += split[6 + d] * (180.0 + 100.0 * (d + 1))
+        F, prod = d + 1, 2.0 * d
+        f += split[d] * (36 + prod + (16 + 32 * F if arcs else 4 * (2 * F + min(F, 2) + 3)))
+        f += split[3 + d] * (164 + 24 * F * (4 if arcs else 3))
+        f += split[6 + d] * (42 + prod + (24 + 32 * F if arcs else 8 * F))
     return f
 
 
@@ -592,7 +597,7 @@ def batching_sample(torch, C, api, geometry, lib, nk=16, peak=None):
     launches, a_ms, a_l, a_pts = (C.ctypes.c_longlong(), C.ctypes.c_double(), C.ctypes.c_longlong(),
                                   C.ctypes.c_longlong())
     lib.hbem_stats_read(C.ctypes.byref(launches), C.ctypes.byref(a_ms), C.ctypes.byref(a_l), C.ctypes.byref(a_pts))
-    flops = assembly_flops(C, lib)
+    flops = assembly_flops(C, lib, False)
     m_asm, m_rs = e0.elapsed_time(e1), e1.elapsed_time(e2)
     tf = flops / (a_ms.value * 1e-3) / 1e12 if a_ms.value > 0 else None
     diff = max(abs(float(o.min()) - p["sigma_min_min"]) / p["sigma_min_min"] for o, p in zip(outs, per))
@@ -689,7 +694,9 @@ def arnoldi_at_scale(torch, C, api, geometry, lib):
     return res, (small_host, small_sig, large_host, large_sig)
 
 
-FIELD_FLOPS_PER_PAIR = 200.0   # per (grid point, boundary node): Hankel pair ~170, geometry + terms ~30
+# FP64 operations executed per (grid point, boundary node): distance and u 6, the two Hankel functions
+# of u 30, projection and two complex products 21
+FIELD_FLOPS_PER_PAIR = 57.0
 
 
 def field_at_scale(torch, C, api, geometry, lib, peak):
@@ -908,7 +915,7 @@ def run_gpu(args):
     d2h = int(roots.nbytes + CFG["npoints"] * 3 * 8 + 2 * roots.size * 8)   # roots, grid, the roots' checks
 
     # roofline of the dominant kernel (panel-pair assembly, FP64 CUDA-core bound):
-    # algorithmic work of the timed launches by derivative order and point kind, on one
+    # executed operations of the timed launches by derivative order and point kind, on one
     # search of the workload with the Newton candidates in lock step, so that the timed
     # assembly launches do not overlap (on per-candidate streams a launch's event
     # interval would also cover other candidates' kernels)
@@ -922,7 +929,7 @@ def run_gpu(args):
         lib.hbem_stats_read(None, C.ctypes.byref(asm_ms), C.ctypes.byref(asm_l), C.ctypes.byref(asm_pts))
     finally:
         C.check(lib.hbem_set_option(b"plain_async", 1))
-    flops = assembly_flops(C, lib)
+    flops = assembly_flops(C, lib, True)
     achieved = flops / (asm_ms.value * 1e-3) / 1e12 if asm_ms.value > 0 else 0.0
     peak = fp64_peak_tflops()
     roofline = {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
@@ -938,10 +945,9 @@ def run_gpu(args):
                 "avg_launch_ms": asm_ms.value / max(1, asm_l.value),
                 # nominal FP64 peak: 2 DFMA per cycle per SM x 152 SMs at the sampled SM clock
                 "peak_nominal": nominal_fp64_tflops(), "frac_of_nominal": achieved / nominal_fp64_tflops(),
-                # FP64 instructions the kernels execute (ncu: DFMA x 2 + DMUL + DADD per cycle
-                # x SM clock), from profiles/assembly_kernels_circle_N50_p11_d2.md; the
-                # algorithmic count above uses the reference's per-point work, which this
-                # build's Hankel pair undercuts, so the algorithmic rate reads above these
+                "work": "FP64 operations executed per quadrature point (FMA = 2), library functions' own not counted",
+                # the same from counters (ncu: DFMA x 2 + DMUL + DADD per cycle x SM clock), all
+                # FP64 instructions of a launch: profiles/assembly_kernels_circle_N50_p11_d2.md
                 "ncu_executed_fp64_tflops": {"k_general<0> grid": 0.83, "k_singular_nodes<0> grid": 0.35,
                                              "k_general<1> Newton": 0.74}}
 

@@ -68,8 +68,9 @@ __device__ __forceinline__ float warp_sumf(float x) {
 // 128 B a cycle), so the columns are read once, into registers, for the inner products and the
 // rotation, and ld keeps the groups of a warp on different banks.  With the FP64 stage's shorter
 // chains (one warp per norm, look-ahead LU, half-warps in the Ritz step's rotations) k_svd_fast
-// went from 7.80 to 5.70 ms for 100 matrices of n = 96 and from 2.24 to 1.79 ms for n = 50;
-// every operation and its order are as they were.  (Sweeps on the triangular factor of a
+// went from 7.80 to 5.70 ms for 100 matrices of n = 96 and from 2.24 to 1.79 ms for n = 50; this
+// stage's operations and their order did not change, in the FP64 stage the sums of gemv_h and the
+// tangents of the Ritz step's rotations round differently.  (Sweeps on the triangular factor of a
 // pivoted QR instead take half the time of this stage, but leave other FP32 noise in the start
 // block, which reaches sigma' and sigma'' at nearly degenerate matrices, where the inverse
 // iterations' count is capped: 1.25 times the error on average.)

@@ -456,8 +456,8 @@ static __device__ void permute_cols(cplx* X, int n, int s, const int* perm, cplx
     }
 }
 
-// X <- T^-1 X.  wide (optional): n x s scratch for a one-pass row permutation;
-// inv_diag: A's diagonal holds 1 / u_kk (multiplications instead of divisions).
+// X <- T^-1 X with the factors of lu_smem, A's diagonal holding 1 / u_kk (lu_inv_diag).  wide
+// (optional): n x s scratch for a one-pass row permutation.
 static __device__ void solve_lu_blk(const cplx* A, const int* perm, int n, cplx* X, int s, cplx* buf,
                                     cplx* wide = nullptr) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
