@@ -35,9 +35,10 @@
 // A CTA takes 128 rows and a run of 16-column tiles: A's digits are cut once (112 KB of
 // 128-byte-swizzled K-major shared memory), B's per tile (28 KB, two buffers).  Tensor memory:
 // the eight sums of a tile are 256 columns, so two tiles fit, and a tile's products run while
-// the sums of the one before are read, joined and subtracted.  That epilogue is what bounds the
-// kernel: per real entry eight 32-bit conversions and two FP64 instructions (a conversion and an
-// FMA) instead of 128.  The first update of four matrices of order 1500 takes 174 us (with
+// the sums of the one before are read, joined and subtracted: per real entry eight 32-bit
+// conversions and two FP64 instructions (a conversion and an FMA) instead of 128.  What bounds the
+// kernel is that work and the cutting of the next digits, dependent instructions of eight warps (FP64
+// pipe 39 % active, tensor pipe 22 %, issue slots 30 %).  The first update of four matrices of order 1500 takes 174 us (with
 // the masks of every column loaded and tested by every thread 189, by warp reductions of half
 // warps 215; without masks 171); with tiles of 32 columns in one buffer, C read in the epilogue and
 // a product per digit pair, 362.
@@ -297,8 +298,8 @@ __global__ void __launch_bounds__(kZThreads, 1) k_zgemm_tc(ZJob J) {
     };
     // one thread: the digit products of buffer u into its half of the tensor memory.  Digit a of A
     // times digits 0 .. of B is one product: B's digits lie one behind the other, 32 rows each, and
-    // so do the sums a + b.  29 products of up to 224 columns, where digit by digit 136 products of
-    // 32 columns took 75 ns each whatever their width.
+    // so do the sums a + b: 29 products of up to 224 columns (digit by digit, 136 products of 32
+    // columns, the first update of four matrices of order 1500 took 317 us where it then took 196).
     auto products = [&](int u) {
         const uint32_t taddr = tmem_slot + u * kZSums * kZN;
         const uint64_t ad = z_desc(z_smem(As)), bd = z_desc(z_smem(Bs) + u * kZDig * kZBBytes);
